@@ -106,7 +106,7 @@ typedef struct sph_stats {
     uint64_t steps;             /* steps taken since upload */
     uint64_t relayouts;         /* storage re-orderings performed */
     uint64_t device_bytes;      /* device memory held by the context */
-    uint64_t cell_rebuilds;     /* steps whose cell list was rebuilt (a particle changed cell) */
+    uint64_t cell_rebuilds;     /* steps whose cell list was rebuilt (their contact search swept cells) */
 } sph_stats;
 
 /* Options for sph_set_option. */

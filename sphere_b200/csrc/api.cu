@@ -510,7 +510,9 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
 
 int do_relayout(sph_ctx *c, cudaStream_t st)
 {
-    // the cell list must describe the current positions before storage follows it
+    // the cell list must describe the current positions before storage follows
+    // it (it may be stale: any nonzero flag rebuilds it)
+    CK(cudaMemsetAsync(c->d.rebuild, 1, 4, st));
     launch_rebuild(c->d, c->np_all, c->ncells_all, c->a, st);
     relayout(c->d, c->np_all, c->a, c->scratch, st);
     // the bonds follow their particles' new storage indices
@@ -518,7 +520,6 @@ int do_relayout(sph_ctx *c, cudaStream_t st)
     // the slot rows moved: every chunk may hold a contact until the next
     // force pass has looked
     CK(cudaMemsetAsync(c->d.cflag, 1, div_up(c->np_all, 32), st));
-    CK(cudaMemsetAsync(c->d.settled, 0, c->np_all, st));
     CK(cudaGetLastError());
     c->relayouts++;
     c->since_relayout = 0;
@@ -654,7 +655,7 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     AL(d.vel0, npad); AL(d.angvel0, npad); AL(d.angpos, npad); AL(d.xysum, npad); AL(d.esv, np);
     AL(d.w_user, WLANES * np); AL(d.fixed, npad);
     AL(d.force, np); AL(d.torque, np); AL(d.acc, np); AL(d.angacc, np); AL(d.edp, np);
-    AL(d.uid, np); AL(d.sidx, np); AL(d.cell, npad); AL(d.outside, np);
+    AL(d.uid, np); AL(d.sidx, np); AL(d.cell, npad);
     AL(d.contacts, tiled_size(np, NC)); AL(d.dmc, np); AL(d.delta_t, tiled_size(np, NC));
     AL(d.cmask, np);
     AL(d.cflag, div_up(np, 32));
@@ -662,8 +663,7 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     AL(d.scan_tiles, scan_tile_count(c->ncells_all));
     AL(d.alias_any, 1);
     AL(d.vl, tiled_size(np, VL_CAP)); AL(d.vl_meta, tiled_size(np, VL_CAP)); AL(d.vl_len, np);
-    AL(d.disp, npad);
-    AL(d.vl_gap, np); AL(d.settled, np);
+    AL(d.vl_held, np); AL(d.due, np);
     AL(d.movers, MOVER_CAP); AL(d.dirty, ncells + 1); AL(d.vs, 1);
     AL(d.wf_pp, np); AL(d.wtouch, npad); AL(d.wf_partial, div_up(np, 256));
     AL(d.wf_flag, div_up(np, 256));
@@ -808,7 +808,21 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
             Q.rmax = rmax;
             rmax_all = std::fmax(rmax_all, rmax);
         }
-        for (auto &Q : c->hps) Q.skin = c->skin_rel * rmax_all;
+        for (auto &Q : c->hps) {
+            Q.skin = c->skin_rel * rmax_all;
+            // the reach of a candidate list, against the cells (see Verlet)
+            const double reach = (2.0 * Q.rmax + Q.skin + Q.reach_extra) * (1.0 + 1e-5) + Q.prune_pad;
+            Q.set_lists = Q.skin > 0.0 ? 1u : 0u;
+            Q.wide = 0u;
+            for (int k = 0; k < 3; ++k) {
+                const bool wraps = (k == 0 && Q.periodic != 0) || (k == 1 && Q.periodic == 1);
+                if (2.0 * Q.cellsize[k] < reach || (wraps && Q.num[k] < 3)) Q.set_lists = 0u;
+                if (Q.cellsize[k] < reach) Q.wide = 1u;
+            }
+            if (!Q.set_lists) Q.wide = 0u;
+            // without lists every step sweeps; the Darcy flow reads the cell list
+            Q.eager = (!(Q.skin > 0.0) || c->darcy_on) ? 1u : 0u;
+        }
         // a zero energy rate may skip the es/ev update only if no sum is -0.0
         bool negzero = false;
         for (size_t i = 0; i < np && !negzero; ++i)
@@ -1191,7 +1205,34 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
     CK(cudaMallocAsync(&b, words * 4, c->stream));
     uint32_t *cs = b, *pm = b + np, *st = b + 2 * (size_t)np, *en = st + nc;
     const unsigned int n = (np > nc + 1 ? np : nc + 1);
-    k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(c->d, cs, pm, st, en);
+    if (c->since_relayout == 0) {
+        k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(c->d, cs, pm, st, en);
+    } else {
+        // the steps keep the list only as far as they need it: it is made
+        // here, in arrays of its own, from the start positions of the last
+        // step, which that step left in the other buffer
+        Dev q = c->d;
+        char *tmp = nullptr;
+        size_t bytes = 0;
+        auto part = [&](size_t count) { const size_t at = bytes; bytes += (count + 31) / 32 * 128; return at; };
+        const size_t o_cell = part(np), o_order = part(np), o_pos = part(np), o_xs = part(4 * (size_t)np),
+                     o_start = part((size_t)nc + 2), o_fill = part((size_t)nc + 1),
+                     o_scan = part(scan_tile_count(nc)), o_word = part(4), o_vs = part(32);
+        CK(cudaMallocAsync(&tmp, bytes, c->stream));
+        CK(cudaMemsetAsync(tmp + o_fill, 0, bytes - o_fill, c->stream));
+        auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
+        q.cell = at(o_cell); q.cellorder = at(o_order); q.pos = at(o_pos);
+        q.xs[0] = q.xs[1] = reinterpret_cast<float4 *>(tmp + o_xs);
+        q.cell_start = at(o_start); q.cell_fill = at(o_fill); q.scan_tiles = at(o_scan);
+        q.status = at(o_word); q.alias_any = at(o_word) + 1; q.rebuild = at(o_word) + 2;
+        q.vs = reinterpret_cast<Verlet *>(tmp + o_vs);
+        CK(cudaMemsetAsync(q.rebuild, 1, 4, c->stream));
+        launch_cell_init(q, np, c->a ^ 1, c->stream);
+        launch_rebuild(q, np, nc, c->a ^ 1, c->stream);
+        k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);
+        CK(cudaFreeAsync(tmp, c->stream));
+    }
+    CK(cudaGetLastError());
     if (cell_sorted) CK(cudaMemcpyAsync(cell_sorted, cs, (size_t)np * 4, cudaMemcpyDeviceToHost, c->stream));
     if (perm) CK(cudaMemcpyAsync(perm, pm, (size_t)np * 4, cudaMemcpyDeviceToHost, c->stream));
     if (cell_start) CK(cudaMemcpyAsync(cell_start, st, (size_t)nc * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1323,7 +1364,6 @@ static int restore_ckpt(sph_ctx *c, const sph_ctx::Ckpt &k)
     launch_cell_init(d, c->np_all, k.a, c->stream);
     CK(cudaMemsetAsync(d.dirty, 0, ((size_t)c->ncells_all + 1) * sizeof(uint32_t), c->stream));
     CK(cudaMemsetAsync(d.cflag, 1, div_up(c->np_all, 32), c->stream));
-    CK(cudaMemsetAsync(d.settled, 0, c->np_all, c->stream));
     // stream-ordered: the host enqueues the next work without waiting
     launch_epoch_reset(d, c->stream);
     CK(cudaGetLastError());
@@ -1496,7 +1536,9 @@ int sph_diff_end(sph_ctx *c)
     free_diff(c);
     drop_graphs(c);
     CK(cudaMemsetAsync(c->d.cflag, 1, div_up(c->np_all, 32), c->stream));
-    CK(cudaMemsetAsync(c->d.settled, 0, c->np_all, c->stream));
+    // every list is looked at again (due below 0)
+    CK(cudaMemsetAsync(c->d.due, 0xbf, (size_t)c->np_all * 4, c->stream));
+    CK(cudaMemsetAsync(c->d.vl_held, 0, (size_t)c->np_all * 4, c->stream));
     c->diff = false;
     c->relayout_every = c->relayout_saved;
     return SPH_OK;
@@ -1545,6 +1587,11 @@ int sph_darcy_upload(sph_ctx *c, double nu, const sph_darcy_state *h)
         CK(cudaEventCreateWithFlags(&c->darcy_join, cudaEventDisableTiming));
     }
     c->darcy_on = true;
+    // the flow reads the cell list and the float positions of every step: the
+    // steps so far may have left them behind
+    c->hp.eager = c->hps[0].eager = 1u;
+    CK(cudaMemcpyAsync(c->d.prm, c->hps.data(), sizeof(Params), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(c->d.rebuild, 1, 4, c->stream));
     drop_graphs(c);   // the step graphs gain the Darcy kernels
     CK(cudaStreamSynchronize(c->stream));   // the caller's arrays are complete
     return SPH_OK;

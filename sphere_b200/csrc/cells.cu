@@ -32,7 +32,6 @@ __global__ void k_cell_init(Dev d, int A)
     if (s >= d.np_all) return;
     const Params &P = prm_of(d, s);
     const double4 x = d.xr[A][s];
-    d.outside[s] = cell_outside(P, x.x, x.y, x.z) ? 1 : 0;
     uint32_t c;
     if (!grid_cell(P, x.x, x.y, x.z, c)) {
         atomicOr(d.status, ST_OUT_OF_GRID);
@@ -181,10 +180,10 @@ __global__ void k_post_sort(Dev d, int A)
         atomicOr(d.alias_any, 1u);
 }
 
-// Verlet lists: every cell of the 27-cell neighbourhood of a cell that
-// gained or lost a member is stamped with this step's number; particles in
-// stamped cells re-sweep their stencil (their list's membership or order may
-// have changed).  Periodic axes wrap as in findDistMod.
+// Candidate lists: every cell whose particles' lists a move can have upset
+// (the 27 cells around the old and the new cell, or with Params::wide the 125)
+// is stamped with this step's number; particles in stamped cells sweep their
+// stencil again.  Periodic axes wrap as in findDistMod.
 __global__ void k_mark_dirty(Dev d)
 {
     if (*d.rebuild == 0u) return;
@@ -193,7 +192,7 @@ __global__ void k_mark_dirty(Dev d)
     if (blockIdx.x == 0 && threadIdx.x == 0) V.rebuilds += 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0 && V.movers_overflow) {
         V.all_rebuild = 1u;
-        V.dmax_bits = 0u;
+        V.moved = 0.0f;
     }
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < 2 * n; e += gridDim.x * blockDim.x) {
         const uint2 mv = d.movers[e >> 1];
@@ -213,16 +212,17 @@ __global__ void k_mark_dirty(Dev d)
         const uint32_t c = cg - P.cell_base;
         const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
         const int32_t cx = (int32_t)(c % nx), cy = (int32_t)((c / nx) % ny), cz = (int32_t)(c / (nx * ny));
-        for (int oz = -1; oz < 2; ++oz) {
+        const int R = P.wide ? 2 : 1;
+        for (int oz = -R; oz <= R; ++oz) {
             const int32_t z = cz + oz;
             if (z < 0 || z >= (int32_t)nz) continue;
-            for (int oy = -1; oy < 2; ++oy) {
+            for (int oy = -R; oy <= R; ++oy) {
                 int32_t y = cy + oy;
                 if (y < 0 || y >= (int32_t)ny) {
                     if (P.periodic != 1) continue;
                     y = (y + (int32_t)ny) % (int32_t)ny;
                 }
-                for (int ox = -1; ox < 2; ++ox) {
+                for (int ox = -R; ox <= R; ++ox) {
                     int32_t x = cx + ox;
                     if (x < 0 || x >= (int32_t)nx) {
                         if (P.periodic != 1 && P.periodic != 2) continue;
@@ -346,7 +346,7 @@ __global__ void k_relayout_finish(Dev d, int A)
     if (k == 0) {
         // storage indices changed: every Verlet list is stale
         d.vs->all_rebuild = 1u;
-        d.vs->dmax_bits = 0u;
+        d.vs->moved = 0.0f;
     }
     const double4 x = d.xr[A][k];
     d.xs[A][k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
@@ -386,7 +386,6 @@ void relayout(const Dev &d, uint32_t np, int a, void *scratch, cudaStream_t st)
     gather_back(d.uid, scratch, order, np, st);
     gather_back(d.cell, scratch, order, np, st);
     gather_back(d.fixed, scratch, order, np, st);
-    gather_back(d.outside, scratch, order, np, st);
     gather_back(d.cmask, scratch, order, np, st);
     gather_back(d.dmc, scratch, order, np, st);
     gather_back(d.wtouch, scratch, order, np, st);

@@ -66,6 +66,9 @@ struct Params {
     double skin;        // Verlet-list skin (metres); 0 disables the lists
     double reach_extra; // model 1: db, the capillary reach beyond contact (metres)
     uint32_t esv_skip;  // no es/ev is -0.0: adding a zero rate may be skipped exactly
+    uint32_t set_lists; // the candidate lists outlive moves between cells (see Verlet)
+    uint32_t wide;      // with set_lists: a near pair may be two cells apart
+    uint32_t eager;     // the cell list and xs are kept up to date in every step
     uint32_t cell_base; // batched contexts: first global cell id of this instance
     uint32_t uid_base;  // batched contexts: first global particle index of this instance
 };
@@ -79,7 +82,7 @@ struct ForceConsts {
     uint32_t nw, nb0, ncells, cell_base;
     int32_t periodic;
     uint32_t num[3];
-    uint32_t esv_skip;
+    uint32_t esv_skip, set_lists, eager;
     uint32_t pad;
     double origo[3], L[3], cellsize[3];
     double dt, g[3], rho, skin;
@@ -93,6 +96,8 @@ inline ForceConsts force_consts(const Params &P)
     c.cell_base = P.cell_base;
     c.periodic = P.periodic;
     c.esv_skip = P.esv_skip;
+    c.set_lists = P.set_lists;
+    c.eager = P.eager;
     for (int i = 0; i < 3; ++i) {
         c.num[i] = P.num[i];
         c.origo[i] = P.origo[i];
@@ -110,18 +115,32 @@ constexpr int VL_CAP = 32;              // candidates kept per particle
 constexpr uint8_t VL_NONE = 0xff;       // no usable list: sweep the stencil
 constexpr uint32_t MOVER_CAP = 1u << 16;
 
-// State of the Verlet-list epoch, device resident.  An epoch starts with a
-// full sweep of every particle; lists stay exact while 4 * dmax < skin, where
-// dmax bounds how far any particle moved since the epoch started.
+// State of the Verlet-list epoch, device resident.
+//
+// An epoch starts with a sweep of every particle, which records the pairs
+// within ra + rb + skin.  `moved` is the epoch's clock: the sum over its
+// steps of the largest displacement of any particle, so no particle has
+// moved farther than it advanced and no pair has closed by more than twice
+// that.  A pair missing from the lists cannot overlap while 2 moved < skin,
+// and a listed pair with a gap g at moment S not before S + g / 2.
+//
+// With Params::set_lists (cells at least (2 rmax + skin) / 2 wide, three of
+// them on a periodic axis) the lists hold every such pair whatever its cells,
+// two cells apart included (wide), so they outlive particles changing cell;
+// the cell list then goes stale until a sweep needs it (`rebuild`).  Without,
+// they hold the pairs of the 27-cell stencils and every change of cell makes
+// the cells around it sweep again.
 struct Verlet {
     uint32_t step;          // number of the step about to run (dirty stamps)
     uint32_t all_rebuild;   // every particle sweeps in this step
-    uint32_t dmax_bits;     // float bits of the displacement bound (atomicMax)
-    uint32_t nmovers;       // particles that changed cell in the last step
+    float moved;            // the epoch's clock at the start of the step
+    uint32_t want_cells;    // a particle without a list sweeps in the next step too
+    uint32_t nmovers;       // particles whose change of cell makes cells sweep
     uint32_t movers_overflow;
     uint32_t dirty_step;    // the last step in which any cell was stamped dirty
     uint32_t rebuilds;      // cell-list rebuilds performed since upload
-    uint32_t pad;
+    uint32_t inc2_bits;     // float bits of the step's largest squared displacement
+    uint32_t pad[3];
 };
 
 // Wall state (src/datatypes.h:95-100), device resident.
@@ -168,7 +187,8 @@ struct Dev {
     double4 *xr[2];       // x, y, z, radius
     P3 *vel[2];           // vx, vy, vz (fixvel in `fixed`, the host lane in w_user)
     P3 *angvel[2];        // wx, wy, wz (the host lane in w_user)
-    float4 *xs[2];        // float copy of xr in cell-list order, for the neighbour cull
+    float4 *xs[2];        // float copy of xr in cell-list order, for the neighbour cull (up to
+                          // date after a rebuild; in every step with Params::eager)
     // private per-particle state (updated in place); three doubles each, the
     // fourth lane of the host rows (never changed by a step) is kept apart in
     // w_user
@@ -182,7 +202,6 @@ struct Dev {
     double4 *edp;         // es_dot, ev_dot, p, 0
     uint32_t *uid, *sidx;
     uint32_t *cell;       // cell id (calcCellID semantics) of the current positions
-    uint8_t *outside;     // the position's floored cell coordinates leave the grid
     // contacts
     uint32_t *contacts;   // tiled, NC per particle (tile_at)
     ulonglong2 *dmc;      // [np] 4-bit periodic shift code of each of the NC slots
@@ -205,13 +224,11 @@ struct Dev {
     uint32_t *alias_any;  // some particle sits outside its cell's box (set by the rebuild)
     // Verlet lists
     uint32_t *vl;         // tiled, VL_CAP per particle: candidate storage indices, in visiting order
-    uint32_t *vl_meta;    // tiled, VL_CAP per particle: vl_meta_of(stencil cell, shift code, gap)
+    uint32_t *vl_meta;    // tiled, VL_CAP per particle: vl_meta_of(shift code, moment)
     uint8_t *vl_len;      // [np] list length or VL_NONE
-    float *vl_gap;        // [np] lower bound of the smallest gap to a listed candidate
-    float *disp;          // [np] displacement bound since the epoch started
-    uint8_t *settled;     // [np] every candidate of the valid list holds its slot (k_topo sets
-                          // it; a freed slot, a new list, upload or relayout clears it)
-    uint2 *movers;        // [MOVER_CAP] (old cell, new cell) of the last step
+    uint32_t *vl_held;    // [np] entries known to hold a slot through their image; 0 says nothing
+    float *due;           // [np] the moment after which the particle is searched; below 0: next step
+    uint2 *movers;        // [MOVER_CAP] (old cell, new cell) of the last step's moves that make cells sweep
     uint32_t *dirty;      // [ncells + 1] step stamp: a neighbour cell changed members
     Verlet *vs;
     // walls
@@ -422,17 +439,15 @@ constexpr uint64_t BULK_WAIT_NS = 1000000000ull;
 #endif
 constexpr uint32_t PF_SLOTS = SPHK_PF_SLOTS;
 
-// The metadata of a Verlet-list entry: bits 0-4 the stencil cell (0..26),
-// 5-15 the periodic shift code, 16-31 the top half of the float gap to the
-// candidate when the list was recorded (a lower bound: the float's low half
-// is dropped, toward zero, and a negative gap is kept as 0).
-__device__ __forceinline__ uint32_t vl_meta_of(uint32_t slot, uint32_t code, float gap)
+// The metadata of a Verlet-list entry: bits 0-3 the periodic shift code, the
+// rest the float moment (Verlet::moved) after which the pair can overlap, its
+// low four bits dropped (toward zero: still a lower bound).
+__device__ __forceinline__ uint32_t vl_meta_of(uint32_t code, float when)
 {
-    const uint32_t g = __float_as_uint(fmaxf(gap, 0.0f)) & 0xffff0000u;
-    return slot | (code << 5) | g;
+    return code | (__float_as_uint(when) & 0xfffffff0u);
 }
-__device__ __forceinline__ uint32_t vl_code(uint32_t meta) { return (meta & 0xffffu) >> 5; }
-__device__ __forceinline__ float vl_gap_of(uint32_t meta) { return __uint_as_float(meta & 0xffff0000u); }
+__device__ __forceinline__ uint32_t vl_code(uint32_t meta) { return meta & 0xfu; }
+__device__ __forceinline__ float vl_when(uint32_t meta) { return __uint_as_float(meta & 0xfffffff0u); }
 
 // Entry e of particle s's Verlet list (Dev::vl, Dev::vl_meta): tiled like
 // the slots, or (SPHK_VL_ROWS) one row of VL_CAP entries per particle.

@@ -382,11 +382,19 @@ __device__ __forceinline__ void dm_set(unsigned long long &lo, unsigned long lon
 
 // findDistMod for one axis that may be periodic (src/contactsearch.cuh:12-74):
 // wraps -1 -> num-1 (shift +L, code bit lo) and num -> 0 (shift -L, bit hi).
+// far: a cell beyond the stencil, which only the candidate lists look at.
 __device__ __forceinline__ void wrap_axis(int32_t &c, uint32_t num, uint32_t &code,
-                                          uint32_t bit_lo, uint32_t bit_hi)
+                                          uint32_t bit_lo, uint32_t bit_hi, bool far)
 {
+    if (far && c == -2) { c += (int32_t)num; code |= bit_lo; return; }
+    if (far && c == (int32_t)num + 1) { c = 1; code |= bit_hi; return; }
     if (c < 0) { c = (int32_t)(num - 1); code |= bit_lo; }
     if ((uint32_t)c == num) { c = 0; code |= bit_hi; }
+}
+// Whether a stencil cell lies past an axis that is not periodic.
+__device__ __forceinline__ bool past_axis(int32_t c, uint32_t num, bool far)
+{
+    return c < 0 || (uint32_t)c == num || (far && (uint32_t)c > num);
 }
 
 // Slot state of one particle during contact detection.
@@ -473,17 +481,16 @@ __device__ __noinline__ bool topo_insert(const Dev &d, uint32_t *srow, int tid, 
     return ++ts.nc <= NC;
 }
 
-// The reference's overlap predicate, float_sqrt(dot) - (ra + rb) < 0, for
-// candidate t through a stencil cell with shift `code`
-// (src/contactsearch.cuh:233-248).
-__device__ __forceinline__ bool overlaps(const Params &P, const double4 *xr, uint32_t t,
-                                         uint32_t code, double4 xa)
+// The reference's overlap, float_sqrt(dot) - (ra + rb), of candidate row xb
+// through a stencil cell with shift `code` (src/contactsearch.cuh:233-248);
+// it overlaps where this is below 0.0f.
+__device__ __forceinline__ double pair_gap(const Params &P, double4 xb, uint32_t code, double4 xa,
+                                           double &len)
 {
-    const double4 xb = xr[t];
     const d3 dm = decode_dm(code, P);
     const d3 xab = add(mk(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z), dm);
-    const double delta = flen(xab) - (xa.w + xb.w);
-    return delta < 0.0f;
+    len = flen(xab);
+    return len - (xa.w + xb.w);
 }
 
 // Contact model 1 processes each candidate as soon as it is found
@@ -507,36 +514,82 @@ __device__ __noinline__ void visc_pair(const Dev &d, int A, uint32_t s, uint32_t
     }
 }
 
-// How far particle s and any partner can have closed their gap since s's list
-// was recorded: its own displacement bound plus the largest of any particle,
-// rounded up.  While that stays below the list's smallest gap (Dev::vl_gap)
-// no listed candidate can overlap, and the list need not be tested.
-__device__ __forceinline__ float moved_bound(const Dev &d, uint32_t s, const Verlet &V)
+// A moment on the epoch's clock (Verlet::moved) before which a pair whose
+// gap is `gap` now, at moment S, cannot overlap: each of the two moves at
+// most as far as the clock advances.  `slack` covers the float roundings of
+// this length and of the later one.  Rounded down.
+__device__ __forceinline__ float pair_when(float S, double gap, double slack)
 {
-    return __fadd_ru(d.disp[s], __uint_as_float(V.dmax_bits));
+    const float g = __double2float_rd(gap - slack);
+    return g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
 }
 
-// k_topo: one thread per particle s (storage order, which relayout keeps close
-// to cell order); its cell-list position k = pos[s] locates it in the runs.
+// The stencil slot (0..26, z y x) through which the search of a particle in
+// grid cell gp reaches a candidate in global cell `cell` through image
+// `code`, or -1 where its stencil does not.
+__device__ __forceinline__ int stencil_slot(const Params &P, const int32_t gp[3], uint32_t cell,
+                                            uint32_t code)
+{
+    const uint32_t c = cell - P.cell_base;
+    if (c >= P.ncells) return -1;
+    const uint32_t nx = P.num[0], ny = P.num[1];
+    int32_t x = (int32_t)(c % nx) - gp[0], y = (int32_t)((c / nx) % ny) - gp[1];
+    const int32_t z = (int32_t)(c / (nx * ny)) - gp[2];
+    if (code & 1u) x -= (int32_t)nx;
+    if (code & 2u) x += (int32_t)nx;
+    if (code & 4u) y -= (int32_t)ny;
+    if (code & 8u) y += (int32_t)ny;
+    if (x < -1 || x > 1 || y < -1 || y > 1 || z < -1 || z > 1) return -1;
+    return (z + 1) * 9 + (y + 1) * 3 + (x + 1);
+}
+
+// The entry of `set` (a mask over s's candidate list) that the reference's
+// search visits first: by stencil cell, then by particle index.  Entries
+// outside the stencil are dropped from `set`; returns -1 when none is left.
+// `slot`: the stencil slot of the entry.
+__device__ __noinline__ int first_visited(const Dev &d, const Params &P, const int32_t gp[3],
+                                          uint32_t s, uint32_t &set, int &slot)
+{
+    int best = -1;
+    uint64_t bkey = ~0ull;
+    for (uint32_t m = set; m; m &= m - 1u) {
+        const int e = __ffs(m) - 1;
+        const size_t at = vl_at(s, (uint32_t)e);
+        const uint32_t t = d.vl[at];
+        const int k = stencil_slot(P, gp, d.cell[t], vl_code(d.vl_meta[at]));
+        if (k < 0) { set &= ~(1u << e); continue; }
+        const uint64_t key = ((uint64_t)k << 32) | d.uid[t];
+        if (key < bkey) { bkey = key; best = e; slot = k; }
+    }
+    if (best >= 0) set &= ~(1u << best);
+    return best;
+}
+
+// The contact search of one particle s that is due (k_topo); sweep: its
+// candidate list cannot be used.
 //
-// List mode: while the particle's Verlet list is valid (no epoch restart, no
-// cell of its neighbourhood changed members this step) only the listed
-// candidates are tested, in their recorded order.  The list holds, in the
-// reference's visiting order, every member of the stencil cells that was
-// within ra + rb + skin when it was recorded; a pair missing from it is at
-// least skin - 4 dmax > 0 apart now, so it cannot overlap.
+// List mode: the list holds every candidate that can overlap while the epoch
+// lasts, each with the earliest moment it can (vl_when).  Candidates known to
+// hold their slot (Dev::vl_held) need no test: the reference leaves such a
+// slot as it is, and a separated one is freed by the force pass.  The others
+// that are due are measured, and either overlap or get a new moment.  The
+// order of new overlaps is the reference's visiting order, taken from their
+// present cells; with one, the usual case, there is no order to find.  The
+// reference's count nc matters only once a row can fill up: while the
+// occupied slots plus the list length stay within NC none can (`simple`);
+// otherwise every overlap is walked in order, as the reference does.
 //
 // Sweep mode: the 27 stencil cells are scanned as in the reference (z, y, x;
-// members by particle index) and the list is recorded on the way.
+// members by particle index) and the list is recorded on the way, together
+// with the near candidates two cells away where cells are that small
+// (Params::wide).
 //
 // VISC (contact model 1): no slots; every candidate within ra + rb + db is
 // processed in visiting order and the contact force and pressure sums are
 // left in Dev::c1acc for k_force_tiles.
-// The contact search of one particle s whose list decision (k_topo) did not
-// settle it: list_ok, its Verlet list is valid; held, Dev::settled[s].
 template <bool VISC, bool BATCH, int TB>
 __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int tid, uint32_t *srow,
-                                            bool list_ok, bool held)
+                                            bool sweep)
 {
     const Params &P = prm_at<BATCH>(d, s);
     const uint32_t len = d.vl_len[s];
@@ -545,15 +598,17 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     // the edge cells, where the stencil sweep grows with the square of their
     // count.  The search stays off until an upload clears the status.  A
     // batch goes on, since its other scenes are still sound.  Tested only
-    // here, past the list decision, so that the particles the decision
-    // settles do not wait for the status word.
+    // here, past the decision, so that the particles it settles do not wait
+    // for the status word.
     // The slot mask and the position are loaded with the status word, so
     // the three wait out one memory latency together.
     const uint32_t occ_in = d.cmask[s];
     const double4 xa = d.xr[A][s];
+    uint32_t held = VISC ? 0u : d.vl_held[s];
     if (!BATCH && (*(volatile const uint32_t *)d.status & ST_OUT_OF_GRID)) return;
     const double ra = xa.w;
     const double4 *__restrict__ xr = d.xr[A];
+    const float S = d.vs->moved;
     TopoSlots ts{occ_in, occ_in, 0u, 0ull, 0ull, 0, false, false};
     const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
     int32_t gp[3];
@@ -565,27 +620,15 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const bool use_lists = P.skin > 0.0 && gp_in;
     d3 F1 = mk(0.0, 0.0, 0.0);   // model 1 sums
     double p1 = 0.0f;
+    float due = 3.0e38f;         // the particle's next moment
 
-    if (VISC && list_ok) {
-        for (uint32_t e = 0; e < len; ++e) {
-            const size_t at = vl_at(s, e);
-            visc_pair(d, A, s, d.vl[at], vl_code(d.vl_meta[at]), F1, p1);
-        }
-    } else if (list_ok) {
+    if (use_lists && !sweep && len != VL_NONE) {
+        const bool simple = VISC || len + (uint32_t)__popc(ts.occ) <= (uint32_t)NC;
+        if (!simple) held = 0u;
+        const bool rows = !VISC && simple && held == 0u && ts.occ != 0u;
+        uint32_t act = 0;   // entries that overlap (or act, model 1)
         // the list is read four entries at a time, so that their loads are
         // in flight together
-        // A candidate that already holds a slot through the same image needs
-        // no test: overlapping or not, the reference's topology leaves its
-        // slot as it is (a separated one is freed by the force pass).  The
-        // test only feeds the count nc, which matters once a row fills up;
-        // while the occupied slots plus the list length stay within NC, no
-        // row can fill, so the filter changes nothing.
-        const bool filter = ts.occ != 0u && len + (uint32_t)__popc(ts.occ) <= (uint32_t)NC;
-        // A candidate whose own recorded gap exceeds the displacement bound
-        // cannot overlap (nor hold a slot taken since the list was
-        // recorded): its position is not fetched.  Skipping it leaves the
-        // order of the others, and so the slot choice, unchanged.
-        const float bound = moved_bound(d, s, *d.vs);
         uint32_t tv[4], mv[4];
         auto load4 = [&](uint32_t e0) {
 #pragma unroll
@@ -595,33 +638,68 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 mv[j] = d.vl_meta[at];
             }
         };
-        load4(0);   // the first four entries are in flight with the slot row
-        if (filter) topo_load_row<TB>(d, srow, tid, s, ts);
-        int skip_slot = -1;
-        uint32_t found = 0;   // candidates found in their slots
+        if (len) load4(0);   // the first four entries are in flight with the slot row
+        if (rows) topo_load_row<TB>(d, srow, tid, s, ts);
         for (uint32_t e0 = 0; e0 < len; e0 += 4) {
             if (e0) load4(e0);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (e0 + (uint32_t)j >= len) break;
-                const uint32_t meta = mv[j];
-                const int slot = (int)(meta & 31u);
-                if (slot == skip_slot) continue;   // nc > NC: rest of that cell
-                const uint32_t t = tv[j], code = vl_code(meta);
-                if (filter && in_slot<TB>(srow, tid, ts, t, code)) {
-                    ++found;
+                const uint32_t e = e0 + (uint32_t)j;
+                if (e >= len) break;
+                if ((held >> e) & 1u) continue;
+                const uint32_t t = tv[j], code = vl_code(mv[j]);
+                if (rows && in_slot<TB>(srow, tid, ts, t, code)) {
+                    held |= 1u << e;
                     continue;
                 }
-                if (vl_gap_of(meta) > bound) continue;
-                if (overlaps(P, xr, t, code, xa) && !topo_insert<TB>(d, srow, tid, s, t, code, ts))
-                    skip_slot = slot;
+                const float w = vl_when(mv[j]);
+                // (a pair of model 1 acts in every step, at rest too)
+                if (VISC ? !(S >= w) : !(S > w)) { due = fminf(due, w); continue; }
+                double ln;
+                const double gap = pair_gap(P, xr[t], code, xa, ln);
+                if (VISC ? (gap < 0.0f || gap < P.db) : (gap < 0.0f)) {
+                    act |= 1u << e;
+                } else {
+                    const uint32_t meta =
+                        vl_meta_of(code, pair_when(S, gap, 1e-6 * ln + (VISC ? P.reach_extra : 0.0)));
+                    d.vl_meta[vl_at(s, e)] = meta;
+                    due = fminf(due, vl_when(meta));
+                }
             }
         }
-        // every candidate already held its slot: settled until a slot is
-        // freed (k_contact) or the list is recorded again
-        if (!VISC && filter && found == len && len != 0) d.settled[s] = 1;
+        if (act) {
+            uint32_t left = act;
+            int slot = 0, skip_slot = -1;
+            if (!VISC && simple && (act & (act - 1u)) == 0u) {
+                // one new overlap: its slot does not depend on any order
+                const size_t at = vl_at(s, (uint32_t)(__ffs(act) - 1));
+                const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
+                if (stencil_slot(P, gp, d.cell[t], code) >= 0) {
+                    topo_insert<TB>(d, srow, tid, s, t, code, ts);
+                    held |= act;
+                } else {
+                    due = -1.0f;   // not in the stencil yet: looked at again next step
+                }
+            } else {
+                for (int e; (e = first_visited(d, P, gp, s, left, slot)) >= 0;) {
+                    const size_t at = vl_at(s, (uint32_t)e);
+                    const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
+                    if constexpr (VISC) {
+                        visc_pair(d, A, s, t, code, F1, p1);
+                    } else {
+                        if (slot == skip_slot) continue;   // nc > NC: rest of that cell
+                        if (!topo_insert<TB>(d, srow, tid, s, t, code, ts)) skip_slot = slot;
+                        held |= 1u << e;
+                    }
+                }
+                if (VISC || (held & act) != act) due = -1.0f;
+            }
+        }
+        if (!simple) {
+            held = 0u;
+            due = -1.0f;
+        }
     } else {
-        if (held) d.settled[s] = 0;   // the list is recorded again
         const float4 *__restrict__ xs = d.xs[A];
         const uint32_t k = d.pos[s];
         const float4 xaf = xs[k];
@@ -631,14 +709,15 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         const float extraf = (float)P.reach_extra;
         uint32_t nlist = 0;
         bool list_overflow = false;
-        float gmin = 3.0e38f;   // smallest gap to a listed candidate, bounded below
+        held = 0u;
 
         // A run [beg, end) of cell-list positions (one cell, or the three
-        // cells of an x-row whose inner boundaries are bnd1 <= bnd2, stencil
-        // slots slot0 .. slot0 + 2), culled four candidates at a time so the
-        // four loads are in flight together; hits are handled in list order.
+        // cells of an x-row whose inner boundaries are bnd1 <= bnd2), culled
+        // four candidates at a time so the four loads are in flight
+        // together; hits are handled in list order.  far: cells outside the
+        // stencil, whose candidates are only recorded.
         auto scan_run = [&](uint32_t beg, uint32_t end, uint32_t code, uint32_t bnd1,
-                            uint32_t bnd2, uint32_t slot0) {
+                            uint32_t bnd2, bool far) {
             const float sx = (code & 1u) ? Lf0 : ((code & 2u) ? -Lf0 : 0.0f);
             const float sy = (code & 4u) ? Lf1 : ((code & 8u) ? -Lf1 : 0.0f);
             uint32_t base = beg;
@@ -660,14 +739,10 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                     const float rs = (rsum + skinf) * 1.000004f + eps;
                     const uint32_t k2 = base + (uint32_t)j;
                     const bool ok = k2 < end && k2 != k;
-                    if (ok && d2 < rs * rs) {
-                        near |= 1u << j;
-                        // the gap, with the cull's float slack taken against
-                        // it (over every near candidate: at least the listed)
-                        gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
-                        gmin = fminf(gmin, gj[j]);
-                    }
-                    if (ok && d2 < rr * rr) hit |= 1u << j;
+                    // the gap, with the cull's float slack taken against it
+                    gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
+                    if (ok && d2 < rs * rs) near |= 1u << j;
+                    if (ok && !far && d2 < rr * rr) hit |= 1u << j;
                 }
                 uint32_t next = base + 4;
                 while (near) {
@@ -675,27 +750,37 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                     near &= near - 1;
                     const uint32_t k2 = base + (uint32_t)j;
                     const uint32_t t = __ldg(&d.cellorder[k2]);
-                    const uint32_t slot = slot0 + ((k2 < bnd1) ? 0u : ((k2 < bnd2) ? 1u : 2u));
+                    const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
+                    float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
+                    if (VISC) {
+                        if ((hit >> j) & 1u) {
+                            visc_pair(d, A, s, t, code, F1, p1);
+                            w = -1.0f;
+                        }
+                    } else if ((hit >> j) & 1u) {
+                        double ln;
+                        if (pair_gap(P, xr[t], code, xa, ln) < 0.0f) {
+                            if (!topo_insert<TB>(d, srow, tid, s, t, code, ts)) {
+                                // nc > NC: skip the rest of this cell; the list
+                                // would not describe the skipped part
+                                next = (k2 < bnd1) ? bnd1 : ((k2 < bnd2) ? bnd2 : end);
+                                near = 0;
+                                list_overflow = true;
+                            }
+                            if (nlist < VL_CAP) held |= 1u << nlist;
+                            w = 3.0e38f;
+                        }
+                    }
+                    due = fminf(due, w);
                     if (!use_lists) {
                     } else if (nlist < VL_CAP) {
                         const size_t at = vl_at(s, nlist);
                         d.vl[at] = t;
-                        d.vl_meta[at] = vl_meta_of(slot, code, gj[j]);
+                        // a held entry that loses its slot is due at once
+                        d.vl_meta[at] = vl_meta_of(code, w > 1.0e38f ? S : fmaxf(w, 0.0f));
                         ++nlist;
                     } else {
                         list_overflow = true;
-                    }
-                    if (VISC) {
-                        if ((hit >> j) & 1u) visc_pair(d, A, s, t, code, F1, p1);
-                    } else if ((hit >> j) & 1u) {
-                        if (overlaps(P, xr, t, code, xa) &&
-                            !topo_insert<TB>(d, srow, tid, s, t, code, ts)) {
-                            // nc > NC: skip the rest of this cell; the list
-                            // would not describe the skipped part
-                            next = (k2 < bnd1) ? bnd1 : ((k2 < bnd2) ? bnd2 : end);
-                            near = 0;
-                            list_overflow = true;
-                        }
                     }
                 }
                 base = next;
@@ -709,72 +794,89 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         // while the particle's own cell is inside the grid and every
         // particle sits inside its cell's box (alias_any clear).
         const bool prune = gp_in && (*d.alias_any == 0u);
-        float flo[3], fhi[3];
+        // squared distances to the cells one and two away on each axis
+        float lo1[3], hi1[3], lo2[3], hi2[3];
         {
             const double xc[3] = {xa.x, xa.y, xa.z};
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 const double lo = xc[q] - (P.origo[q] + (double)gp[q] * P.cellsize[q]);
                 const double hi = (P.origo[q] + (double)(gp[q] + 1) * P.cellsize[q]) - xc[q];
-                flo[q] = lo > 0.0 ? (float)(lo * lo) * 0.99999f : 0.0f;
-                fhi[q] = hi > 0.0 ? (float)(hi * hi) * 0.99999f : 0.0f;
+                const double l2 = lo + P.cellsize[q], h2 = hi + P.cellsize[q];
+                lo1[q] = lo > 0.0 ? (float)(lo * lo) * 0.99999f : 0.0f;
+                hi1[q] = hi > 0.0 ? (float)(hi * hi) * 0.99999f : 0.0f;
+                lo2[q] = l2 > 0.0 ? (float)(l2 * l2) * 0.99999f : 0.0f;
+                hi2[q] = h2 > 0.0 ? (float)(h2 * h2) * 0.99999f : 0.0f;
             }
         }
+        auto dist2 = [&](int q, int o) {
+            return o == 0 ? 0.0f : (o < 0 ? (o == -1 ? lo1[q] : lo2[q]) : (o == 1 ? hi1[q] : hi2[q]));
+        };
         const double extra = VISC ? P.reach_extra : 0.0;
         const float reach = (float)((ra + P.rmax + P.skin + extra) * (1.0 + 1e-5) + P.prune_pad);
         const float reach2 = prune ? reach * reach : 3.0e38f;
+        const int R = (P.wide && use_lists) ? 2 : 1;
 
-        for (int oz = -1; oz < 2; ++oz) {
+        for (int oz = -R; oz <= R; ++oz) {
             const int32_t cz = (int32_t)((uint32_t)gp[2] + (uint32_t)oz);
-            if (cz < 0 || (uint32_t)cz == nz) continue;
-            const float dz2 = oz < 0 ? flo[2] : (oz > 0 ? fhi[2] : 0.0f);
+            if (past_axis(cz, nz, R == 2)) continue;
+            const float dz2 = dist2(2, oz);
             if (dz2 > reach2) continue;
-            for (int oy = -1; oy < 2; ++oy) {
-                const float dyz2 = dz2 + (oy < 0 ? flo[1] : (oy > 0 ? fhi[1] : 0.0f));
+            for (int oy = -R; oy <= R; ++oy) {
+                const float dyz2 = dz2 + dist2(1, oy);
                 if (dyz2 > reach2) continue;
                 int32_t cy = (int32_t)((uint32_t)gp[1] + (uint32_t)oy);
                 uint32_t ycode = 0;
                 if (P.periodic == 1) {
-                    wrap_axis(cy, ny, ycode, 4u, 8u);
-                } else if (cy < 0 || (uint32_t)cy == ny) {
+                    wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
+                } else if (past_axis(cy, ny, R == 2)) {
                     continue;
                 }
                 const uint32_t rowbase = (uint32_t)cy * nx + (nx * ny) * (uint32_t)cz;
-                const uint32_t slot0 = (uint32_t)((oz + 1) * 9 + (oy + 1) * 3);
-                const int32_t c0 = gp[0] - 1;
-                if (c0 >= 0 && (uint32_t)c0 + 2 < nx) {
-                    // the three x cells are consecutive ids: one run of xs
-                    const uint32_t cid0 = (uint32_t)c0 + rowbase;
-                    if (cid0 + 2 >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
-                    const uint32_t g0 = cid0 + P.cell_base;
-                    const uint32_t b0 = d.cell_start[g0], b1 = d.cell_start[g0 + 1];
-                    const uint32_t b2 = d.cell_start[g0 + 2], b3 = d.cell_start[g0 + 3];
-                    const uint32_t lo = (dyz2 + flo[0] <= reach2) ? b0 : b1;
-                    const uint32_t hi = (dyz2 + fhi[0] <= reach2) ? b3 : b2;
-                    scan_run(lo, hi, ycode, b1, b2, slot0);
-                } else {
-                    for (int ox = -1; ox < 2; ++ox) {
-                        if (dyz2 + (ox < 0 ? flo[0] : (ox > 0 ? fhi[0] : 0.0f)) > reach2) continue;
-                        int32_t cx = (int32_t)((uint32_t)gp[0] + (uint32_t)ox);
-                        uint32_t code = ycode;
+                const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
+                for (int ox = -R; ox <= R; ++ox) {
+                    int32_t cx = (int32_t)((uint32_t)gp[0] + (uint32_t)ox);
+                    uint32_t beg, end, b1, b2, code = ycode;
+                    const bool far = far_row || ox < -1 || ox > 1;
+                    if (!far && ox == -1 && cx >= 0 && (uint32_t)cx + 2 < nx) {
+                        // the three x cells are consecutive ids: one run of xs
+                        ox = 1;
+                        const uint32_t cid0 = (uint32_t)cx + rowbase;
+                        if (cid0 + 2 >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
+                        const uint32_t g0 = cid0 + P.cell_base;
+                        const uint32_t b0 = d.cell_start[g0], b3 = d.cell_start[g0 + 3];
+                        b1 = d.cell_start[g0 + 1];
+                        b2 = d.cell_start[g0 + 2];
+                        beg = (dyz2 + lo1[0] <= reach2) ? b0 : b1;
+                        end = (dyz2 + hi1[0] <= reach2) ? b3 : b2;
+                    } else {
+                        if (dyz2 + dist2(0, ox) > reach2) continue;
                         if (P.periodic == 1 || P.periodic == 2) {
-                            wrap_axis(cx, nx, code, 1u, 2u);
-                        } else if (cx < 0 || (uint32_t)cx == nx) {
+                            wrap_axis(cx, nx, code, 1u, 2u, R == 2);
+                        } else if (past_axis(cx, nx, R == 2)) {
                             continue;
                         }
                         const uint32_t cid = (uint32_t)cx + rowbase;
                         if (cid >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
                         const uint32_t g = cid + P.cell_base;
-                        const uint32_t e = d.cell_start[g + 1];
-                        scan_run(d.cell_start[g], e, code, e, e, slot0 + (uint32_t)(ox + 1));
+                        beg = d.cell_start[g];
+                        end = b1 = b2 = d.cell_start[g + 1];
                     }
+                    scan_run(beg, end, code, b1, b2, far);
                 }
             }
         }
-        d.vl_len[s] = (use_lists && !list_overflow) ? (uint8_t)nlist : VL_NONE;
-        if (use_lists) d.vl_gap[s] = gmin;
+        const bool listed = use_lists && !list_overflow;
+        d.vl_len[s] = listed ? (uint8_t)nlist : VL_NONE;
+        if (!listed) {
+            // sweeps again next step, over a cell list of that step
+            due = -1.0f;
+            if (P.skin > 0.0) d.vs->want_cells = 1u;
+        }
     }
 
+    d.due[s] = due;
+    if (!VISC) d.vl_held[s] = held;
     if (VISC) d.c1acc[s] = make_double4(F1.x, F1.y, F1.z, p1);
     if (ts.dirty) {
         // the search only fills empty slots (and may change a code): the
@@ -792,32 +894,30 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     if (ts.err) atomicOr(d.status, ts.err);
 }
 
-// Most particles whose list decision each lane of k_topo makes in one go.
+// Most particles whose decision each lane of k_topo makes in one go.
 constexpr uint32_t TOPO_SPAN_MAX = 4;
 
 // k_topo: the contact search, one warp per span x 32 consecutive storage
 // indices (storage order, which relayout keeps close to cell order), span
-// <= TOPO_SPAN_MAX.  First every lane makes the list decision of its span
-// particles (particle base + 32 j + lane), their loads in flight together;
-// the particles it does not settle are then dealt to the warp's lanes in
-// order, 32 at a time, each searched by topo_search.
+// <= TOPO_SPAN_MAX.  First every lane decides for its span particles (particle
+// base + 32 j + lane), their loads in flight together: a particle is searched
+// only when the epoch's clock has passed the moment Dev::due kept for it, the
+// earliest at which anything can change for it.  The particles that are due
+// are then dealt to the warp's lanes in order, 32 at a time, each searched by
+// topo_search.
 //
-// List mode: while the particle's Verlet list is valid (no epoch restart, no
-// cell of its neighbourhood changed members this step) only the listed
-// candidates are tested, in their recorded order.  The list holds, in the
-// reference's visiting order, every member of the stencil cells that was
-// within ra + rb + skin when it was recorded; a pair missing from it is at
-// least skin - 4 dmax > 0 apart now, so it cannot overlap.
-//
-// Sweep mode: the 27 stencil cells are scanned as in the reference (z, y, x;
-// members by particle index) and the list is recorded on the way.
-//
-// VISC (contact model 1): no slots; every candidate within ra + rb + db is
-// processed in visiting order and the contact force and pressure sums are
-// left in Dev::c1acc for k_force_tiles.
+// What bounds it: the latency of the few searches (three dependent L2 round
+// trips in a warp with one), not bytes -- the decision reads 4 a particle.
+// The lists used to be tied to the cells (a particle that changed cell made
+// the 54 cells around it sweep, and the cell list was sorted anew in each
+// such step) and tested against the largest displacement in every step.  Per
+// step, search + cell list, then and now: 1M loose grains in motion 44 + 60
+// -> 11.3 + 0.1 us; 50k in a rapid flow 36 + 25 -> 15 + 2 us; 64 jammed
+// scenes of 330k grains 233 + 62 -> 5.3 + 0.1 us; the 1M jammed column 13.9
+// -> 8.7 us.
 template <bool VISC, bool BATCH, int TB>
 __global__ void __launch_bounds__(TB, TOPO_THREADS_PER_SM / TB)
-k_topo(Dev d, int A, uint32_t span)
+k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ uint32_t srow[NC * TB];
@@ -831,52 +931,37 @@ k_topo(Dev d, int A, uint32_t span)
         d.vs->movers_overflow = 0u;
     }
     const Verlet &V = *d.vs;
-    // bit j: particle base + 32 j + lane needs the search / has a valid
-    // list / is marked settled
-    uint32_t need = 0, lok = 0, hld = 0;
+    const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == V.step;
+    const float S = V.moved;
+    // bit j: particle base + 32 j + lane is searched / must sweep
+    uint32_t need = 0, swp = 0;
 #pragma unroll
     for (uint32_t j = 0; j < TOPO_SPAN_MAX; ++j) {
         const uint32_t s = base + 32u * j + lane;
         if (j >= span) break;
         if (s >= np) continue;
-        const Params &P = prm_at<BATCH>(d, s);
-        // The list decision, from a few bytes: a valid list whose gap bound
-        // rules out every contact ends the particle's work here.  Its
-        // per-particle loads are unconditional so that they (and those of
-        // the lane's other particles) are in flight together.
-        const uint8_t len = d.vl_len[s];
-        const uint8_t outs = d.outside[s];
-        const float gap = d.vl_gap[s];
-        const uint8_t held = VISC ? 0 : d.settled[s];
-        const float bound = moved_bound(d, s, V);
-        bool list_ok = P.skin > 0.0 && !V.all_rebuild && len != VL_NONE && outs == 0;
-        if (list_ok && V.dirty_step == V.step) list_ok = d.dirty[d.cell[s]] != V.step;
-        // A valid list whose candidates all hold their slots (Dev::settled) is
-        // settled too: the reference's topology would find every overlap among
-        // them (the list holds every possible one) already in its slot and
-        // change nothing.
-        if (list_ok && (gap > bound || held)) {
+        const float due = d.due[s];
+        const bool sw = all || (dirty && d.dirty[d.cell[s]] == V.step);
+        if (!sw && !(S > due)) {
             if (VISC) d.c1acc[s] = make_double4(0.0, 0.0, 0.0, 0.0);
             continue;
         }
         need |= 1u << j;
-        if (list_ok) lok |= 1u << j;
-        if (held) hld |= 1u << j;
+        if (sw) swp |= 1u << j;
     }
     // the warp's particles that need the search, in (j, lane) order: the
     // k-th goes to lane k % 32 in round k / 32
-    uint32_t m[TOPO_SPAN_MAX], ml[TOPO_SPAN_MAX], mh[TOPO_SPAN_MAX];
+    uint32_t m[TOPO_SPAN_MAX], ms[TOPO_SPAN_MAX];
     uint32_t total = 0;
 #pragma unroll
     for (uint32_t j = 0; j < TOPO_SPAN_MAX; ++j) {
-        // need, lok and hld have no bit j >= span: those masks are zero
+        // need and swp have no bit j >= span: those masks are zero
         m[j] = __ballot_sync(FULL, (need >> j) & 1u);
-        ml[j] = __ballot_sync(FULL, (lok >> j) & 1u);
-        mh[j] = __ballot_sync(FULL, (hld >> j) & 1u);
+        ms[j] = __ballot_sync(FULL, (swp >> j) & 1u);
         total += (uint32_t)__popc(m[j]);
     }
     for (uint32_t k = lane; k < total; k += 32u) {
-        uint32_t rem = k, sel = 0, selj = 0, sel_l = 0, sel_h = 0;
+        uint32_t rem = k, sel = 0, selj = 0, sel_s = 0;
         bool got = false;
 #pragma unroll
         for (uint32_t j = 0; j < TOPO_SPAN_MAX; ++j) {
@@ -884,8 +969,7 @@ k_topo(Dev d, int A, uint32_t span)
             if (!got) {
                 if (rem < c) {
                     sel = m[j];
-                    sel_l = ml[j];
-                    sel_h = mh[j];
+                    sel_s = ms[j];
                     selj = j;
                     got = true;
                 } else {
@@ -895,7 +979,7 @@ k_topo(Dev d, int A, uint32_t span)
         }
         const uint32_t bit = __fns(sel, 0, (int)rem + 1);
         const uint32_t s = base + 32u * selj + bit;
-        topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_l >> bit) & 1u, (sel_h >> bit) & 1u);
+        topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u);
     }
 }
 
@@ -920,8 +1004,6 @@ struct GlobalRows {
     __device__ P3 angvel0() const { return d.angvel0[s]; }
     __device__ P3 vel0() const { return d.vel0[s]; }
     __device__ double2 xysum() const { return d.xysum[s]; }
-    __device__ uint32_t pos() const { return d.pos[s]; }
-    __device__ float disp() const { return d.disp[s]; }
     __device__ uint32_t cell() const { return d.cell[s]; }
     __device__ uint8_t fixed() const { return d.fixed[s]; }
     __device__ uint8_t wtouch() const { return d.wtouch[s]; }
@@ -945,8 +1027,7 @@ struct __align__(16) ForceTile {
     double4 xr[FT_TILE];
     P3 vel[FT_TILE], angvel[FT_TILE], angpos[FT_TILE], angvel0[FT_TILE], vel0[FT_TILE];
     double2 xysum[FT_TILE];
-    uint32_t pos[FT_TILE], cell[FT_TILE];
-    float disp[FT_TILE];
+    uint32_t cell[FT_TILE];
     uint8_t fixed[FT_TILE], wtouch[FT_TILE];
 };
 static_assert(sizeof(ForceTile) % 16 == 0 && (FT_TILE % 16) == 0, "bulk copies are multiples of 16 bytes");
@@ -969,8 +1050,6 @@ struct TileRows {
     __device__ P3 angvel0() const { return T.angvel0[r]; }
     __device__ P3 vel0() const { return T.vel0[r]; }
     __device__ double2 xysum() const { return T.xysum[r]; }
-    __device__ uint32_t pos() const { return T.pos[r]; }
-    __device__ float disp() const { return T.disp[r]; }
     __device__ uint32_t cell() const { return T.cell[r]; }
     __device__ uint8_t fixed() const { return T.fixed[r]; }
     __device__ uint8_t wtouch() const { return T.wtouch[r]; }
@@ -988,10 +1067,9 @@ struct TileRows {
 // angvel_a4 are the particle's start-of-step rows of buffer A, R reads its
 // other rows; the new state goes to buffer 1 - A.
 // P: the particle's scene constants (Params, or a launch's ForceConsts);
-// restart: this step starts a Verlet epoch (Verlet::all_rebuild).
 template <bool BATCH, bool DIFF, class Rows, class PS>
 __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_t s, int A,
-                                              int write_outputs, bool restart, double4 xa,
+                                              int write_outputs, double4 xa,
                                               double4 vel_a, double4 angvel_a4, d3 F, d3 T,
                                               double p, double ev_dot, double es_dot,
                                               const Rows &R)
@@ -1150,19 +1228,19 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     d.xr[B][s] = x;
     d.vel[B][s] = p3of(vel);
     d.vel0[s] = vel0;
-    // float copy for the next step's contact search, at this particle's
-    // cell-list position (rewritten by the rebuild when the order changes)
-    d.xs[B][R.pos()] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+    // float copy in cell-list order, where every step needs it
+    if (P.eager) d.xs[B][d.pos[s]] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
 
-    // ---- displacement bound since the Verlet epoch started ----------------
+    // ---- the largest displacement of the step, squared, rounded up ---------
     Verlet &V = *d.vs;
     if (P.skin > 0.0) {
-        const double ix = vel0.x * dt, iy = vel0.y * dt, iz = vel0.z * dt;
-        const float inc = __fadd_ru(__fmul_ru((float)sqrt(ix * ix + iy * iy + iz * iz), 1.0001f), 1e-15f);
-        const float dnew = __fadd_ru(restart ? 0.0f : R.disp(), inc);
-        d.disp[s] = dnew;
-        const uint32_t bits = __reduce_max_sync(__activemask(), __float_as_uint(dnew));
-        if ((threadIdx.x & 31u) == (uint32_t)(__ffs(__activemask()) - 1)) atomicMax(&V.dmax_bits, bits);
+        const float fx = __double2float_ru(fabs(vel0.x * dt)), fy = __double2float_ru(fabs(vel0.y * dt)),
+                    fz = __double2float_ru(fabs(vel0.z * dt));
+        const float d2 = __fmaf_ru(fx, fx, __fmaf_ru(fy, fy, __fmul_ru(fz, fz)));
+        const uint32_t bits = __reduce_max_sync(__activemask(), __float_as_uint(d2) & 0x7fffffffu);
+        if ((threadIdx.x & 31u) == (uint32_t)(__ffs(__activemask()) - 1) &&
+            bits > *(volatile uint32_t *)&V.inc2_bits)
+            atomicMax(&V.inc2_bits, bits);
     }
 
     // ---- cell of the new position, for the next step's cell list -----------
@@ -1171,12 +1249,31 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     uint32_t c;
     if (!grid_cell(P, x.x, x.y, x.z, c)) { err |= ST_OUT_OF_GRID; c = d.ncells_all; }
     else c += P.cell_base;
-    d.outside[s] = cell_outside(P, x.x, x.y, x.z) ? 1 : 0;
+    const bool out = cell_outside(P, x.x, x.y, x.z);
     const uint32_t c_old = R.cell();
+    if (out) {
+        // outside its cell's box: its own search sweeps, over a fresh list
+        *d.rebuild = 1u;
+        d.due[s] = -1.0f;
+    }
     if (c != c_old) {
         d.cell[s] = c;
-        *d.rebuild = 1u;
-        if (P.skin > 0.0) {
+        // A move between neighbouring cells inside the grid leaves every
+        // candidate list as it is (the lists are sets of near pairs, ordered
+        // by their cells only when needed).  Any other -- through a periodic
+        // boundary, or from or to a place outside the cells' boxes -- changes
+        // images or what a stencil reaches: the cells around sweep again.
+        bool hard = out || !P.set_lists || c == d.ncells_all || c_old == d.ncells_all ||
+                    cell_outside(P, xa.x, xa.y, xa.z);
+        if (!hard) {
+            const uint32_t p = c_old - P.cell_base, q = c - P.cell_base;
+            const uint32_t nx = P.num[0], ny = P.num[1];
+            const int dx = (int)(q % nx) - (int)(p % nx), dy = (int)(q / nx % ny) - (int)(p / nx % ny),
+                      dz = (int)(q / (nx * ny)) - (int)(p / (nx * ny));
+            hard = dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1;
+        }
+        if (hard || P.eager) *d.rebuild = 1u;
+        if (hard && P.skin > 0.0) {
             const uint32_t m = atomicAdd(&V.nmovers, 1u);
             if (m < MOVER_CAP) d.movers[m] = make_uint2(c_old, c);
             else V.movers_overflow = 1u;
@@ -1188,10 +1285,10 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
 // Everything of one particle s after the contact search, outside the
 // differentiable step: its slot sums (k_contact's, or k_topo's for model 1)
 // and particle_tail.  f: the chunk flag of s (Dev::cflag[s / 32], read by
-// the caller ahead of the rows); restart: Verlet::all_rebuild.
+// the caller ahead of the rows).
 template <int MODEL, bool BATCH, class Rows>
 __device__ __forceinline__ void force_row(const ForceArgs &args, uint32_t s, const Rows &R,
-                                          uint8_t f, bool restart)
+                                          uint8_t f)
 {
     const Dev &d = args.d;
     // A chunk k_contact visited (flag 2: a contact remains, 3: none does)
@@ -1226,10 +1323,10 @@ __device__ __forceinline__ void force_row(const ForceArgs &args, uint32_t s, con
         es_dot = d.csum_es[s];
     }
     if constexpr (BATCH)
-        particle_tail<true, false>(d, prm_at<true>(d, s), s, args.a, args.write_outputs, restart, xa,
+        particle_tail<true, false>(d, prm_at<true>(d, s), s, args.a, args.write_outputs, xa,
                                    vel_a, angvel_a4, F, T, p, ev_dot, es_dot, R);
     else
-        particle_tail<false, false>(d, args.fc, s, args.a, args.write_outputs, restart, xa, vel_a,
+        particle_tail<false, false>(d, args.fc, s, args.a, args.write_outputs, xa, vel_a,
                                     angvel_a4, F, T, p, ev_dot, es_dot, R);
 }
 
@@ -1253,15 +1350,12 @@ k_force_diff(ForceArgs args)
         bulk_prefetch_l2(d.angvel0 + s, 32 * sizeof(P3));
         bulk_prefetch_l2(d.vel0 + s, 32 * sizeof(P3));
         bulk_prefetch_l2(d.xysum + s, 32 * sizeof(double2));
-        bulk_prefetch_l2(d.pos + s, 32 * sizeof(uint32_t));
-        bulk_prefetch_l2(d.disp + s, 32 * sizeof(float));
         bulk_prefetch_l2(d.cell + s, 32 * sizeof(uint32_t));
         bulk_prefetch_l2(d.fixed + s, 32);
         bulk_prefetch_l2(d.wtouch + s, 32);
     }
 #endif
     const GlobalRows R{d, args.a, s};
-    const bool restart = d.vs->all_rebuild != 0u;
     {
         const Params &P = *d.prm;
         const int A = args.a;
@@ -1318,7 +1412,8 @@ k_force_diff(ForceArgs args)
         }
         if (occ != occ0) {
             d.cmask[s] = occ;
-            d.settled[s] = 0;   // a listed candidate left its slot
+            d.vl_held[s] = 0u;   // a listed candidate left its slot: the
+            d.due[s] = -1.0f;    // next search looks at the list
         }
         if (j >= 0) {
             d.tp_x[row] = xa;
@@ -1327,7 +1422,7 @@ k_force_diff(ForceArgs args)
             d.tp_mask[row] = lawmask;
             d.tp_dmc[row] = dmw;
         }
-        particle_tail<false, true>(d, P, s, A, args.write_outputs, restart, xa, vel_a, angvel_a4, F,
+        particle_tail<false, true>(d, P, s, A, args.write_outputs, xa, vel_a, angvel_a4, F,
                                    T, p, ev_dot, es_dot, R);
     }
 }
@@ -1345,9 +1440,7 @@ __device__ __forceinline__ void stage_force_tile(const Dev &d, int A, uint32_t t
     bulk_load(T.angvel0, d.angvel0 + s0, sizeof(T.angvel0), bar);
     bulk_load(T.vel0, d.vel0 + s0, sizeof(T.vel0), bar);
     bulk_load(T.xysum, d.xysum + s0, sizeof(T.xysum), bar);
-    bulk_load(T.pos, d.pos + s0, sizeof(T.pos), bar);
     bulk_load(T.cell, d.cell + s0, sizeof(T.cell), bar);
-    bulk_load(T.disp, d.disp + s0, sizeof(T.disp), bar);
     bulk_load(T.fixed, d.fixed + s0, sizeof(T.fixed), bar);
     bulk_load(T.wtouch, d.wtouch + s0, sizeof(T.wtouch), bar);
 }
@@ -1390,7 +1483,6 @@ k_force_tiles(ForceArgs args)
         }
     }
     __syncthreads();
-    const bool restart = d.vs->all_rebuild != 0u;
     uint32_t t = blockIdx.x;
     for (uint32_t it = 0; t < ntiles; t += gridDim.x, ++it) {
         const uint32_t k = it % FT_STAGES;
@@ -1398,7 +1490,7 @@ k_force_tiles(ForceArgs args)
         // the chunk flag comes from global memory: asked for before the wait
         const uint8_t f = (MODEL != 1 && s < np) ? d.cflag[s >> 5] : (uint8_t)0;
         const bool ready = mbar_wait(&full[k], (it / FT_STAGES) & 1u, BULK_WAIT_NS);
-        if (ready && s < np) force_row<MODEL, BATCH>(args, s, TileRows{tiles[k], tid}, f, restart);
+        if (ready && s < np) force_row<MODEL, BATCH>(args, s, TileRows{tiles[k], tid}, f);
         if (__syncthreads_or(!ready)) {
             if (tid == 0) {
                 atomicOr(d.status, ST_TIMEOUT);
@@ -1659,7 +1751,8 @@ k_contact(ContactArgs args)
                 d.csum_es[s] = sm[8][lane];
                 if (occ != occ0) {
                     d.cmask[s] = occ;
-                    d.settled[s] = 0;   // a listed candidate left its slot
+                    d.vl_held[s] = 0u;   // a listed candidate left its slot: the
+            d.due[s] = -1.0f;    // next search looks at the list
                 }
             }
             // visited (2: a slot is still held, 3: none is); k_force_tiles reads

@@ -28,16 +28,23 @@ namespace sphk {
 
 constexpr int WALL_BLOCK = 256;
 
-// Verlet epoch decision for the next step: lists stay exact while
-// 4 * dmax < skin; otherwise every particle sweeps and a new epoch starts.
+// The epoch's clock and the decision for the next step: the lists hold every
+// pair that can overlap while 2 moved < skin; otherwise (a clock that is not a
+// number included) every particle sweeps and a new epoch starts.
 __device__ void step_tail(const Dev &d)
 {
     const Params &P = *d.prm;
     Verlet &V = *d.vs;
-    const float dmax = __uint_as_float(V.dmax_bits);
-    const bool restart = P.skin > 0.0 && 4.0 * (double)dmax >= 0.999 * P.skin;
+    float moved = V.moved;
+    const float inc = __fmul_ru(__fsqrt_ru(__uint_as_float(V.inc2_bits)), 1.00001f);
+    if (inc != 0.0f) moved = __fadd_ru(moved, __fadd_ru(inc, 1e-15f));
+    V.inc2_bits = 0u;
+    const bool restart = P.skin > 0.0 && !(2.02 * (double)moved < 0.999 * P.skin);
     V.all_rebuild = restart ? 1u : 0u;
-    if (restart) V.dmax_bits = 0u;
+    V.moved = restart ? 0.0f : moved;
+    // a sweep needs the cell list of its own step
+    if (restart || V.want_cells) *d.rebuild = 1u;
+    V.want_cells = 0u;
     V.step += 1u;
 }
 

@@ -1,0 +1,94 @@
+"""The candidate lists across changes of cell: grains that cross cells while
+their lists stay in use, several new contacts of one grain in one step (whose
+slots follow the reference's visiting order), cells of every size against the
+reach of a list, grids of two and three periodic cells, lists that overflow
+and grains outside their cells' boxes.  Everything bit for bit against the
+oracle, the cell list of the last step included."""
+import numpy as np
+import pytest
+
+from helpers import OUTPUT_FIELDS, STATE_FIELDS, WALL_FIELDS, mismatches, run_oracle, with_model
+from sphere_b200 import scenes
+from sphere_b200.sphk import BatchSimulation, Simulation
+from sphere_b200.state import config_from_spherebin, state_from_spherebin
+
+pytestmark = pytest.mark.gpu
+
+ALL = STATE_FIELDS + OUTPUT_FIELDS + ("contacts", "delta_t") + WALL_FIELDS
+
+
+def _flow(cell, periodic, n=900, seed=91, r=(0.8e-3, 1.6e-3), nw=0, **kw):
+    """Soft grains in fast motion; cells `cell` times the largest radius wide."""
+    sb = scenes.collision(n=n, seed=seed, periodic=periodic, r=r, nw=nw, vmax=6.0, k_n=500.0,
+                          k_t=500.0, gamma_n=0.01, straddle=periodic != 0, **kw)
+    sb.num = np.maximum(1, np.floor(sb.L / (cell * r[1]))).astype(np.uint32)
+    return sb
+
+
+SCENES = {
+    # two radii a cell: pairs of a list can be two cells apart
+    "cells_2r": lambda: _flow(2.0, 0),
+    "cells_2r_periodic": lambda: _flow(2.0, 1, box=(0.032, 0.032, 0.06)),
+    "cells_2r_periodic_x": lambda: _flow(2.0, 2, box=(0.032, 0.06, 0.06)),
+    # cells that hold the whole reach of a list
+    "cells_3r": lambda: _flow(3.0, 0, nw=1),
+    # below a diameter: overlapping grains the stencil does not reach
+    "cells_1.5r": lambda: _flow(1.5, 0),
+    # too small for any list to outlive a change of cell
+    "cells_1.05r": lambda: _flow(1.05, 0, n=500),
+    # three and two cells around a periodic axis
+    "three_cells": lambda: _flow(3.0, 1, n=400, box=(0.0165, 0.0165, 0.05)),
+    "two_cells": lambda: _flow(4.5, 1, n=400, box=(0.0165, 0.0165, 0.05)),
+    # grains four times their neighbours' size: more candidates than a list holds
+    "overflow": lambda: _flow(2.0, 0, n=1200, r=(0.35e-3, 2.0e-3)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+@pytest.mark.parametrize("skin", [0.1, 0.5])
+def test_lists_outlive_changes_of_cell(oracle_libs, name, skin):
+    sb = SCENES[name]()
+    rc, want, orun = run_oracle(oracle_libs["orc"], sb, 90)
+    assert rc == 0
+    cfg = config_from_spherebin(sb)
+    with Simulation(cfg, verlet_skin=skin) as sim:
+        sim.upload(state_from_spherebin(sb))
+        for k in (33, 1, 56):
+            sim.step(k)
+        sim.sync()
+        got = sim.download()
+        cell_sorted, perm, cstart, cend = sim.cells()
+    assert mismatches(got, want, ALL) == []
+    assert np.array_equal(perm, orun.perm) and np.array_equal(cell_sorted, orun.cell_sorted)
+    assert np.array_equal(cstart, orun.cell_start)
+    occ = orun.cell_start != 0xFFFFFFFF
+    assert np.array_equal(cend[occ], orun.cell_end[occ])
+
+
+@pytest.mark.parametrize("name", ["cells_2r", "cells_2r_periodic", "cells_1.5r", "two_cells"])
+def test_model1_lists_outlive_changes_of_cell(oracle_libs, name):
+    """Contact model 1 sums its pairs in visiting order: the order of a list
+    follows the grains' present cells."""
+    sb = with_model(SCENES[name](), 1)
+    rc, want, _ = run_oracle(oracle_libs["orc"], sb, 60)
+    assert rc == 0
+    with Simulation(config_from_spherebin(sb), verlet_skin=0.3) as sim:
+        sim.upload(state_from_spherebin(sb))
+        sim.step(60)
+        sim.sync()
+        got = sim.download()
+    assert mismatches(got, want, ALL) == []
+
+
+def test_batched_scenes_of_either_kind(oracle_libs):
+    """Scenes whose lists outlive changes of cell beside scenes whose do not."""
+    sbs = [SCENES[k]() for k in ("cells_2r", "cells_1.05r", "two_cells", "cells_2r_periodic_x")]
+    with BatchSimulation([config_from_spherebin(sb) for sb in sbs], verlet_skin=0.3) as sim:
+        sim.upload([state_from_spherebin(sb) for sb in sbs])
+        sim.step(50)
+        sim.sync()
+        got = sim.download_all()
+    for sb, st in zip(sbs, got):
+        rc, want, _ = run_oracle(oracle_libs["orc"], sb, 50)
+        assert rc == 0
+        assert mismatches(st, want, STATE_FIELDS + OUTPUT_FIELDS + ("contacts", "delta_t")) == []
