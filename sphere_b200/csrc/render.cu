@@ -28,14 +28,16 @@
 // products, two squarings, a subtraction), so a positive result needs
 //   dist^2 < R^2 (1 + 6u) + 16 u |ec|^2.
 // The box is the image of the ball around c with radius
-//   sqrt(R^2 (1 + 1e-6) + 4e-6 |ec|^2) + 2e-6 (|e| + |c| + |ec| (1 + P / D)),
-// about four times those bounds plus the rounding of c, e and d (P: the
-// image-plane half extent, D: the focal distance), projected through the
-// eye onto the image plane, widened by two pixels.  A ball that reaches the
+//   sqrt(R^2 (1 + 1e-6) + 1.1e-6 |ec|^2) + 2e-6 (|e| + |c| + |ec| (1 + P / D)),
+// a tenth above those bounds (16 u = 0.954e-6; what they leave out is of
+// order u^2) plus the rounding of c, e and d (P: the image-plane half
+// extent, D: the focal distance), projected through the eye onto the image
+// plane, widened by half a pixel.  A ball that reaches the
 // plane through the eye parallel to the image plane projects without bound:
 // such a sphere is tested against every pixel.
 #include "sphk_internal.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -104,21 +106,6 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rt_rays(RenderArgs g, fl3 *A, fl3 
     B[t] = p_v * V;
 }
 
-// the reference's intersection (src/raytracer.cuh:84-108): true when the
-// discriminant is positive and |t_minus| < 1e10, with |t_minus| in *t
-__device__ __forceinline__ bool intersect(fl3 d, fl3 ec, float R, float *t)
-{
-    const float Delta = (2.0f * fdot(d, ec)) * (2.0f * fdot(d, ec)) -
-                        4.0f * fdot(d, d) * (fdot(ec, ec) - R * R);
-    if (!(Delta > 0.0f)) return false;
-    const float t_minus =
-        ((fdot(-d, ec) - sqrtf(fdot(d, ec) * fdot(d, ec) - fdot(d, d) * (fdot(ec, ec) - R * R))) /
-         fdot(d, d));
-    *t = fabsf(t_minus);
-    if (!(*t < 1e10f)) return false;   // NaN, or beyond the initial distance
-    return true;
-}
-
 // DEM::render's colour-map values (src/raytracer.cuh:396-452), by storage index
 __global__ void __launch_bounds__(RT_BLOCK) k_rt_values(Dev d, int A, int method, double *out)
 {
@@ -138,16 +125,17 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rt_values(Dev d, int A, int method
 }
 
 // DEM::maxPos (src/sphere.cpp:520-548): the largest coordinate on each axis,
-// starting from zero; a max is order-free, so any reduction order gives it
+// starting from zero; a max is order-free, so any reduction order gives it.
+// A resident grid, so that each axis takes a few atomics an SM (one a warp of
+// 32 particles queued 94,000 on three words: 62 us at 1M, 12 now).
 __global__ void __launch_bounds__(RT_BLOCK) k_rt_maxpos(Dev d, int A, unsigned long long *mx)
 {
-    const uint32_t s = blockIdx.x * RT_BLOCK + threadIdx.x;
     double m[3] = {0.0, 0.0, 0.0};
-    if (s < d.np_all) {
+    for (uint32_t s = blockIdx.x * RT_BLOCK + threadIdx.x; s < d.np_all; s += gridDim.x * RT_BLOCK) {
         const double4 x = d.xr[A][s];
-        m[0] = x.x > 0.0 ? x.x : 0.0;
-        m[1] = x.y > 0.0 ? x.y : 0.0;
-        m[2] = x.z > 0.0 ? x.z : 0.0;
+        m[0] = x.x > m[0] ? x.x : m[0];
+        m[1] = x.y > m[1] ? x.y : m[1];
+        m[2] = x.z > m[2] ? x.z : m[2];
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -158,9 +146,15 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rt_maxpos(Dev d, int A, unsigned l
     }
 }
 
+// A sphere's pixels.  What bounds it: instructions, a discriminant for each
+// pixel of the box.  A pixel whose key is already nearer than the sphere can
+// be (a plain read, possibly out of date: keys only fall) takes no root and
+// no atomic.  1M spheres, 800 x 800: 542 us with a box four times the bound's
+// and a root and an atomic for every hit, 164 us now.
 __global__ void __launch_bounds__(RT_BLOCK)
-k_rt_splat(Dev d, int A, RenderArgs g, const double *values, const fl3 *__restrict__ colA,
-           const fl3 *__restrict__ rowB, unsigned long long *keys)
+k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderArgs g,
+           const double *values, const fl3 *__restrict__ colA, const fl3 *__restrict__ rowB,
+           unsigned long long *keys)
 {
     const uint32_t s = blockIdx.x * RT_BLOCK + threadIdx.x;
     if (s >= d.np_all) return;
@@ -187,7 +181,7 @@ k_rt_splat(Dev d, int A, RenderArgs g, const double *values, const fl3 *__restri
     const float *ip = g.cam.imgplane;
     const double P = fmax(fmax(fabs((double)ip[0]), fabs((double)ip[1])),
                           fmax(fabs((double)ip[2]), fabs((double)ip[3])));
-    const double rho = sqrt((double)R * R * (1.0 + 1e-6) + 4e-6 * nb * nb) +
+    const double rho = sqrt((double)R * R * (1.0 + 1e-6) + 1.1e-6 * nb * nb) +
                        2e-6 * (ne + nc + nb * (1.0 + P / D));
     const double a0 = qx * g.cam.u[0] + qy * g.cam.u[1] + qz * g.cam.u[2];
     const double b0 = qx * g.cam.v[0] + qy * g.cam.v[1] + qz * g.cam.v[2];
@@ -196,13 +190,19 @@ k_rt_splat(Dev d, int A, RenderArgs g, const double *values, const fl3 *__restri
     const int W = (int)g.W;
     int i0 = 0, i1 = W - 1, j0 = 0, j1 = W - 1;   // j: the wrapped row index
     const double r2 = rho * (1.0 + 1e-6);
+    // no hit's |t| is below this (0: not known).  The ray t d passes within
+    // rho of c, and the float root errs on t by less than rho / |d| more, so
+    // |t| |d| > |ec| - 3 rho; |d| is at most its length at the box's far corner.
+    float t_low = 0.0f;
     if (c0 * c0 > r2 * r2) {
         // image-plane coordinate -D * (along / depth) over the ball
+        double far2 = 0.0;   // squares of the box's largest plane coordinates
         auto range = [&](double p0, double lo_img, double hi_img, int n, int &lo, int &hi) {
             const double den = c0 * c0 - r2 * r2;
             const double root = r2 * sqrt(p0 * p0 + c0 * c0 - r2 * r2);
             const double k1 = (p0 * c0 + root) / den, k2 = (p0 * c0 - root) / den;
             const double pa = -D * k1, pb = -D * k2;
+            far2 += isfinite(pa) && isfinite(pb) ? fmax(pa * pa, pb * pb) : 1e300;
             if (!isfinite(pa) || !isfinite(pb)) return;   // keep the whole range
             const double plo = fmin(pa, pb), phi = fmax(pa, pb);
             const double span = hi_img - lo_img;
@@ -214,10 +214,10 @@ k_rt_splat(Dev d, int A, RenderArgs g, const double *values, const fl3 *__restri
                 return;
             }
             const double f_lo = (plo - lo_img) * n / span - 0.5, f_hi = (phi - lo_img) * n / span - 0.5;
-            if (!isfinite(f_lo) || !isfinite(f_hi)) return;
+            if (!isfinite(f_lo) || !isfinite(f_hi)) { far2 = 1e300; return; }
             const double a = fmin(f_lo, f_hi), b = fmax(f_lo, f_hi);
-            lo = (int)fmax(-1.0, fmin((double)n, floor(a) - 2.0));
-            hi = (int)fmax(-1.0, fmin((double)n, ceil(b) + 2.0));
+            lo = (int)fmax(-1.0, fmin((double)n, ceil(a - 0.5)));
+            hi = (int)fmax(-1.0, fmin((double)n, floor(b + 0.5)));
         };
         range(a0, ip[0], ip[1], (int)g.W, i0, i1);
         range(b0, ip[2], ip[3], (int)g.H, j0, j1);
@@ -225,31 +225,39 @@ k_rt_splat(Dev d, int A, RenderArgs g, const double *values, const fl3 *__restri
         i1 = min(i1, W - 1);
         j0 = max(j0, 0);
         j1 = min(j1, W - 1);
+        // the widening by half a pixel and the float directions: one more
+        // pixel's extent and 1e-5
+        const double px = fmax(fabs((double)ip[1] - ip[0]) / g.W, fabs((double)ip[3] - ip[2]) / g.H);
+        const double dmax = sqrt(D * D + far2) + 2.0 * px;
+        const double low = (nb - 3.0 * rho) / dmax * (1.0 - 1e-5);
+        if (low > 0.0 && low < 1e30) t_low = __double2float_rd(low);
     }
     if (i0 > i1 || j0 > j1) return;
-    // rows y whose wrapped index y mod W lies within [j0 - 1, j1 + 1]; the
-    // exact row index of each pixel is recomputed as the reference does
+    const float *key_t = reinterpret_cast<const float *>(keys) + 1;   // the |t| of a key
+    // Rows y with y mod W in [j0, j1].  The reference's row index of pixel m
+    // is floor((float)m / W) mod W: m is below 2^24, so the quotient errs by
+    // at most H 2^-24 < 1 / W and the floor is y for every pixel of row y.
     const uint32_t H = g.H;
     for (uint32_t base = 0; base < H; base += (uint32_t)W) {
-        const int ylo = (int)base + max(j0 - 1, 0), yhi = (int)base + min(j1 + 1, W - 1);
-        for (int y = ylo; y <= yhi && y < (int)H; ++y) {
-            // the row index floor((float)m / W) mod W does not decrease with
-            // m: equal at both ends of the box's row, it is the row's own
-            const uint32_t mrow = (uint32_t)y * g.W;
-            const uint32_t ja = (uint32_t)((int)floorf((float)(mrow + i0) / g.W) % (int)g.W);
-            const uint32_t jb = (uint32_t)((int)floorf((float)(mrow + i1) / g.W) % (int)g.W);
-            const fl3 Bj = rowB[ja];
+        for (int j = j0; j <= j1 && base + (uint32_t)j < H; ++j) {
+            const uint32_t mrow = (base + (uint32_t)j) * g.W;
+            const fl3 Bj = rowB[j];
             for (int xi = i0; xi <= i1; ++xi) {
                 const uint32_t m = mrow + (uint32_t)xi;
-                fl3 dir;
-                if (ja == jb) {
-                    dir = colA[xi] + Bj;
-                } else {
-                    const uint32_t j = (uint32_t)((int)floorf((float)m / g.W) % (int)g.W);
-                    dir = colA[xi] + rowB[j];
-                }
-                float t;
-                if (!intersect(dir, ec, R, &t)) continue;
+                const fl3 dir = colA[xi] + Bj;
+                // the reference's intersection (src/raytracer.cuh:84-108): a
+                // positive discriminant and |t_minus| < 1e10
+                const float Delta = (2.0f * fdot(dir, ec)) * (2.0f * fdot(dir, ec)) -
+                                    4.0f * fdot(dir, dir) * (fdot(ec, ec) - R * R);
+                if (!(Delta > 0.0f)) continue;
+                // no hit yet reads as NaN, which is not below
+                if (key_t[2 * (size_t)m] < t_low) continue;
+                const float t_minus =
+                    ((fdot(-dir, ec) -
+                      sqrtf(fdot(dir, ec) * fdot(dir, ec) - fdot(dir, dir) * (fdot(ec, ec) - R * R))) /
+                     fdot(dir, dir));
+                const float t = fabsf(t_minus);
+                if (!(t < 1e10f)) continue;   // NaN, or beyond the initial distance
                 const unsigned long long key = ((unsigned long long)__float_as_uint(t) << 32) | idx;
                 atomicMin(&keys[m], key);
             }
@@ -310,7 +318,8 @@ k_rt_resolve(Dev d, int A, RenderArgs g, const double *values, const unsigned lo
 
 void launch_maxpos(const Dev &d, uint32_t np, int a, unsigned long long *mx, cudaStream_t st)
 {
-    k_rt_maxpos<<<div_up(np, RT_BLOCK), RT_BLOCK, 0, st>>>(d, a, mx);
+    const unsigned resident = 8u * 148u;
+    k_rt_maxpos<<<std::min(div_up(np, RT_BLOCK), resident), RT_BLOCK, 0, st>>>(d, a, mx);
 }
 
 // DEM::render's camera (src/raytracer.cuh:351-367) and DEM::cameraInit
