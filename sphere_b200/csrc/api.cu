@@ -28,7 +28,8 @@ void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStrea
 unsigned int scan_tile_count(uint32_t ncells);
 void relayout(const Dev &d, uint32_t np, int a, void *scratch, cudaStream_t st);
 void launch_rebuild_gate(cudaGraphConditionalHandle h, const uint32_t *rebuild, cudaStream_t st);
-void launch_darcy(const Dev &d, const DarcyDev &f, const Params &hp, int a, int hs, cudaStream_t st);
+void launch_darcy(const Dev &d, const DarcyDev &f, const Params &hp, int a, int hs, int last,
+                  cudaStream_t st);
 struct RenderArgs;
 void launch_maxpos(const Dev &d, uint32_t np, int a, unsigned long long *mx, cudaStream_t st);
 int render_image(const Dev &d, uint32_t np, int a, const double L[3], const double maxpos[3],
@@ -373,7 +374,7 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
     if (branch) {
         CK(cudaEventRecord(c->darcy_fork, st));
         CK(cudaStreamWaitEvent(c->darcy_stream, c->darcy_fork, 0));
-        launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, c->darcy_stream);
+        launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, c->darcy_stream);
         CK(cudaEventRecord(c->darcy_join, c->darcy_stream));
     }
     const int model = (int)c->hp.contactmodel;
@@ -386,7 +387,7 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
         c->wall_pending = false;
     }
     launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, st);
-    if (c->darcy_on && !branch) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, st);
+    if (c->darcy_on && !branch) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
     if (capturing && c->hp.nw > 0 && !c->batched) {
         CK(cudaEventRecord(c->wall_fork, st));
         CK(cudaStreamWaitEvent(c->wall_stream, c->wall_fork, 0));
@@ -495,7 +496,7 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
     CK(cudaEventRecord(c->ev[5], st));
     launch_walls(c->d, c->np_all, c->hp.nw, st);
     CK(cudaEventRecord(c->ev[6], st));
-    if (c->darcy_on) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, st);
+    if (c->darcy_on) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
     CK(cudaEventRecord(c->ev[7], st));
     CK(cudaGetLastError());
     CK(cudaEventSynchronize(c->ev[7]));
