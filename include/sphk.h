@@ -265,8 +265,11 @@ int sph_render(sph_ctx *ctx, const sph_render_opts *opts, uint8_t *rgba);
  * gradient with respect to k_n, k_t and gamma_n (grad_params[3]), per-
  * particle friction (grad_mu[np]) and the starting positions and velocities
  * (x0_bar, v0_bar, np*3); any output may be NULL.  The context's state after
- * the call is the state before it.  sph_diff_end returns to the plain step
- * and frees the checkpoints and tape. */
+ * the call is the state before it.  sph_diff_end returns to the plain step;
+ * the context keeps the checkpoints' memory, and the tape's while the
+ * contexts of the process together keep no more of those than an eighth of
+ * the device's memory, for its next sph_diff_begin (a calibration loop's);
+ * sph_destroy frees both. */
 int sph_diff_begin(sph_ctx *ctx, const double *mu, uint32_t checkpoint_every);
 int sph_diff_backward(sph_ctx *ctx, const double *x_bar, const double *v_bar, double *grad_params,
                       double *grad_mu, double *x0_bar, double *v0_bar);

@@ -4,6 +4,7 @@
 #include "../../include/sphk.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -70,9 +71,13 @@ struct sph_ctx {
     size_t scratch_bytes = 0;
     std::vector<void *> allocs;
     size_t device_bytes = 0;
-    cudaGraphExec_t g_multi[2] = {nullptr, nullptr};
-    cudaGraphExec_t g_single[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    int graphs_for_k = 0;
+    // the graphs of a step, of the plain and of the differentiable one
+    struct StepGraphs {
+        cudaGraphExec_t multi[2] = {nullptr, nullptr};
+        cudaGraphExec_t single[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+        int for_k = 0;
+        ForceConsts fc{};   // the force kernel's constants in them
+    } graphs[2];
     std::string err;
     int sticky = SPH_OK;
     // profile mode: events bracket each phase of each step
@@ -109,7 +114,6 @@ struct sph_ctx {
     cudaStream_t wall_stream = nullptr;
     cudaEvent_t wall_fork = nullptr, wall_join = nullptr;
     bool wall_pending = false;
-    ForceConsts graph_fc{};          // the force kernel's constants in the step graphs
     int dflip = 0;
     double mean_radius = 0.0;        // of the uploaded particles, summed in caller order
     // ray tracer scratch: per-pixel keys and image, per-particle values
@@ -117,16 +121,35 @@ struct sph_ctx {
     size_t rt_bytes = 0;
     size_t ckpt_bytes = 0;                // size of one pooled buffer
     cudaEvent_t ckpt_ev = nullptr;        // orders a checkpoint copy against the caller's stream
+    // the tape and the adjoint arrays; sph_diff_end keeps them (and the graphs
+    // that hold them) for the next session with the same checkpoint interval,
+    // within KEPT_SHARE of the device's memory over all contexts
     std::vector<void *> diff_allocs;
     size_t diff_bytes = 0;
+    uint32_t diff_K = 0;                  // the interval they are sized for (0: none)
+    size_t kept_bytes = 0;                // counted in g_kept_bytes
+    struct {
+        double *mu_p;
+        double4 *x, *v, *w;
+        P3 *dt0;
+        uint32_t *mask, *partner;
+        ulonglong2 *dmc;
+        double *tmp;
+    } tape{};
     double *bwd_scratch = nullptr;        // the backward's seeds and results, 13 np doubles
     AdjDev adj{};
     // graphs of one segment's re-run with the tape and of its reverse, by
     // (segment length, starting buffer)
     std::map<std::pair<int, int>, cudaGraphExec_t> diff_graphs;
+    ForceConsts diff_fc{};                // the scene constants they were captured with
 };
 
 namespace {
+
+// Bytes of differentiable sessions kept after their end, over all contexts
+// of the process: at most 1 / KEPT_SHARE of the device's memory.
+constexpr size_t KEPT_SHARE = 8;
+std::atomic<size_t> g_kept_bytes{0};
 
 int fail(sph_ctx *c, int code, const std::string &msg)
 {
@@ -145,13 +168,13 @@ int fail(sph_ctx *c, int code, const std::string &msg)
     } while (0)
 
 template <typename T>
-int dalloc(sph_ctx *c, T **p, size_t count, std::vector<void *> *owner = nullptr)
+int dalloc(sph_ctx *c, T **p, size_t count, std::vector<void *> *owner = nullptr, bool clear = true)
 {
     const size_t bytes = sizeof(T) * (count ? count : 1);
     void *q = nullptr;
     cudaError_t e = cudaMalloc(&q, bytes);
     if (e != cudaSuccess) return fail(c, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    e = cudaMemsetAsync(q, 0, bytes, c->stream);
+    e = clear ? cudaMemsetAsync(q, 0, bytes, c->stream) : cudaSuccess;
     if (e != cudaSuccess) return fail(c, SPH_ERR_CUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
     (owner ? owner : &c->allocs)->push_back(q);
     (owner ? c->diff_bytes : c->device_bytes) += bytes;
@@ -442,14 +465,29 @@ int capture(sph_ctx *c, cudaGraphExec_t *out, int a, int nsteps, int write_last)
     return SPH_OK;
 }
 
-void drop_graphs(sph_ctx *c)
+void drop_step_graphs(sph_ctx::StepGraphs &S)
 {
-    for (auto &g : c->g_multi)
+    for (auto &g : S.multi)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-    for (auto &row : c->g_single)
+    for (auto &row : S.single)
         for (auto &g : row)
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-    c->graphs_for_k = 0;
+    S.for_k = 0;
+}
+
+// the graphs of the differentiable step and of the backward's segments
+void drop_diff_graphs(sph_ctx *c)
+{
+    drop_step_graphs(c->graphs[1]);
+    for (auto &kv : c->diff_graphs)
+        if (kv.second) cudaGraphExecDestroy(kv.second);
+    c->diff_graphs.clear();
+}
+
+void drop_graphs(sph_ctx *c)
+{
+    drop_step_graphs(c->graphs[0]);
+    drop_diff_graphs(c);
 }
 
 int ensure_graphs(sph_ctx *c)
@@ -457,18 +495,18 @@ int ensure_graphs(sph_ctx *c)
     // graphs carry the force kernel's constants: an upload that changed one
     // (the skin, esv_skip) captures them again
     const ForceConsts fc = force_consts(c->hp);
-    if (c->graphs_for_k == c->graph_steps && c->g_single[0][0] &&
-        std::memcmp(&fc, &c->graph_fc, sizeof(fc)) == 0)
+    sph_ctx::StepGraphs &S = c->graphs[c->diff ? 1 : 0];
+    if (S.for_k == c->graph_steps && S.single[0][0] && std::memcmp(&fc, &S.fc, sizeof(fc)) == 0)
         return SPH_OK;
-    drop_graphs(c);
+    drop_step_graphs(S);
     for (int a = 0; a < 2; ++a) {
         int rc;
-        if ((rc = capture(c, &c->g_multi[a], a, c->graph_steps, 0)) != SPH_OK) return rc;
+        if ((rc = capture(c, &S.multi[a], a, c->graph_steps, 0)) != SPH_OK) return rc;
         for (int w = 0; w < 2; ++w)
-            if ((rc = capture(c, &c->g_single[a][w], a, 1, w)) != SPH_OK) return rc;
+            if ((rc = capture(c, &S.single[a][w], a, 1, w)) != SPH_OK) return rc;
     }
-    c->graphs_for_k = c->graph_steps;
-    c->graph_fc = force_consts(c->hp);
+    S.for_k = c->graph_steps;
+    S.fc = fc;
     return SPH_OK;
 }
 
@@ -1069,14 +1107,14 @@ static int step_plain(sph_ctx *c, uint64_t nsteps, void *stream)
         const bool last_chunk = (i + room == nsteps);
         // multi-step graphs while more than one graph's worth remains
         while (room > K || (room == K && !last_chunk)) {
-            CK(cudaGraphLaunch(c->g_multi[c->a], st));
+            CK(cudaGraphLaunch(c->graphs[c->diff ? 1 : 0].multi[c->a], st));
             c->a ^= (int)(K & 1u);
             room -= K; i += K; c->since_relayout += K; c->steps += K;
             for (uint64_t k = 0; k < K; ++k) c->t_host += c->hp.dt;
         }
         while (room > 0) {
             const int w = (room == 1 && last_chunk) ? 1 : 0;
-            CK(cudaGraphLaunch(c->g_single[c->a][w], st));
+            CK(cudaGraphLaunch(c->graphs[c->diff ? 1 : 0].single[c->a][w], st));
             c->a ^= 1;
             room -= 1; i += 1; c->since_relayout += 1; c->steps += 1;
             c->t_host += c->hp.dt;
@@ -1405,24 +1443,33 @@ static int capture_segment(sph_ctx *c, int len, int a, cudaGraphExec_t *out)
     return SPH_OK;
 }
 
-static void free_diff(sph_ctx *c)
+// Ends a differentiable session: the checkpoints go back to their pool, and
+// the step's kernels lose the session's arrays.
+static void leave_diff(sph_ctx *c)
 {
-    for (auto &kv : c->diff_graphs)
-        if (kv.second) cudaGraphExecDestroy(kv.second);
-    c->diff_graphs.clear();
-    for (void *p : c->diff_allocs) cudaFree(p);
-    c->diff_allocs.clear();
-    c->bwd_scratch = nullptr;
-    c->diff_bytes = 0;
     for (auto &k : c->ckpts) ckpt_release(c, k.buf);
     c->ckpts.clear();
-    c->adj = AdjDev{};
     Dev &d = c->d;
     d.mu_p = nullptr;
     d.tp_x = d.tp_v = d.tp_w = nullptr;
     d.tp_dt0 = nullptr;
     d.tp_mask = d.tp_partner = nullptr;
     d.tp_dmc = nullptr;
+}
+
+// Frees the session's arrays with the graphs that hold them.
+static void free_diff(sph_ctx *c)
+{
+    leave_diff(c);
+    drop_diff_graphs(c);
+    for (void *p : c->diff_allocs) cudaFree(p);
+    c->diff_allocs.clear();
+    c->bwd_scratch = nullptr;
+    c->diff_bytes = 0;
+    c->diff_K = 0;
+    c->adj = AdjDev{};
+    g_kept_bytes -= c->kept_bytes;
+    c->kept_bytes = 0;
 }
 
 int sph_diff_begin(sph_ctx *c, const double *mu, uint32_t checkpoint_every)
@@ -1440,24 +1487,35 @@ int sph_diff_begin(sph_ctx *c, const double *mu, uint32_t checkpoint_every)
     const size_t np = c->np_all, K = checkpoint_every;
     Dev &d = c->d;
     AdjDev &A = c->adj;
+    auto &T = c->tape;
     std::vector<void *> *own = &c->diff_allocs;
     int rc = SPH_OK;
-#define ALD(ptr, n) if ((rc = dalloc(c, &(ptr), (n), own)) != SPH_OK) { free_diff(c); return rc; }
-    ALD(d.mu_p, np);
-    ALD(d.tp_x, K * np); ALD(d.tp_v, K * np); ALD(d.tp_w, K * np);
-    ALD(d.tp_mask, K * np); ALD(d.tp_dmc, K * np);
-    ALD(d.tp_partner, K * tiled_size(np, NC)); ALD(d.tp_dt0, K * tiled_size(np, NC));
-    ALD(A.xb, np); ALD(A.vb, np); ALD(A.wb, np); ALD(A.v0b, np); ALD(A.w0b, np);
-    ALD(A.Fb, np); ALD(A.Tb, np); ALD(A.dtb, tiled_size(np, NC)); ALD(A.mub, np); ALD(A.theta_b, 3);
-    ALD(A.dtb_mask, np);
-    double *tmp = nullptr;
-    ALD(tmp, np);
+    if (c->diff_K != checkpoint_every) {
+        free_diff(c);
+        // the tape's rows are written before they are read
+#define ALD(ptr, n, clear) \
+    if ((rc = dalloc(c, &(ptr), (n), own, clear)) != SPH_OK) { free_diff(c); return rc; }
+        ALD(T.mu_p, np, true);
+        ALD(T.x, K * np, false); ALD(T.v, K * np, false); ALD(T.w, K * np, false);
+        ALD(T.mask, K * np, false); ALD(T.dmc, K * np, false);
+        ALD(T.partner, K * tiled_size(np, NC), false); ALD(T.dt0, K * tiled_size(np, NC), false);
+        ALD(A.xb, np, true); ALD(A.vb, np, true); ALD(A.wb, np, true); ALD(A.v0b, np, true);
+        ALD(A.w0b, np, true); ALD(A.Fb, np, true); ALD(A.Tb, np, true);
+        ALD(A.dtb, tiled_size(np, NC), true); ALD(A.mub, np, true); ALD(A.theta_b, 3, true);
+        ALD(A.dtb_mask, np, true);
+        ALD(T.tmp, np, true);
 #undef ALD
+        c->diff_K = checkpoint_every;
+    }
+    d.mu_p = T.mu_p;
+    d.tp_x = T.x; d.tp_v = T.v; d.tp_w = T.w;
+    d.tp_dt0 = T.dt0;
+    d.tp_mask = T.mask; d.tp_partner = T.partner;
+    d.tp_dmc = T.dmc;
+    double *tmp = T.tmp;
     if (mu) CK(cudaMemcpyAsync(tmp, mu, np * 8, cudaMemcpyHostToDevice, c->stream));
     launch_user_to_storage1(mu ? tmp : nullptr, d.mu_p, d.uid, P.mu_s, (uint32_t)np, c->stream);
     CK(cudaStreamSynchronize(c->stream));
-    // kernels and graphs take Dev by value: capture again with the new arrays
-    drop_graphs(c);
     c->relayout_saved = c->relayout_every;
     c->relayout_every = 0;   // the tape and checkpoints are storage-indexed
     c->diff = true;
@@ -1503,6 +1561,14 @@ int sph_diff_backward(sph_ctx *c, const double *x_bar, const double *v_bar, doub
     CK(cudaMemsetAsync(A.dtb_mask, 0, (size_t)np * 4, st));
     CK(cudaMemsetAsync(A.mub, 0, (size_t)np * 8, st));
     CK(cudaMemsetAsync(A.theta_b, 0, 24, st));
+    // the graphs of a segment carry the scene constants, which an upload can change
+    const ForceConsts fc = force_consts(c->hp);
+    if (std::memcmp(&fc, &c->diff_fc, sizeof(fc)) != 0) {
+        for (auto &kv : c->diff_graphs)
+            if (kv.second) cudaGraphExecDestroy(kv.second);
+        c->diff_graphs.clear();
+        c->diff_fc = fc;
+    }
     const uint64_t nseg = (N + K - 1) / K;
     for (uint64_t seg = nseg; seg-- > 0;) {
         // adjoints survive the restore: they live apart from the state
@@ -1534,8 +1600,16 @@ int sph_diff_end(sph_ctx *c)
     if (!c->diff) return SPH_OK;
     CK(cudaSetDevice(c->device));
     CK(cudaDeviceSynchronize());
-    free_diff(c);
-    drop_graphs(c);
+    leave_diff(c);
+    // the session's arrays stay for the next one while all contexts together
+    // keep no more than their share of the device's memory
+    if (c->kept_bytes != c->diff_bytes) {
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        g_kept_bytes -= c->kept_bytes;
+        c->kept_bytes = c->diff_bytes;
+        if ((g_kept_bytes += c->kept_bytes) > total_b / KEPT_SHARE) free_diff(c);
+    }
     CK(cudaMemsetAsync(c->d.cflag, 1, div_up(c->np_all, 32), c->stream));
     // every list is looked at again (due below 0)
     CK(cudaMemsetAsync(c->d.due, 0xbf, (size_t)c->np_all * 4, c->stream));
