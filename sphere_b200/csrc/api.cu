@@ -15,14 +15,14 @@
 namespace sphk {
 void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st);
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  cudaStream_t st);
-void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                    cudaStream_t st);
+                  const NextStep &next, cudaStream_t st);
+void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st);
+bool small_step(const Dev &d, uint32_t np);
+void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                  const NextStep &next, cudaStream_t st);
 void launch_bonds(const Dev &d, const Params &hp, uint32_t nb0, int a, cudaStream_t st);
 void launch_bond_storage(const Dev &d, uint32_t nb0, uint32_t np, cudaStream_t st);
 void launch_walls(const Dev &d, uint32_t np, uint32_t nw, cudaStream_t st);
-void launch_wall_motion(const Dev &d, uint32_t np, cudaStream_t st);
-void launch_tail(const Dev &d, cudaStream_t st);
 void launch_cell_init(const Dev &d, uint32_t np, int a, cudaStream_t st);
 void launch_epoch_reset(const Dev &d, cudaStream_t st);
 void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st);
@@ -36,7 +36,8 @@ void launch_maxpos(const Dev &d, uint32_t np, int a, unsigned long long *mx, cud
 int render_image(const Dev &d, uint32_t np, int a, const double L[3], const double maxpos[3],
                  const sph_render_opts &o, double *values, unsigned long long *keys, uchar4 *img,
                  float *rays, cudaStream_t st);
-void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStream_t st);
+void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, const NextStep &next,
+                       cudaStream_t st);
 void launch_rev_step(const Dev &d, const AdjDev &a, uint32_t np, int j, cudaStream_t st);
 void launch_user_to_storage3(const double *src, double4 *dst, const uint32_t *uid, uint32_t n,
                              cudaStream_t st);
@@ -351,23 +352,42 @@ int sync_status(sph_ctx *c)
     return SPH_OK;
 }
 
-// Inside a stream capture: the rebuild as a conditional node whose body the
-// side stream captures, gated by k_rebuild_gate.
-int capture_rebuild_conditional(sph_ctx *c, int a, cudaStream_t st)
+// The condition handles of a graph's steps while it is captured: each step's
+// end sets that of the next, a kernel of its own (k_rebuild_gate) the first's.
+struct StepGate {
+    bool on = false;     // capturing, with conditional nodes
+    bool first = true;   // no step captured yet
+    NextStep here{};     // this step's handle
+};
+
+int captured_graph(sph_ctx *c, cudaStream_t st, cudaGraph_t *g, const cudaGraphNode_t **deps, size_t *nd)
 {
     cudaStreamCaptureStatus cs;
     unsigned long long id;
+    CK(cudaStreamGetCaptureInfo(st, &cs, &id, g, deps, nd));
+    return SPH_OK;
+}
+
+// Inside a stream capture: the rebuild as a conditional node whose body the
+// side stream captures, and the handle that the step's end sets for the next
+// step (`last`: there is none).
+int capture_rebuild_conditional(sph_ctx *c, int a, bool last, StepGate &gate, NextStep &next,
+                                cudaStream_t st)
+{
     cudaGraph_t g;
     const cudaGraphNode_t *deps;
     size_t nd;
-    CK(cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd));
-    cudaGraphConditionalHandle h;
-    CK(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
-    launch_rebuild_gate(h, c->d.rebuild, st);
-    CK(cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd));
+    int rc;
+    if ((rc = captured_graph(c, st, &g, &deps, &nd)) != SPH_OK) return rc;
+    if (gate.first) {
+        CK(cudaGraphConditionalHandleCreate(&gate.here.handle, g, 0, 0));
+        launch_rebuild_gate(gate.here.handle, c->d.rebuild, st);
+        gate.first = false;
+    }
+    if ((rc = captured_graph(c, st, &g, &deps, &nd)) != SPH_OK) return rc;
     cudaGraphNodeParams np{};
     np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = h;
+    np.conditional.handle = gate.here.handle;
     np.conditional.type = cudaGraphCondTypeIf;
     np.conditional.size = 1;
     cudaGraphNode_t node;
@@ -377,13 +397,22 @@ int capture_rebuild_conditional(sph_ctx *c, int a, cudaStream_t st)
     launch_rebuild(c->d, c->np_all, c->ncells_all, a, c->side);
     CK(cudaStreamEndCapture(c->side, &body));
     CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+    next = NextStep{};
+    if (!last) {
+        CK(cudaGraphConditionalHandleCreate(&next.handle, g, 0, 0));
+        next.gated = 1;
+        gate.here = next;
+    }
     return SPH_OK;
 }
 
-int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool capturing = false)
+// gate: of the graph being captured, or nullptr; last: its last step.
+int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, StepGate *gate, bool last)
 {
-    if (capturing && c->cond_rebuild) {
-        const int rc = capture_rebuild_conditional(c, a, st);
+    const bool capturing = gate != nullptr;
+    NextStep next{};
+    if (capturing && gate->on) {
+        const int rc = capture_rebuild_conditional(c, a, last, *gate, next, st);
         if (rc != SPH_OK) return rc;
     } else {
         launch_rebuild(c->d, c->np_all, c->ncells_all, a, st);
@@ -401,23 +430,30 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
         CK(cudaEventRecord(c->darcy_join, c->darcy_stream));
     }
     const int model = (int)c->hp.contactmodel;
-    launch_topo(c->d, c->np_all, model == 1, a, st);
-    launch_contact(c->d, c->hp, c->np_all, model, a, write_outputs, st);
-    if (c->wall_pending) {
-        // the walls moved by the previous step's branch, before this step's
-        // wall forces read them
-        CK(cudaStreamWaitEvent(st, c->wall_join, 0));
+    // walls moved by the previous step's branch, before this step's wall
+    // forces read them
+    auto join_walls = [&]() -> int {
+        if (c->wall_pending) CK(cudaStreamWaitEvent(st, c->wall_join, 0));
         c->wall_pending = false;
+        return SPH_OK;
+    };
+    int rc;
+    if (!c->diff && small_step(c->d, c->np_all)) {
+        if ((rc = join_walls()) != SPH_OK) return rc;
+        launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, next, st);
+    } else {
+        launch_topo(c->d, c->np_all, model == 1, a, st);
+        launch_contact(c->d, c->hp, c->np_all, model, a, st);
+        if ((rc = join_walls()) != SPH_OK) return rc;
+        launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, next, st);
     }
-    launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, st);
     if (c->darcy_on && !branch) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
     if (capturing && c->hp.nw > 0 && !c->batched) {
         CK(cudaEventRecord(c->wall_fork, st));
         CK(cudaStreamWaitEvent(c->wall_stream, c->wall_fork, 0));
-        launch_wall_motion(c->d, c->np_all, c->wall_stream);
+        launch_walls(c->d, c->np_all, c->hp.nw, c->wall_stream);
         CK(cudaEventRecord(c->wall_join, c->wall_stream));
         c->wall_pending = true;
-        launch_tail(c->d, st);
     } else {
         launch_walls(c->d, c->np_all, c->hp.nw, st);
     }
@@ -432,8 +468,11 @@ int capture(sph_ctx *c, cudaGraphExec_t *out, int a, int nsteps, int write_last)
     int aa = a;
     int rc = SPH_OK;
     c->wall_pending = false;
+    StepGate gate;
+    gate.on = c->cond_rebuild;
     for (int i = 0; i < nsteps && rc == SPH_OK; ++i) {
-        rc = enqueue_one_step(c, aa, (write_last && i == nsteps - 1) ? 1 : 0, c->stream, true);
+        const bool last = i == nsteps - 1;
+        rc = enqueue_one_step(c, aa, (write_last && last) ? 1 : 0, c->stream, &gate, last);
         aa ^= 1;
     }
     if (c->wall_pending) {
@@ -528,9 +567,9 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
     CK(cudaEventRecord(c->ev[2], st));
     launch_topo(c->d, c->np_all, c->hp.contactmodel == 1, a, st);
     CK(cudaEventRecord(c->ev[3], st));
-    launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, st);
+    launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, st);
     CK(cudaEventRecord(c->ev[4], st));
-    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, st);
+    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, NextStep{}, st);
     CK(cudaEventRecord(c->ev[5], st));
     launch_walls(c->d, c->np_all, c->hp.nw, st);
     CK(cudaEventRecord(c->ev[6], st));
@@ -1421,12 +1460,13 @@ static int capture_segment(sph_ctx *c, int len, int a, cudaGraphExec_t *out)
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int rc = SPH_OK;
     int aa = a;
+    StepGate gate;
     for (int j = 0; j < len && rc == SPH_OK; ++j) {
-        if (c->cond_rebuild) rc = capture_rebuild_conditional(c, aa, st);
+        NextStep next{};
+        if (c->cond_rebuild) rc = capture_rebuild_conditional(c, aa, j == len - 1, gate, next, st);
         else launch_rebuild(d, np, c->ncells_all, aa, st);
         launch_topo(d, np, false, aa, st);
-        launch_force_tape(d, np, aa, j, st);
-        launch_walls(d, np, 0, st);
+        launch_force_tape(d, np, aa, j, next, st);
         aa ^= 1;
     }
     for (int j = len - 1; j >= 0 && rc == SPH_OK; --j) launch_rev_step(d, c->adj, np, j, st);

@@ -186,7 +186,7 @@ __global__ void k_post_sort(Dev d, int A)
 // stencil again.  Periodic axes wrap as in findDistMod.
 __global__ void k_mark_dirty(Dev d)
 {
-    if (*d.rebuild == 0u) return;
+    if (*d.rebuild == 0u) return;   // cleared, with the movers, by the last launch of a rebuild
     Verlet &V = *d.vs;
     const uint32_t n = min(V.nmovers, MOVER_CAP);
     if (blockIdx.x == 0 && threadIdx.x == 0) V.rebuilds += 1u;
@@ -270,6 +270,14 @@ void launch_epoch_reset(const Dev &d, cudaStream_t st)
     k_epoch_reset<<<1, 1, 0, st>>>(d);
 }
 
+// the flag and the movers of the last step, consumed
+__global__ void k_rebuild_done(Dev d)
+{
+    *d.rebuild = 0u;
+    d.vs->nmovers = 0u;
+    d.vs->movers_overflow = 0u;
+}
+
 void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st)
 {
     const unsigned int ntiles = div_up((unsigned long long)ncells + 1, SCAN_TILE);
@@ -280,7 +288,7 @@ void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStrea
     k_cellsort<<<div_up((unsigned long long)ncells + 1, CELL_BLOCK), CELL_BLOCK, 0, st>>>(d);
     k_post_sort<<<div_up(np, CELL_BLOCK), CELL_BLOCK, 0, st>>>(d, a);
     k_mark_dirty<<<64, CELL_BLOCK, 0, st>>>(d);
-    cudaMemsetAsync(d.rebuild, 0, sizeof(uint32_t), st);
+    k_rebuild_done<<<1, 1, 0, st>>>(d);
 }
 
 unsigned int scan_tile_count(uint32_t ncells)

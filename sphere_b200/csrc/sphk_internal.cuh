@@ -87,7 +87,7 @@ struct ForceConsts {
     double origo[3], L[3], cellsize[3];
     double dt, g[3], rho, skin;
 };
-inline ForceConsts force_consts(const Params &P)
+__host__ __device__ inline ForceConsts force_consts(const Params &P)
 {
     ForceConsts c{};
     c.nw = P.nw;
@@ -140,7 +140,16 @@ struct Verlet {
     uint32_t dirty_step;    // the last step in which any cell was stamped dirty
     uint32_t rebuilds;      // cell-list rebuilds performed since upload
     uint32_t inc2_bits;     // float bits of the step's largest squared displacement
-    uint32_t pad[3];
+    uint32_t done_blocks;   // blocks of the step's force kernel that are through
+    uint32_t came_apart;    // a position had left the grid when the last step ended
+    uint32_t pad;
+};
+
+// What the end of a step sets for the next one in a graph: the condition of
+// the cell-list node in front of it.
+struct NextStep {
+    cudaGraphConditionalHandle handle;
+    int gated;   // there is such a node
 };
 
 // Wall state (src/datatypes.h:95-100), device resident.
@@ -285,6 +294,12 @@ struct LawParams {
     double k_n, k_t, gamma_n, gamma_t, gamma_r, mu_s, mu_d, mu_r, kappa, dt;
     double L[2];
 };
+
+__host__ __device__ inline LawParams law_params(const Params &P)
+{
+    return LawParams{P.k_n, P.k_t, P.gamma_n, P.gamma_t, P.gamma_r, P.mu_s, P.mu_d,
+                     P.mu_r, P.kappa, P.dt, {P.L[0], P.L[1]}};
+}
 
 // periodic shift code: bits 0-1 x (1: +L, 2: -L), bits 2-3 y.  PR is Params
 // or LawParams.

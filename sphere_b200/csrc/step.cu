@@ -525,13 +525,14 @@ __device__ __forceinline__ float pair_when(float S, double gap, double slack)
 }
 
 // The stencil slot (0..26, z y x) through which the search of a particle in
-// grid cell gp reaches a candidate in global cell `cell` through image
-// `code`, or -1 where its stencil does not.
-__device__ __forceinline__ int stencil_slot(const Params &P, const int32_t gp[3], uint32_t cell,
+// grid cell gp reaches a candidate at xb through image `code`, or -1 where its
+// stencil does not.  The candidate's cell is computed from its start-of-step
+// position: in k_small, Dev::cell may be the next step's by now.
+__device__ __forceinline__ int stencil_slot(const Params &P, const int32_t gp[3], double4 xb,
                                             uint32_t code)
 {
-    const uint32_t c = cell - P.cell_base;
-    if (c >= P.ncells) return -1;
+    uint32_t c;
+    if (!grid_cell(P, xb.x, xb.y, xb.z, c)) return -1;
     const uint32_t nx = P.num[0], ny = P.num[1];
     int32_t x = (int32_t)(c % nx) - gp[0], y = (int32_t)((c / nx) % ny) - gp[1];
     const int32_t z = (int32_t)(c / (nx * ny)) - gp[2];
@@ -547,7 +548,7 @@ __device__ __forceinline__ int stencil_slot(const Params &P, const int32_t gp[3]
 // search visits first: by stencil cell, then by particle index.  Entries
 // outside the stencil are dropped from `set`; returns -1 when none is left.
 // `slot`: the stencil slot of the entry.
-__device__ __noinline__ int first_visited(const Dev &d, const Params &P, const int32_t gp[3],
+__device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, const int32_t gp[3],
                                           uint32_t s, uint32_t &set, int &slot)
 {
     int best = -1;
@@ -556,7 +557,7 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, const i
         const int e = __ffs(m) - 1;
         const size_t at = vl_at(s, (uint32_t)e);
         const uint32_t t = d.vl[at];
-        const int k = stencil_slot(P, gp, d.cell[t], vl_code(d.vl_meta[at]));
+        const int k = stencil_slot(P, gp, d.xr[A][t], vl_code(d.vl_meta[at]));
         if (k < 0) { set &= ~(1u << e); continue; }
         const uint64_t key = ((uint64_t)k << 32) | d.uid[t];
         if (key < bkey) { bkey = key; best = e; slot = k; }
@@ -598,14 +599,14 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     // the edge cells, where the stencil sweep grows with the square of their
     // count.  The search stays off until an upload clears the status.  A
     // batch goes on, since its other scenes are still sound.  Tested only
-    // here, past the decision, so that the particles it settles do not wait
-    // for the status word.
-    // The slot mask and the position are loaded with the status word, so
-    // the three wait out one memory latency together.
+    // here, past the decision, and from the word the last step's end left
+    // (k_small's integration may be setting the status already).  The slot
+    // mask and the position are loaded with it, so the three wait out one
+    // memory latency together.
     const uint32_t occ_in = d.cmask[s];
     const double4 xa = d.xr[A][s];
     uint32_t held = VISC ? 0u : d.vl_held[s];
-    if (!BATCH && (*(volatile const uint32_t *)d.status & ST_OUT_OF_GRID)) return;
+    if (!BATCH && d.vs->came_apart != 0u) return;
     const double ra = xa.w;
     const double4 *__restrict__ xr = d.xr[A];
     const float S = d.vs->moved;
@@ -674,14 +675,14 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 // one new overlap: its slot does not depend on any order
                 const size_t at = vl_at(s, (uint32_t)(__ffs(act) - 1));
                 const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
-                if (stencil_slot(P, gp, d.cell[t], code) >= 0) {
+                if (stencil_slot(P, gp, xr[t], code) >= 0) {
                     topo_insert<TB>(d, srow, tid, s, t, code, ts);
                     held |= act;
                 } else {
                     due = -1.0f;   // not in the stencil yet: looked at again next step
                 }
             } else {
-                for (int e; (e = first_visited(d, P, gp, s, left, slot)) >= 0;) {
+                for (int e; (e = first_visited(d, P, A, gp, s, left, slot)) >= 0;) {
                     const size_t at = vl_at(s, (uint32_t)e);
                     const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
                     if constexpr (VISC) {
@@ -925,11 +926,6 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
     const int tid = threadIdx.x;
     const uint32_t lane = (uint32_t)tid & 31u;
     const uint32_t base = ((blockIdx.x * TB + (uint32_t)tid) >> 5) * (32u * span);
-    if (blockIdx.x == 0 && tid == 0) {
-        // the movers of the last step have been consumed by the rebuild
-        d.vs->nmovers = 0u;
-        d.vs->movers_overflow = 0u;
-    }
     const Verlet &V = *d.vs;
     const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == V.step;
     const float S = V.moved;
@@ -989,7 +985,45 @@ struct ForceArgs {
     int write_outputs;  // store force/torque/acc/angacc/edp of this step
     int tape_step;      // differentiable step: tape row to record, or -1
     ForceConsts fc;     // single-scene contexts: the scene's constants
+    NextStep next;
 };
+
+// The epoch's clock and the decision for the next step: the lists hold every
+// pair that can overlap while 2 moved < skin; otherwise (a clock that is not a
+// number included) every particle sweeps and a new epoch starts.  One thread,
+// after everything else of the step's force kernel.
+__device__ void step_tail(const Dev &d, const NextStep &next)
+{
+    const Params &P = *d.prm;
+    Verlet &V = *d.vs;
+    float moved = V.moved;
+    const float inc = __fmul_ru(__fsqrt_ru(__uint_as_float(atomicExch(&V.inc2_bits, 0u))), 1.00001f);
+    if (inc != 0.0f) moved = __fadd_ru(moved, __fadd_ru(inc, 1e-15f));
+    const bool restart = P.skin > 0.0 && !(2.02 * (double)moved < 0.999 * P.skin);
+    V.all_rebuild = restart ? 1u : 0u;
+    V.moved = restart ? 0.0f : moved;
+    // a sweep needs the cell list of its own step
+    const bool want = atomicExch(&V.want_cells, 0u) != 0u;
+    if (restart || want) *d.rebuild = 1u;
+    V.came_apart = *(volatile const uint32_t *)d.status & ST_OUT_OF_GRID;
+    V.step += 1u;
+    if (next.gated)
+        cudaGraphSetConditional(next.handle, (restart || want || *(volatile uint32_t *)d.rebuild) ? 1u : 0u);
+}
+
+// The last block of a force kernel ends the step (a launch of its own took
+// 1.8 us and a gap, and another one in front of every step's cell list to
+// read its flag).  Called by all threads of every block.
+__device__ __forceinline__ void end_of_step(const Dev &d, const NextStep &next)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&d.vs->done_blocks, 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    d.vs->done_blocks = 0u;
+    step_tail(d, next);
+}
 
 // Where the force kernels read a particle's own start-of-step rows: global
 // memory (GlobalRows) or a tile of rows staged in shared memory (TileRows).
@@ -1286,9 +1320,10 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
 // differentiable step: its slot sums (k_contact's, or k_topo's for model 1)
 // and particle_tail.  f: the chunk flag of s (Dev::cflag[s / 32], read by
 // the caller ahead of the rows).
+// fc: the constants of s's scene.
 template <int MODEL, bool BATCH, class Rows>
-__device__ __forceinline__ void force_row(const ForceArgs &args, uint32_t s, const Rows &R,
-                                          uint8_t f)
+__device__ __forceinline__ void force_row(const ForceArgs &args, const ForceConsts &fc, uint32_t s,
+                                          const Rows &R, uint8_t f)
 {
     const Dev &d = args.d;
     // A chunk k_contact visited (flag 2: a contact remains, 3: none does)
@@ -1322,12 +1357,8 @@ __device__ __forceinline__ void force_row(const ForceArgs &args, uint32_t s, con
         ev_dot = ct.w;
         es_dot = d.csum_es[s];
     }
-    if constexpr (BATCH)
-        particle_tail<true, false>(d, prm_at<true>(d, s), s, args.a, args.write_outputs, xa,
-                                   vel_a, angvel_a4, F, T, p, ev_dot, es_dot, R);
-    else
-        particle_tail<false, false>(d, args.fc, s, args.a, args.write_outputs, xa, vel_a,
-                                    angvel_a4, F, T, p, ev_dot, es_dot, R);
+    particle_tail<BATCH, false>(d, fc, s, args.a, args.write_outputs, xa, vel_a, angvel_a4, F, T, p,
+                                ev_dot, es_dot, R);
 }
 
 // The differentiable step's force kernel: one thread per particle, rows
@@ -1339,7 +1370,7 @@ k_force_diff(ForceArgs args)
     const Dev &d = args.d;
     const uint32_t np = d.np_all;
     const uint32_t s = blockIdx.x * FORCE_BLOCK + threadIdx.x;
-    if (s >= np) return;
+    if (s < np) {
 #ifndef SPHK_NO_PREFETCH
     // The state the integration reads comes after the contact work and
     // after stores the compiler may not move loads across, so each of its
@@ -1425,6 +1456,8 @@ k_force_diff(ForceArgs args)
         particle_tail<false, true>(d, P, s, A, args.write_outputs, xa, vel_a, angvel_a4, F,
                                    T, p, ev_dot, es_dot, R);
     }
+    }
+    end_of_step(d, args.next);
 }
 
 // Issues the bulk copies of tile t's rows into T, completing on `bar`.
@@ -1443,6 +1476,32 @@ __device__ __forceinline__ void stage_force_tile(const Dev &d, int A, uint32_t t
     bulk_load(T.cell, d.cell + s0, sizeof(T.cell), bar);
     bulk_load(T.fixed, d.fixed + s0, sizeof(T.fixed), bar);
     bulk_load(T.wtouch, d.wtouch + s0, sizeof(T.wtouch), bar);
+}
+
+// Calls `run` for the lanes of the (converged) warp with `on` set, the
+// constants of their scene in `slot`, the warp's own place in shared memory:
+// scene by scene, which is once for nearly every warp (storage is in scene
+// order).  `have`: the scene in the slot.  Read through their pointer the
+// constants would be loaded again after every store to global memory, which
+// might alias them.
+template <class Consts, class Fill, class Run>
+__device__ __forceinline__ void by_scene(Consts &slot, uint32_t &have, uint32_t inst, bool on,
+                                         Fill fill, Run run)
+{
+    uint32_t left = __ballot_sync(0xffffffffu, on);
+    while (left) {
+        const uint32_t i = __shfl_sync(0xffffffffu, inst, __ffs(left) - 1);
+        const bool mine = on && inst == i;
+        if (i != have) {
+            __syncwarp();
+            if ((threadIdx.x & 31u) == 0) fill(slot, i);
+            have = i;
+            __syncwarp();
+        }
+        left &= ~__ballot_sync(0xffffffffu, mine);
+        if (mine) run(slot);
+        __syncwarp();
+    }
 }
 
 // Shared-memory stages of k_force_tiles: tiles a block has in flight.
@@ -1468,6 +1527,8 @@ k_force_tiles(ForceArgs args)
 {
     __shared__ ForceTile tiles[FT_STAGES];
     __shared__ uint64_t full[FT_STAGES];
+    __shared__ ForceConsts scene[BATCH ? FT_TILE / 32 : 1];   // a batch's, one a warp
+    uint32_t have = 0xffffffffu;
     const Dev &d = args.d;
     const uint32_t np = d.np_all;
     const uint32_t ntiles = (np + FT_TILE - 1) / FT_TILE;
@@ -1490,7 +1551,16 @@ k_force_tiles(ForceArgs args)
         // the chunk flag comes from global memory: asked for before the wait
         const uint8_t f = (MODEL != 1 && s < np) ? d.cflag[s >> 5] : (uint8_t)0;
         const bool ready = mbar_wait(&full[k], (it / FT_STAGES) & 1u, BULK_WAIT_NS);
-        if (ready && s < np) force_row<MODEL, BATCH>(args, s, TileRows{tiles[k], tid}, f);
+        if constexpr (BATCH) {
+            const uint32_t inst = s < np ? d.inst[s] : 0u;
+            by_scene(scene[tid >> 5], have, inst, ready && s < np,
+                     [&](ForceConsts &c, uint32_t i) { c = force_consts(d.prm[i]); },
+                     [&](const ForceConsts &c) {
+                         force_row<MODEL, true>(args, c, s, TileRows{tiles[k], tid}, f);
+                     });
+        } else if (ready && s < np) {
+            force_row<MODEL, false>(args, args.fc, s, TileRows{tiles[k], tid}, f);
+        }
         if (__syncthreads_or(!ready)) {
             if (tid == 0) {
                 atomicOr(d.status, ST_TIMEOUT);
@@ -1512,12 +1582,12 @@ k_force_tiles(ForceArgs args)
             stage_force_tile(d, A, tn, tiles[k], &full[k]);
         }
     }
+    end_of_step(d, args.next);
 }
 
 struct ContactArgs {
     Dev d;
     int a;               // read buffer (start of step)
-    int write_outputs;   // store force/torque/acc/angacc/edp of this step
     LawParams lp;        // single-scene contexts; a batch reads each scene's Params
 };
 
@@ -1527,8 +1597,201 @@ struct ContactArgs {
 #endif
 constexpr uint32_t CT_CAP = SPHK_CONTACT_CAP;
 
+// A warp's shared memory for one chunk's contacts.
+struct ContactWarp {
+    double terms[9][CT_CAP];       // law terms held: F xyz, T xyz, p, ev_dot, es_dot
+    double sums[9][32];            // each particle's running sums
+    LawParams law;                 // a batch's scene
+    uint32_t smask[NC];            // the particles holding each slot
+    uint32_t hitw[CT_CAP / 32], slipw[CT_CAP / 32];   // which held contacts overlapped, slipped
+    uint16_t expand[32 * NC];      // the chunk's list of (lane | slot << 5)
+    uint16_t sbase[NC];            // first list entry of each slot
+};
+
+// The slot loop of a chunk, 32 consecutive storage indices from s0, by one
+// warp: lane l's particle s0 + l held the slots occ0, still holds occ after
+// this step, and where occ0 is not zero its sums are cs.sums[.][l].  have: the
+// scene in cs.law.  Returns whether a particle of the chunk still holds a slot.
+//
+// The occupied slots form a list of directed contacts, written once into
+// shared memory as (lane, slot) pairs in slot-major order.  The list is
+// evaluated 32 contacts at a time, one per lane, so every lane runs a force
+// law whatever the spread of contact counts, and the terms of up to CT_CAP
+// contacts are kept in shared memory.  Then every particle's own lane adds its
+// terms in slot order, the reference's summation order, all lanes at once.  A
+// slot whose partner no longer overlaps is freed and its history zeroed, as in
+// the reference.  A chunk's rows are contiguous, its slot tiles too, and a
+// round's lanes mostly read one slot of consecutive particles, so their loads
+// coalesce.
+template <int MODEL, bool BATCH>
+__device__ __forceinline__ bool contact_chunk(const Dev &d, int A, const LawParams &lp, uint32_t s0,
+                                              ContactWarp &cs, uint32_t &have, uint32_t &occ0,
+                                              uint32_t &occ)
+{
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t np = d.np_all, lane = threadIdx.x & 31u, s = s0 + lane;
+    double (*tm)[CT_CAP] = cs.terms;
+    double (*sm)[32] = cs.sums;
+    uint16_t *ex = cs.expand;
+    occ0 = (s < np) ? d.cmask[s] : 0u;
+    const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
+    const uint32_t n = __popc(occ0);
+    const uint32_t total = __reduce_add_sync(FULL, n);   // the chunk's contacts
+    // The list in slot-major order: slot by slot, and within a slot
+    // by particle.  The lanes of a round then mostly share a slot and
+    // touch consecutive particles: consecutive entries of the slot
+    // tiles and consecutive particle rows.  A particle's contacts stay
+    // in ascending slot order along the list; slot i's first entry is
+    // sbase[i], and a particle finds its own entry of slot i from
+    // smask[i], the particles holding it.
+    {
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t k = 0;
+        for (uint32_t u = __reduce_or_sync(FULL, occ0); u; u &= u - 1u) {
+            const uint32_t i = (uint32_t)(__ffs(u) - 1);
+            const uint32_t m = __ballot_sync(FULL, (occ0 >> i) & 1u);
+            if ((occ0 >> i) & 1u) ex[k + __popc(m & lt)] = (uint16_t)(lane | (i << 5));
+            if (lane == 0) {
+                cs.sbase[i] = (uint16_t)k;
+                cs.smask[i] = m;
+            }
+            k += __popc(m);
+        }
+    }
+    __syncwarp();
+
+    // the particle's running sums live in shared memory between the
+    // passes, so no register holds them while the laws run
+    if (n) {
+#pragma unroll
+        for (int f = 0; f < 9; ++f) sm[f][lane] = 0.0;
+    }
+    occ = occ0;   // slots still held after this step
+    uint32_t rem = occ0;   // slots whose terms are still to be added
+    // the partner of this lane's contact, loaded a round ahead
+    uint32_t t_next = 0;
+    if (lane < total) {
+        const uint32_t x = ex[lane];
+        t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
+    }
+    for (uint32_t base = 0; base < total; base += 32u) {
+        const uint32_t c = base + lane;
+        const uint32_t t = t_next;
+        if (c + 32u < total) {
+            const uint32_t x = ex[c + 32u];
+            t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
+        }
+        const uint32_t pb = base - base % CT_CAP;   // first contact of this pass
+        bool hit = false, slip = false;
+        auto evaluate = [&](const auto &P) {
+            const uint32_t x = ex[c];
+            const uint32_t sq = s0 + (x & 31u), i = x >> 5;
+            const size_t e = tile_at(sq, i, NC);
+            const ulonglong2 dmw = d.dmc[sq];
+            const P3 dtp = d.delta_t[e];
+            const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
+            const double4 xa = d.xr[A][sq];
+            const double4 vel_a = ld4(d.vel[A], sq);
+            const d3 angvel_a = xyz(ld4(d.angvel[A], sq));
+            const double4 xb = d.xr[A][t];
+            const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
+            LawOut o;
+            const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)i), P);
+            const double ra = xa.w, rb = xb.w;
+            const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y,
+                              xa.z - xb.z + dm.z);
+            const double xlen = flen(xab);
+            const double delta_n = xlen - (ra + rb);
+            const bool touch = delta_n < 0.0f;
+            if (touch) {
+                o = (MODEL == 2)
+                    ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
+                                     xlen, delta_n, dt0)
+                    : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
+                                    xlen, delta_n, dt0);
+            }
+            if (touch) {
+                const uint32_t k = c - pb;
+                d.delta_t[e] = P3{o.dt4.x, o.dt4.y, o.dt4.z};
+                tm[0][k] = o.f.x;
+                tm[1][k] = o.f.y;
+                tm[2][k] = o.f.z;
+                tm[3][k] = o.t.x;
+                tm[4][k] = o.t.y;
+                tm[5][k] = o.t.z;
+                tm[6][k] = o.pr;
+                tm[7][k] = o.ev;
+                tm[8][k] = o.es;
+                hit = true;
+                slip = o.es_set;
+            } else {
+                // separated: free the slot and zero its history
+                d.contacts[e] = np;
+                d.delta_t[e] = P3{0.0, 0.0, 0.0};
+            }
+        };
+        if constexpr (BATCH) {
+            const uint32_t q = __shfl_sync(FULL, inst, c < total ? (ex[c] & 31u) : 0u);
+            by_scene(cs.law, have, q, c < total,
+                     [&](LawParams &l, uint32_t i) { l = law_params(d.prm[i]); }, evaluate);
+        } else if (c < total) {
+            evaluate(lp);
+        }
+        const uint32_t hb = __ballot_sync(FULL, hit);
+        const uint32_t sb = __ballot_sync(FULL, slip);
+        if (lane == 0) {
+            cs.hitw[(base - pb) >> 5] = hb;
+            cs.slipw[(base - pb) >> 5] = sb;
+        }
+        const uint32_t pe = min(total, pb + CT_CAP);
+        if (base + 32u < pe) continue;
+        __syncwarp();
+        // the pass is complete: every particle adds its terms of the
+        // pass, in slot order
+        const uint32_t lt = (1u << lane) - 1u;
+        auto entry = [&](uint32_t i) { return (uint32_t)cs.sbase[i] + __popc(cs.smask[i] & lt); };
+        if (rem && entry((uint32_t)(__ffs(rem) - 1)) < pe) {
+            d3 F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);
+            d3 T = mk(sm[3][lane], sm[4][lane], sm[5][lane]);
+            double p = sm[6][lane], ev_dot = sm[7][lane], es_dot = sm[8][lane];
+            while (rem) {
+                const uint32_t i = (uint32_t)(__ffs(rem) - 1);
+                const uint32_t j = entry(i);
+                if (j >= pe) break;   // in a later pass
+                const uint32_t k = j - pb;
+                rem &= rem - 1u;
+                if ((cs.hitw[k >> 5] >> (k & 31u)) & 1u) {
+                    F = add(F, mk(tm[0][k], tm[1][k], tm[2][k]));
+                    T = add(T, mk(tm[3][k], tm[4][k], tm[5][k]));
+                    p += tm[6][k];
+                    ev_dot += tm[7][k];
+                    if ((cs.slipw[k >> 5] >> (k & 31u)) & 1u) es_dot += tm[8][k];
+                } else {
+                    occ &= ~(1u << i);
+                }
+            }
+            sm[0][lane] = F.x;
+            sm[1][lane] = F.y;
+            sm[2][lane] = F.z;
+            sm[3][lane] = T.x;
+            sm[4][lane] = T.y;
+            sm[5][lane] = T.z;
+            sm[6][lane] = p;
+            sm[7][lane] = ev_dot;
+            sm[8][lane] = es_dot;
+        }
+        __syncwarp();
+    }
+    if (occ != occ0) {
+        d.cmask[s] = occ;
+        d.vl_held[s] = 0u;   // a listed candidate left its slot: the next
+        d.due[s] = -1.0f;    // search looks at the list
+    }
+    return __any_sync(FULL, occ != 0u);
+}
+
 // k_contact: interact's slot loop (src/contactsearch.cuh:468-543) for
-// contact models 2 and 3, one lane per directed contact.
+// contact models 2 and 3, one lane per directed contact (contact_chunk).
 //
 // The unit of work is a chunk of 32 consecutive storage indices, and a chunk
 // is visited only while its flag (Dev::cflag) says it may hold a contact:
@@ -1537,41 +1800,21 @@ constexpr uint32_t CT_CAP = SPHK_CONTACT_CAP;
 // is resident (a few blocks per SM); warp g takes chunks g, g + W, g + 2W,
 // ... of the W warps, reading the flags of 32 of them in one load, so a
 // contact-free scene costs about one memory latency.
-//
-// In a chunk, the occupied slots form a list of directed contacts, written
-// once into shared memory as (lane, slot) pairs in slot-major order.  The
-// list is evaluated 32 contacts at a time, one per lane, so every lane runs
-// a force law whatever the spread of contact counts, and the terms of up to
-// CT_CAP contacts are kept in shared memory.  Then every particle's own lane
-// adds its terms in slot order, the reference's summation order, all lanes
-// at once, and at the end stores the sums for k_force_tiles.  A slot whose partner
-// no longer overlaps is freed and its history zeroed, as in the reference.
-// A chunk's rows are contiguous, its slot tiles too, and a round's lanes
-// mostly read one slot of consecutive particles, so their loads coalesce.
 template <int MODEL, bool BATCH, int CB>
 __global__ void __launch_bounds__(CB, CONTACT_THREADS_PER_SM / CB)
 k_contact(ContactArgs args)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = CB / 32;
-    // per warp: the law terms of the contacts held (F xyz, T xyz, p, ev_dot,
-    // es_dot), the chunk's list of (lane | slot << 5), and which held
-    // contacts overlapped (hits) and slipped
-    __shared__ double terms[WARPS][9][CT_CAP];
-    __shared__ uint16_t expand[WARPS][32 * NC];
-    __shared__ uint32_t hitw[WARPS][CT_CAP / 32], slipw[WARPS][CT_CAP / 32];
-    __shared__ double sums[WARPS][9][32];   // each particle's running sums
-    __shared__ uint16_t sbase[WARPS][NC];    // first list entry of each slot
-    __shared__ uint32_t smask[WARPS][NC];    // the particles holding each slot
+    __shared__ ContactWarp warps[WARPS];
+    uint32_t have = 0xffffffffu;
     const Dev &d = args.d;
     const int A = args.a;
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t np = d.np_all;
     const uint32_t nchunk = (np + 31u) >> 5;
     const uint32_t gw = blockIdx.x * WARPS + w, nwarps = gridDim.x * WARPS;
-    double (*tm)[CT_CAP] = terms[w];
-    double (*sm)[32] = sums[w];
-    uint16_t *ex = expand[w];
+    double (*sm)[32] = warps[w].sums;
     // A chunk's rows are contiguous (its slot tiles too), so one lane asks
     // the copy engine to bring a chunk that is coming up into L2 while the
     // warp works: the chain of loads of each round then waits on L2, not on
@@ -1599,169 +1842,152 @@ k_contact(ContactArgs args)
             if (todo) prefetch_chunk(g + (uint32_t)(__ffs(todo) - 1) * nwarps);
             const uint32_t s0 = chunk << 5;
             const uint32_t s = s0 + lane;
-            const uint32_t occ0 = (s < np) ? d.cmask[s] : 0u;
-            const uint32_t n = __popc(occ0);
-            const uint32_t total = __reduce_add_sync(FULL, n);   // the chunk's contacts
-            // The list in slot-major order: slot by slot, and within a slot
-            // by particle.  The lanes of a round then mostly share a slot and
-            // touch consecutive particles: consecutive entries of the slot
-            // tiles and consecutive particle rows.  A particle's contacts stay
-            // in ascending slot order along the list; slot i's first entry is
-            // sbase[i], and a particle finds its own entry of slot i from
-            // smask[i], the particles holding it.
-            {
-                const uint32_t lt = (1u << lane) - 1u;
-                uint32_t k = 0;
-                for (uint32_t u = __reduce_or_sync(FULL, occ0); u; u &= u - 1u) {
-                    const uint32_t i = (uint32_t)(__ffs(u) - 1);
-                    const uint32_t m = __ballot_sync(FULL, (occ0 >> i) & 1u);
-                    if ((occ0 >> i) & 1u) ex[k + __popc(m & lt)] = (uint16_t)(lane | (i << 5));
-                    if (lane == 0) {
-                        sbase[w][i] = (uint16_t)k;
-                        smask[w][i] = m;
-                    }
-                    k += __popc(m);
-                }
-            }
-            __syncwarp();
-
-            // the particle's running sums live in shared memory between the
-            // passes, so no register holds them while the laws run
-            if (n) {
-#pragma unroll
-                for (int f = 0; f < 9; ++f) sm[f][lane] = 0.0;
-            }
-            uint32_t occ = occ0;   // slots still held after this step
-            uint32_t rem = occ0;   // slots whose terms are still to be added
-            // the partner of this lane's contact, loaded a round ahead
-            uint32_t t_next = 0;
-            if (lane < total) {
-                const uint32_t x = ex[lane];
-                t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
-            }
-            for (uint32_t base = 0; base < total; base += 32u) {
-                const uint32_t c = base + lane;
-                const uint32_t t = t_next;
-                if (c + 32u < total) {
-                    const uint32_t x = ex[c + 32u];
-                    t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
-                }
-                const uint32_t pb = base - base % CT_CAP;   // first contact of this pass
-                bool hit = false, slip = false;
-                if (c < total) {
-                    const uint32_t x = ex[c];
-                    const uint32_t sq = s0 + (x & 31u), i = x >> 5;
-                    const size_t e = tile_at(sq, i, NC);
-                    const ulonglong2 dmw = d.dmc[sq];
-                    const P3 dtp = d.delta_t[e];
-                    const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
-                    const double4 xa = d.xr[A][sq];
-                    const double4 vel_a = ld4(d.vel[A], sq);
-                    const d3 angvel_a = xyz(ld4(d.angvel[A], sq));
-                    const double4 xb = d.xr[A][t];
-                    const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
-                    LawOut o;
-                    bool touch;
-                    auto eval = [&](const auto &P) {
-                        const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)i), P);
-                        const double ra = xa.w, rb = xb.w;
-                        const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y,
-                                          xa.z - xb.z + dm.z);
-                        const double xlen = flen(xab);
-                        const double delta_n = xlen - (ra + rb);
-                        touch = delta_n < 0.0f;
-                        if (touch) {
-                            o = (MODEL == 2)
-                                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
-                                                 xlen, delta_n, dt0)
-                                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
-                                                xlen, delta_n, dt0);
-                        }
-                    };
-                    if constexpr (BATCH) eval(prm_at<true>(d, sq));
-                    else eval(args.lp);
-                    if (touch) {
-                        const uint32_t k = c - pb;
-                        d.delta_t[e] = P3{o.dt4.x, o.dt4.y, o.dt4.z};
-                        tm[0][k] = o.f.x;
-                        tm[1][k] = o.f.y;
-                        tm[2][k] = o.f.z;
-                        tm[3][k] = o.t.x;
-                        tm[4][k] = o.t.y;
-                        tm[5][k] = o.t.z;
-                        tm[6][k] = o.pr;
-                        tm[7][k] = o.ev;
-                        tm[8][k] = o.es;
-                        hit = true;
-                        slip = o.es_set;
-                    } else {
-                        // separated: free the slot and zero its history
-                        d.contacts[e] = np;
-                        d.delta_t[e] = P3{0.0, 0.0, 0.0};
-                    }
-                }
-                const uint32_t hb = __ballot_sync(FULL, hit);
-                const uint32_t sb = __ballot_sync(FULL, slip);
-                if (lane == 0) {
-                    hitw[w][(base - pb) >> 5] = hb;
-                    slipw[w][(base - pb) >> 5] = sb;
-                }
-                const uint32_t pe = min(total, pb + CT_CAP);
-                if (base + 32u < pe) continue;
-                __syncwarp();
-                // the pass is complete: every particle adds its terms of the
-                // pass, in slot order
-                const uint32_t lt = (1u << lane) - 1u;
-                auto entry = [&](uint32_t i) { return (uint32_t)sbase[w][i] + __popc(smask[w][i] & lt); };
-                if (rem && entry((uint32_t)(__ffs(rem) - 1)) < pe) {
-                    d3 F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);
-                    d3 T = mk(sm[3][lane], sm[4][lane], sm[5][lane]);
-                    double p = sm[6][lane], ev_dot = sm[7][lane], es_dot = sm[8][lane];
-                    while (rem) {
-                        const uint32_t i = (uint32_t)(__ffs(rem) - 1);
-                        const uint32_t j = entry(i);
-                        if (j >= pe) break;   // in a later pass
-                        const uint32_t k = j - pb;
-                        rem &= rem - 1u;
-                        if ((hitw[w][k >> 5] >> (k & 31u)) & 1u) {
-                            F = add(F, mk(tm[0][k], tm[1][k], tm[2][k]));
-                            T = add(T, mk(tm[3][k], tm[4][k], tm[5][k]));
-                            p += tm[6][k];
-                            ev_dot += tm[7][k];
-                            if ((slipw[w][k >> 5] >> (k & 31u)) & 1u) es_dot += tm[8][k];
-                        } else {
-                            occ &= ~(1u << i);
-                        }
-                    }
-                    sm[0][lane] = F.x;
-                    sm[1][lane] = F.y;
-                    sm[2][lane] = F.z;
-                    sm[3][lane] = T.x;
-                    sm[4][lane] = T.y;
-                    sm[5][lane] = T.z;
-                    sm[6][lane] = p;
-                    sm[7][lane] = ev_dot;
-                    sm[8][lane] = es_dot;
-                }
-                __syncwarp();
-            }
-            if (n) {
+            uint32_t occ0, occ;
+            const bool held = contact_chunk<MODEL, BATCH>(d, A, args.lp, s0, warps[w], have, occ0, occ);
+            if (occ0) {
                 d.csum_f[s] = make_double4(sm[0][lane], sm[1][lane], sm[2][lane], sm[6][lane]);
                 d.csum_t[s] = make_double4(sm[3][lane], sm[4][lane], sm[5][lane], sm[7][lane]);
                 d.csum_es[s] = sm[8][lane];
-                if (occ != occ0) {
-                    d.cmask[s] = occ;
-                    d.vl_held[s] = 0u;   // a listed candidate left its slot: the
-            d.due[s] = -1.0f;    // next search looks at the list
-                }
             }
             // visited (2: a slot is still held, 3: none is); k_force_tiles reads
             // the sums of a visited chunk and sets its flag back to 1 or 0
             // for the next step's search
-            const bool held = __any_sync(FULL, occ != 0u);
             if (lane == 0) d.cflag[chunk] = held ? 2 : 3;
         }
     }
+}
+
+// A particle's rows, loaded together.
+struct RegRows {
+    double4 x;
+    P3 v, w, ap, w0, v0;
+    double2 xy;
+    uint32_t c;
+    uint8_t fx, wt;
+    __device__ RegRows(const Dev &d, int A, uint32_t s)
+        : x(d.xr[A][s]), v(d.vel[A][s]), w(d.angvel[A][s]), ap(d.angpos[s]), w0(d.angvel0[s]),
+          v0(d.vel0[s]), xy(d.xysum[s]), c(d.cell[s]), fx(d.fixed[s]), wt(d.wtouch[s])
+    {
+    }
+    __device__ P3 angpos() const { return ap; }
+    __device__ P3 angvel0() const { return w0; }
+    __device__ P3 vel0() const { return v0; }
+    __device__ double2 xysum() const { return xy; }
+    __device__ uint32_t cell() const { return c; }
+    __device__ uint8_t fixed() const { return fx; }
+    __device__ uint8_t wtouch() const { return wt; }
+};
+
+// k_small: the step of a scene small enough that every chunk of 32 particles
+// has a warp of its own on the device at once.  A particle's search, contact
+// forces and integration need its neighbours' start-of-step rows (buffer A)
+// and its own results only, so the warp of a chunk runs all three, and the
+// step is one launch: the slot sums stay in shared memory, the last block
+// ends the step.
+//
+// What bounds it: latency, one chain of the search, the laws' rounds and the
+// integration.  As three kernels each of their launches, ramps and drains
+// stood in that chain: whole runs of 500 grains 7.05 -> 6.45 ms (200 steps), of
+// 10,000 10.8 -> 8.4 ms (500 steps).
+constexpr int SMALL_BLOCK = 64, SMALL_BLOCKS_PER_SM = 8;
+template <int MODEL, bool BATCH>
+__global__ void __launch_bounds__(SMALL_BLOCK, SMALL_BLOCKS_PER_SM)
+k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParams lp)
+{
+    constexpr uint32_t FULL = 0xffffffffu;
+    constexpr int WARPS = SMALL_BLOCK / 32;
+    constexpr bool VISC = MODEL == 1;
+    union Warp {
+        uint32_t srow[NC * 32];   // the search's slot rows
+        ContactWarp cs;
+    };
+    __shared__ __align__(16) unsigned char mem[WARPS][sizeof(Warp)];
+    __shared__ ForceConsts scene[BATCH ? WARPS : 1];
+    const Dev &d = args.d;
+    const int A = args.a;
+    const uint32_t np = d.np_all, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
+    Warp &sh = *reinterpret_cast<Warp *>(mem[w]);
+    if (s0 < np) {
+        // ---- the search (k_topo) ----
+        {
+            const Verlet &V = *d.vs;
+            bool need = false, sweep = false;
+            if (s < np) {
+                sweep = V.all_rebuild != 0u || (V.dirty_step == V.step && d.dirty[d.cell[s]] == V.step);
+                need = sweep || V.moved > d.due[s];
+                if (VISC && !need) d.c1acc[s] = make_double4(0.0, 0.0, 0.0, 0.0);
+            }
+            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, sh.srow, sweep);
+            __syncwarp();
+        }
+        // ---- the slot forces (k_contact) ----
+        uint32_t have = 0xffffffffu, occ0 = 0u, occ = 0u;
+        if (!VISC && d.cflag[chunk] != 0) {
+            const bool held = contact_chunk<MODEL, BATCH>(d, A, lp, s0, sh.cs, have, occ0, occ);
+            if (lane == 0) d.cflag[chunk] = held ? 1 : 0;
+        }
+        // ---- the rest of the step (k_force_tiles) ----
+        const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
+        auto integrate = [&](const ForceConsts &fc) {
+            const RegRows R(d, A, s);
+            d3 F = mk(0.0, 0.0, 0.0), T = mk(0.0, 0.0, 0.0);
+            double es_dot = 0.0f, ev_dot = 0.0f, p = 0.0f;
+            if (VISC) {
+                const double4 c = d.c1acc[s];
+                F = mk(c.x, c.y, c.z);
+                p = c.w;
+            } else if (occ != 0u) {
+                const double (*sm)[32] = sh.cs.sums;
+                F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);
+                T = mk(sm[3][lane], sm[4][lane], sm[5][lane]);
+                p = sm[6][lane];
+                ev_dot = sm[7][lane];
+                es_dot = sm[8][lane];
+            }
+            particle_tail<BATCH, false>(d, fc, s, A, args.write_outputs, R.x,
+                                        make_double4(R.v.x, R.v.y, R.v.z, 0.0),
+                                        make_double4(R.w.x, R.w.y, R.w.z, 0.0), F, T, p, ev_dot,
+                                        es_dot, R);
+        };
+        if constexpr (BATCH) {
+            have = 0xffffffffu;
+            by_scene(scene[w], have, inst, s < np,
+                     [&](ForceConsts &c, uint32_t i) { c = force_consts(d.prm[i]); }, integrate);
+        } else if (s < np) {
+            integrate(args.fc);
+        }
+    }
+    end_of_step(d, args.next);
+}
+
+// Whether a context's steps run as k_small: its chunks have a resident warp
+// each (75,776 particles on 148 SMs), and no shape or span of the split
+// kernels was asked for.  Above, the split kernels balance the work over the
+// device and stream the integration; below, they were slower (50,000 grains in
+// a flow, 200 steps: 11.1 ms against 10.1).
+bool small_step(const Dev &d, uint32_t np)
+{
+    if (d.shape != 0 || d.topo_span != 0) return false;
+    static int nsm = 0;
+    if (nsm == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return np <= (uint32_t)nsm * SMALL_BLOCKS_PER_SM * SMALL_BLOCK;
+}
+
+void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                  const NextStep &next, cudaStream_t st)
+{
+    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp), next};
+    const LawParams lp = law_params(hp);
+    const unsigned grid = div_up(np, SMALL_BLOCK);
+    if (d.inst) k_small<2, true><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
+    else if (model == 1) k_small<1, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
+    else if (model == 3) k_small<3, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
+    else k_small<2, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
 }
 
 // A resident grid of k_contact: the SMs times the blocks of this
@@ -1848,9 +2074,9 @@ static void launch_force_tiles(const ForceArgs &args, uint32_t np, cudaStream_t 
 }
 
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  cudaStream_t st)
+                  const NextStep &next, cudaStream_t st)
 {
-    ForceArgs args{d, a, write_outputs, -1, force_consts(hp)};
+    ForceArgs args{d, a, write_outputs, -1, force_consts(hp), next};
     if (d.inst) {   // batched contexts: contact model 2 only
         launch_force_tiles<2, true>(args, np, st);
     } else if (d.mu_p) {   // the differentiable step
@@ -1865,22 +2091,20 @@ void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a,
 }
 
 // The differentiable step, recording tape row `tape_step`.
-void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStream_t st)
+void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, const NextStep &next,
+                       cudaStream_t st)
 {
-    ForceArgs args{d, a, 0, tape_step, ForceConsts{}};
+    ForceArgs args{d, a, 0, tape_step, ForceConsts{}, next};
     k_force_diff<<<div_up(np, FORCE_BLOCK), FORCE_BLOCK, 0, st>>>(args);
 }
 
 // The slot forces of contact models 2 and 3; model 1 has no slots (k_topo
 // sums its forces) and the differentiable step evaluates its own law in
 // k_force_diff, recording the tape.
-void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a,
-                    int write_outputs, cudaStream_t st)
+void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st)
 {
     if (model == 1 || d.mu_p) return;
-    ContactArgs args{d, a, write_outputs,
-                     LawParams{hp.k_n, hp.k_t, hp.gamma_n, hp.gamma_t, hp.gamma_r, hp.mu_s, hp.mu_d,
-                               hp.mu_r, hp.kappa, hp.dt, {hp.L[0], hp.L[1]}}};
+    ContactArgs args{d, a, law_params(hp)};
     if (d.shape) launch_contact_as<contact_block(1)>(args, np, model, st);
     else launch_contact_as<contact_block(0)>(args, np, model, st);
 }

@@ -1,12 +1,9 @@
 // walls.cu -- wall-force reduction and wall integration (summation and
 // integrateWalls, src/integration.cuh:191-295), in one launch.
 //
-// The launch also ends the step's Verlet bookkeeping (step_tail) when it
-// runs on the step's own stream.  In the step graphs it runs on a branch
-// instead, forked after the force kernel and joined before the next step's
-// force kernel (the only reader of the wall rows), so that its serial tail
-// overlaps the next step's contact search; the bookkeeping, which that
-// search reads, is then a one-thread launch on the step's stream (k_tail).
+// In the step graphs it runs on a branch, forked after the force kernel and
+// joined before the next step's force kernel (the only reader of the wall
+// rows), so that its serial tail overlaps the next step's contact search.
 //
 // The wall-0 force of every particle is summed in the reference's exact
 // order: 256-particle blocks in particle-index order reduced by a halving
@@ -28,31 +25,10 @@ namespace sphk {
 
 constexpr int WALL_BLOCK = 256;
 
-// The epoch's clock and the decision for the next step: the lists hold every
-// pair that can overlap while 2 moved < skin; otherwise (a clock that is not a
-// number included) every particle sweeps and a new epoch starts.
-__device__ void step_tail(const Dev &d)
-{
-    const Params &P = *d.prm;
-    Verlet &V = *d.vs;
-    float moved = V.moved;
-    const float inc = __fmul_ru(__fsqrt_ru(__uint_as_float(V.inc2_bits)), 1.00001f);
-    if (inc != 0.0f) moved = __fadd_ru(moved, __fadd_ru(inc, 1e-15f));
-    V.inc2_bits = 0u;
-    const bool restart = P.skin > 0.0 && !(2.02 * (double)moved < 0.999 * P.skin);
-    V.all_rebuild = restart ? 1u : 0u;
-    V.moved = restart ? 0.0f : moved;
-    // a sweep needs the cell list of its own step
-    if (restart || V.want_cells) *d.rebuild = 1u;
-    V.want_cells = 0u;
-    V.step += 1u;
-}
-
 constexpr int REF_BLOCK = 256;               // the reference's summation block
 constexpr int WARPS = WALL_BLOCK / 32;        // reference blocks per CUDA block
 constexpr int FOLD = 16;                      // partials per thread in the fold
 
-template <bool TAIL>
 __global__ void __launch_bounds__(WALL_BLOCK)
 k_walls(Dev d)
 {
@@ -165,37 +141,14 @@ k_walls(Dev d)
     if (t == 0) {
         W.t_current += P.dt;
         W.done_blocks = 0;
-        if (TAIL) step_tail(d);
     }
-}
-
-// End of a step without walls: only the Verlet epoch bookkeeping.
-__global__ void k_tail(Dev d)
-{
-    if (threadIdx.x == 0) step_tail(d);
 }
 
 void launch_walls(const Dev &d, uint32_t np, uint32_t nw, cudaStream_t st)
 {
-    if (nw == 0) {
-        k_tail<<<1, 32, 0, st>>>(d);
-        return;
-    }
+    if (nw == 0) return;
     const unsigned int nref = div_up(np, REF_BLOCK);
-    k_walls<true><<<div_up(nref, WARPS), WALL_BLOCK, 0, st>>>(d);
-}
-
-// The wall reduction and integration alone (nw > 0), for a graph branch.
-void launch_wall_motion(const Dev &d, uint32_t np, cudaStream_t st)
-{
-    const unsigned int nref = div_up(np, REF_BLOCK);
-    k_walls<false><<<div_up(nref, WARPS), WALL_BLOCK, 0, st>>>(d);
-}
-
-// The Verlet bookkeeping alone.
-void launch_tail(const Dev &d, cudaStream_t st)
-{
-    k_tail<<<1, 32, 0, st>>>(d);
+    k_walls<<<div_up(nref, WARPS), WALL_BLOCK, 0, st>>>(d);
 }
 
 }  // namespace sphk
