@@ -29,6 +29,7 @@
 // visiting order is the reference's: stencil cells z, y, x, members of a cell
 // by particle index.
 #include <algorithm>
+#include <type_traits>
 
 #include "sphk_internal.cuh"
 #include "diff_step.cuh"
@@ -253,11 +254,10 @@ __device__ __forceinline__ double f32_powf(double x, float y)
 
 // contactLinearViscous, src/contactmodels.cuh:114-253 (contact model 1): no
 // tangential history, and the torque is left alone (its update is commented
-// out in the reference, :244).
-__device__ __noinline__ void contact_viscous(const Params &P, d3 &F, double &p, double4 vel_a,
-                                                double4 vel_b, d3 angvel_a, d3 angvel_b,
-                                                double ra, double rb, d3 x_ab,
-                                                double x_ab_length, double delta)
+// out in the reference, :244).  Returns the force on a; pr: the pressure.
+__device__ __forceinline__ d3 contact_viscous(const Params &P, double &pr, d3 vel_a, d3 vel_b,
+                                              d3 angvel_a, d3 angvel_b, double ra, double rb,
+                                              d3 x_ab, double x_ab_length, double delta)
 {
     const d3 n = divs(x_ab, x_ab_length);
     const d3 vel_linear = mk(vel_a.x - vel_b.x, vel_a.y - vel_b.y, vel_a.z - vel_b.z);
@@ -279,13 +279,13 @@ __device__ __noinline__ void contact_viscous(const Params &P, d3 &F, double &p, 
         if (f_t_visc < f_t_limit) f_t = divs(smul(-f_t_visc, vel_t), vel_t_length);
         else f_t = divs(smul(-f_t_limit, vel_t), vel_t_length);
     }
-    F = add(F, add(add(f_n, f_t), f_c));
-    p += f_n_length / (4.0f * REF_PI * ra * ra);
+    pr = f_n_length / (4.0f * REF_PI * ra * ra);
+    return add(add(f_n, f_t), f_c);
 }
 
 // capillaryCohesion_exp, src/cohesion.cuh:314-350
-__device__ __noinline__ void capillary_exp(const Params &P, d3 &F, double ra, double rb,
-                                              double delta, d3 x_ab, double x_ab_length)
+__device__ __forceinline__ d3 capillary_exp(const Params &P, double ra, double rb, double delta,
+                                            d3 x_ab, double x_ab_length)
 {
     const d3 n = divs(x_ab, x_ab_length);
     double r;
@@ -295,8 +295,7 @@ __device__ __noinline__ void capillary_exp(const Params &P, d3 &F, double ra, do
     const double R_har = (2.0f * ra * rb) / (ra + rb);
     const double R_geo = fsqrt_of(ra * rb);
     const double lambda = 0.9f * h * fsqrt_of(P.V_b / R_har);
-    const d3 f_c = smul(-P.kappa * R_geo * f32_expf(-delta / lambda), n);
-    F = add(F, f_c);
+    return smul(-P.kappa * R_geo * f32_expf(-delta / lambda), n);
 }
 
 // contactHertz, src/contactmodels.cuh:499-666 (contact model 3).  As in the
@@ -495,22 +494,121 @@ __device__ __forceinline__ double pair_gap(const Params &P, double4 xb, uint32_t
 
 // Contact model 1 processes each candidate as soon as it is found
 // (findAndProcessContactsInCell, src/contactsearch.cuh:81-175): overlap ->
-// contactLinearViscous, else a gap below db -> capillaryCohesion_exp.  Out of
-// line, with every operand loaded here, so the candidate loop stays lean.
-__device__ __noinline__ void visc_pair(const Dev &d, int A, uint32_t s, uint32_t t,
-                                       uint32_t code, d3 &F, double &p)
+// contactLinearViscous, else a gap below db -> capillaryCohesion_exp.  One
+// pair's force on s in f (where the return is not 0), and its pressure in pr
+// (where the return is 2).
+__device__ __forceinline__ int visc_pair(const Dev &d, const Params &P, int A, uint32_t s, uint32_t t,
+                                         uint32_t code, d3 &f, double &pr)
 {
-    const Params &P = prm_of(d, s);
     const double4 xa = d.xr[A][s], xb = d.xr[A][t];
+    const d3 va = xyz(ld4(d.vel[A], s)), vb = xyz(ld4(d.vel[A], t));
+    const d3 wa = xyz(ld4(d.angvel[A], s)), wb = xyz(ld4(d.angvel[A], t));
     const d3 dm = decode_dm(code, P);
     const d3 xab = add(mk(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z), dm);
     const double len = flen(xab);
     const double delta = len - (xa.w + xb.w);
     if (delta < 0.0f) {
-        contact_viscous(P, F, p, ld4(d.vel[A], s), ld4(d.vel[A], t), xyz(ld4(d.angvel[A], s)),
-                        xyz(ld4(d.angvel[A], t)), xa.w, xb.w, xab, len, delta);
-    } else if (delta < P.db) {
-        capillary_exp(P, F, xa.w, xb.w, delta, xab, len);
+        f = contact_viscous(P, pr, va, vb, wa, wb, xa.w, xb.w, xab, len, delta);
+        return 2;
+    }
+    if (delta < P.db) {
+        f = capillary_exp(P, xa.w, xb.w, delta, xab, len);
+        return 1;
+    }
+    return 0;
+}
+
+// The pairs of model 1 that a particle's search found, in visiting order, are
+// kept as (storage index | shift code << 27) in its column of shared memory
+// (act) and worked on by the whole warp (visc_warp).  A particle with more
+// than VISC_CAP of them works them off itself, out of line.
+constexpr uint32_t VISC_CAP = 32;
+struct ViscAct {
+    uint32_t n;      // pairs in the column
+    d3 F;            // what has been summed up already
+    double p;
+};
+__device__ __noinline__ void visc_spill(const Dev &d, const Params &P, int A, uint32_t s,
+                                        const uint32_t *col, uint32_t stride, ViscAct &v)
+{
+    for (uint32_t k = 0; k < v.n; ++k) {
+        const uint32_t e = col[k * stride];
+        d3 f;
+        double pr;
+        const int does = visc_pair(d, P, A, s, e & 0x7ffffffu, e >> 27, f, pr);
+        if (does) v.F = add(v.F, f);
+        if (does == 2) v.p += pr;
+    }
+    v.n = 0u;
+}
+
+// A warp's shared memory for the pairs of its lanes' particles.
+struct ViscWarp {
+    double terms[4][64];          // force terms held, pressure
+    uint32_t smask[VISC_CAP];     // the lanes with a k-th pair
+    uint32_t hitw[2], touchw[2];  // which held pairs act, overlap
+    uint16_t expand[32 * VISC_CAP];
+    uint16_t sbase[VISC_CAP];
+};
+
+// The pairs of the warp's particles (lane's particle s, its column act),
+// evaluated 32 at a time, one a lane, and added up by each particle's own lane
+// in visiting order, as contact_chunk does for the slots.  All lanes.
+__device__ __forceinline__ void visc_warp(const Dev &d, int A, uint32_t s, const uint32_t *act,
+                                          uint32_t stride, ViscWarp &vs, ViscAct &v)
+{
+    constexpr uint32_t FULL = 0xffffffffu;
+    const Params &P = *d.prm;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t total = __reduce_add_sync(FULL, v.n);
+    uint32_t most = __reduce_max_sync(FULL, v.n);
+    for (uint32_t k = 0, at = 0; k < most; ++k) {
+        const uint32_t m = __ballot_sync(FULL, v.n > k);
+        if (v.n > k) vs.expand[at + __popc(m & lt)] = (uint16_t)(lane | (k << 5));
+        if (lane == 0) {
+            vs.sbase[k] = (uint16_t)at;
+            vs.smask[k] = m;
+        }
+        at += __popc(m);
+    }
+    __syncwarp();
+    uint32_t done = 0;   // of this lane's pairs
+    for (uint32_t base = 0; base < total; base += 32u) {
+        const uint32_t c = base + lane, pb = base - base % 64u;
+        const uint32_t x = c < total ? vs.expand[c] : 0u;
+        const uint32_t sq = __shfl_sync(FULL, s, x & 31u);
+        int does = 0;
+        if (c < total) {
+            const uint32_t e = act[(x >> 5) * stride + (x & 31u)];
+            d3 f;
+            double pr = 0.0;
+            does = visc_pair(d, P, A, sq, e & 0x7ffffffu, e >> 27, f, pr);
+            if (does) {
+                const uint32_t k = c - pb;
+                vs.terms[0][k] = f.x;
+                vs.terms[1][k] = f.y;
+                vs.terms[2][k] = f.z;
+                vs.terms[3][k] = pr;
+            }
+        }
+        const uint32_t hb = __ballot_sync(FULL, does != 0), tb = __ballot_sync(FULL, does == 2);
+        if (lane == 0) {
+            vs.hitw[(base - pb) >> 5] = hb;
+            vs.touchw[(base - pb) >> 5] = tb;
+        }
+        const uint32_t pe = min(total, pb + 64u);
+        if (base + 32u < pe) continue;
+        __syncwarp();
+        while (done < v.n) {
+            const uint32_t j = vs.sbase[done] + __popc(vs.smask[done] & lt);
+            if (j >= pe) break;
+            const uint32_t k = j - pb;
+            ++done;
+            if ((vs.hitw[k >> 5] >> (k & 31u)) & 1u)
+                v.F = add(v.F, mk(vs.terms[0][k], vs.terms[1][k], vs.terms[2][k]));
+            if ((vs.touchw[k >> 5] >> (k & 31u)) & 1u) v.p += vs.terms[3][k];
+        }
+        __syncwarp();
     }
 }
 
@@ -585,12 +683,11 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
 // with the near candidates two cells away where cells are that small
 // (Params::wide).
 //
-// VISC (contact model 1): no slots; every candidate within ra + rb + db is
-// processed in visiting order and the contact force and pressure sums are
-// left in Dev::c1acc for k_force_tiles.
+// VISC (contact model 1): no slots; every candidate within ra + rb + db acts,
+// in visiting order: they are left in `va` and the lane's column of srow.
 template <bool VISC, bool BATCH, int TB>
 __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int tid, uint32_t *srow,
-                                            bool sweep)
+                                            bool sweep, ViscAct &va)
 {
     const Params &P = prm_at<BATCH>(d, s);
     const uint32_t len = d.vl_len[s];
@@ -619,8 +716,11 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const bool gp_in = gp[0] >= 0 && (uint32_t)gp[0] < nx && gp[1] >= 0 && (uint32_t)gp[1] < ny &&
                        gp[2] >= 0 && (uint32_t)gp[2] < nz;
     const bool use_lists = P.skin > 0.0 && gp_in;
-    d3 F1 = mk(0.0, 0.0, 0.0);   // model 1 sums
-    double p1 = 0.0f;
+    // one more acting pair of model 1
+    auto act_on = [&](uint32_t t, uint32_t code) {
+        if (va.n == VISC_CAP) visc_spill(d, P, A, s, srow + tid, TB, va);
+        srow[va.n++ * TB + tid] = t | (code << 27);
+    };
     float due = 3.0e38f;         // the particle's next moment
 
     if (use_lists && !sweep && len != VL_NONE) {
@@ -671,7 +771,29 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         if (act) {
             uint32_t left = act;
             int slot = 0, skip_slot = -1;
-            if (!VISC && simple && (act & (act - 1u)) == 0u) {
+            if constexpr (VISC) {
+                // by stencil cell, then particle index: the keys sorted in the
+                // column (slot << 27 | uid, both fit), then the pairs they name
+                for (; left; left &= left - 1u) {
+                    const size_t at = vl_at(s, (uint32_t)(__ffs(left) - 1));
+                    const uint32_t t = d.vl[at];
+                    const int k = stencil_slot(P, gp, xr[t], vl_code(d.vl_meta[at]));
+                    if (k < 0) continue;   // not in the stencil: not visited
+                    const uint32_t key = ((uint32_t)k << 27) | d.uid[t];
+                    uint32_t q = va.n++;
+                    for (; q > 0u && srow[(q - 1u) * TB + tid] > key; --q)
+                        srow[q * TB + tid] = srow[(q - 1u) * TB + tid];
+                    srow[q * TB + tid] = key;
+                }
+                for (uint32_t q = 0; q < va.n; ++q) {
+                    const uint32_t key = srow[q * TB + tid], k = key >> 27;
+                    const int32_t cx = gp[0] + (int32_t)(k % 3u) - 1, cy = gp[1] + (int32_t)(k / 3u % 3u) - 1;
+                    const uint32_t code = (cx < 0 ? 1u : (cx == (int32_t)nx ? 2u : 0u)) |
+                                          (cy < 0 ? 4u : (cy == (int32_t)ny ? 8u : 0u));
+                    srow[q * TB + tid] = d.sidx[key & 0x7ffffffu] | (code << 27);
+                }
+                due = -1.0f;
+            } else if (simple && (act & (act - 1u)) == 0u) {
                 // one new overlap: its slot does not depend on any order
                 const size_t at = vl_at(s, (uint32_t)(__ffs(act) - 1));
                 const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
@@ -685,15 +807,11 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 for (int e; (e = first_visited(d, P, A, gp, s, left, slot)) >= 0;) {
                     const size_t at = vl_at(s, (uint32_t)e);
                     const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
-                    if constexpr (VISC) {
-                        visc_pair(d, A, s, t, code, F1, p1);
-                    } else {
-                        if (slot == skip_slot) continue;   // nc > NC: rest of that cell
-                        if (!topo_insert<TB>(d, srow, tid, s, t, code, ts)) skip_slot = slot;
-                        held |= 1u << e;
-                    }
+                    if (slot == skip_slot) continue;   // nc > NC: rest of that cell
+                    if (!topo_insert<TB>(d, srow, tid, s, t, code, ts)) skip_slot = slot;
+                    held |= 1u << e;
                 }
-                if (VISC || (held & act) != act) due = -1.0f;
+                if ((held & act) != act) due = -1.0f;
             }
         }
         if (!simple) {
@@ -755,7 +873,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                     float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
                     if (VISC) {
                         if ((hit >> j) & 1u) {
-                            visc_pair(d, A, s, t, code, F1, p1);
+                            act_on(t, code);
                             w = -1.0f;
                         }
                     } else if ((hit >> j) & 1u) {
@@ -878,7 +996,6 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
 
     d.due[s] = due;
     if (!VISC) d.vl_held[s] = held;
-    if (VISC) d.c1acc[s] = make_double4(F1.x, F1.y, F1.z, p1);
     if (ts.dirty) {
         // the search only fills empty slots (and may change a code): the
         // partners of the newly occupied slots are the entries to write;
@@ -922,6 +1039,7 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ uint32_t srow[NC * TB];
+    __shared__ ViscWarp visc[VISC ? TB / 32 : 1];
     const uint32_t np = d.np_all;
     const int tid = threadIdx.x;
     const uint32_t lane = (uint32_t)tid & 31u;
@@ -956,26 +1074,36 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
         ms[j] = __ballot_sync(FULL, (swp >> j) & 1u);
         total += (uint32_t)__popc(m[j]);
     }
-    for (uint32_t k = lane; k < total; k += 32u) {
-        uint32_t rem = k, sel = 0, selj = 0, sel_s = 0;
-        bool got = false;
+    for (uint32_t k0 = 0; k0 < total; k0 += 32u) {
+        const uint32_t k = k0 + lane;
+        uint32_t s = 0;
+        ViscAct va{0u, mk(0.0, 0.0, 0.0), 0.0};
+        if (k < total) {
+            uint32_t rem = k, sel = 0, selj = 0, sel_s = 0;
+            bool got = false;
 #pragma unroll
-        for (uint32_t j = 0; j < TOPO_SPAN_MAX; ++j) {
-            const uint32_t c = (uint32_t)__popc(m[j]);
-            if (!got) {
-                if (rem < c) {
-                    sel = m[j];
-                    sel_s = ms[j];
-                    selj = j;
-                    got = true;
-                } else {
-                    rem -= c;
+            for (uint32_t j = 0; j < TOPO_SPAN_MAX; ++j) {
+                const uint32_t c = (uint32_t)__popc(m[j]);
+                if (!got) {
+                    if (rem < c) {
+                        sel = m[j];
+                        sel_s = ms[j];
+                        selj = j;
+                        got = true;
+                    } else {
+                        rem -= c;
+                    }
                 }
             }
+            const uint32_t bit = __fns(sel, 0, (int)rem + 1);
+            s = base + 32u * selj + bit;
+            topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u, va);
         }
-        const uint32_t bit = __fns(sel, 0, (int)rem + 1);
-        const uint32_t s = base + 32u * selj + bit;
-        topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u);
+        if constexpr (VISC) {
+            __syncwarp();
+            visc_warp(d, A, s, srow + (tid & ~31), TB, visc[tid >> 5], va);
+            if (k < total) d.c1acc[s] = make_double4(va.F.x, va.F.y, va.F.z, va.p);
+        }
     }
 }
 
@@ -1897,10 +2025,17 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = SMALL_BLOCK / 32;
     constexpr bool VISC = MODEL == 1;
-    union Warp {
-        uint32_t srow[NC * 32];   // the search's slot rows
+    // model 1: the acting pairs and their evaluation; otherwise the search's
+    // slot rows, then the contacts
+    struct Visc {
+        uint32_t srow[NC * 32];
+        ViscWarp vs;
+    };
+    union Slots {
+        uint32_t srow[NC * 32];
         ContactWarp cs;
     };
+    using Warp = std::conditional_t<VISC, Visc, Slots>;
     __shared__ __align__(16) unsigned char mem[WARPS][sizeof(Warp)];
     __shared__ ForceConsts scene[BATCH ? WARPS : 1];
     const Dev &d = args.d;
@@ -1909,6 +2044,7 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
     const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
     Warp &sh = *reinterpret_cast<Warp *>(mem[w]);
     if (s0 < np) {
+        ViscAct va{0u, mk(0.0, 0.0, 0.0), 0.0};   // model 1's sums
         // ---- the search (k_topo) ----
         {
             const Verlet &V = *d.vs;
@@ -1916,16 +2052,18 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
             if (s < np) {
                 sweep = V.all_rebuild != 0u || (V.dirty_step == V.step && d.dirty[d.cell[s]] == V.step);
                 need = sweep || V.moved > d.due[s];
-                if (VISC && !need) d.c1acc[s] = make_double4(0.0, 0.0, 0.0, 0.0);
             }
-            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, sh.srow, sweep);
+            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, sh.srow, sweep, va);
             __syncwarp();
+            if constexpr (VISC) visc_warp(d, A, s, sh.srow, 32u, sh.vs, va);
         }
         // ---- the slot forces (k_contact) ----
         uint32_t have = 0xffffffffu, occ0 = 0u, occ = 0u;
-        if (!VISC && d.cflag[chunk] != 0) {
-            const bool held = contact_chunk<MODEL, BATCH>(d, A, lp, s0, sh.cs, have, occ0, occ);
-            if (lane == 0) d.cflag[chunk] = held ? 1 : 0;
+        if constexpr (!VISC) {
+            if (d.cflag[chunk] != 0) {
+                const bool held = contact_chunk<MODEL, BATCH>(d, A, lp, s0, sh.cs, have, occ0, occ);
+                if (lane == 0) d.cflag[chunk] = held ? 1 : 0;
+            }
         }
         // ---- the rest of the step (k_force_tiles) ----
         const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
@@ -1933,10 +2071,9 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
             const RegRows R(d, A, s);
             d3 F = mk(0.0, 0.0, 0.0), T = mk(0.0, 0.0, 0.0);
             double es_dot = 0.0f, ev_dot = 0.0f, p = 0.0f;
-            if (VISC) {
-                const double4 c = d.c1acc[s];
-                F = mk(c.x, c.y, c.z);
-                p = c.w;
+            if constexpr (VISC) {
+                F = va.F;
+                p = va.p;
             } else if (occ != 0u) {
                 const double (*sm)[32] = sh.cs.sums;
                 F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);

@@ -3,7 +3,9 @@ their lists stay in use, several new contacts of one grain in one step (whose
 slots follow the reference's visiting order), cells of every size against the
 reach of a list, grids of two and three periodic cells, lists that overflow
 and grains outside their cells' boxes.  Everything bit for bit against the
-oracle, the cell list of the last step included."""
+oracle, the cell list of the last step included.  Each with the step in one
+kernel, as scenes of this size run, and in the split kernels of larger ones
+(which asking for a search span selects)."""
 import numpy as np
 import pytest
 
@@ -44,14 +46,18 @@ SCENES = {
 }
 
 
+both_kernels = pytest.mark.parametrize("span", [None, 1], ids=["one_kernel", "split"])
+
+
+@both_kernels
 @pytest.mark.parametrize("name", sorted(SCENES))
 @pytest.mark.parametrize("skin", [0.1, 0.5])
-def test_lists_outlive_changes_of_cell(oracle_libs, name, skin):
+def test_lists_outlive_changes_of_cell(oracle_libs, name, skin, span):
     sb = SCENES[name]()
     rc, want, orun = run_oracle(oracle_libs["orc"], sb, 90)
     assert rc == 0
     cfg = config_from_spherebin(sb)
-    with Simulation(cfg, verlet_skin=skin) as sim:
+    with Simulation(cfg, verlet_skin=skin, topo_span=span) as sim:
         sim.upload(state_from_spherebin(sb))
         for k in (33, 1, 56):
             sim.step(k)
@@ -65,14 +71,17 @@ def test_lists_outlive_changes_of_cell(oracle_libs, name, skin):
     assert np.array_equal(cend[occ], orun.cell_end[occ])
 
 
+@both_kernels
+@pytest.mark.parametrize("db, V_b, kappa", [(1e-4, 1e-12, 0.05), (1.2e-3, 1e-9, 1e-3)], ids=["near", "far"])
 @pytest.mark.parametrize("name", ["cells_2r", "cells_2r_periodic", "cells_1.5r", "two_cells"])
-def test_model1_lists_outlive_changes_of_cell(oracle_libs, name):
+def test_model1_lists_outlive_changes_of_cell(oracle_libs, name, db, V_b, kappa, span):
     """Contact model 1 sums its pairs in visiting order: the order of a list
-    follows the grains' present cells."""
-    sb = with_model(SCENES[name](), 1)
+    follows the grains' present cells.  With the wide reach some grains have
+    more acting pairs than a list, or the warp's shared memory, holds."""
+    sb = with_model(SCENES[name](), 1, kappa=kappa, V_b=V_b, db=db)
     rc, want, _ = run_oracle(oracle_libs["orc"], sb, 60)
     assert rc == 0
-    with Simulation(config_from_spherebin(sb), verlet_skin=0.3) as sim:
+    with Simulation(config_from_spherebin(sb), verlet_skin=0.3, topo_span=span) as sim:
         sim.upload(state_from_spherebin(sb))
         sim.step(60)
         sim.sync()
@@ -80,10 +89,12 @@ def test_model1_lists_outlive_changes_of_cell(oracle_libs, name):
     assert mismatches(got, want, ALL) == []
 
 
-def test_batched_scenes_of_either_kind(oracle_libs):
+@both_kernels
+def test_batched_scenes_of_either_kind(oracle_libs, span):
     """Scenes whose lists outlive changes of cell beside scenes whose do not."""
     sbs = [SCENES[k]() for k in ("cells_2r", "cells_1.05r", "two_cells", "cells_2r_periodic_x")]
-    with BatchSimulation([config_from_spherebin(sb) for sb in sbs], verlet_skin=0.3) as sim:
+    with BatchSimulation([config_from_spherebin(sb) for sb in sbs], verlet_skin=0.3,
+                         topo_span=span) as sim:
         sim.upload([state_from_spherebin(sb) for sb in sbs])
         sim.step(50)
         sim.sync()
