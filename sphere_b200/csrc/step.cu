@@ -29,7 +29,6 @@
 // visiting order is the reference's: stencil cells z, y, x, members of a cell
 // by particle index.
 #include <algorithm>
-#include <type_traits>
 
 #include "sphk_internal.cuh"
 #include "diff_step.cuh"
@@ -50,14 +49,14 @@ constexpr int FORCE_BLOCK = SPHK_FORCE_BLOCK;
 // shapes each, and a context picks one pair (Dev::shape, SPH_OPT_BLOCK_SHAPES;
 // the ensemble's autotuner times both).  Shape 0, the default: k_topo in
 // blocks of 64 threads, 16 per SM, whose threads leave at different times;
-// k_contact in blocks of 4 warps, 5 per SM.  Shape 1: k_topo in 128 x 8,
-// k_contact in 2 warps x 10.  The threads resident per SM are the same.
+// k_contact in blocks of 4 warps, 4 per SM.  Shape 1: k_topo in 128 x 8,
+// k_contact in 2 warps x 8.  The threads resident per SM are the same.
 #ifndef SPHK_TOPO_THREADS_PER_SM
 #define SPHK_TOPO_THREADS_PER_SM 1024
 #endif
 constexpr int TOPO_THREADS_PER_SM = SPHK_TOPO_THREADS_PER_SM;
 #ifndef SPHK_CONTACT_THREADS_PER_SM
-#define SPHK_CONTACT_THREADS_PER_SM 640
+#define SPHK_CONTACT_THREADS_PER_SM 512
 #endif
 constexpr int CONTACT_THREADS_PER_SM = SPHK_CONTACT_THREADS_PER_SM;
 __host__ __device__ constexpr int topo_block(uint32_t shape) { return shape ? 128 : 64; }
@@ -1719,222 +1718,94 @@ struct ContactArgs {
     LawParams lp;        // single-scene contexts; a batch reads each scene's Params
 };
 
-// Contacts of one chunk whose law terms a warp holds at once (a multiple of 32).
-#ifndef SPHK_CONTACT_CAP
-#define SPHK_CONTACT_CAP 64
-#endif
-constexpr uint32_t CT_CAP = SPHK_CONTACT_CAP;
-
-// A warp's shared memory for one chunk's contacts.
-struct ContactWarp {
-    double terms[9][CT_CAP];       // law terms held: F xyz, T xyz, p, ev_dot, es_dot
-    double sums[9][32];            // each particle's running sums
-    LawParams law;                 // a batch's scene
-    uint32_t smask[NC];            // the particles holding each slot
-    uint32_t hitw[CT_CAP / 32], slipw[CT_CAP / 32];   // which held contacts overlapped, slipped
-    uint16_t expand[32 * NC];      // the chunk's list of (lane | slot << 5)
-    uint16_t sbase[NC];            // first list entry of each slot
+// A particle's slot sums.
+struct SlotSums {
+    d3 F, T;
+    double p, ev, es;
 };
 
-// The slot loop of a chunk, 32 consecutive storage indices from s0, by one
-// warp: lane l's particle s0 + l held the slots occ0, still holds occ after
-// this step, and where occ0 is not zero its sums are cs.sums[.][l].  have: the
-// scene in cs.law.  Returns whether a particle of the chunk still holds a slot.
-//
-// The occupied slots form a list of directed contacts, written once into
-// shared memory as (lane, slot) pairs in slot-major order.  The list is
-// evaluated 32 contacts at a time, one per lane, so every lane runs a force
-// law whatever the spread of contact counts, and the terms of up to CT_CAP
-// contacts are kept in shared memory.  Then every particle's own lane adds its
-// terms in slot order, the reference's summation order, all lanes at once.  A
-// slot whose partner no longer overlaps is freed and its history zeroed, as in
-// the reference.  A chunk's rows are contiguous, its slot tiles too, and a
-// round's lanes mostly read one slot of consecutive particles, so their loads
-// coalesce.
-template <int MODEL, bool BATCH>
-__device__ __forceinline__ bool contact_chunk(const Dev &d, int A, const LawParams &lp, uint32_t s0,
-                                              ContactWarp &cs, uint32_t &have, uint32_t &occ0,
-                                              uint32_t &occ)
+// interact's slot loop (src/contactsearch.cuh:468-543) for particle s, whose
+// occupied slots are occ0: the sums of the laws' terms in slot order, the
+// slots' new history, and in occ the slots still held.  A slot whose partner
+// no longer overlaps is freed and its history zeroed, as in the reference.
+template <int MODEL, class PR>
+__device__ __forceinline__ void contact_slots(const Dev &d, int A, const PR &P, uint32_t s,
+                                              uint32_t occ0, uint32_t &occ, SlotSums &o)
 {
-    constexpr uint32_t FULL = 0xffffffffu;
-    const uint32_t np = d.np_all, lane = threadIdx.x & 31u, s = s0 + lane;
-    double (*tm)[CT_CAP] = cs.terms;
-    double (*sm)[32] = cs.sums;
-    uint16_t *ex = cs.expand;
-    occ0 = (s < np) ? d.cmask[s] : 0u;
-    const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
-    const uint32_t n = __popc(occ0);
-    const uint32_t total = __reduce_add_sync(FULL, n);   // the chunk's contacts
-    // The list in slot-major order: slot by slot, and within a slot
-    // by particle.  The lanes of a round then mostly share a slot and
-    // touch consecutive particles: consecutive entries of the slot
-    // tiles and consecutive particle rows.  A particle's contacts stay
-    // in ascending slot order along the list; slot i's first entry is
-    // sbase[i], and a particle finds its own entry of slot i from
-    // smask[i], the particles holding it.
-    {
-        const uint32_t lt = (1u << lane) - 1u;
-        uint32_t k = 0;
-        for (uint32_t u = __reduce_or_sync(FULL, occ0); u; u &= u - 1u) {
-            const uint32_t i = (uint32_t)(__ffs(u) - 1);
-            const uint32_t m = __ballot_sync(FULL, (occ0 >> i) & 1u);
-            if ((occ0 >> i) & 1u) ex[k + __popc(m & lt)] = (uint16_t)(lane | (i << 5));
-            if (lane == 0) {
-                cs.sbase[i] = (uint16_t)k;
-                cs.smask[i] = m;
-            }
-            k += __popc(m);
+    const double4 xa = d.xr[A][s];
+    const double4 vel_a = ld4(d.vel[A], s);
+    const d3 angvel_a = xyz(ld4(d.angvel[A], s));
+    const ulonglong2 dmw = d.dmc[s];
+    o = SlotSums{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
+    occ = occ0;
+    // the partner of the next slot, loaded a slot ahead
+    uint32_t i = (uint32_t)(__ffs(occ0) - 1);
+    uint32_t t = d.contacts[tile_at(s, i, NC)];
+    for (uint32_t m = occ0; m;) {
+        const size_t e = tile_at(s, i, NC);
+        const double4 xb = d.xr[A][t];
+        const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
+        const P3 dtp = d.delta_t[e];
+        const uint32_t bit = m & (0u - m), slot = i;
+        m &= m - 1u;
+        if (m) {
+            i = (uint32_t)(__ffs(m) - 1);
+            t = d.contacts[tile_at(s, i, NC)];
         }
-    }
-    __syncwarp();
-
-    // the particle's running sums live in shared memory between the
-    // passes, so no register holds them while the laws run
-    if (n) {
-#pragma unroll
-        for (int f = 0; f < 9; ++f) sm[f][lane] = 0.0;
-    }
-    occ = occ0;   // slots still held after this step
-    uint32_t rem = occ0;   // slots whose terms are still to be added
-    // the partner of this lane's contact, loaded a round ahead
-    uint32_t t_next = 0;
-    if (lane < total) {
-        const uint32_t x = ex[lane];
-        t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
-    }
-    for (uint32_t base = 0; base < total; base += 32u) {
-        const uint32_t c = base + lane;
-        const uint32_t t = t_next;
-        if (c + 32u < total) {
-            const uint32_t x = ex[c + 32u];
-            t_next = d.contacts[tile_at(s0 + (x & 31u), x >> 5, NC)];
-        }
-        const uint32_t pb = base - base % CT_CAP;   // first contact of this pass
-        bool hit = false, slip = false;
-        auto evaluate = [&](const auto &P) {
-            const uint32_t x = ex[c];
-            const uint32_t sq = s0 + (x & 31u), i = x >> 5;
-            const size_t e = tile_at(sq, i, NC);
-            const ulonglong2 dmw = d.dmc[sq];
-            const P3 dtp = d.delta_t[e];
+        const double ra = xa.w, rb = xb.w;
+        const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)slot), P);
+        const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
+        const double xlen = flen(xab);
+        const double delta_n = xlen - (ra + rb);
+        if (delta_n < 0.0f) {
             const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
-            const double4 xa = d.xr[A][sq];
-            const double4 vel_a = ld4(d.vel[A], sq);
-            const d3 angvel_a = xyz(ld4(d.angvel[A], sq));
-            const double4 xb = d.xr[A][t];
-            const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
-            LawOut o;
-            const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)i), P);
-            const double ra = xa.w, rb = xb.w;
-            const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y,
-                              xa.z - xb.z + dm.z);
-            const double xlen = flen(xab);
-            const double delta_n = xlen - (ra + rb);
-            const bool touch = delta_n < 0.0f;
-            if (touch) {
-                o = (MODEL == 2)
-                    ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
-                                     xlen, delta_n, dt0)
-                    : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab,
-                                    xlen, delta_n, dt0);
-            }
-            if (touch) {
-                const uint32_t k = c - pb;
-                d.delta_t[e] = P3{o.dt4.x, o.dt4.y, o.dt4.z};
-                tm[0][k] = o.f.x;
-                tm[1][k] = o.f.y;
-                tm[2][k] = o.f.z;
-                tm[3][k] = o.t.x;
-                tm[4][k] = o.t.y;
-                tm[5][k] = o.t.z;
-                tm[6][k] = o.pr;
-                tm[7][k] = o.ev;
-                tm[8][k] = o.es;
-                hit = true;
-                slip = o.es_set;
-            } else {
-                // separated: free the slot and zero its history
-                d.contacts[e] = np;
-                d.delta_t[e] = P3{0.0, 0.0, 0.0};
-            }
-        };
-        if constexpr (BATCH) {
-            const uint32_t q = __shfl_sync(FULL, inst, c < total ? (ex[c] & 31u) : 0u);
-            by_scene(cs.law, have, q, c < total,
-                     [&](LawParams &l, uint32_t i) { l = law_params(d.prm[i]); }, evaluate);
-        } else if (c < total) {
-            evaluate(lp);
+            const LawOut l = (MODEL == 2)
+                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0)
+                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0);
+            d.delta_t[e] = P3{l.dt4.x, l.dt4.y, l.dt4.z};
+            o.F = add(o.F, l.f);
+            o.T = add(o.T, l.t);
+            o.p += l.pr;
+            o.ev += l.ev;
+            if (l.es_set) o.es += l.es;
+        } else {
+            // separated: free the slot and zero its history
+            d.contacts[e] = d.np_all;
+            d.delta_t[e] = P3{0.0, 0.0, 0.0};
+            occ &= ~bit;
         }
-        const uint32_t hb = __ballot_sync(FULL, hit);
-        const uint32_t sb = __ballot_sync(FULL, slip);
-        if (lane == 0) {
-            cs.hitw[(base - pb) >> 5] = hb;
-            cs.slipw[(base - pb) >> 5] = sb;
-        }
-        const uint32_t pe = min(total, pb + CT_CAP);
-        if (base + 32u < pe) continue;
-        __syncwarp();
-        // the pass is complete: every particle adds its terms of the
-        // pass, in slot order
-        const uint32_t lt = (1u << lane) - 1u;
-        auto entry = [&](uint32_t i) { return (uint32_t)cs.sbase[i] + __popc(cs.smask[i] & lt); };
-        if (rem && entry((uint32_t)(__ffs(rem) - 1)) < pe) {
-            d3 F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);
-            d3 T = mk(sm[3][lane], sm[4][lane], sm[5][lane]);
-            double p = sm[6][lane], ev_dot = sm[7][lane], es_dot = sm[8][lane];
-            while (rem) {
-                const uint32_t i = (uint32_t)(__ffs(rem) - 1);
-                const uint32_t j = entry(i);
-                if (j >= pe) break;   // in a later pass
-                const uint32_t k = j - pb;
-                rem &= rem - 1u;
-                if ((cs.hitw[k >> 5] >> (k & 31u)) & 1u) {
-                    F = add(F, mk(tm[0][k], tm[1][k], tm[2][k]));
-                    T = add(T, mk(tm[3][k], tm[4][k], tm[5][k]));
-                    p += tm[6][k];
-                    ev_dot += tm[7][k];
-                    if ((cs.slipw[k >> 5] >> (k & 31u)) & 1u) es_dot += tm[8][k];
-                } else {
-                    occ &= ~(1u << i);
-                }
-            }
-            sm[0][lane] = F.x;
-            sm[1][lane] = F.y;
-            sm[2][lane] = F.z;
-            sm[3][lane] = T.x;
-            sm[4][lane] = T.y;
-            sm[5][lane] = T.z;
-            sm[6][lane] = p;
-            sm[7][lane] = ev_dot;
-            sm[8][lane] = es_dot;
-        }
-        __syncwarp();
     }
     if (occ != occ0) {
         d.cmask[s] = occ;
         d.vl_held[s] = 0u;   // a listed candidate left its slot: the next
         d.due[s] = -1.0f;    // search looks at the list
     }
-    return __any_sync(FULL, occ != 0u);
 }
 
-// k_contact: interact's slot loop (src/contactsearch.cuh:468-543) for
-// contact models 2 and 3, one lane per directed contact (contact_chunk).
+// k_contact: the slot forces of contact models 2 and 3.
 //
-// The unit of work is a chunk of 32 consecutive storage indices, and a chunk
-// is visited only while its flag (Dev::cflag) says it may hold a contact:
-// the contact search sets the flag when it writes a row with an occupied
-// slot, and this kernel clears it when the chunk ends without one.  The grid
-// is resident (a few blocks per SM); warp g takes chunks g, g + W, g + 2W,
-// ... of the W warps, reading the flags of 32 of them in one load, so a
-// contact-free scene costs about one memory latency.
+// The unit of work is a chunk of 32 consecutive storage indices, a lane a
+// particle, and a chunk is visited only while its flag (Dev::cflag) says it
+// may hold a contact: the contact search sets the flag when it writes a row
+// with an occupied slot, and this kernel clears it when the chunk ends without
+// one.  The grid is resident (a few blocks per SM); warp g takes chunks g,
+// g + W, g + 2W, ... of the W warps, reading the flags of 32 of them in one
+// load, so a contact-free scene costs about one memory latency.  A chunk's
+// rows are contiguous, its slot tiles too, and its lanes mostly walk the same
+// slots, so their loads coalesce.
+//
+// What bounds it: the laws' FP64 chains at 16 warps an SM and L1, 54 B of
+// history and 80 B of the partner's rows a contact.  A lane a contact, which
+// kept every lane busy whatever the spread of contact counts, loaded the
+// particle's own rows again for each of its contacts and passed nine terms
+// through shared memory (L1 79% busy): the jammed 1M column 189 -> 166 us.
 template <int MODEL, bool BATCH, int CB>
 __global__ void __launch_bounds__(CB, CONTACT_THREADS_PER_SM / CB)
 k_contact(ContactArgs args)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = CB / 32;
-    __shared__ ContactWarp warps[WARPS];
+    __shared__ LawParams law[BATCH ? WARPS : 1];   // a batch's scene, one a warp
     uint32_t have = 0xffffffffu;
     const Dev &d = args.d;
     const int A = args.a;
@@ -1942,7 +1813,6 @@ k_contact(ContactArgs args)
     const uint32_t np = d.np_all;
     const uint32_t nchunk = (np + 31u) >> 5;
     const uint32_t gw = blockIdx.x * WARPS + w, nwarps = gridDim.x * WARPS;
-    double (*sm)[32] = warps[w].sums;
     // A chunk's rows are contiguous (its slot tiles too), so one lane asks
     // the copy engine to bring a chunk that is coming up into L2 while the
     // warp works: the chain of loads of each round then waits on L2, not on
@@ -1970,13 +1840,22 @@ k_contact(ContactArgs args)
             if (todo) prefetch_chunk(g + (uint32_t)(__ffs(todo) - 1) * nwarps);
             const uint32_t s0 = chunk << 5;
             const uint32_t s = s0 + lane;
-            uint32_t occ0, occ;
-            const bool held = contact_chunk<MODEL, BATCH>(d, A, args.lp, s0, warps[w], have, occ0, occ);
-            if (occ0) {
-                d.csum_f[s] = make_double4(sm[0][lane], sm[1][lane], sm[2][lane], sm[6][lane]);
-                d.csum_t[s] = make_double4(sm[3][lane], sm[4][lane], sm[5][lane], sm[7][lane]);
-                d.csum_es[s] = sm[8][lane];
+            const uint32_t occ0 = (s < np) ? d.cmask[s] : 0u;
+            uint32_t occ = 0u;
+            auto slots = [&](const auto &P) {
+                SlotSums o;
+                contact_slots<MODEL>(d, A, P, s, occ0, occ, o);
+                d.csum_f[s] = make_double4(o.F.x, o.F.y, o.F.z, o.p);
+                d.csum_t[s] = make_double4(o.T.x, o.T.y, o.T.z, o.ev);
+                d.csum_es[s] = o.es;
+            };
+            if constexpr (BATCH) {
+                by_scene(law[w], have, s < np ? d.inst[s] : 0u, occ0 != 0u,
+                         [&](LawParams &l, uint32_t i) { l = law_params(d.prm[i]); }, slots);
+            } else if (occ0) {
+                slots(args.lp);
             }
+            const bool held = __any_sync(FULL, occ != 0u);
             // visited (2: a slot is still held, 3: none is); k_force_tiles reads
             // the sums of a visited chunk and sets its flag back to 1 or 0
             // for the next step's search
@@ -2025,24 +1904,14 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = SMALL_BLOCK / 32;
     constexpr bool VISC = MODEL == 1;
-    // model 1: the acting pairs and their evaluation; otherwise the search's
-    // slot rows, then the contacts
-    struct Visc {
-        uint32_t srow[NC * 32];
-        ViscWarp vs;
-    };
-    union Slots {
-        uint32_t srow[NC * 32];
-        ContactWarp cs;
-    };
-    using Warp = std::conditional_t<VISC, Visc, Slots>;
-    __shared__ __align__(16) unsigned char mem[WARPS][sizeof(Warp)];
+    __shared__ uint32_t srow[WARPS][NC * 32];   // the search's slot rows; model 1's acting pairs
+    __shared__ ViscWarp visc[VISC ? WARPS : 1];
+    __shared__ LawParams law[BATCH ? WARPS : 1];
     __shared__ ForceConsts scene[BATCH ? WARPS : 1];
     const Dev &d = args.d;
     const int A = args.a;
     const uint32_t np = d.np_all, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
-    Warp &sh = *reinterpret_cast<Warp *>(mem[w]);
     if (s0 < np) {
         ViscAct va{0u, mk(0.0, 0.0, 0.0), 0.0};   // model 1's sums
         // ---- the search (k_topo) ----
@@ -2053,20 +1922,29 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
                 sweep = V.all_rebuild != 0u || (V.dirty_step == V.step && d.dirty[d.cell[s]] == V.step);
                 need = sweep || V.moved > d.due[s];
             }
-            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, sh.srow, sweep, va);
+            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, va);
             __syncwarp();
-            if constexpr (VISC) visc_warp(d, A, s, sh.srow, 32u, sh.vs, va);
+            if constexpr (VISC) visc_warp(d, A, s, srow[w], 32u, visc[w], va);
         }
         // ---- the slot forces (k_contact) ----
-        uint32_t have = 0xffffffffu, occ0 = 0u, occ = 0u;
+        const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
+        uint32_t have = 0xffffffffu, occ = 0u;
+        SlotSums o{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
         if constexpr (!VISC) {
             if (d.cflag[chunk] != 0) {
-                const bool held = contact_chunk<MODEL, BATCH>(d, A, lp, s0, sh.cs, have, occ0, occ);
+                const uint32_t occ0 = (s < np) ? d.cmask[s] : 0u;
+                auto slots = [&](const auto &P) { contact_slots<MODEL>(d, A, P, s, occ0, occ, o); };
+                if constexpr (BATCH) {
+                    by_scene(law[w], have, inst, occ0 != 0u,
+                             [&](LawParams &l, uint32_t i) { l = law_params(d.prm[i]); }, slots);
+                } else if (occ0) {
+                    slots(lp);
+                }
+                const bool held = __any_sync(FULL, occ != 0u);
                 if (lane == 0) d.cflag[chunk] = held ? 1 : 0;
             }
         }
         // ---- the rest of the step (k_force_tiles) ----
-        const uint32_t inst = (BATCH && s < np) ? d.inst[s] : 0u;
         auto integrate = [&](const ForceConsts &fc) {
             const RegRows R(d, A, s);
             d3 F = mk(0.0, 0.0, 0.0), T = mk(0.0, 0.0, 0.0);
@@ -2075,12 +1953,11 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
                 F = va.F;
                 p = va.p;
             } else if (occ != 0u) {
-                const double (*sm)[32] = sh.cs.sums;
-                F = mk(sm[0][lane], sm[1][lane], sm[2][lane]);
-                T = mk(sm[3][lane], sm[4][lane], sm[5][lane]);
-                p = sm[6][lane];
-                ev_dot = sm[7][lane];
-                es_dot = sm[8][lane];
+                F = o.F;
+                T = o.T;
+                p = o.p;
+                ev_dot = o.ev;
+                es_dot = o.es;
             }
             particle_tail<BATCH, false>(d, fc, s, A, args.write_outputs, R.x,
                                         make_double4(R.v.x, R.v.y, R.v.z, 0.0),
