@@ -15,20 +15,19 @@
 namespace sphk {
 void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st);
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  const NextStep &next, cudaStream_t st);
+                  cudaStream_t st);
 void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st);
 bool small_step(const Dev &d, uint32_t np);
 void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  const NextStep &next, cudaStream_t st);
+                  bool own_list, cudaStream_t st);
+void launch_tail(const Dev &d, cudaStream_t st);
 void launch_bonds(const Dev &d, const Params &hp, uint32_t nb0, int a, cudaStream_t st);
 void launch_bond_storage(const Dev &d, uint32_t nb0, uint32_t np, cudaStream_t st);
 void launch_walls(const Dev &d, uint32_t np, uint32_t nw, cudaStream_t st);
 void launch_cell_init(const Dev &d, uint32_t np, int a, cudaStream_t st);
 void launch_epoch_reset(const Dev &d, cudaStream_t st);
 void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st);
-unsigned int scan_tile_count(uint32_t ncells);
 void relayout(const Dev &d, uint32_t np, int a, void *scratch, cudaStream_t st);
-void launch_rebuild_gate(cudaGraphConditionalHandle h, const uint32_t *rebuild, cudaStream_t st);
 void launch_darcy(const Dev &d, const DarcyDev &f, const Params &hp, int a, int hs, int last,
                   cudaStream_t st);
 struct RenderArgs;
@@ -36,8 +35,7 @@ void launch_maxpos(const Dev &d, uint32_t np, int a, unsigned long long *mx, cud
 int render_image(const Dev &d, uint32_t np, int a, const double L[3], const double maxpos[3],
                  const sph_render_opts &o, double *values, unsigned long long *keys, uchar4 *img,
                  float *rays, cudaStream_t st);
-void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, const NextStep &next,
-                       cudaStream_t st);
+void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStream_t st);
 void launch_rev_step(const Dev &d, const AdjDev &a, uint32_t np, int j, cudaStream_t st);
 void launch_user_to_storage3(const double *src, double4 *dst, const uint32_t *uid, uint32_t n,
                              cudaStream_t st);
@@ -59,8 +57,6 @@ struct sph_ctx {
     bool batched = false;
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;     // captures the bodies of conditional graph nodes
-    bool cond_rebuild = true;        // graphs skip the rebuild kernels when no cell changed
     int a = 0;                       // buffer holding the current state
     uint64_t steps = 0, relayouts = 0, since_relayout = 0;
     double t_host = 0.0;
@@ -352,71 +348,13 @@ int sync_status(sph_ctx *c)
     return SPH_OK;
 }
 
-// The condition handles of a graph's steps while it is captured: each step's
-// end sets that of the next, a kernel of its own (k_rebuild_gate) the first's.
-struct StepGate {
-    bool on = false;     // capturing, with conditional nodes
-    bool first = true;   // no step captured yet
-    NextStep here{};     // this step's handle
-};
-
-int captured_graph(sph_ctx *c, cudaStream_t st, cudaGraph_t *g, const cudaGraphNode_t **deps, size_t *nd)
+// One step on `st`; capturing: into a graph.
+int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool capturing = false)
 {
-    cudaStreamCaptureStatus cs;
-    unsigned long long id;
-    CK(cudaStreamGetCaptureInfo(st, &cs, &id, g, deps, nd));
-    return SPH_OK;
-}
-
-// Inside a stream capture: the rebuild as a conditional node whose body the
-// side stream captures, and the handle that the step's end sets for the next
-// step (`last`: there is none).
-int capture_rebuild_conditional(sph_ctx *c, int a, bool last, StepGate &gate, NextStep &next,
-                                cudaStream_t st)
-{
-    cudaGraph_t g;
-    const cudaGraphNode_t *deps;
-    size_t nd;
-    int rc;
-    if ((rc = captured_graph(c, st, &g, &deps, &nd)) != SPH_OK) return rc;
-    if (gate.first) {
-        CK(cudaGraphConditionalHandleCreate(&gate.here.handle, g, 0, 0));
-        launch_rebuild_gate(gate.here.handle, c->d.rebuild, st);
-        gate.first = false;
-    }
-    if ((rc = captured_graph(c, st, &g, &deps, &nd)) != SPH_OK) return rc;
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = gate.here.handle;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    CK(cudaGraphAddNode(&node, g, deps, nd, &np));
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    CK(cudaStreamBeginCaptureToGraph(c->side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    launch_rebuild(c->d, c->np_all, c->ncells_all, a, c->side);
-    CK(cudaStreamEndCapture(c->side, &body));
-    CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    next = NextStep{};
-    if (!last) {
-        CK(cudaGraphConditionalHandleCreate(&next.handle, g, 0, 0));
-        next.gated = 1;
-        gate.here = next;
-    }
-    return SPH_OK;
-}
-
-// gate: of the graph being captured, or nullptr; last: its last step.
-int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, StepGate *gate, bool last)
-{
-    const bool capturing = gate != nullptr;
-    NextStep next{};
-    if (capturing && gate->on) {
-        const int rc = capture_rebuild_conditional(c, a, last, *gate, next, st);
-        if (rc != SPH_OK) return rc;
-    } else {
-        launch_rebuild(c->d, c->np_all, c->ncells_all, a, st);
-    }
+    // the small scenes' kernel makes its own cell list, unless the flow reads it too
+    const bool small = !c->diff && small_step(c->d, c->np_all);
+    const bool own_list = small && !c->darcy_on;
+    if (!own_list) launch_rebuild(c->d, c->np_all, c->ncells_all, a, st);
     launch_bonds(c->d, c->hp, c->hp.nb0, a, st);
     // The Darcy block reads the step's start positions (buffer a) and its
     // cell list, which nothing changes before the next step's rebuild, and
@@ -438,14 +376,15 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, Step
         return SPH_OK;
     };
     int rc;
-    if (!c->diff && small_step(c->d, c->np_all)) {
+    if (small) {
         if ((rc = join_walls()) != SPH_OK) return rc;
-        launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, next, st);
+        launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, own_list, st);
     } else {
         launch_topo(c->d, c->np_all, model == 1, a, st);
         launch_contact(c->d, c->hp, c->np_all, model, a, st);
         if ((rc = join_walls()) != SPH_OK) return rc;
-        launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, next, st);
+        launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, st);
+        launch_tail(c->d, st);
     }
     if (c->darcy_on && !branch) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
     if (capturing && c->hp.nw > 0 && !c->batched) {
@@ -468,12 +407,13 @@ int capture(sph_ctx *c, cudaGraphExec_t *out, int a, int nsteps, int write_last)
     int aa = a;
     int rc = SPH_OK;
     c->wall_pending = false;
-    StepGate gate;
-    gate.on = c->cond_rebuild;
     for (int i = 0; i < nsteps && rc == SPH_OK; ++i) {
-        const bool last = i == nsteps - 1;
-        rc = enqueue_one_step(c, aa, (write_last && last) ? 1 : 0, c->stream, &gate, last);
+        rc = enqueue_one_step(c, aa, (write_last && i == nsteps - 1) ? 1 : 0, c->stream, true);
         aa ^= 1;
+    }
+    if (rc == SPH_OK) {
+        const cudaError_t e = cudaGetLastError();   // of the launches
+        if (e != cudaSuccess) rc = fail(c, SPH_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
     }
     if (c->wall_pending) {
         // the last step's walls are part of the graph's work (and a capture
@@ -484,17 +424,11 @@ int capture(sph_ctx *c, cudaGraphExec_t *out, int a, int nsteps, int write_last)
     }
     c->wall_pending = false;
     if (rc != SPH_OK) {
-        // conditional nodes unavailable: end the broken capture and capture
-        // the plain rebuild instead
+        // end the broken capture
         cudaStreamEndCapture(c->stream, &g);
         if (g) cudaGraphDestroy(g);
-        if (c->side) cudaStreamEndCapture(c->side, &g);
         cudaGetLastError();
-        if (!c->cond_rebuild) return rc;
-        c->cond_rebuild = false;
-        c->sticky = SPH_OK;
-        c->err.clear();
-        return capture(c, out, a, nsteps, write_last);
+        return rc;
     }
     CK(cudaStreamEndCapture(c->stream, &g));
     cudaError_t e = cudaGraphInstantiate(out, g, 0);
@@ -569,8 +503,9 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
     CK(cudaEventRecord(c->ev[3], st));
     launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, st);
     CK(cudaEventRecord(c->ev[4], st));
-    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, NextStep{}, st);
+    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, st);
     CK(cudaEventRecord(c->ev[5], st));
+    launch_tail(c->d, st);
     launch_walls(c->d, c->np_all, c->hp.nw, st);
     CK(cudaEventRecord(c->ev[6], st));
     if (c->darcy_on) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
@@ -590,7 +525,7 @@ int do_relayout(sph_ctx *c, cudaStream_t st)
 {
     // the cell list must describe the current positions before storage follows
     // it (it may be stale: any nonzero flag rebuilds it)
-    CK(cudaMemsetAsync(c->d.rebuild, 1, 4, st));
+    CK(cudaMemsetAsync(&c->d.rebuild[REBUILD_NOW], 1, 4, st));
     launch_rebuild(c->d, c->np_all, c->ncells_all, c->a, st);
     relayout(c->d, c->np_all, c->a, c->scratch, st);
     // the bonds follow their particles' new storage indices
@@ -712,7 +647,6 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     c->device = cfgs[0].device;
     CK(cudaSetDevice(c->device));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&c->wall_stream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->wall_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->wall_join, cudaEventDisableTiming));
@@ -738,7 +672,7 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     AL(d.cmask, np);
     AL(d.cflag, div_up(np, 32));
     AL(d.cell_start, ncells + 2); AL(d.cellorder, np); AL(d.pos, npad); AL(d.cell_fill, ncells + 1);
-    AL(d.scan_tiles, scan_tile_count(c->ncells_all));
+    AL(d.scan_tiles, SCAN_TILES);
     AL(d.alias_any, 1);
     AL(d.vl, tiled_size(np, VL_CAP)); AL(d.vl_meta, tiled_size(np, VL_CAP)); AL(d.vl_len, np);
     AL(d.vl_held, np); AL(d.due, np);
@@ -754,7 +688,7 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     } else {
         AL(d.csum_f, np); AL(d.csum_t, np); AL(d.csum_es, np);
     }
-    AL(d.status, 1); AL(d.rebuild, 1); AL(d.prm, ninst);
+    AL(d.status, 1); AL(d.rebuild, 2); AL(d.prm, ninst);
     if (batched) {
         AL(d.inst, np);
         AL(d.inst_cell_base, (size_t)ninst + 1);
@@ -1052,8 +986,7 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
         CK(cudaStreamSynchronize(c->stream));   // the CSR built above goes out of scope
     }
     CK(cudaMemsetAsync(d.status, 0, 4, c->stream));
-    const uint32_t one = 1;
-    CK(cudaMemcpyAsync(d.rebuild, &one, 4, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(d.rebuild, 0, 8, c->stream));
     c->sticky = SPH_OK;
     c->err.clear();
     c->t_host = h->t_current;
@@ -1295,7 +1228,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         auto part = [&](size_t count) { const size_t at = bytes; bytes += (count + 31) / 32 * 128; return at; };
         const size_t o_cell = part(np), o_order = part(np), o_pos = part(np), o_xs = part(4 * (size_t)np),
                      o_start = part((size_t)nc + 2), o_fill = part((size_t)nc + 1),
-                     o_scan = part(scan_tile_count(nc)), o_word = part(4), o_vs = part(32);
+                     o_scan = part(SCAN_TILES), o_word = part(4), o_vs = part(32);
         CK(cudaMallocAsync(&tmp, bytes, c->stream));
         CK(cudaMemsetAsync(tmp + o_fill, 0, bytes - o_fill, c->stream));
         auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
@@ -1304,7 +1237,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         q.cell_start = at(o_start); q.cell_fill = at(o_fill); q.scan_tiles = at(o_scan);
         q.status = at(o_word); q.alias_any = at(o_word) + 1; q.rebuild = at(o_word) + 2;
         q.vs = reinterpret_cast<Verlet *>(tmp + o_vs);
-        CK(cudaMemsetAsync(q.rebuild, 1, 4, c->stream));
+        CK(cudaMemsetAsync(&q.rebuild[REBUILD_NOW], 1, 4, c->stream));
         launch_cell_init(q, np, c->a ^ 1, c->stream);
         launch_rebuild(q, np, nc, c->a ^ 1, c->stream);
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);
@@ -1460,13 +1393,11 @@ static int capture_segment(sph_ctx *c, int len, int a, cudaGraphExec_t *out)
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int rc = SPH_OK;
     int aa = a;
-    StepGate gate;
     for (int j = 0; j < len && rc == SPH_OK; ++j) {
-        NextStep next{};
-        if (c->cond_rebuild) rc = capture_rebuild_conditional(c, aa, j == len - 1, gate, next, st);
-        else launch_rebuild(d, np, c->ncells_all, aa, st);
+        launch_rebuild(d, np, c->ncells_all, aa, st);
         launch_topo(d, np, false, aa, st);
-        launch_force_tape(d, np, aa, j, next, st);
+        launch_force_tape(d, np, aa, j, st);
+        launch_tail(d, st);
         aa ^= 1;
     }
     for (int j = len - 1; j >= 0 && rc == SPH_OK; --j) launch_rev_step(d, c->adj, np, j, st);
@@ -1706,7 +1637,7 @@ int sph_darcy_upload(sph_ctx *c, double nu, const sph_darcy_state *h)
     // steps so far may have left them behind
     c->hp.eager = c->hps[0].eager = 1u;
     CK(cudaMemcpyAsync(c->d.prm, c->hps.data(), sizeof(Params), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(c->d.rebuild, 1, 4, c->stream));
+    CK(cudaMemsetAsync(&c->d.rebuild[REBUILD_NOW], 1, 4, c->stream));
     drop_graphs(c);   // the step graphs gain the Darcy kernels
     CK(cudaStreamSynchronize(c->stream));   // the caller's arrays are complete
     return SPH_OK;
@@ -1794,7 +1725,6 @@ int sph_destroy(sph_ctx *c)
     if (c->wall_stream) cudaStreamDestroy(c->wall_stream);
     for (void *p : c->allocs) cudaFree(p);
     if (c->stream) cudaStreamDestroy(c->stream);
-    if (c->side) cudaStreamDestroy(c->side);
     delete c;
     return SPH_OK;
 }

@@ -1,0 +1,232 @@
+// rebuild.cuh -- the cell list as a device function of a whole grid, called by
+// the kernel that only makes the list (cells.cu) and by the small scenes' step
+// (k_small, step.cu):
+//   count      histogram of cell ids                  (atomics in L2)
+//   scan       exclusive scan of the histogram        (two passes)
+//   scatter    each particle claims a position in its cell's range
+//   sort       each cell orders its few members by particle index
+//   finish     inverse order, the float position copy in list order, and the
+//              stamps of the cells whose particles' lists a move upset
+// The blocks wait for one another between the passes, so the kernel is
+// launched cooperatively.  Arrays that a pass changes after another read them
+// in the same launch are read past L1 (__ldcg).
+#ifndef SPHK_REBUILD_CUH_
+#define SPHK_REBUILD_CUH_
+
+#include "sphk_internal.cuh"
+
+namespace sphk {
+
+// Waits until every block of the grid is here; false when that did not happen
+// within BULK_WAIT_NS (ST_TIMEOUT: the caller leaves).  bar: a counter that
+// only this kernel's launches use, a multiple of the grid's blocks before.
+__device__ __forceinline__ bool grid_barrier(const Dev &d, uint32_t *bar)
+{
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t ticket = atomicAdd(bar, 1u);
+        const uint32_t target = (ticket / gridDim.x + 1u) * gridDim.x;
+        const uint64_t t0 = global_ns();
+        ok = 1;
+        while ((int32_t)(*(volatile const uint32_t *)bar - target) < 0) {
+            if (global_ns() - t0 > BULK_WAIT_NS) {
+                atomicOr(d.status, ST_TIMEOUT);
+                ok = 0;
+                break;
+            }
+            __nanosleep(64);   // leaves the counter to those still arriving
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// Every cell of the neighbourhood of the cells that a move left and entered
+// (27 cells each, or with Params::wide 125) is stamped with this step's
+// number; particles in stamped cells sweep their stencil again.  Periodic axes
+// wrap as in findDistMod.
+__device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32_t stride)
+{
+    Verlet &V = *d.vs;
+    const uint32_t n = min(__ldcg(&V.nmovers), MOVER_CAP), step = __ldcg(&V.step);
+    for (uint32_t e = first; e < 2 * n; e += stride) {
+        const uint2 mv = __ldcg(&d.movers[e >> 1]);
+        const uint32_t cg = (e & 1u) ? mv.y : mv.x;
+        if (cg >= d.ncells_all) continue;
+        // the instance owning global cell cg (batched contexts)
+        uint32_t inst = 0;
+        if (d.inst) {
+            uint32_t lo = 0, hi = d.ninst;
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (d.inst_cell_base[mid] <= cg) lo = mid; else hi = mid;
+            }
+            inst = lo;
+        }
+        const Params &P = d.prm[inst];
+        const uint32_t c = cg - P.cell_base;
+        const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
+        const int32_t cx = (int32_t)(c % nx), cy = (int32_t)((c / nx) % ny), cz = (int32_t)(c / (nx * ny));
+        const int R = P.wide ? 2 : 1;
+        for (int oz = -R; oz <= R; ++oz) {
+            const int32_t z = cz + oz;
+            if (z < 0 || z >= (int32_t)nz) continue;
+            for (int oy = -R; oy <= R; ++oy) {
+                int32_t y = cy + oy;
+                if (y < 0 || y >= (int32_t)ny) {
+                    if (P.periodic != 1) continue;
+                    y = (y + (int32_t)ny) % (int32_t)ny;
+                }
+                for (int ox = -R; ox <= R; ++ox) {
+                    int32_t x = cx + ox;
+                    if (x < 0 || x >= (int32_t)nx) {
+                        if (P.periodic != 1 && P.periodic != 2) continue;
+                        x = (x + (int32_t)nx) % (int32_t)nx;
+                    }
+                    d.dirty[P.cell_base + (uint32_t)x + (uint32_t)y * nx + (nx * ny) * (uint32_t)z] = step;
+                    V.dirty_step = step;
+                }
+            }
+        }
+    }
+}
+
+// The exclusive scan over the block's threads of one value each, and their sum.
+template <int BLOCK>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t &total)
+{
+    __shared__ uint32_t warp_tot[BLOCK / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (unsigned)o) inc += y;
+    }
+    if (lane == 31) warp_tot[warp] = inc;
+    __syncthreads();
+    uint32_t off = 0, sum = 0;
+#pragma unroll
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        const uint32_t t = warp_tot[w];
+        if ((unsigned)w < warp) off += t;
+        sum += t;
+    }
+    __syncthreads();
+    total = sum;
+    return off + inc - v;
+}
+
+// The cell list of the positions in buffer A, by all blocks of the grid; false
+// after a timeout.  BLOCK: the threads of a block.
+template <int BLOCK>
+__device__ __noinline__ bool rebuild_grid(const Dev &d, int A, uint32_t *bar)
+{
+    const uint32_t first = blockIdx.x * BLOCK + threadIdx.x, stride = gridDim.x * BLOCK;
+    const uint32_t np = d.np_all, n = d.ncells_all + 1u;   // buckets, the last for the outside
+    if (first == 0) *d.alias_any = 0u;
+    for (uint32_t s = first; s < np; s += stride) atomicAdd(&d.cell_fill[d.cell[s]], 1u);
+    if (!grid_barrier(d, bar)) return false;
+    // the block's run of buckets: its sum, then after every block's the scan
+    const uint32_t per = (n + gridDim.x - 1u) / gridDim.x;
+    const uint32_t lo = min(n, blockIdx.x * per), hi = min(n, lo + per);
+    uint32_t sum = 0, total = 0;
+    for (uint32_t c = lo + threadIdx.x; c < hi; c += BLOCK) sum += __ldcg(&d.cell_fill[c]);
+    block_scan<BLOCK>(sum, total);
+    if (threadIdx.x == 0) d.scan_tiles[blockIdx.x] = total;
+    if (!grid_barrier(d, bar)) return false;
+    uint32_t run = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += BLOCK) run += __ldcg(&d.scan_tiles[b]);
+    block_scan<BLOCK>(run, total);
+    run = total;
+    for (uint32_t c0 = lo; c0 < hi; c0 += BLOCK) {
+        const uint32_t c = c0 + threadIdx.x;
+        const uint32_t v = c < hi ? __ldcg(&d.cell_fill[c]) : 0u;
+        const uint32_t at = run + block_scan<BLOCK>(v, total);
+        if (c < hi) d.cell_start[c] = at;
+        run += total;
+    }
+    if (first == 0) d.cell_start[n] = np;
+    if (!grid_barrier(d, bar)) return false;
+    // each particle takes a place of its cell's range; counters return to zero
+    for (uint32_t s = first; s < np; s += stride) {
+        const uint32_t c = d.cell[s];
+        const uint32_t k = atomicSub(&d.cell_fill[c], 1u) - 1u;
+        __stcg(&d.cellorder[d.cell_start[c] + k], s);
+    }
+    if (!grid_barrier(d, bar)) return false;
+    // the members of each cell by particle index (insertion sort)
+    for (uint32_t c = first; c < n; c += stride) {
+        const uint32_t beg = d.cell_start[c], end = d.cell_start[c + 1];
+        for (uint32_t i = beg + 1; i < end; ++i) {
+            const uint32_t s = __ldcg(&d.cellorder[i]);
+            const uint32_t key = d.uid[s];
+            uint32_t j = i;
+            while (j > beg) {
+                const uint32_t o = __ldcg(&d.cellorder[j - 1]);
+                if (d.uid[o] <= key) break;
+                __stcg(&d.cellorder[j], o);
+                --j;
+            }
+            __stcg(&d.cellorder[j], s);
+        }
+    }
+    if (!grid_barrier(d, bar)) return false;
+    // inverse of the new order and the float copy of the positions in list order
+    for (uint32_t k = first; k < np; k += stride) {
+        const uint32_t s = __ldcg(&d.cellorder[k]);
+        const Params &P = prm_of(d, s);
+        d.pos[s] = k;
+        const double4 x = d.xr[A][s];
+        d.xs[A][k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+        // a particle whose floored coordinates leave the grid sits outside
+        // its cell's box (saturated or aliased cell id): contact search must
+        // then not prune cells by geometry
+        if (cell_outside(P, x.x, x.y, x.z)) atomicOr(d.alias_any, 1u);
+    }
+    stamp_moves(d, first, stride);
+    if (first == 0) {
+        Verlet &V = *d.vs;
+        V.rebuilds += 1u;
+        if (__ldcg(&V.movers_overflow)) {
+            V.all_rebuild = 1u;
+            V.moved = 0.0f;
+        }
+    }
+    if (!grid_barrier(d, bar)) return false;
+    if (first == 0) {
+        // the flag and the movers, consumed
+        d.rebuild[REBUILD_NOW] = 0u;
+        d.vs->nmovers = 0u;
+        d.vs->movers_overflow = 0u;
+    }
+    return true;
+}
+
+// A launch whose blocks are all on the device together.
+template <class T>
+struct SameType {
+    using type = T;
+};
+template <class... Args>
+inline void launch_together(void (*kernel)(Args...), unsigned grid, unsigned block, cudaStream_t st,
+                            typename SameType<Args>::type... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+}  // namespace sphk
+
+#endif

@@ -111,6 +111,8 @@ __host__ __device__ inline ForceConsts force_consts(const Params &P)
     return c;
 }
 
+// Blocks that a rebuild's grid can have (8 an SM, with room).
+constexpr uint32_t SCAN_TILES = 4096;
 constexpr int VL_CAP = 32;              // candidates kept per particle
 constexpr uint8_t VL_NONE = 0xff;       // no usable list: sweep the stencil
 constexpr uint32_t MOVER_CAP = 1u << 16;
@@ -142,15 +144,12 @@ struct Verlet {
     uint32_t inc2_bits;     // float bits of the step's largest squared displacement
     uint32_t done_blocks;   // blocks of the step's force kernel that are through
     uint32_t came_apart;    // a position had left the grid when the last step ended
-    uint32_t pad;
+    uint32_t bar_rebuild, bar_small;   // grid_barrier's counters, one a kernel
 };
 
-// What the end of a step sets for the next one in a graph: the condition of
-// the cell-list node in front of it.
-struct NextStep {
-    cudaGraphConditionalHandle handle;
-    int gated;   // there is such a node
-};
+// Dev::rebuild: the cell list must be made before this step; before the next.
+// The end of a step turns the second into the first.
+constexpr int REBUILD_NOW = 0, REBUILD_NEXT = 1;
 
 // Wall state (src/datatypes.h:95-100), device resident.
 struct Walls {
@@ -229,7 +228,7 @@ struct Dev {
     uint32_t *cellorder;  // [np] cell-list position -> storage index
     uint32_t *pos;        // [np] storage index -> cell-list position
     uint32_t *cell_fill;  // [ncells + 1] scratch
-    uint32_t *scan_tiles; // scratch for the scan
+    uint32_t *scan_tiles; // [SCAN_TILES] scratch for the scan: a total for each block
     uint32_t *alias_any;  // some particle sits outside its cell's box (set by the rebuild)
     // Verlet lists
     uint32_t *vl;         // tiled, VL_CAP per particle: candidate storage indices, in visiting order
@@ -266,7 +265,7 @@ struct Dev {
     ulonglong2 *tp_dmc;
     // status
     uint32_t *status;
-    uint32_t *rebuild;          // cell list must be rebuilt before the next step
+    uint32_t *rebuild;          // [2] REBUILD_NOW, REBUILD_NEXT
     Params *prm;
 };
 

@@ -32,6 +32,7 @@
 
 #include "sphk_internal.cuh"
 #include "diff_step.cuh"
+#include "rebuild.cuh"
 
 namespace sphk {
 
@@ -664,7 +665,7 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
 }
 
 // The contact search of one particle s that is due (k_topo); sweep: its
-// candidate list cannot be used.
+// candidate list cannot be used; S: the epoch's clock.
 //
 // List mode: the list holds every candidate that can overlap while the epoch
 // lasts, each with the earliest moment it can (vl_when).  Candidates known to
@@ -686,7 +687,7 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
 // in visiting order: they are left in `va` and the lane's column of srow.
 template <bool VISC, bool BATCH, int TB>
 __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int tid, uint32_t *srow,
-                                            bool sweep, ViscAct &va)
+                                            bool sweep, float S, ViscAct &va)
 {
     const Params &P = prm_at<BATCH>(d, s);
     const uint32_t len = d.vl_len[s];
@@ -702,10 +703,9 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const uint32_t occ_in = d.cmask[s];
     const double4 xa = d.xr[A][s];
     uint32_t held = VISC ? 0u : d.vl_held[s];
-    if (!BATCH && d.vs->came_apart != 0u) return;
+    if (!BATCH && __ldcg(&d.vs->came_apart) != 0u) return;
     const double ra = xa.w;
     const double4 *__restrict__ xr = d.xr[A];
-    const float S = d.vs->moved;
     TopoSlots ts{occ_in, occ_in, 0u, 0ull, 0ull, 0, false, false};
     const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
     int32_t gp[3];
@@ -818,7 +818,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
             due = -1.0f;
         }
     } else {
-        const float4 *__restrict__ xs = d.xs[A];
+        const float4 *xs = d.xs[A];
         const uint32_t k = d.pos[s];
         const float4 xaf = xs[k];
         const float Lf0 = (float)P.L[0], Lf1 = (float)P.L[1];
@@ -843,7 +843,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 const uint32_t last = end - 1;
                 float4 c[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) c[j] = __ldg(&xs[min(base + (uint32_t)j, last)]);
+                for (int j = 0; j < 4; ++j) c[j] = __ldca(&xs[min(base + (uint32_t)j, last)]);
                 uint32_t near = 0, hit = 0;
                 float gj[4];
 #pragma unroll
@@ -867,7 +867,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                     const int j = __ffs(near) - 1;
                     near &= near - 1;
                     const uint32_t k2 = base + (uint32_t)j;
-                    const uint32_t t = __ldg(&d.cellorder[k2]);
+                    const uint32_t t = __ldca(&d.cellorder[k2]);
                     const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
                     float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
                     if (VISC) {
@@ -911,7 +911,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         // it leaves the visiting order of the others unchanged.  Used only
         // while the particle's own cell is inside the grid and every
         // particle sits inside its cell's box (alias_any clear).
-        const bool prune = gp_in && (*d.alias_any == 0u);
+        const bool prune = gp_in && (__ldcg(d.alias_any) == 0u);
         // squared distances to the cells one and two away on each axis
         float lo1[3], hi1[3], lo2[3], hi2[3];
         {
@@ -1096,7 +1096,7 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
             }
             const uint32_t bit = __fns(sel, 0, (int)rem + 1);
             s = base + 32u * selj + bit;
-            topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u, va);
+            topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u, S, va);
         }
         if constexpr (VISC) {
             __syncwarp();
@@ -1112,18 +1112,17 @@ struct ForceArgs {
     int write_outputs;  // store force/torque/acc/angacc/edp of this step
     int tape_step;      // differentiable step: tape row to record, or -1
     ForceConsts fc;     // single-scene contexts: the scene's constants
-    NextStep next;
 };
 
 // The epoch's clock and the decision for the next step: the lists hold every
 // pair that can overlap while 2 moved < skin; otherwise (a clock that is not a
 // number included) every particle sweeps and a new epoch starts.  One thread,
 // after everything else of the step's force kernel.
-__device__ void step_tail(const Dev &d, const NextStep &next)
+__device__ void step_tail(const Dev &d)
 {
     const Params &P = *d.prm;
     Verlet &V = *d.vs;
-    float moved = V.moved;
+    float moved = __ldcg(&V.moved);
     const float inc = __fmul_ru(__fsqrt_ru(__uint_as_float(atomicExch(&V.inc2_bits, 0u))), 1.00001f);
     if (inc != 0.0f) moved = __fadd_ru(moved, __fadd_ru(inc, 1e-15f));
     const bool restart = P.skin > 0.0 && !(2.02 * (double)moved < 0.999 * P.skin);
@@ -1131,17 +1130,26 @@ __device__ void step_tail(const Dev &d, const NextStep &next)
     V.moved = restart ? 0.0f : moved;
     // a sweep needs the cell list of its own step
     const bool want = atomicExch(&V.want_cells, 0u) != 0u;
-    if (restart || want) *d.rebuild = 1u;
+    const bool next = atomicExch(&d.rebuild[REBUILD_NEXT], 0u) != 0u;
+    d.rebuild[REBUILD_NOW] = (restart || want || next) ? 1u : 0u;
     V.came_apart = *(volatile const uint32_t *)d.status & ST_OUT_OF_GRID;
-    V.step += 1u;
-    if (next.gated)
-        cudaGraphSetConditional(next.handle, (restart || want || *(volatile uint32_t *)d.rebuild) ? 1u : 0u);
+    V.step = __ldcg(&V.step) + 1u;
+}
+// Large scenes end a step in a launch of their own: in the force kernel's
+// last block it took longer (the fence of every block behind its stores, 4 us
+// at 1M against 1.8 for the launch).
+__global__ void k_tail(const __grid_constant__ Dev d)
+{
+    if (threadIdx.x == 0) step_tail(d);
+}
+void launch_tail(const Dev &d, cudaStream_t st)
+{
+    k_tail<<<1, 32, 0, st>>>(d);
 }
 
-// The last block of a force kernel ends the step (a launch of its own took
-// 1.8 us and a gap, and another one in front of every step's cell list to
-// read its flag).  Called by all threads of every block.
-__device__ __forceinline__ void end_of_step(const Dev &d, const NextStep &next)
+// The last block of a kernel ends the step.  Called by all threads of every
+// block.
+__device__ __forceinline__ void end_of_step(const Dev &d)
 {
     __syncthreads();
     if (threadIdx.x != 0) return;
@@ -1149,7 +1157,7 @@ __device__ __forceinline__ void end_of_step(const Dev &d, const NextStep &next)
     if (atomicAdd(&d.vs->done_blocks, 1u) != gridDim.x - 1u) return;
     __threadfence();
     d.vs->done_blocks = 0u;
-    step_tail(d, next);
+    step_tail(d);
 }
 
 // Where the force kernels read a particle's own start-of-step rows: global
@@ -1414,7 +1422,7 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     const uint32_t c_old = R.cell();
     if (out) {
         // outside its cell's box: its own search sweeps, over a fresh list
-        *d.rebuild = 1u;
+        d.rebuild[REBUILD_NEXT] = 1u;
         d.due[s] = -1.0f;
     }
     if (c != c_old) {
@@ -1433,7 +1441,7 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
                       dz = (int)(q / (nx * ny)) - (int)(p / (nx * ny));
             hard = dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1;
         }
-        if (hard || P.eager) *d.rebuild = 1u;
+        if (hard || P.eager) d.rebuild[REBUILD_NEXT] = 1u;
         if (hard && P.skin > 0.0) {
             const uint32_t m = atomicAdd(&V.nmovers, 1u);
             if (m < MOVER_CAP) d.movers[m] = make_uint2(c_old, c);
@@ -1497,7 +1505,7 @@ k_force_diff(ForceArgs args)
     const Dev &d = args.d;
     const uint32_t np = d.np_all;
     const uint32_t s = blockIdx.x * FORCE_BLOCK + threadIdx.x;
-    if (s < np) {
+    if (s >= np) return;
 #ifndef SPHK_NO_PREFETCH
     // The state the integration reads comes after the contact work and
     // after stores the compiler may not move loads across, so each of its
@@ -1583,8 +1591,6 @@ k_force_diff(ForceArgs args)
         particle_tail<false, true>(d, P, s, A, args.write_outputs, xa, vel_a, angvel_a4, F,
                                    T, p, ev_dot, es_dot, R);
     }
-    }
-    end_of_step(d, args.next);
 }
 
 // Issues the bulk copies of tile t's rows into T, completing on `bar`.
@@ -1709,7 +1715,6 @@ k_force_tiles(ForceArgs args)
             stage_force_tile(d, A, tn, tiles[k], &full[k]);
         }
     }
-    end_of_step(d, args.next);
 }
 
 struct ContactArgs {
@@ -1896,10 +1901,13 @@ struct RegRows {
 // integration.  As three kernels each of their launches, ramps and drains
 // stood in that chain: whole runs of 500 grains 7.05 -> 6.45 ms (200 steps), of
 // 10,000 10.8 -> 8.4 ms (500 steps).
-constexpr int SMALL_BLOCK = 64, SMALL_BLOCKS_PER_SM = 8;
+//
+// Blocks of 128 threads: with 64, twice as many meet at the barriers of a cell
+// list (50,000 grains in a flow 37.4 us a step, 36.1 with 128).
+constexpr int SMALL_BLOCK = 128, SMALL_BLOCKS_PER_SM = 4;
 template <int MODEL, bool BATCH>
 __global__ void __launch_bounds__(SMALL_BLOCK, SMALL_BLOCKS_PER_SM)
-k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParams lp)
+k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParams lp, int own_list)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = SMALL_BLOCK / 32;
@@ -1912,17 +1920,27 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
     const int A = args.a;
     const uint32_t np = d.np_all, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
+    // the cell list first, where this step needs it (REBUILD_NOW does not
+    // change before the step ends)
+    if (own_list && *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u) {
+        uint32_t *bar = &d.vs->bar_small;
+        if (!rebuild_grid<SMALL_BLOCK>(d, A, bar) || !grid_barrier(d, bar)) return;
+    }
     if (s0 < np) {
         ViscAct va{0u, mk(0.0, 0.0, 0.0), 0.0};   // model 1's sums
         // ---- the search (k_topo) ----
         {
+            // past L1: the rebuild above may have changed them
             const Verlet &V = *d.vs;
+            const uint32_t step = __ldcg(&V.step);
+            const float S = __ldcg(&V.moved);
             bool need = false, sweep = false;
             if (s < np) {
-                sweep = V.all_rebuild != 0u || (V.dirty_step == V.step && d.dirty[d.cell[s]] == V.step);
-                need = sweep || V.moved > d.due[s];
+                sweep = __ldcg(&V.all_rebuild) != 0u ||
+                        (__ldcg(&V.dirty_step) == step && __ldcg(&d.dirty[d.cell[s]]) == step);
+                need = sweep || S > d.due[s];
             }
-            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, va);
+            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, S, va);
             __syncwarp();
             if constexpr (VISC) visc_warp(d, A, s, srow[w], 32u, visc[w], va);
         }
@@ -1972,7 +1990,19 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
             integrate(args.fc);
         }
     }
-    end_of_step(d, args.next);
+    end_of_step(d);
+}
+
+// Particles that k_small's resident threads hold.
+static uint32_t small_np()
+{
+    static int nsm = 0;
+    if (nsm == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return (uint32_t)nsm * SMALL_BLOCKS_PER_SM * SMALL_BLOCK;
 }
 
 // Whether a context's steps run as k_small: its chunks have a resident warp
@@ -1982,26 +2012,23 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
 // a flow, 200 steps: 11.1 ms against 10.1).
 bool small_step(const Dev &d, uint32_t np)
 {
-    if (d.shape != 0 || d.topo_span != 0) return false;
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return np <= (uint32_t)nsm * SMALL_BLOCKS_PER_SM * SMALL_BLOCK;
+    return d.shape == 0 && d.topo_span == 0 && np <= small_np();
 }
 
+// own_list: the kernel makes the cell list itself when it is due.
 void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  const NextStep &next, cudaStream_t st)
+                  bool own_list, cudaStream_t st)
 {
-    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp), next};
+    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp)};
     const LawParams lp = law_params(hp);
-    const unsigned grid = div_up(np, SMALL_BLOCK);
-    if (d.inst) k_small<2, true><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
-    else if (model == 1) k_small<1, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
-    else if (model == 3) k_small<3, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
-    else k_small<2, false><<<grid, SMALL_BLOCK, 0, st>>>(args, lp);
+    // more blocks than chunks need where the cells are many: they share the list
+    const unsigned most = (unsigned)(small_np() / SMALL_BLOCK);
+    const unsigned grid = std::min(most, std::max(div_up(np, SMALL_BLOCK), div_up(d.ncells_all, 32 * SMALL_BLOCK)));
+    const int own = own_list ? 1 : 0;
+    if (d.inst) launch_together(k_small<2, true>, grid, SMALL_BLOCK, st, args, lp, own);
+    else if (model == 1) launch_together(k_small<1, false>, grid, SMALL_BLOCK, st, args, lp, own);
+    else if (model == 3) launch_together(k_small<3, false>, grid, SMALL_BLOCK, st, args, lp, own);
+    else launch_together(k_small<2, false>, grid, SMALL_BLOCK, st, args, lp, own);
 }
 
 // A resident grid of k_contact: the SMs times the blocks of this
@@ -2088,9 +2115,9 @@ static void launch_force_tiles(const ForceArgs &args, uint32_t np, cudaStream_t 
 }
 
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  const NextStep &next, cudaStream_t st)
+                  cudaStream_t st)
 {
-    ForceArgs args{d, a, write_outputs, -1, force_consts(hp), next};
+    ForceArgs args{d, a, write_outputs, -1, force_consts(hp)};
     if (d.inst) {   // batched contexts: contact model 2 only
         launch_force_tiles<2, true>(args, np, st);
     } else if (d.mu_p) {   // the differentiable step
@@ -2105,10 +2132,9 @@ void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a,
 }
 
 // The differentiable step, recording tape row `tape_step`.
-void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, const NextStep &next,
-                       cudaStream_t st)
+void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStream_t st)
 {
-    ForceArgs args{d, a, 0, tape_step, ForceConsts{}, next};
+    ForceArgs args{d, a, 0, tape_step, ForceConsts{}};
     k_force_diff<<<div_up(np, FORCE_BLOCK), FORCE_BLOCK, 0, st>>>(args);
 }
 
