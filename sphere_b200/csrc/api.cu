@@ -15,7 +15,7 @@
 namespace sphk {
 void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st);
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  cudaStream_t st);
+                  bool slots, cudaStream_t st);
 void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st);
 bool small_step(const Dev &d, uint32_t np);
 void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
@@ -381,9 +381,12 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
         launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, own_list, st);
     } else {
         launch_topo(c->d, c->np_all, model == 1, a, st);
-        launch_contact(c->d, c->hp, c->np_all, model, a, st);
+        // the slot forces in the force kernel, unless the shapes of the split
+        // kernels were asked for
+        const bool slots = c->d.shape == 0;
+        if (!slots) launch_contact(c->d, c->hp, c->np_all, model, a, st);
         if ((rc = join_walls()) != SPH_OK) return rc;
-        launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, st);
+        launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, slots, st);
         launch_tail(c->d, st);
     }
     if (c->darcy_on && !branch) launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, st);
@@ -503,7 +506,7 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
     CK(cudaEventRecord(c->ev[3], st));
     launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, st);
     CK(cudaEventRecord(c->ev[4], st));
-    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, st);
+    launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, false, st);
     CK(cudaEventRecord(c->ev[5], st));
     launch_tail(c->d, st);
     launch_walls(c->d, c->np_all, c->hp.nw, st);

@@ -44,7 +44,7 @@ namespace sphk {
 #endif
 constexpr int FORCE_BLOCK = SPHK_FORCE_BLOCK;
 #ifndef SPHK_FORCE_MIN_BLOCKS
-#define SPHK_FORCE_MIN_BLOCKS 8
+#define SPHK_FORCE_MIN_BLOCKS 6
 #endif
 // The contact search and the contact forces are compiled in two block
 // shapes each, and a context picks one pair (Dev::shape, SPH_OPT_BLOCK_SHAPES;
@@ -1112,6 +1112,7 @@ struct ForceArgs {
     int write_outputs;  // store force/torque/acc/angacc/edp of this step
     int tape_step;      // differentiable step: tape row to record, or -1
     ForceConsts fc;     // single-scene contexts: the scene's constants
+    LawParams lp;
 };
 
 // The epoch's clock and the decision for the next step: the lists hold every
@@ -1178,16 +1179,15 @@ struct GlobalRows {
     __device__ uint8_t wtouch() const { return d.wtouch[s]; }
 };
 
-// Particles per tile of the tiled force kernel (one thread each), a multiple
-// of 32; the per-particle arrays it stages are allocated in whole tiles.
-#ifndef SPHK_FORCE_TILE
-#define SPHK_FORCE_TILE 128
-#endif
-constexpr uint32_t FT_TILE = SPHK_FORCE_TILE;
-static_assert(FT_TILE % 32 == 0 && ROW_PAD % FT_TILE == 0, "force tiles are whole warps of a padded array");
-// Resident blocks per SM: two stages of a tile are ~45.5 KB of shared memory.
+// The tiled force kernel: blocks of FORCE_WARPS warps, each with tiles of its
+// own, a chunk of 32 particles (one lane each); the per-particle arrays it
+// stages are allocated in whole tiles.
+constexpr uint32_t FT_TILE = 32;
+static_assert(ROW_PAD % FT_TILE == 0, "force tiles are whole chunks of a padded array");
+constexpr int FORCE_WARPS = 4;
+// Resident blocks per SM: two stages of a warp's tile are 11 KB of shared memory.
 #ifndef SPHK_FORCE_TILE_BLOCKS
-#define SPHK_FORCE_TILE_BLOCKS (512 / SPHK_FORCE_TILE)
+#define SPHK_FORCE_TILE_BLOCKS 4
 #endif
 
 // The start-of-step rows of FT_TILE consecutive particles, each array one
@@ -1451,49 +1451,102 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     if (err) atomicOr(d.status, err);
 }
 
-// Everything of one particle s after the contact search, outside the
-// differentiable step: its slot sums (k_contact's, or k_topo's for model 1)
-// and particle_tail.  f: the chunk flag of s (Dev::cflag[s / 32], read by
-// the caller ahead of the rows).
-// fc: the constants of s's scene.
-template <int MODEL, bool BATCH, class Rows>
-__device__ __forceinline__ void force_row(const ForceArgs &args, const ForceConsts &fc, uint32_t s,
-                                          const Rows &R, uint8_t f)
+// A particle's slot sums.
+struct SlotSums {
+    d3 F, T;
+    double p, ev, es;
+};
+
+// interact's slot loop (src/contactsearch.cuh:468-543) for particle s, whose
+// occupied slots are occ0: the sums of the laws' terms in slot order, the
+// slots' new history, and in occ the slots still held.  A slot whose partner
+// no longer overlaps is freed and its history zeroed, as in the reference.
+// xa, vel_a and angvel_a are its own rows.
+template <int MODEL, class PR>
+__device__ __forceinline__ void contact_slots(const Dev &d, int A, const PR &P, uint32_t s,
+                                              double4 xa, double4 vel_a, d3 angvel_a,
+                                              uint32_t occ0, uint32_t &occ, SlotSums &o)
 {
-    const Dev &d = args.d;
-    // A chunk k_contact visited (flag 2: a contact remains, 3: none does)
-    // has the slot sums of its particles in Dev::csum_*; its flag goes back
-    // to 1 or 0 for the next step's search.  A warp is one chunk, so the
-    // flag is the warp's.
-    bool visited = false;
-    if constexpr (MODEL != 1) {
-        visited = f >= 2;
-        if (visited) {
-            __syncwarp(__activemask());
-            if ((s & 31u) == 0) d.cflag[s >> 5] = (f == 2) ? 1 : 0;
+    const ulonglong2 dmw = d.dmc[s];
+    o = SlotSums{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
+    occ = occ0;
+    // the partner of the next slot, loaded a slot ahead
+    uint32_t i = (uint32_t)(__ffs(occ0) - 1);
+    uint32_t t = d.contacts[tile_at(s, i, NC)];
+    for (uint32_t m = occ0; m;) {
+        const size_t e = tile_at(s, i, NC);
+        const double4 xb = d.xr[A][t];
+        const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
+        const P3 dtp = d.delta_t[e];
+        const uint32_t bit = m & (0u - m), slot = i;
+        m &= m - 1u;
+        if (m) {
+            i = (uint32_t)(__ffs(m) - 1);
+            t = d.contacts[tile_at(s, i, NC)];
+        }
+        const double ra = xa.w, rb = xb.w;
+        const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)slot), P);
+        const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
+        const double xlen = flen(xab);
+        const double delta_n = xlen - (ra + rb);
+        if (delta_n < 0.0f) {
+            const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
+            const LawOut l = (MODEL == 2)
+                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0)
+                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0);
+            d.delta_t[e] = P3{l.dt4.x, l.dt4.y, l.dt4.z};
+            o.F = add(o.F, l.f);
+            o.T = add(o.T, l.t);
+            o.p += l.pr;
+            o.ev += l.ev;
+            if (l.es_set) o.es += l.es;
+        } else {
+            // separated: free the slot and zero its history
+            d.contacts[e] = d.np_all;
+            d.delta_t[e] = P3{0.0, 0.0, 0.0};
+            occ &= ~bit;
         }
     }
+    if (occ != occ0) {
+        d.cmask[s] = occ;
+        d.vl_held[s] = 0u;   // a listed candidate left its slot: the next
+        d.due[s] = -1.0f;    // search looks at the list
+    }
+}
+
+// Everything of one particle s after the contact search: its slot sums and
+// particle_tail.  The sums are k_topo's for model 1; with SLOTS they are made
+// here; otherwise they are k_contact's, in Dev::csum_* for the chunks it
+// visited.  f: the chunk flag of s (Dev::cflag[s / 32], read by the caller
+// ahead of the rows, the same for the warp); fc, lp: the constants of s's
+// scene; occ: with SLOTS, the slots still held.
+template <int MODEL, bool BATCH, bool SLOTS, class Rows>
+__device__ __forceinline__ void force_row(const ForceArgs &args, const ForceConsts &fc,
+                                          const LawParams &lp, uint32_t s, const Rows &R, uint8_t f,
+                                          uint32_t &occ)
+{
+    const Dev &d = args.d;
     const double4 xa = R.xr();
     const double4 vel_a = R.vel();
     const double4 angvel_a4 = R.angvel();
-    d3 F = mk(0.0, 0.0, 0.0), T = mk(0.0, 0.0, 0.0);
-    double es_dot = 0.0f, ev_dot = 0.0f, p = 0.0f;
-    if (MODEL == 1) {
+    SlotSums o{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
+    if constexpr (MODEL == 1) {
         const double4 c = d.c1acc[s];
-        F = mk(c.x, c.y, c.z);
-        p = c.w;
-    } else if (visited && d.cmask[s] != 0u) {
+        o.F = mk(c.x, c.y, c.z);
+        o.p = c.w;
+    } else if constexpr (SLOTS) {
+        if (f != 0) {
+            const uint32_t occ0 = d.cmask[s];
+            if (occ0) contact_slots<MODEL>(d, args.a, lp, s, xa, vel_a, xyz(angvel_a4), occ0, occ, o);
+        }
+    } else if (f >= 2 && d.cmask[s] != 0u) {
         // the sums of a particle that still holds a slot (with every slot
         // freed nothing was added: the sums are zero)
         const double4 cf = d.csum_f[s], ct = d.csum_t[s];
-        F = mk(cf.x, cf.y, cf.z);
-        p = cf.w;
-        T = mk(ct.x, ct.y, ct.z);
-        ev_dot = ct.w;
-        es_dot = d.csum_es[s];
+        o = SlotSums{mk(cf.x, cf.y, cf.z), mk(ct.x, ct.y, ct.z), cf.w, ct.w, d.csum_es[s]};
     }
-    particle_tail<BATCH, false>(d, fc, s, args.a, args.write_outputs, xa, vel_a, angvel_a4, F, T, p,
-                                ev_dot, es_dot, R);
+    particle_tail<BATCH, false>(d, fc, s, args.a, args.write_outputs, xa, vel_a, angvel_a4, o.F, o.T,
+                                o.p, o.ev, o.es, R);
 }
 
 // The differentiable step's force kernel: one thread per particle, rows
@@ -1593,6 +1646,20 @@ k_force_diff(ForceArgs args)
     }
 }
 
+// Asks for the slot rows of chunk t, if it may hold a contact, so that they
+// are in L2 when its turn comes: its slot tiles are contiguous, and the top
+// PF_SLOTS slots are the ones in use.  Only a whole chunk, so that no request
+// passes an array's end.
+__device__ __forceinline__ void prefetch_slots(const Dev &d, uint32_t t)
+{
+    const uint32_t b = t * FT_TILE;
+    if (b + FT_TILE > d.np_all || d.cflag[t] == 0) return;
+    bulk_prefetch_l2(d.cmask + b, 32 * sizeof(uint32_t));
+    bulk_prefetch_l2(d.dmc + b, 32 * sizeof(ulonglong2));
+    bulk_prefetch_l2(d.contacts + tile_at(b, NC - PF_SLOTS, NC), PF_SLOTS * 32 * sizeof(uint32_t));
+    bulk_prefetch_l2(d.delta_t + tile_at(b, NC - PF_SLOTS, NC), PF_SLOTS * 32 * sizeof(P3));
+}
+
 // Issues the bulk copies of tile t's rows into T, completing on `bar`.
 __device__ __forceinline__ void stage_force_tile(const Dev &d, int A, uint32_t t, ForceTile &T,
                                                  uint64_t *bar)
@@ -1637,82 +1704,104 @@ __device__ __forceinline__ void by_scene(Consts &slot, uint32_t &have, uint32_t 
     }
 }
 
-// Shared-memory stages of k_force_tiles: tiles a block has in flight.
+// Shared-memory stages of k_force_tiles: tiles a warp has in flight.
 #ifndef SPHK_FORCE_STAGES
 #define SPHK_FORCE_STAGES 2
 #endif
 constexpr uint32_t FT_STAGES = SPHK_FORCE_STAGES;
 
-// k_force_tiles: force_row over tiles of FT_TILE particles, a resident grid
-// of blocks (one thread per particle of a tile), each taking tiles
-// blockIdx.x, blockIdx.x + gridDim.x, ...  The particle's own rows (372 of
-// the 372 + 189 bytes a particle moves) arrive by bulk copies into a ring of
-// FT_STAGES shared-memory stages: while a block integrates one tile, the
-// copy engine fetches its next ones, so the bytes in flight do not depend on
-// how many threads are resident.  A stage is refilled, FT_STAGES tiles
-// ahead, once the block's barrier shows its tile consumed.  The
-// per-particle arrays are allocated in whole tiles (ROW_PAD), so every copy
-// is a whole tile.  A copy that has not landed after BULK_WAIT_NS stops the
-// block with ST_TIMEOUT, after the copies it issued have landed.
-template <int MODEL, bool BATCH>
-__global__ void __launch_bounds__(FT_TILE, SPHK_FORCE_TILE_BLOCKS)
-k_force_tiles(ForceArgs args)
+// k_force_tiles: force_row over tiles of 32 particles (SLOTS: with the slot
+// forces, which the graphs of a step use; profile mode and the second block
+// shapes run them as k_contact), a resident grid whose warps each take tiles
+// g, g + W, g + 2 W, ... of the W warps.  The particles' own rows (364 of the
+// 364 + 172 bytes a particle moves) arrive by bulk copies into a ring of
+// FT_STAGES shared-memory stages of the warp: while it integrates one tile,
+// the copy engine fetches its next ones, so the bytes in flight do not depend
+// on how many threads are resident.  A stage is refilled, FT_STAGES tiles
+// ahead, once the warp is past its tile.  The per-particle arrays are
+// allocated in whole tiles (ROW_PAD), so every copy is a whole tile.  A copy
+// that has not landed after BULK_WAIT_NS stops the warp with ST_TIMEOUT, after
+// the copies it issued have landed.
+//
+// The warps of a block wait for nothing of one another: with tiles of the
+// block a chunk with contacts held up the three beside it (64 jammed scenes
+// 113 us a step, 109 so; the 1M scenes the same).
+template <int MODEL, bool BATCH, bool SLOTS>
+__global__ void __launch_bounds__(32 * FORCE_WARPS, SPHK_FORCE_TILE_BLOCKS)
+k_force_tiles(const __grid_constant__ ForceArgs args)
 {
-    __shared__ ForceTile tiles[FT_STAGES];
-    __shared__ uint64_t full[FT_STAGES];
-    __shared__ ForceConsts scene[BATCH ? FT_TILE / 32 : 1];   // a batch's, one a warp
+    struct Scene {
+        ForceConsts fc;
+        LawParams lp;
+    };
+    __shared__ ForceTile tiles[FORCE_WARPS][FT_STAGES];
+    __shared__ uint64_t full[FORCE_WARPS][FT_STAGES];
+    __shared__ Scene scene[BATCH ? FORCE_WARPS : 1];   // a batch's, one a warp
+    constexpr uint32_t FULL = 0xffffffffu;
     uint32_t have = 0xffffffffu;
     const Dev &d = args.d;
     const uint32_t np = d.np_all;
     const uint32_t ntiles = (np + FT_TILE - 1) / FT_TILE;
-    const uint32_t tid = threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t first = blockIdx.x * FORCE_WARPS + w, stride = gridDim.x * FORCE_WARPS;
     const int A = args.a;
-    if (tid == 0) {
-        for (uint32_t k = 0; k < FT_STAGES; ++k) mbar_init(&full[k], 1);
+    if (lane == 0) {
+        for (uint32_t k = 0; k < FT_STAGES; ++k) mbar_init(&full[w][k], 1);
         mbar_init_fence();
-        // the block's first FT_STAGES tiles
+        // the warp's first FT_STAGES tiles
         for (uint32_t k = 0; k < FT_STAGES; ++k) {
-            const uint32_t tk = blockIdx.x + k * gridDim.x;
-            if (tk < ntiles) stage_force_tile(d, A, tk, tiles[k], &full[k]);
+            const uint32_t tk = first + k * stride;
+            if (tk >= ntiles) continue;
+            stage_force_tile(d, A, tk, tiles[w][k], &full[w][k]);
+            if (SLOTS) prefetch_slots(d, tk);
         }
     }
-    __syncthreads();
-    uint32_t t = blockIdx.x;
-    for (uint32_t it = 0; t < ntiles; t += gridDim.x, ++it) {
+    __syncwarp();
+    uint32_t t = first;
+    for (uint32_t it = 0; t < ntiles; t += stride, ++it) {
         const uint32_t k = it % FT_STAGES;
-        const uint32_t s = t * FT_TILE + tid;
+        const uint32_t s = t * FT_TILE + lane;
         // the chunk flag comes from global memory: asked for before the wait
-        const uint8_t f = (MODEL != 1 && s < np) ? d.cflag[s >> 5] : (uint8_t)0;
-        const bool ready = mbar_wait(&full[k], (it / FT_STAGES) & 1u, BULK_WAIT_NS);
-        if constexpr (BATCH) {
-            const uint32_t inst = s < np ? d.inst[s] : 0u;
-            by_scene(scene[tid >> 5], have, inst, ready && s < np,
-                     [&](ForceConsts &c, uint32_t i) { c = force_consts(d.prm[i]); },
-                     [&](const ForceConsts &c) {
-                         force_row<MODEL, true>(args, c, s, TileRows{tiles[k], tid}, f);
-                     });
-        } else if (ready && s < np) {
-            force_row<MODEL, false>(args, args.fc, s, TileRows{tiles[k], tid}, f);
-        }
-        if (__syncthreads_or(!ready)) {
-            if (tid == 0) {
+        const uint8_t f = MODEL != 1 ? d.cflag[t] : (uint8_t)0;
+        const bool ready = mbar_wait(&full[w][k], (it / FT_STAGES) & 1u, BULK_WAIT_NS);
+        if (!__all_sync(FULL, ready)) {
+            if (lane == 0) {
                 atomicOr(d.status, ST_TIMEOUT);
                 // this tile's copies and those issued for the next ones land
-                // before the block leaves
+                // before the warp leaves
                 for (uint32_t q = 0; q < FT_STAGES; ++q) {
                     const uint32_t iq = it + q;
-                    if (t + q * gridDim.x < ntiles)
-                        mbar_wait(&full[iq % FT_STAGES], (iq / FT_STAGES) & 1u, BULK_WAIT_NS);
+                    if (t + q * stride < ntiles)
+                        mbar_wait(&full[w][iq % FT_STAGES], (iq / FT_STAGES) & 1u, BULK_WAIT_NS);
                 }
             }
             return;
         }
-        // every thread is past its reads of stage k: it takes the tile
+        uint32_t occ = 0u;   // slots that the particle still holds
+        if constexpr (BATCH) {
+            const uint32_t inst = s < np ? d.inst[s] : 0u;
+            by_scene(scene[w], have, inst, s < np,
+                     [&](Scene &c, uint32_t i) { c = Scene{force_consts(d.prm[i]), law_params(d.prm[i])}; },
+                     [&](const Scene &c) {
+                         force_row<MODEL, true, SLOTS>(args, c.fc, c.lp, s, TileRows{tiles[w][k], lane}, f, occ);
+                     });
+        } else if (s < np) {
+            force_row<MODEL, false, SLOTS>(args, args.fc, args.lp, s, TileRows{tiles[w][k], lane}, f, occ);
+        }
+        // the chunk's flag for the next step's search: 1 while it holds a
+        // contact (k_contact left 2 for that, 3 for none)
+        if (MODEL != 1 && f >= (SLOTS ? 1 : 2)) {
+            const bool held = SLOTS ? __any_sync(FULL, occ != 0u) : f == 2;
+            if (lane == 0) d.cflag[t] = held ? 1 : 0;
+        }
+        // every lane is past its reads of stage k: it takes the tile
         // FT_STAGES rounds ahead
-        const uint32_t tn = t + FT_STAGES * gridDim.x;
-        if (tid == 0 && tn < ntiles) {
+        __syncwarp();
+        const uint32_t tn = t + FT_STAGES * stride;
+        if (lane == 0 && tn < ntiles) {
             fence_proxy_async_smem();
-            stage_force_tile(d, A, tn, tiles[k], &full[k]);
+            stage_force_tile(d, A, tn, tiles[w][k], &full[w][k]);
+            if (SLOTS) prefetch_slots(d, tn);
         }
     }
 }
@@ -1722,70 +1811,6 @@ struct ContactArgs {
     int a;               // read buffer (start of step)
     LawParams lp;        // single-scene contexts; a batch reads each scene's Params
 };
-
-// A particle's slot sums.
-struct SlotSums {
-    d3 F, T;
-    double p, ev, es;
-};
-
-// interact's slot loop (src/contactsearch.cuh:468-543) for particle s, whose
-// occupied slots are occ0: the sums of the laws' terms in slot order, the
-// slots' new history, and in occ the slots still held.  A slot whose partner
-// no longer overlaps is freed and its history zeroed, as in the reference.
-template <int MODEL, class PR>
-__device__ __forceinline__ void contact_slots(const Dev &d, int A, const PR &P, uint32_t s,
-                                              uint32_t occ0, uint32_t &occ, SlotSums &o)
-{
-    const double4 xa = d.xr[A][s];
-    const double4 vel_a = ld4(d.vel[A], s);
-    const d3 angvel_a = xyz(ld4(d.angvel[A], s));
-    const ulonglong2 dmw = d.dmc[s];
-    o = SlotSums{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
-    occ = occ0;
-    // the partner of the next slot, loaded a slot ahead
-    uint32_t i = (uint32_t)(__ffs(occ0) - 1);
-    uint32_t t = d.contacts[tile_at(s, i, NC)];
-    for (uint32_t m = occ0; m;) {
-        const size_t e = tile_at(s, i, NC);
-        const double4 xb = d.xr[A][t];
-        const double4 vel_b = ld4(d.vel[A], t), angvel_b = ld4(d.angvel[A], t);
-        const P3 dtp = d.delta_t[e];
-        const uint32_t bit = m & (0u - m), slot = i;
-        m &= m - 1u;
-        if (m) {
-            i = (uint32_t)(__ffs(m) - 1);
-            t = d.contacts[tile_at(s, i, NC)];
-        }
-        const double ra = xa.w, rb = xb.w;
-        const d3 dm = decode_dm(dm_get(dmw.x, dmw.y, (int)slot), P);
-        const d3 xab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
-        const double xlen = flen(xab);
-        const double delta_n = xlen - (ra + rb);
-        if (delta_n < 0.0f) {
-            const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
-            const LawOut l = (MODEL == 2)
-                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0)
-                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0);
-            d.delta_t[e] = P3{l.dt4.x, l.dt4.y, l.dt4.z};
-            o.F = add(o.F, l.f);
-            o.T = add(o.T, l.t);
-            o.p += l.pr;
-            o.ev += l.ev;
-            if (l.es_set) o.es += l.es;
-        } else {
-            // separated: free the slot and zero its history
-            d.contacts[e] = d.np_all;
-            d.delta_t[e] = P3{0.0, 0.0, 0.0};
-            occ &= ~bit;
-        }
-    }
-    if (occ != occ0) {
-        d.cmask[s] = occ;
-        d.vl_held[s] = 0u;   // a listed candidate left its slot: the next
-        d.due[s] = -1.0f;    // search looks at the list
-    }
-}
 
 // k_contact: the slot forces of contact models 2 and 3.
 //
@@ -1849,7 +1874,8 @@ k_contact(ContactArgs args)
             uint32_t occ = 0u;
             auto slots = [&](const auto &P) {
                 SlotSums o;
-                contact_slots<MODEL>(d, A, P, s, occ0, occ, o);
+                contact_slots<MODEL>(d, A, P, s, d.xr[A][s], ld4(d.vel[A], s), xyz(ld4(d.angvel[A], s)),
+                                     occ0, occ, o);
                 d.csum_f[s] = make_double4(o.F.x, o.F.y, o.F.z, o.p);
                 d.csum_t[s] = make_double4(o.T.x, o.T.y, o.T.z, o.ev);
                 d.csum_es[s] = o.es;
@@ -1907,7 +1933,7 @@ struct RegRows {
 constexpr int SMALL_BLOCK = 128, SMALL_BLOCKS_PER_SM = 4;
 template <int MODEL, bool BATCH>
 __global__ void __launch_bounds__(SMALL_BLOCK, SMALL_BLOCKS_PER_SM)
-k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParams lp, int own_list)
+k_small(const __grid_constant__ ForceArgs args, int own_list)
 {
     constexpr uint32_t FULL = 0xffffffffu;
     constexpr int WARPS = SMALL_BLOCK / 32;
@@ -1951,12 +1977,15 @@ k_small(const __grid_constant__ ForceArgs args, const __grid_constant__ LawParam
         if constexpr (!VISC) {
             if (d.cflag[chunk] != 0) {
                 const uint32_t occ0 = (s < np) ? d.cmask[s] : 0u;
-                auto slots = [&](const auto &P) { contact_slots<MODEL>(d, A, P, s, occ0, occ, o); };
+                auto slots = [&](const auto &P) {
+                    contact_slots<MODEL>(d, A, P, s, d.xr[A][s], ld4(d.vel[A], s),
+                                         xyz(ld4(d.angvel[A], s)), occ0, occ, o);
+                };
                 if constexpr (BATCH) {
                     by_scene(law[w], have, inst, occ0 != 0u,
                              [&](LawParams &l, uint32_t i) { l = law_params(d.prm[i]); }, slots);
                 } else if (occ0) {
-                    slots(lp);
+                    slots(args.lp);
                 }
                 const bool held = __any_sync(FULL, occ != 0u);
                 if (lane == 0) d.cflag[chunk] = held ? 1 : 0;
@@ -2019,16 +2048,15 @@ bool small_step(const Dev &d, uint32_t np)
 void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                   bool own_list, cudaStream_t st)
 {
-    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp)};
-    const LawParams lp = law_params(hp);
+    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp), law_params(hp)};
     // more blocks than chunks need where the cells are many: they share the list
     const unsigned most = (unsigned)(small_np() / SMALL_BLOCK);
     const unsigned grid = std::min(most, std::max(div_up(np, SMALL_BLOCK), div_up(d.ncells_all, 32 * SMALL_BLOCK)));
     const int own = own_list ? 1 : 0;
-    if (d.inst) launch_together(k_small<2, true>, grid, SMALL_BLOCK, st, args, lp, own);
-    else if (model == 1) launch_together(k_small<1, false>, grid, SMALL_BLOCK, st, args, lp, own);
-    else if (model == 3) launch_together(k_small<3, false>, grid, SMALL_BLOCK, st, args, lp, own);
-    else launch_together(k_small<2, false>, grid, SMALL_BLOCK, st, args, lp, own);
+    if (d.inst) launch_together(k_small<2, true>, grid, SMALL_BLOCK, st, args, own);
+    else if (model == 1) launch_together(k_small<1, false>, grid, SMALL_BLOCK, st, args, own);
+    else if (model == 3) launch_together(k_small<3, false>, grid, SMALL_BLOCK, st, args, own);
+    else launch_together(k_small<2, false>, grid, SMALL_BLOCK, st, args, own);
 }
 
 // A resident grid of k_contact: the SMs times the blocks of this
@@ -2098,7 +2126,7 @@ void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st)
 
 // Blocks of k_force_tiles: as many as fit on the device at once, no more
 // than there are tiles.
-template <int MODEL, bool BATCH>
+template <int MODEL, bool BATCH, bool SLOTS>
 static void launch_force_tiles(const ForceArgs &args, uint32_t np, cudaStream_t st)
 {
     static int per_sm = 0, nsm = 0;
@@ -2106,35 +2134,44 @@ static void launch_force_tiles(const ForceArgs &args, uint32_t np, cudaStream_t 
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_force_tiles<MODEL, BATCH>, FT_TILE, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_force_tiles<MODEL, BATCH, SLOTS>,
+                                                      32 * FORCE_WARPS, 0);
         if (per_sm < 1) per_sm = 1;
     }
-    const uint32_t ntiles = div_up(np, FT_TILE);
-    const uint32_t grid = std::min<uint32_t>(ntiles, (uint32_t)(per_sm * nsm));
-    if (grid) k_force_tiles<MODEL, BATCH><<<grid, FT_TILE, 0, st>>>(args);
+    const uint32_t grid = std::min<uint32_t>(div_up(np, FT_TILE * FORCE_WARPS), (uint32_t)(per_sm * nsm));
+    if (grid) k_force_tiles<MODEL, BATCH, SLOTS><<<grid, 32 * FORCE_WARPS, 0, st>>>(args);
 }
 
-void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  cudaStream_t st)
+template <bool SLOTS>
+static void launch_force_as(const ForceArgs &args, uint32_t np, int model, cudaStream_t st)
 {
-    ForceArgs args{d, a, write_outputs, -1, force_consts(hp)};
-    if (d.inst) {   // batched contexts: contact model 2 only
-        launch_force_tiles<2, true>(args, np, st);
-    } else if (d.mu_p) {   // the differentiable step
+    if (args.d.inst)   // batched contexts: contact model 2 only
+        launch_force_tiles<2, true, SLOTS>(args, np, st);
+    else if (model == 1)
+        launch_force_tiles<1, false, false>(args, np, st);
+    else if (model == 3)
+        launch_force_tiles<3, false, SLOTS>(args, np, st);
+    else
+        launch_force_tiles<2, false, SLOTS>(args, np, st);
+}
+
+// slots: the kernel does k_contact's work too.
+void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                  bool slots, cudaStream_t st)
+{
+    const ForceArgs args{d, a, write_outputs, -1, force_consts(hp), law_params(hp)};
+    if (d.mu_p)   // the differentiable step
         k_force_diff<<<div_up(np, FORCE_BLOCK), FORCE_BLOCK, 0, st>>>(args);
-    } else if (model == 1) {
-        launch_force_tiles<1, false>(args, np, st);
-    } else if (model == 3) {
-        launch_force_tiles<3, false>(args, np, st);
-    } else {
-        launch_force_tiles<2, false>(args, np, st);
-    }
+    else if (slots)
+        launch_force_as<true>(args, np, model, st);
+    else
+        launch_force_as<false>(args, np, model, st);
 }
 
 // The differentiable step, recording tape row `tape_step`.
 void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStream_t st)
 {
-    ForceArgs args{d, a, 0, tape_step, ForceConsts{}};
+    ForceArgs args{d, a, 0, tape_step, ForceConsts{}, LawParams{}};
     k_force_diff<<<div_up(np, FORCE_BLOCK), FORCE_BLOCK, 0, st>>>(args);
 }
 
