@@ -16,7 +16,8 @@ namespace sphk {
 void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st);
 void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                   bool slots, cudaStream_t st);
-void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st);
+void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                    cudaStream_t st);
 bool small_step(const Dev &d, uint32_t np);
 void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                   bool own_list, cudaStream_t st);
@@ -384,7 +385,7 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
         // the slot forces in the force kernel, unless the shapes of the split
         // kernels were asked for
         const bool slots = c->d.shape == 0;
-        if (!slots) launch_contact(c->d, c->hp, c->np_all, model, a, st);
+        if (!slots) launch_contact(c->d, c->hp, c->np_all, model, a, write_outputs, st);
         if ((rc = join_walls()) != SPH_OK) return rc;
         launch_force(c->d, c->hp, c->np_all, model, a, write_outputs, slots, st);
         launch_tail(c->d, st);
@@ -504,7 +505,7 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
     CK(cudaEventRecord(c->ev[2], st));
     launch_topo(c->d, c->np_all, c->hp.contactmodel == 1, a, st);
     CK(cudaEventRecord(c->ev[3], st));
-    launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, st);
+    launch_contact(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, st);
     CK(cudaEventRecord(c->ev[4], st));
     launch_force(c->d, c->hp, c->np_all, (int)c->hp.contactmodel, a, write_outputs, false, st);
     CK(cudaEventRecord(c->ev[5], st));

@@ -1,4 +1,5 @@
-// step.cu -- the per-particle DEM step of libsphk, in three launches.
+// step.cu -- the per-particle DEM step of libsphk: two launches, or one for
+// the whole step of a small scene.
 //
 // k_topo   contact detection into the persistent slots (topology,
 //          src/contactsearch.cuh:181-355): a lane's list decisions for one
@@ -8,17 +9,19 @@
 //          the 27-cell stencil are three adjacent runs of one array and a
 //          candidate costs one coalesced 16-byte load; the particle's own slot
 //          row is fetched only when an overlap is found.
-// k_contact the force laws of the occupied slots (interact's slot loop,
-//          src/contactsearch.cuh:468-543), one lane per directed contact;
-//          each particle's sums, in slot order, are left for k_force_tiles.
 // k_force_tiles  everything per particle after it (src/device.cu:829-1058):
-//          the slot sums, the walls (interact, contactsearch.cuh:578-663),
-//          the per-bond forces of bondsLinear (cohesion.cuh:8-233, computed
-//          by bonds.cu and gathered here in bond order), and the half-step
-//          leapfrog (integrate, integration.cuh:9-187).  A resident grid over
-//          tiles of 128 particles whose rows arrive by bulk copies.  The
-//          differentiable step runs k_force_diff instead of k_contact and
-//          k_force_tiles.
+//          the force laws of the occupied slots (interact's slot loop,
+//          src/contactsearch.cuh:468-543), a lane a particle, summed in slot
+//          order in registers; the walls (interact,
+//          contactsearch.cuh:578-663); the per-bond forces of bondsLinear
+//          (cohesion.cuh:8-233, computed by bonds.cu and gathered here in
+//          bond order); and the half-step leapfrog (integrate,
+//          integration.cuh:9-187).  Warps of a resident grid take tiles of 32
+//          particles whose rows arrive by bulk copies.
+// k_contact  the slot forces by themselves, where they are timed apart or a
+//          block size was asked for; k_force_tiles then reads its sums.
+// k_force_diff  the differentiable step's forces and integration.
+// k_small  the whole step in one cooperative launch.
 // Kinematics of step n are read from buffer A and step n+1 is written to
 // buffer B, so neighbours always see start-of-step values.
 //
@@ -184,13 +187,29 @@ __device__ __noinline__ WallSums wall_forces(const Params &P, const Walls &W, ui
     return r;
 }
 
-// contactLinear, src/contactmodels.cuh:283-493 (contact model 2).  Inlined
-// into k_contact, the one kernel that evaluates it.
+// Whether flen(a) > 0, without the square root.
+__device__ __forceinline__ bool has_length(d3 a) { return __double2float_rn(dot(a, a)) > 0.0f; }
+
+// The pressure term of a contact: only a call's last step stores it.
+__device__ __forceinline__ double contact_pressure(double f_n_length, double ra)
+{
+    return f_n_length / (4.0f * REF_PI * ra * ra);
+}
+
+// contactLinear, src/contactmodels.cuh:283-493 (contact model 2).
+//
+// What it does not evaluate: the pressure where it is not stored (want_p), the
+// lengths that are only compared with zero, and the capillary force f_c where
+// it is a zero vector, which changes no sum (they start at +0) and no length.
+// f_c is one where kappa is 0 and its other factors are finite: radii in
+// [0, 2^62) and centres apart (n is finite).  k_force_tiles on the jammed 1M
+// column 237 -> 218 us, on 64 jammed scenes 109 -> 103; k_small on 500
+// colliding grains 24 -> 21.
 template <class PR>
 __device__ __forceinline__ LawOut contact_linear(const PR &P, double4 vel_a, d3 angvel_a,
                                               double4 vel_b4, double4 angvel_b4, double ra,
                                               double rb, d3 x, double x_length, double delta,
-                                              double4 dt4)
+                                              double4 dt4, bool want_p)
 {
     LawOut o;
     o.es = 0.0;
@@ -198,41 +217,46 @@ __device__ __forceinline__ LawOut contact_linear(const PR &P, double4 vel_a, d3 
     const double dt = P.dt;
     const d3 vel_b = xyz(vel_b4), angvel_b = xyz(angvel_b4);
     const d3 dt0u = xyz(dt4);
+    const bool no_f_c = P.kappa == 0.0 && (uint32_t)__double2hiint(ra) < 0x43d00000u &&
+                        (uint32_t)__double2hiint(rb) < 0x43d00000u && __double2hiint(x_length) > 0;
     const d3 n = divs(x, x_length);
     const d3 vel_linear = mk(vel_a.x - vel_b.x, vel_a.y - vel_b.y, vel_a.z - vel_b.z);
     const d3 vel = add(add(vel_linear, smul(ra + delta / 2.0, cross(n, angvel_a))),
                        smul(rb + delta / 2.0, cross(n, angvel_b)));
     const double vel_n = -dot(vel_linear, n);
     const d3 vel_t = sub(vel, muls(n, dot(n, vel)));
-    const double vel_t_length = flen(vel_t);
     const d3 delta_t0 = sub(dt0u, muls(n, dot(n, dt0u)));
-    const double delta_t0_length = flen(delta_t0);
     d3 delta_t = mk(0.0, 0.0, 0.0);   // the reference leaves it unset when unused
     d3 f_n = smul(-P.k_n * delta - P.gamma_n * vel_n, n);
     o.ev = P.gamma_n * vel_n * vel_n;
     if (dot(f_n, n) < 0.0f) f_n = mk(0.0, 0.0, 0.0);
-    const double f_n_length = flen(f_n);
-    const d3 f_c = smul(-P.kappa * fsqrt_of(ra * rb), n);
+    d3 f_c = mk(0.0, 0.0, 0.0), f_nc = f_n;   // f_n - f_c
+    if (!no_f_c) {
+        f_c = smul(-P.kappa * fsqrt_of(ra * rb), n);
+        f_nc = sub(f_n, f_c);
+    }
     d3 f_t = mk(0.0, 0.0, 0.0);
-    if (delta_t0_length > 0.0 || vel_t_length > 0.0) {
+    if (has_length(delta_t0) || has_length(vel_t)) {
         delta_t = add(delta_t0, muls(vel_t, dt));
         const d3 f_t_elast = smul(-P.k_t, delta_t);
         const d3 f_t_visc = smul(-P.gamma_t, vel_t);
         f_t = add(f_t_elast, f_t_visc);
         const double f_t_length = flen(f_t);
-        const double f_t_limit = P.mu_s * flen(sub(f_n, f_c));
+        const double f_nc_length = flen(f_nc);
+        const double f_t_limit = P.mu_s * f_nc_length;
         if (f_t_length > f_t_limit) {
-            const d3 t = divs(f_t, flen(f_t));
+            const d3 t = divs(f_t, f_t_length);
             f_t = smul(f_t_limit, t);
             delta_t = smul(-1.0 / P.k_t,
-                           add(smul(P.mu_d * flen(sub(f_n, f_c)), t), smul(P.gamma_t, vel_t)));
+                           add(smul(P.mu_d * f_nc_length, t), smul(P.gamma_t, vel_t)));
             o.es = flen(muls(smul(flen(f_t), vel_t), dt)) / dt;
             o.es_set = true;
         }
     }
-    o.f = add(add(f_n, f_t), f_c);
+    o.f = add(f_n, f_t);
+    if (!no_f_c) o.f = add(o.f, f_c);
     o.t = cross(smul(-(ra + delta * 0.5), n), f_t);
-    o.pr = f_n_length / (4.0f * REF_PI * ra * ra);
+    o.pr = want_p ? contact_pressure(flen(f_n), ra) : 0.0;
     o.dt4 = make_double4(delta_t.x, delta_t.y, delta_t.z, 0.0f);
     return o;
 }
@@ -305,7 +329,7 @@ template <class PR>
 __device__ __forceinline__ LawOut contact_hertz(const PR &P, double4 vel_a, d3 angvel_a,
                                              double4 vel_b4, double4 angvel_b4, double ra,
                                              double rb, d3 x, double x_length, double delta,
-                                             double4 dt4)
+                                             double4 dt4, bool want_p)
 {
     LawOut o;
     o.es = 0.0;
@@ -359,7 +383,7 @@ __device__ __forceinline__ LawOut contact_hertz(const PR &P, double4 vel_a, d3 a
     }
     o.f = add(add(f_n, f_t), f_c);
     o.t = add(smul(-(ra + delta / 2.0), cross(n, f_t)), T_res);
-    o.pr = f_n_length / (4.0f * REF_PI * ra * ra);
+    o.pr = want_p ? contact_pressure(f_n_length, ra) : 0.0;
     o.dt4 = make_double4(delta_t.x, delta_t.y, delta_t.z, 0.0f);
     return o;
 }
@@ -1461,11 +1485,12 @@ struct SlotSums {
 // occupied slots are occ0: the sums of the laws' terms in slot order, the
 // slots' new history, and in occ the slots still held.  A slot whose partner
 // no longer overlaps is freed and its history zeroed, as in the reference.
-// xa, vel_a and angvel_a are its own rows.
+// xa, vel_a and angvel_a are its own rows; want_p: the pressure is stored.
 template <int MODEL, class PR>
 __device__ __forceinline__ void contact_slots(const Dev &d, int A, const PR &P, uint32_t s,
                                               double4 xa, double4 vel_a, d3 angvel_a,
-                                              uint32_t occ0, uint32_t &occ, SlotSums &o)
+                                              uint32_t occ0, uint32_t &occ, SlotSums &o,
+                                              bool want_p)
 {
     const ulonglong2 dmw = d.dmc[s];
     o = SlotSums{mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0.0, 0.0, 0.0};
@@ -1492,8 +1517,10 @@ __device__ __forceinline__ void contact_slots(const Dev &d, int A, const PR &P, 
         if (delta_n < 0.0f) {
             const double4 dt0 = make_double4(dtp.x, dtp.y, dtp.z, 0.0);
             const LawOut l = (MODEL == 2)
-                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0)
-                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0);
+                ? contact_linear(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0,
+                                 want_p)
+                : contact_hertz(P, vel_a, angvel_a, vel_b, angvel_b, ra, rb, xab, xlen, delta_n, dt0,
+                                 want_p);
             d.delta_t[e] = P3{l.dt4.x, l.dt4.y, l.dt4.z};
             o.F = add(o.F, l.f);
             o.T = add(o.T, l.t);
@@ -1537,7 +1564,9 @@ __device__ __forceinline__ void force_row(const ForceArgs &args, const ForceCons
     } else if constexpr (SLOTS) {
         if (f != 0) {
             const uint32_t occ0 = d.cmask[s];
-            if (occ0) contact_slots<MODEL>(d, args.a, lp, s, xa, vel_a, xyz(angvel_a4), occ0, occ, o);
+            if (occ0)
+                contact_slots<MODEL>(d, args.a, lp, s, xa, vel_a, xyz(angvel_a4), occ0, occ, o,
+                                     args.write_outputs != 0);
         }
     } else if (f >= 2 && d.cmask[s] != 0u) {
         // the sums of a particle that still holds a slot (with every slot
@@ -1809,6 +1838,7 @@ k_force_tiles(const __grid_constant__ ForceArgs args)
 struct ContactArgs {
     Dev d;
     int a;               // read buffer (start of step)
+    int write_outputs;   // the pressure is read after this step
     LawParams lp;        // single-scene contexts; a batch reads each scene's Params
 };
 
@@ -1875,7 +1905,7 @@ k_contact(ContactArgs args)
             auto slots = [&](const auto &P) {
                 SlotSums o;
                 contact_slots<MODEL>(d, A, P, s, d.xr[A][s], ld4(d.vel[A], s), xyz(ld4(d.angvel[A], s)),
-                                     occ0, occ, o);
+                                     occ0, occ, o, args.write_outputs != 0);
                 d.csum_f[s] = make_double4(o.F.x, o.F.y, o.F.z, o.p);
                 d.csum_t[s] = make_double4(o.T.x, o.T.y, o.T.z, o.ev);
                 d.csum_es[s] = o.es;
@@ -1979,7 +2009,8 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
                 const uint32_t occ0 = (s < np) ? d.cmask[s] : 0u;
                 auto slots = [&](const auto &P) {
                     contact_slots<MODEL>(d, A, P, s, d.xr[A][s], ld4(d.vel[A], s),
-                                         xyz(ld4(d.angvel[A], s)), occ0, occ, o);
+                                         xyz(ld4(d.angvel[A], s)), occ0, occ, o,
+                                         args.write_outputs != 0);
                 };
                 if constexpr (BATCH) {
                     by_scene(law[w], have, inst, occ0 != 0u,
@@ -2037,8 +2068,10 @@ static uint32_t small_np()
 // Whether a context's steps run as k_small: its chunks have a resident warp
 // each (75,776 particles on 148 SMs), and no shape or span of the split
 // kernels was asked for.  Above, the split kernels balance the work over the
-// device and stream the integration; below, they were slower (50,000 grains in
-// a flow, 200 steps: 11.1 ms against 10.1).
+// device and stream the integration.  Microseconds a step, one kernel against
+// split, on a B200: in a flow 24.7 / 29.0 at 1,000 grains, 32.6 / 38.3 at
+// 10,000, 37.8 / 45.0 at 50,000, 44.8 / 53.3 at 75,000; in a jammed packing
+// 20.1 / 20.9 at 1,000, 23.3 / 24.7 at 29,791, 28.5 / 29.0 at 74,088.
 bool small_step(const Dev &d, uint32_t np)
 {
     return d.shape == 0 && d.topo_span == 0 && np <= small_np();
@@ -2178,10 +2211,11 @@ void launch_force_tape(const Dev &d, uint32_t np, int a, int tape_step, cudaStre
 // The slot forces of contact models 2 and 3; model 1 has no slots (k_topo
 // sums its forces) and the differentiable step evaluates its own law in
 // k_force_diff, recording the tape.
-void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, cudaStream_t st)
+void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                    cudaStream_t st)
 {
     if (model == 1 || d.mu_p) return;
-    ContactArgs args{d, a, law_params(hp)};
+    ContactArgs args{d, a, write_outputs, law_params(hp)};
     if (d.shape) launch_contact_as<contact_block(1)>(args, np, model, st);
     else launch_contact_as<contact_block(0)>(args, np, model, st);
 }
