@@ -7,7 +7,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import OUTPUT_FIELDS, STATE_FIELDS, mismatches, run_oracle
+from helpers import BOND_FIELDS, OUTPUT_FIELDS, STATE_FIELDS, mismatches, run_oracle
 from sphere_b200 import scenes, sphk
 from sphere_b200.sphk import Simulation
 from sphere_b200.spherebin import Spherebin
@@ -128,3 +128,50 @@ def test_linear_law_leaves_out_only_what_changes_nothing(oracle_libs, kappa, spe
             rc, want, _ = run_oracle(oracle_libs["orc"], sb, done)
             assert rc == 0
             assert mismatches(sim.download(), want, fields) == [], done
+
+
+# grains on the vertices of the grid, a few units in the last place and 2^-20
+# of a cell to either side: the cell of a position beside a boundary
+@pytest.mark.parametrize("span", [None, 1], ids=["one_kernel", "split"])
+@pytest.mark.parametrize("num, L, origo", [((7, 11, 13), (0.1, 0.2, 0.3), (0.0, 0.0, 0.0)),
+                                           ((9, 5, 6), (0.07, 0.011, 1.3), (0.013, 0.001, 0.1)),
+                                           ((4, 4, 8), (1.0, 1.0, 2.0), (0.0, 0.0, 0.0))])
+def test_cells_of_positions_at_cell_boundaries(oracle_libs, num, L, origo, span):
+    rng = np.random.default_rng(num[0])
+    k = np.stack(np.meshgrid(*(np.arange(1, m) for m in num), indexing="ij"), -1).reshape(-1, 3)
+    cell = np.array(L) / np.array(num)
+    x = np.array(origo) + k * cell
+    side = rng.integers(-3, 4, x.shape)
+    x = x + side * np.spacing(np.abs(x))
+    far = rng.random(x.shape) < 0.3
+    x = np.where(far, x + side * 2.0 ** -21 * cell, x)
+    x = x[np.all(x < np.array(L) - 1e-4, axis=1)]   # clear of the default walls at L
+    sb = scenes.collision(n=len(x), seed=1, vmax=0.0, wmax=0.0, g=(0.0, 0.0, 0.0))
+    sb.x, sb.radius = x, np.full(len(x), 1e-5)
+    sb.origo, sb.L, sb.num = np.array(origo), np.array(L), np.array(num, dtype=np.uint32)
+    rc, want, orun = run_oracle(oracle_libs["orc"], sb, 5)
+    with Simulation(config_from_spherebin(sb), topo_span=span) as sim:
+        sim.upload(state_from_spherebin(sb))
+        sim.step(5)
+        sim.sync()
+        got = sim.download()
+        cell_sorted, perm, _, _ = sim.cells()
+    assert rc == 0 and mismatches(got, want, STATE_FIELDS + OUTPUT_FIELDS) == []
+    assert np.array_equal(perm, orun.perm) and np.array_equal(cell_sorted, orun.cell_sorted)
+
+
+# the bonds' screens: viscous terms that are there or not, strengths that some
+# bonds, all and none reach, and strengths outside the screen's range
+@pytest.mark.parametrize("gamma_n, gamma_t", [(0.0, 0.0), (3.0, 0.0), (0.0, 2.0), (3.0, 2.0), (-0.0, -0.0)])
+@pytest.mark.parametrize("sigma_b, tau_b", [(3e-3, 3e-3), (1.0, 1e-3), (1e-130, 1e-130), (1e130, 1e130),
+                                            (np.inf, np.inf), (-1.0, 1.0)])
+def test_bond_breaking_and_viscosity(oracle_libs, gamma_n, gamma_t, sigma_b, tau_b):
+    sb = scenes.tension(nx=7, ny=4, nz=5, seed=3, sigma_b=sigma_b, tau_b=tau_b)
+    sb.gamma_n, sb.gamma_t = gamma_n, gamma_t
+    rc, want, _ = run_oracle(oracle_libs["orc"], sb, 120)
+    assert rc == 0
+    with Simulation(config_from_spherebin(sb)) as sim:
+        sim.upload(state_from_spherebin(sb))
+        sim.step(120)
+        sim.sync()
+        assert mismatches(sim.download(), want, STATE_FIELDS + OUTPUT_FIELDS + BOND_FIELDS) == []
