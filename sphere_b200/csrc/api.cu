@@ -580,6 +580,7 @@ void fill_params(const sph_config *cfg, Params &P)
         P.origo[k] = cfg->origo[k];
         P.L[k] = cfg->L[k];
         P.cellsize[k] = cfg->L[k] / (double)cfg->num[k];
+        P.rcell[k] = cell_rcp(P.cellsize[k]);
         P.g[k] = cfg->g[k];
         ext = std::fmax(ext, std::fmax(std::fabs(cfg->origo[k]), std::fabs(cfg->L[k])));
     }

@@ -1248,6 +1248,16 @@ struct TileRows {
     __device__ uint8_t wtouch() const { return T.wtouch[r]; }
 };
 
+// Whether every component is a zero; whether v is a positive normal number.
+__device__ __forceinline__ bool is_zero(d3 a)
+{
+    return ((__double_as_longlong(a.x) | __double_as_longlong(a.y) | __double_as_longlong(a.z)) << 1) == 0;
+}
+__device__ __forceinline__ bool positive(double v)
+{
+    return (uint32_t)__double2hiint(v) - 0x00100000u < 0x7fe00000u;
+}
+
 // MODEL: the contact model (1, 2 or 3), a template argument so that each
 // model's kernel carries only its own force law.
 // DIFF: the differentiable step (contact model 2 in exact FP64 with
@@ -1347,17 +1357,21 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     // ---- integrate, src/integration.cuh:9-187 -------------------------------
     // The rotation and the translation are independent; each is finished and
     // stored before the other starts, so fewer values are live at once.
-    // Every expression keeps the reference's operands and order.
+    // Every expression keeps the reference's operands and order; a zero over
+    // a positive number is that zero, which a warp of particles without a
+    // contact finds without dividing.
     const double radius = xa.w;
     const double m = 4.0 / 3.0 * REF_PI * radius * radius * radius * P.rho;
     const bool fixed = R.fixed() != 0;   // fixvel > 0
     {
         P3 angpos = R.angpos(), angvel0 = R.angvel0();
-        double4 angacc;
-        angacc.x = T.x * 1.0 / (2.0 / 5.0 * m * radius * radius);
-        angacc.y = T.y * 1.0 / (2.0 / 5.0 * m * radius * radius);
-        angacc.z = T.z * 1.0 / (2.0 / 5.0 * m * radius * radius);
-        angacc.w = 0.0;
+        const double I = 2.0 / 5.0 * m * radius * radius;
+        double4 angacc = make_double4(T.x, T.y, T.z, 0.0);
+        if (!(is_zero(T) && positive(I))) {
+            angacc.x = T.x * 1.0 / I;
+            angacc.y = T.y * 1.0 / I;
+            angacc.z = T.z * 1.0 / I;
+        }
         if (fixed) angacc = make_double4(0.0f, 0.0f, 0.0f, 0.0f);
         angvel0.x += angacc.x * dt;
         angvel0.y += angacc.y * dt;
@@ -1379,11 +1393,12 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     }
     double4 x = xa, vel = vel_a;
     P3 vel0 = R.vel0();
-    double4 acc;
-    acc.x = F.x / m;
-    acc.y = F.y / m;
-    acc.z = F.z / m;
-    acc.w = 0.0;
+    double4 acc = make_double4(F.x, F.y, F.z, 0.0);
+    if (!(is_zero(F) && positive(m))) {
+        acc.x = F.x / m;
+        acc.y = F.y / m;
+        acc.z = F.z / m;
+    }
     acc.x += P.g[0];
     acc.y += P.g[1];
     acc.z += P.g[2];
@@ -1440,9 +1455,9 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     // a position that is not finite (NaN forces, contact model 3) is
     // outside the grid whatever its float-to-integer conversion gives
     uint32_t c;
-    if (!grid_cell(P, x.x, x.y, x.z, c)) { err |= ST_OUT_OF_GRID; c = d.ncells_all; }
+    bool out;
+    if (!cell_at(P, x.x, x.y, x.z, c, out)) { err |= ST_OUT_OF_GRID; c = d.ncells_all; }
     else c += P.cell_base;
-    const bool out = cell_outside(P, x.x, x.y, x.z);
     const uint32_t c_old = R.cell();
     if (out) {
         // outside its cell's box: its own search sweeps, over a fresh list
