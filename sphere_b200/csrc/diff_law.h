@@ -112,6 +112,14 @@ DL_HD void pair_fwd(const Law &P, const PairIn &in, PairOut &out)
     out.dtn = dtn;
 }
 
+// The cohesive force per unit normal, -kappa sqrt(ra rb), without the square
+// root where kappa is 0 and the root is a number.
+DL_HD double cohesion(double kappa, double ra, double rb)
+{
+    const double rr = ra * rb;
+    return (kappa == 0.0 && rr >= 0.0 && rr < 1e300) ? -kappa : -kappa * sqrt(rr);
+}
+
 // Reverse of pair_fwd: from the adjoints of F, T and dtn, the adjoints of
 // the inputs (stored into ib) and of the parameters (added to pb).
 DL_HD void pair_rev(const Law &P, const PairIn &in, V3 Fb, V3 Tb, V3 dtnb, PairBar &ib,
@@ -128,41 +136,29 @@ DL_HD void pair_rev(const Law &P, const PairIn &in, V3 Fb, V3 Tb, V3 dtnb, PairB
     const double vn = -dot(vl, n);
     const double s1 = dot(n, vel);
     const V3 vt = vel - s1 * n;
-    const double Lt = len(vt);
     const double s0 = dot(n, in.d0u);
     const V3 d0 = in.d0u - s0 * n;
-    const double L0 = len(d0);
     const double sfn = -P.kn * delta - P.gn * vn;
     V3 fn = sfn * n;
     const bool clip = dot(fn, n) < 0.0;
     if (clip) fn = v3(0.0, 0.0, 0.0);
-    const double cfc = -P.kappa * sqrt(in.ra * in.rb);
+    const double cfc = cohesion(P.kappa, in.ra, in.rb);
     const V3 fc = cfc * n;
     // The forward skips the tangential law when both d0 and vt vanish; there
     // the sticking branch gives the same values (zero force, zero
     // displacement) and its derivative is the true one, so the reverse always
     // takes the law.
-    (void)L0;
-    (void)Lt;
-    const bool active = true;
-    V3 ft = v3(0.0, 0.0, 0.0), dtn1 = v3(0.0, 0.0, 0.0), ft1 = v3(0.0, 0.0, 0.0);
-    V3 t = v3(0.0, 0.0, 0.0), g = v3(0.0, 0.0, 0.0);
-    double Lft = 0.0, Lg = 0.0, lim = 0.0;
-    bool slip = false;
-    if (active) {
-        dtn1 = d0 + P.dt * vt;
-        ft1 = -P.kt * dtn1 - P.gt * vt;
-        Lft = len(ft1);
-        g = fn - fc;
-        Lg = len(g);
-        lim = P.mu * Lg;
-        slip = Lft > lim;
-        if (slip) {
-            t = ft1 / Lft;
-            ft = lim * t;
-        } else {
-            ft = ft1;
-        }
+    const V3 dtn1 = d0 + P.dt * vt;
+    const V3 ft1 = -P.kt * dtn1 - P.gt * vt;
+    const double Lft = len(ft1);
+    const V3 g = fn - fc;
+    const double Lg = len(g);
+    const double lim = P.mu * Lg;
+    const bool slip = Lft > lim;
+    V3 ft = ft1, t = v3(0.0, 0.0, 0.0);
+    if (slip) {
+        t = ft1 / Lft;
+        ft = lim * t;
     }
     const double hT = -(in.ra + delta * 0.5);
     const V3 u = hT * n;
@@ -179,40 +175,35 @@ DL_HD void pair_rev(const Law &P, const PairIn &in, V3 Fb, V3 Tb, V3 dtnb, PairB
     fnb = Fb;
     ftb += Fb;
     nb += cfc * Fb;
-    if (active) {
-        V3 ft1b, dtn1b = v3(0.0, 0.0, 0.0);
-        double Lgb = 0.0;
-        if (slip) {
-            const V3 q = P.mu * Lg * t + P.gt * vt;
-            const V3 qb = (-1.0 / P.kt) * dtnb;
-            pb.kt += dot(dtnb, q) / (P.kt * P.kt);
-            pb.mu += Lg * dot(qb, t);
-            Lgb += P.mu * dot(qb, t);
-            V3 tb = (P.mu * Lg) * qb;
-            vtb += P.gt * qb;
-            const double limb = dot(ftb, t);
-            tb += lim * ftb;
-            ft1b = (tb - dot(t, tb) * t) / Lft;
-            pb.mu += Lg * limb;
-            Lgb += P.mu * limb;
-        } else {
-            ft1b = ftb;
-            dtn1b = dtnb;
-        }
-        // Lg = |fn - fc|
+    V3 ft1b = ftb, dtn1b = dtnb;
+    if (slip) {
+        const V3 q = P.mu * Lg * t + P.gt * vt;
+        const V3 qb = (-1.0 / P.kt) * dtnb;
+        pb.kt += dot(dtnb, q) / (P.kt * P.kt);
+        pb.mu += Lg * dot(qb, t);
+        double Lgb = P.mu * dot(qb, t);
+        V3 tb = (P.mu * Lg) * qb;
+        vtb += P.gt * qb;
+        const double limb = dot(ftb, t);
+        tb += lim * ftb;
+        ft1b = (tb - dot(t, tb) * t) / Lft;
+        pb.mu += Lg * limb;
+        Lgb += P.mu * limb;
+        dtn1b = v3(0.0, 0.0, 0.0);
+        // Lg = |fn - fc|; in the sticking branch nothing depends on it
         if (Lg > 0.0) {
             const V3 gb = (Lgb / Lg) * g;
             fnb += gb;
             nb += cfc * (-gb);
         }
-        // ft1 = -kt dtn1 - gt vt
-        pb.kt += -dot(ft1b, dtn1);
-        dtn1b += -P.kt * ft1b;
-        vtb += -P.gt * ft1b;
-        // dtn1 = d0 + dt vt
-        d0b = dtn1b;
-        vtb += P.dt * dtn1b;
     }
+    // ft1 = -kt dtn1 - gt vt
+    pb.kt += -dot(ft1b, dtn1);
+    dtn1b += -P.kt * ft1b;
+    vtb += -P.gt * ft1b;
+    // dtn1 = d0 + dt vt
+    d0b = dtn1b;
+    vtb += P.dt * dtn1b;
     double vnb = 0.0;
     if (!clip) {
         const double sfnb = dot(fnb, n);
