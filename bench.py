@@ -350,14 +350,14 @@ def gpu_arm(args, rank, world, local):
     b_step, b_whole, b_tight = algorithmic_bytes(cfg.np, cfg.ncells, C, cfg.nb0)
     peak, peak_kind = measured_peak_hbm()
     achieved = b_step / (step_ms * 1e-3) / 1e9
-    # per step: the rebuild gate, k_bonds (with bonds), k_topo, k_contact
-    # (contact models 2 and 3), k_force_tiles, k_tail, and with dynamic walls
-    # k_walls on its graph branch; the 7 cell-list kernels only in steps
-    # whose cell list changed (a conditional graph node)
+    # Per step of a graph: k_rebuild (which leaves at once unless the cell list
+    # is due), k_topo, k_force_tiles and k_tail, or up to 512 particles an SM
+    # k_small alone; with bonds k_bonds, with dynamic walls k_walls on its
+    # graph branch.
     rebuilt = stats["cell_rebuilds"] - rebuilds0
-    per_step = (4 + (1 if cfg.nb0 else 0) + (1 if cfg.contactmodel in (2, 3) else 0)
-                + (1 if cfg.nw else 0))
-    launches = args.steps * per_step + 7 * rebuilt
+    small = cfg.np <= 512 * torch.cuda.get_device_properties(local).multi_processor_count
+    per_step = (1 if small else 4) + (1 if cfg.nb0 else 0) + (1 if cfg.nw else 0)
+    launches = args.steps * per_step
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
@@ -1127,11 +1127,12 @@ def reference_arm(args, rank, world):
 
 def profile_workload(args):
     """One workload in profile mode only (every kernel a direct launch, one
-    step after another with events between the phases), for ncu: a profiler
-    cannot follow the kernels of the step graphs.  `warmup` steps, then
-    `steps` steps; prints the phase times per step.  Per step the launches
-    are the cell-list kernels, k_bonds (with bonds), k_topo, k_contact (models
-    2 and 3), k_force_tiles and the wall kernel, in that order."""
+    step after another with events between the phases), for ncu.  `warmup`
+    steps, then `steps` steps; prints the phase times per step.  Per step the
+    launches are k_rebuild, k_bonds (with bonds), k_topo, k_contact (models 2
+    and 3), k_force_tiles, k_tail and k_walls (with dynamic walls), in that
+    order; the step graphs run the slot forces in k_force_tiles instead, and
+    small scenes in k_small."""
     import torch
     from sphere_b200 import scenes
     from sphere_b200.sphk import Simulation
