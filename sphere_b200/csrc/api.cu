@@ -1242,7 +1242,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         q.cell_start = at(o_start); q.cell_fill = at(o_fill); q.scan_tiles = at(o_scan);
         q.status = at(o_word); q.alias_any = at(o_word) + 1; q.rebuild = at(o_word) + 2;
         q.vs = reinterpret_cast<Verlet *>(tmp + o_vs);
-        CK(cudaMemsetAsync(&q.rebuild[REBUILD_NOW], 1, 4, c->stream));
+        launch_epoch_reset(q, c->stream);
         launch_cell_init(q, np, c->a ^ 1, c->stream);
         launch_rebuild(q, np, nc, c->a ^ 1, c->stream);
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);

@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(REBUILD_BLOCK, REBUILD_BLOCKS_PER_SM)
 k_rebuild(const __grid_constant__ Dev d, int A)
 {
     if (*(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] == 0u) return;
-    rebuild_grid<REBUILD_BLOCK>(d, A, &d.vs->bar_rebuild);
+    GridBar bar{&d.vs->bar_rebuild, 0};
+    rebuild_grid<REBUILD_BLOCK>(d, A, bar);
 }
 
 void launch_cell_init(const Dev &d, uint32_t np, int a, cudaStream_t st)

@@ -13,24 +13,31 @@
 #ifndef SPHK_REBUILD_CUH_
 #define SPHK_REBUILD_CUH_
 
+#include "barrier_count.h"
 #include "sphk_internal.cuh"
 
 namespace sphk {
 
+// A barrier's counter and the end of this block's last round (thread 0's).
+struct GridBar {
+    unsigned long long *count;
+    uint64_t end;
+};
+
 // Waits until every block of the grid is here; false when that did not happen
-// within BULK_WAIT_NS (ST_TIMEOUT: the caller leaves).  bar: a counter that
-// only this kernel's launches use, a multiple of the grid's blocks before.
-__device__ __forceinline__ bool grid_barrier(const Dev &d, uint32_t *bar)
+// within BULK_WAIT_NS (ST_TIMEOUT: the caller leaves, and no list is made before
+// an upload has cleared the status).  bar: a counter that only this kernel's
+// launches use, always with the same grid.
+__device__ __forceinline__ bool grid_barrier(const Dev &d, GridBar &bar)
 {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        const uint32_t ticket = atomicAdd(bar, 1u);
-        const uint32_t target = (ticket / gridDim.x + 1u) * gridDim.x;
+        bar.end = barrier_round_end(bar.end, atomicAdd(bar.count, 1ull), gridDim.x);
         const uint64_t t0 = global_ns();
         ok = 1;
-        while ((int32_t)(*(volatile const uint32_t *)bar - target) < 0) {
+        while (!barrier_open(*(volatile const unsigned long long *)bar.count, bar.end)) {
             if (global_ns() - t0 > BULK_WAIT_NS) {
                 atomicOr(d.status, ST_TIMEOUT);
                 ok = 0;
@@ -123,7 +130,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t &total)
 // The cell list of the positions in buffer A, by all blocks of the grid; false
 // after a timeout.  BLOCK: the threads of a block.
 template <int BLOCK>
-__device__ __noinline__ bool rebuild_grid(const Dev &d, int A, uint32_t *bar)
+__device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
 {
     const uint32_t first = blockIdx.x * BLOCK + threadIdx.x, stride = gridDim.x * BLOCK;
     const uint32_t np = d.np_all, n = d.ncells_all + 1u;   // buckets, the last for the outside

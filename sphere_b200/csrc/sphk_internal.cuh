@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "barrier_count.h"
+
 namespace sphk {
 
 constexpr int NC = 32;           // contact slots per particle, src/constants.h:24
@@ -146,7 +148,8 @@ struct Verlet {
     uint32_t inc2_bits;     // float bits of the step's largest squared displacement
     uint32_t done_blocks;   // blocks of the step's force kernel that are through
     uint32_t came_apart;    // a position had left the grid when the last step ended
-    uint32_t bar_rebuild, bar_small;   // grid_barrier's counters, one a kernel
+    // grid_barrier's counters, one a kernel
+    unsigned long long bar_rebuild = BARRIER_START, bar_small = BARRIER_START;
 };
 
 // Dev::rebuild: the cell list must be made before this step; before the next.

@@ -1994,7 +1994,7 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
     // the cell list first, where this step needs it (REBUILD_NOW does not
     // change before the step ends)
     if (own_list && *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u) {
-        uint32_t *bar = &d.vs->bar_small;
+        GridBar bar{&d.vs->bar_small, 0};
         if (!rebuild_grid<SMALL_BLOCK>(d, A, bar) || !grid_barrier(d, bar)) return;
     }
     if (s0 < np) {
