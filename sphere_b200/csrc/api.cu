@@ -1232,13 +1232,15 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         size_t bytes = 0;
         auto part = [&](size_t count) { const size_t at = bytes; bytes += (count + 31) / 32 * 128; return at; };
         const size_t o_cell = part(np), o_order = part(np), o_pos = part(np), o_xs = part(4 * (size_t)np),
-                     o_start = part((size_t)nc + 2), o_fill = part((size_t)nc + 1),
-                     o_scan = part(SCAN_TILES), o_word = part(4), o_vs = part(32);
+                     o_members = part(np), o_start = part((size_t)nc + 2),
+                     o_fill = part((size_t)nc + 1), o_scan = part(SCAN_TILES), o_word = part(4),
+                     o_vs = part(sizeof(Verlet) / 4);
         CK(cudaMallocAsync(&tmp, bytes, c->stream));
         CK(cudaMemsetAsync(tmp + o_fill, 0, bytes - o_fill, c->stream));
         auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
         q.cell = at(o_cell); q.cellorder = at(o_order); q.pos = at(o_pos);
-        q.xs[0] = q.xs[1] = reinterpret_cast<float4 *>(tmp + o_xs);
+        q.xs[c->a ^ 1] = reinterpret_cast<float4 *>(tmp + o_xs);
+        q.xs[c->a] = reinterpret_cast<float4 *>(tmp + o_members);
         q.cell_start = at(o_start); q.cell_fill = at(o_fill); q.scan_tiles = at(o_scan);
         q.status = at(o_word); q.alias_any = at(o_word) + 1; q.rebuild = at(o_word) + 2;
         q.vs = reinterpret_cast<Verlet *>(tmp + o_vs);

@@ -4,9 +4,10 @@
 //   count      histogram of cell ids                  (atomics in L2)
 //   scan       exclusive scan of the histogram        (two passes)
 //   scatter    each particle claims a position in its cell's range
-//   sort       each cell orders its few members by particle index
-//   finish     inverse order, the float position copy in list order, and the
-//              stamps of the cells whose particles' lists a move upset
+//   rank       each particle's place is the number of its cell's members with
+//              a smaller index: the list, its inverse and the float position
+//              copy in list order; and the stamps of the cells whose particles'
+//              lists a move upset
 // The blocks wait for one another between the passes, so the kernel is
 // launched cooperatively.  Arrays that a pass changes after another read them
 // in the same launch are read past L1 (__ldcg).
@@ -127,14 +128,33 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t &total)
     return off + inc - v;
 }
 
+// A cell with more members than this is put in order by one block, which looks
+// for them among all particles in index order; below, every member counts the
+// smaller indices of its cell for itself.  The first costs a pass over the
+// particles (1.5 us per 512 of them), the second the square of the members
+// shared by the whole grid: 65,536 of them 2 ms of a million particles' list,
+// and all particles in one cell still well inside the barrier's limit.
+constexpr uint32_t CROWD = 1u << 16;
+// the crowded cells, in the half of scan_tiles that no grid's totals reach
+constexpr uint32_t CROWDED_AT = SCAN_TILES / 2, CROWDED_CAP = SCAN_TILES / 2;
+
 // The cell list of the positions in buffer A, by all blocks of the grid; false
 // after a timeout.  BLOCK: the threads of a block.
+//
+// What bounds it: the barriers (about 2 us each) and L2 latency.  One thread
+// used to sort each cell's members by insertion, one load after another: 190 us
+// a list where cells of four radii hold 12 grains each, 13 ms at 300, and past
+// the barrier's limit of 1 s at about 3,000.
 template <int BLOCK>
 __device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
 {
     const uint32_t first = blockIdx.x * BLOCK + threadIdx.x, stride = gridDim.x * BLOCK;
     const uint32_t np = d.np_all, n = d.ncells_all + 1u;   // buckets, the last for the outside
-    if (first == 0) *d.alias_any = 0u;
+    Verlet &V = *d.vs;
+    if (first == 0) {
+        *d.alias_any = 0u;
+        V.crowded = 0u;
+    }
     for (uint32_t s = first; s < np; s += stride) atomicAdd(&d.cell_fill[d.cell[s]], 1u);
     if (!grid_barrier(d, bar)) return false;
     // the block's run of buckets: its sum, then after every block's the scan
@@ -154,38 +174,28 @@ __device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
         const uint32_t v = c < hi ? __ldcg(&d.cell_fill[c]) : 0u;
         const uint32_t at = run + block_scan<BLOCK>(v, total);
         if (c < hi) d.cell_start[c] = at;
+        if (v > CROWD) {
+            const uint32_t e = atomicAdd(&V.crowded, 1u);
+            if (e < CROWDED_CAP) d.scan_tiles[CROWDED_AT + e] = c;
+        }
         run += total;
     }
     if (first == 0) d.cell_start[n] = np;
     if (!grid_barrier(d, bar)) return false;
-    // each particle takes a place of its cell's range; counters return to zero
+    // each particle takes a place of its cell's range; counters return to zero.
+    // The members lie in the other buffer's float positions, which nothing
+    // reads before this step's end writes them.
+    uint32_t *const members = reinterpret_cast<uint32_t *>(d.xs[A ^ 1]);
     for (uint32_t s = first; s < np; s += stride) {
         const uint32_t c = d.cell[s];
         const uint32_t k = atomicSub(&d.cell_fill[c], 1u) - 1u;
-        __stcg(&d.cellorder[d.cell_start[c] + k], s);
+        members[d.cell_start[c] + k] = s;
     }
     if (!grid_barrier(d, bar)) return false;
-    // the members of each cell by particle index (insertion sort)
-    for (uint32_t c = first; c < n; c += stride) {
-        const uint32_t beg = d.cell_start[c], end = d.cell_start[c + 1];
-        for (uint32_t i = beg + 1; i < end; ++i) {
-            const uint32_t s = __ldcg(&d.cellorder[i]);
-            const uint32_t key = d.uid[s];
-            uint32_t j = i;
-            while (j > beg) {
-                const uint32_t o = __ldcg(&d.cellorder[j - 1]);
-                if (d.uid[o] <= key) break;
-                __stcg(&d.cellorder[j], o);
-                --j;
-            }
-            __stcg(&d.cellorder[j], s);
-        }
-    }
-    if (!grid_barrier(d, bar)) return false;
-    // inverse of the new order and the float copy of the positions in list order
-    for (uint32_t k = first; k < np; k += stride) {
-        const uint32_t s = __ldcg(&d.cellorder[k]);
+    // particle s at place k of the list
+    auto place = [&](uint32_t s, uint32_t k) {
         const Params &P = prm_of(d, s);
+        d.cellorder[k] = s;
         d.pos[s] = k;
         const double4 x = d.xr[A][s];
         d.xs[A][k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
@@ -193,10 +203,31 @@ __device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
         // its cell's box (saturated or aliased cell id): contact search must
         // then not prune cells by geometry
         if (cell_outside(P, x.x, x.y, x.z)) atomicOr(d.alias_any, 1u);
+    };
+    for (uint32_t k = first; k < np; k += stride) {
+        const uint32_t s = members[k], c = d.cell[s], key = d.uid[s];
+        const uint32_t beg = d.cell_start[c], end = d.cell_start[c + 1];
+        if (end - beg > CROWD) continue;
+        uint32_t at = beg;
+#pragma unroll 4
+        for (uint32_t j = beg; j < end; ++j) at += d.uid[members[j]] < key ? 1u : 0u;
+        place(s, at);
+    }
+    const uint32_t crowded = min(__ldcg(&V.crowded), CROWDED_CAP);
+    for (uint32_t e = blockIdx.x; e < crowded; e += gridDim.x) {
+        const uint32_t c = __ldcg(&d.scan_tiles[CROWDED_AT + e]);
+        uint32_t at = d.cell_start[c];
+        for (uint32_t u0 = 0; u0 < np; u0 += BLOCK) {
+            const uint32_t u = u0 + threadIdx.x;
+            const uint32_t s = u < np ? d.sidx[u] : 0u;
+            const bool in = u < np && d.cell[s] == c;
+            const uint32_t k = at + block_scan<BLOCK>(in ? 1u : 0u, total);
+            if (in) place(s, k);
+            at += total;
+        }
     }
     stamp_moves(d, first, stride);
     if (first == 0) {
-        Verlet &V = *d.vs;
         V.rebuilds += 1u;
         if (__ldcg(&V.movers_overflow)) {
             V.all_rebuild = 1u;

@@ -115,7 +115,7 @@ __host__ __device__ inline ForceConsts force_consts(const Params &P)
     return c;
 }
 
-// Blocks that a rebuild's grid can have (8 an SM, with room).
+// Twice the blocks that a rebuild's grid can have (8 an SM, with room).
 constexpr uint32_t SCAN_TILES = 4096;
 constexpr int VL_CAP = 32;              // candidates kept per particle
 constexpr uint8_t VL_NONE = 0xff;       // no usable list: sweep the stencil
@@ -147,6 +147,7 @@ struct Verlet {
     uint32_t rebuilds;      // cell-list rebuilds performed since upload
     uint32_t inc2_bits;     // float bits of the step's largest squared displacement
     uint32_t done_blocks;   // blocks of the step's force kernel that are through
+    uint32_t crowded;       // cells with more than CROWD members (rebuild_grid)
     uint32_t came_apart;    // a position had left the grid when the last step ended
     // grid_barrier's counters, one a kernel
     unsigned long long bar_rebuild = BARRIER_START, bar_small = BARRIER_START;
@@ -201,7 +202,8 @@ struct Dev {
     P3 *vel[2];           // vx, vy, vz (fixvel in `fixed`, the host lane in w_user)
     P3 *angvel[2];        // wx, wy, wz (the host lane in w_user)
     float4 *xs[2];        // float copy of xr in cell-list order, for the neighbour cull (up to
-                          // date after a rebuild; in every step with Params::eager)
+                          // date after a rebuild; in every step with Params::eager); a
+                          // rebuild uses the other buffer's as scratch
     // private per-particle state (updated in place); three doubles each, the
     // fourth lane of the host rows (never changed by a step) is kept apart in
     // w_user
@@ -233,7 +235,7 @@ struct Dev {
     uint32_t *cellorder;  // [np] cell-list position -> storage index
     uint32_t *pos;        // [np] storage index -> cell-list position
     uint32_t *cell_fill;  // [ncells + 1] scratch
-    uint32_t *scan_tiles; // [SCAN_TILES] scratch for the scan: a total for each block
+    uint32_t *scan_tiles; // [SCAN_TILES] scratch for the scan: a total for each block; the crowded cells
     uint32_t *alias_any;  // some particle sits outside its cell's box (set by the rebuild)
     // Verlet lists
     uint32_t *vl;         // tiled, VL_CAP per particle: candidate storage indices, in visiting order
