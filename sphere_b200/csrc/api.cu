@@ -848,10 +848,9 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
         for (auto &Q : c->hps) Q.esv_skip = negzero ? 0u : 1u;
         c->hp = c->hps[0];
         CK(cudaMemcpyAsync(d.prm, c->hps.data(), sizeof(Params) * c->ninst, cudaMemcpyHostToDevice, c->stream));
-        Verlet V{};
-        V.step = 1;
-        V.all_rebuild = 1;
-        CK(cudaMemcpyAsync(d.vs, &V, sizeof(V), cudaMemcpyHostToDevice, c->stream));
+        launch_epoch_reset(d, c->stream);
+        // zero but after a list that was given up
+        CK(cudaMemsetAsync(d.cell_fill, 0, ((size_t)c->ncells_all + 1) * sizeof(uint32_t), c->stream));
         CK(cudaMemsetAsync(d.dirty, 0, ((size_t)c->ncells_all + 1) * sizeof(uint32_t), c->stream));
         CK(cudaMemsetAsync(d.vl_len, VL_NONE, np, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -991,7 +990,6 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
         CK(cudaStreamSynchronize(c->stream));   // the CSR built above goes out of scope
     }
     CK(cudaMemsetAsync(d.status, 0, 4, c->stream));
-    CK(cudaMemsetAsync(d.rebuild, 0, 8, c->stream));
     c->sticky = SPH_OK;
     c->err.clear();
     c->t_host = h->t_current;
@@ -1221,6 +1219,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
     CK(cudaMallocAsync(&b, words * 4, c->stream));
     uint32_t *cs = b, *pm = b + np, *st = b + 2 * (size_t)np, *en = st + nc;
     const unsigned int n = (np > nc + 1 ? np : nc + 1);
+    uint32_t made = 0;   // the status of a list made here
     if (c->since_relayout == 0) {
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(c->d, cs, pm, st, en);
     } else {
@@ -1236,7 +1235,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
                      o_fill = part((size_t)nc + 1), o_scan = part(SCAN_TILES), o_word = part(4),
                      o_vs = part(sizeof(Verlet) / 4);
         CK(cudaMallocAsync(&tmp, bytes, c->stream));
-        CK(cudaMemsetAsync(tmp + o_fill, 0, bytes - o_fill, c->stream));
+        CK(cudaMemsetAsync(tmp, 0, bytes, c->stream));   // a list given up stays in range
         auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
         q.cell = at(o_cell); q.cellorder = at(o_order); q.pos = at(o_pos);
         q.xs[c->a ^ 1] = reinterpret_cast<float4 *>(tmp + o_xs);
@@ -1248,6 +1247,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         launch_cell_init(q, np, c->a ^ 1, c->stream);
         launch_rebuild(q, np, nc, c->a ^ 1, c->stream);
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);
+        CK(cudaMemcpyAsync(&made, q.status, 4, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaFreeAsync(tmp, c->stream));
     }
     CK(cudaGetLastError());
@@ -1257,6 +1257,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
     if (cell_end) CK(cudaMemcpyAsync(cell_end, en, (size_t)nc * 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaFreeAsync(b, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (made & ST_TIMEOUT) return fail(c, SPH_ERR_TIMEOUT, status_msg(SPH_ERR_TIMEOUT));
     return SPH_OK;
 }
 

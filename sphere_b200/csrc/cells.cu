@@ -44,7 +44,7 @@ constexpr int REBUILD_BLOCK = 512, REBUILD_BLOCKS_PER_SM = 2;
 __global__ void __launch_bounds__(REBUILD_BLOCK, REBUILD_BLOCKS_PER_SM)
 k_rebuild(const __grid_constant__ Dev d, int A)
 {
-    if (*(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] == 0u) return;
+    if (*(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] == 0u || lists_given_up(d)) return;
     GridBar bar{&d.vs->bar_rebuild, 0};
     rebuild_grid<REBUILD_BLOCK>(d, A, bar);
 }
@@ -104,7 +104,8 @@ __global__ void k_gather(const T *__restrict__ src, T *__restrict__ dst, const u
 // contact rows: move the row and translate partner indices
 // Tiled slot entries into the new storage order: entry e of the new tiles
 // takes the old particle's entry, partners renamed through `inv` (empty
-// slots keep whatever they held: an empty slot's entry is never read).
+// slots keep whatever they held: an empty slot's entry is never read).  After a
+// list that was given up `inv` may have gaps: a partner stays a particle.
 __device__ __forceinline__ bool tile_entry(uint64_t e, uint32_t np, uint32_t &s, uint32_t &i)
 {
     s = (uint32_t)((e / (32ull * NC)) * 32ull + (e & 31ull));
@@ -120,7 +121,7 @@ __global__ void k_gather_rows(const uint32_t *src, uint32_t *dst, const uint32_t
     uint32_t s, i;
     if (!tile_entry(e, np, s, i)) return;
     const uint32_t v = src[tile_at(order[s], i, NC)];
-    dst[e] = (v < np) ? inv[v] : np;
+    dst[e] = (v < np) ? min(inv[v], np - 1u) : np;
 }
 
 __global__ void k_gather_dt(const P3 *src, P3 *dst, const uint32_t *order, uint32_t np)

@@ -27,7 +27,7 @@ struct GridBar {
 
 // Waits until every block of the grid is here; false when that did not happen
 // within BULK_WAIT_NS (ST_TIMEOUT: the caller leaves, and no list is made before
-// an upload has cleared the status).  bar: a counter that only this kernel's
+// an upload has cleared the status, see lists_given_up).  bar: a counter that only this kernel's
 // launches use, always with the same grid.
 __device__ __forceinline__ bool grid_barrier(const Dev &d, GridBar &bar)
 {
@@ -50,6 +50,16 @@ __device__ __forceinline__ bool grid_barrier(const Dev &d, GridBar &bar)
     }
     __syncthreads();
     return ok != 0;
+}
+
+// Whether a barrier has timed out since the upload.  The counters and cell_fill
+// are then as the blocks that left found them: a list made from them would be
+// written past its arrays.  The kernels that make lists leave at once until an
+// upload has cleared all three.  (A half-made list is safe to read: every entry of
+// every array is in range at any time.)
+__device__ __forceinline__ bool lists_given_up(const Dev &d)
+{
+    return (*(volatile const uint32_t *)d.status & ST_TIMEOUT) != 0u;
 }
 
 // Every cell of the neighbourhood of the cells that a move left and entered

@@ -1993,7 +1993,9 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
     const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
     // the cell list first, where this step needs it (REBUILD_NOW does not
     // change before the step ends)
-    if (own_list && *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u) {
+    const bool due = *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u;
+    if (lists_given_up(d)) return;
+    if (own_list && due) {
         GridBar bar{&d.vs->bar_small, 0};
         if (!rebuild_grid<SMALL_BLOCK>(d, A, bar) || !grid_barrier(d, bar)) return;
     }

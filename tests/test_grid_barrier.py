@@ -75,3 +75,18 @@ def test_lists_past_2_32_arrivals(oracle_libs, span):
     rc, want, _ = run_oracle(oracle_libs["orc"], sb, 150)
     assert rc == 0
     assert mismatches(got, want, fields) == []
+
+
+@pytest.mark.gpu
+def test_barrier_and_list_by_themselves(tmp_path):
+    """Rounds of the barrier on the device past 2^32 arrivals, a block that never
+    comes (the others give up after a second and report it), and the cell list's
+    kernel afterwards: it makes nothing until the status has been cleared."""
+    from sphere_b200 import build
+    exe = tmp_path / "cell_list_driver"
+    subprocess.run([build.NVCC, *build.ARCH, "-O2", "--fmad=false", "-std=c++17", "-I",
+                    str(ROOT / "sphere_b200" / "csrc"), str(HERE / "cell_list_driver.cu"), "-o", str(exe)],
+                   check=True)
+    res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0, res.stdout + res.stderr
+    assert res.stdout.count(": ok") == 11, res.stdout
