@@ -18,16 +18,16 @@ void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a,
                   bool slots, cudaStream_t st);
 void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                     cudaStream_t st);
-bool small_step(const Dev &d, uint32_t np);
-void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  bool own_list, cudaStream_t st);
+bool small_step(const Dev &d, uint32_t np, int model);
+cudaError_t launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                         bool own_list, cudaStream_t st);
 void launch_tail(const Dev &d, cudaStream_t st);
 void launch_bonds(const Dev &d, const Params &hp, uint32_t nb0, int a, cudaStream_t st);
 void launch_bond_storage(const Dev &d, uint32_t nb0, uint32_t np, cudaStream_t st);
 void launch_walls(const Dev &d, uint32_t np, uint32_t nw, cudaStream_t st);
 void launch_cell_init(const Dev &d, uint32_t np, int a, cudaStream_t st);
 void launch_epoch_reset(const Dev &d, cudaStream_t st);
-void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st);
+cudaError_t launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st);
 void relayout(const Dev &d, uint32_t np, int a, void *scratch, cudaStream_t st);
 void launch_darcy(const Dev &d, const DarcyDev &f, const Params &hp, int a, int hs, int last,
                   cudaStream_t st);
@@ -353,9 +353,10 @@ int sync_status(sph_ctx *c)
 int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool capturing = false)
 {
     // the small scenes' kernel makes its own cell list, unless the flow reads it too
-    const bool small = !c->diff && small_step(c->d, c->np_all);
+    const int model = (int)c->hp.contactmodel;
+    const bool small = !c->diff && small_step(c->d, c->np_all, model);
     const bool own_list = small && !c->darcy_on;
-    if (!own_list) launch_rebuild(c->d, c->np_all, c->ncells_all, a, st);
+    if (!own_list) CK(launch_rebuild(c->d, c->np_all, c->ncells_all, a, st));
     launch_bonds(c->d, c->hp, c->hp.nb0, a, st);
     // The Darcy block reads the step's start positions (buffer a) and its
     // cell list, which nothing changes before the next step's rebuild, and
@@ -368,7 +369,6 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
         launch_darcy(c->d, c->darcy, c->hp, a, a ^ c->dflip, write_outputs, c->darcy_stream);
         CK(cudaEventRecord(c->darcy_join, c->darcy_stream));
     }
-    const int model = (int)c->hp.contactmodel;
     // walls moved by the previous step's branch, before this step's wall
     // forces read them
     auto join_walls = [&]() -> int {
@@ -379,7 +379,7 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
     int rc;
     if (small) {
         if ((rc = join_walls()) != SPH_OK) return rc;
-        launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, own_list, st);
+        CK(launch_small(c->d, c->hp, c->np_all, model, a, write_outputs, own_list, st));
     } else {
         launch_topo(c->d, c->np_all, model == 1, a, st);
         // the slot forces in the force kernel, unless the shapes of the split
@@ -499,7 +499,7 @@ int profiled_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st)
                                            SPH_PHASE_CONTACT, SPH_PHASE_FORCE, SPH_PHASE_WALLS,
                                            SPH_PHASE_DARCY};
     CK(cudaEventRecord(c->ev[0], st));
-    launch_rebuild(c->d, c->np_all, c->ncells_all, a, st);
+    CK(launch_rebuild(c->d, c->np_all, c->ncells_all, a, st));
     CK(cudaEventRecord(c->ev[1], st));
     launch_bonds(c->d, c->hp, c->hp.nb0, a, st);
     CK(cudaEventRecord(c->ev[2], st));
@@ -530,7 +530,7 @@ int do_relayout(sph_ctx *c, cudaStream_t st)
     // the cell list must describe the current positions before storage follows
     // it (it may be stale: any nonzero flag rebuilds it)
     CK(cudaMemsetAsync(&c->d.rebuild[REBUILD_NOW], 1, 4, st));
-    launch_rebuild(c->d, c->np_all, c->ncells_all, c->a, st);
+    CK(launch_rebuild(c->d, c->np_all, c->ncells_all, c->a, st));
     relayout(c->d, c->np_all, c->a, c->scratch, st);
     // the bonds follow their particles' new storage indices
     if (!c->batched) launch_bond_storage(c->d, c->hp.nb0, c->np_all, st);
@@ -1245,7 +1245,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         q.vs = reinterpret_cast<Verlet *>(tmp + o_vs);
         launch_epoch_reset(q, c->stream);
         launch_cell_init(q, np, c->a ^ 1, c->stream);
-        launch_rebuild(q, np, nc, c->a ^ 1, c->stream);
+        CK(launch_rebuild(q, np, nc, c->a ^ 1, c->stream));
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);
         CK(cudaMemcpyAsync(&made, q.status, 4, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaFreeAsync(tmp, c->stream));
@@ -1402,7 +1402,11 @@ static int capture_segment(sph_ctx *c, int len, int a, cudaGraphExec_t *out)
     int rc = SPH_OK;
     int aa = a;
     for (int j = 0; j < len && rc == SPH_OK; ++j) {
-        launch_rebuild(d, np, c->ncells_all, aa, st);
+        const cudaError_t e = launch_rebuild(d, np, c->ncells_all, aa, st);
+        if (e != cudaSuccess) {   // the capture ends below
+            rc = fail(c, SPH_ERR_CUDA, std::string("segment launch: ") + cudaGetErrorString(e));
+            break;
+        }
         launch_topo(d, np, false, aa, st);
         launch_force_tape(d, np, aa, j, st);
         launch_tail(d, st);

@@ -71,17 +71,11 @@ void launch_epoch_reset(const Dev &d, cudaStream_t st)
     k_epoch_reset<<<1, 1, 0, st>>>(d);
 }
 
-void launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st)
+cudaError_t launch_rebuild(const Dev &d, uint32_t np, uint32_t ncells, int a, cudaStream_t st)
 {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    }
-    const uint32_t most = (uint32_t)nsm * REBUILD_BLOCKS_PER_SM;
+    const uint32_t most = std::min(resident_blocks<k_rebuild, REBUILD_BLOCK>(), sm_count() * REBUILD_BLOCKS_PER_SM);
     const uint32_t grid = std::min(most, div_up(std::max<uint64_t>(np, (uint64_t)ncells + 1), REBUILD_BLOCK));
-    launch_together(k_rebuild, grid, REBUILD_BLOCK, st, d, a);
+    return launch_together(k_rebuild, grid, REBUILD_BLOCK, st, d, a);
 }
 
 // ---- relayout: storage order := current cell order -----------------------

@@ -260,8 +260,8 @@ struct SameType {
     using type = T;
 };
 template <class... Args>
-inline void launch_together(void (*kernel)(Args...), unsigned grid, unsigned block, cudaStream_t st,
-                            typename SameType<Args>::type... args)
+inline cudaError_t launch_together(void (*kernel)(Args...), unsigned grid, unsigned block, cudaStream_t st,
+                                   typename SameType<Args>::type... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
@@ -272,7 +272,7 @@ inline void launch_together(void (*kernel)(Args...), unsigned grid, unsigned blo
     attr.val.cooperative = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace sphk

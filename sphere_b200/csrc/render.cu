@@ -318,8 +318,7 @@ k_rt_resolve(Dev d, int A, RenderArgs g, const double *values, const unsigned lo
 
 void launch_maxpos(const Dev &d, uint32_t np, int a, unsigned long long *mx, cudaStream_t st)
 {
-    const unsigned resident = 8u * 148u;
-    k_rt_maxpos<<<std::min(div_up(np, RT_BLOCK), resident), RT_BLOCK, 0, st>>>(d, a, mx);
+    k_rt_maxpos<<<std::min(div_up(np, RT_BLOCK), 8u * sm_count()), RT_BLOCK, 0, st>>>(d, a, mx);
 }
 
 // DEM::render's camera (src/raytracer.cuh:351-367) and DEM::cameraInit

@@ -11,6 +11,7 @@
 // root (src/vector_arithmetic.h:317-320).
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -530,6 +531,32 @@ __host__ __device__ __forceinline__ size_t tiled_size(size_t np, uint32_t width)
 __host__ __device__ __forceinline__ size_t tape_slot_at(uint32_t j, uint32_t np, uint32_t s, uint32_t i)
 {
     return (size_t)j * tiled_size(np, NC) + tile_at(s, i, NC);
+}
+
+// The SMs of the current device, and the blocks of a kernel (without dynamic
+// shared memory) that it holds at once, as the runtime sees them: a share of a
+// GPU has fewer.  Looked up once a device.
+inline uint32_t sm_count()
+{
+    static std::atomic<uint32_t> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (const uint32_t k = known[dev].load(std::memory_order_relaxed)) return k;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    known[dev].store((uint32_t)(n > 0 ? n : 1), std::memory_order_relaxed);
+    return (uint32_t)(n > 0 ? n : 1);
+}
+template <auto Kernel, int Block>
+uint32_t resident_blocks()
+{
+    static std::atomic<uint32_t> known[64];
+    int dev = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (const uint32_t k = known[dev].load(std::memory_order_relaxed)) return k;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kernel, Block, 0);
+    const uint32_t k = sm_count() * (uint32_t)(per_sm > 0 ? per_sm : 1);
+    known[dev].store(k, std::memory_order_relaxed);
+    return k;
 }
 
 inline unsigned int div_up(unsigned long long a, unsigned int b)

@@ -2070,16 +2070,17 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
     end_of_step(d);
 }
 
-// Particles that k_small's resident threads hold.
-static uint32_t small_np()
+// Blocks of k_small that the device holds at once.
+template <int MODEL, bool BATCH>
+static uint32_t small_blocks()
 {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return (uint32_t)nsm * SMALL_BLOCKS_PER_SM * SMALL_BLOCK;
+    return std::min(resident_blocks<k_small<MODEL, BATCH>, SMALL_BLOCK>(), sm_count() * SMALL_BLOCKS_PER_SM);
+}
+static uint32_t small_blocks(const Dev &d, int model)
+{
+    if (d.inst) return small_blocks<2, true>();
+    return model == 1 ? small_blocks<1, false>()
+                      : (model == 3 ? small_blocks<3, false>() : small_blocks<2, false>());
 }
 
 // Whether a context's steps run as k_small: its chunks have a resident warp
@@ -2089,41 +2090,33 @@ static uint32_t small_np()
 // split, on a B200: in a flow 24.7 / 29.0 at 1,000 grains, 32.6 / 38.3 at
 // 10,000, 37.8 / 45.0 at 50,000, 44.8 / 53.3 at 75,000; in a jammed packing
 // 20.1 / 20.9 at 1,000, 23.3 / 24.7 at 29,791, 28.5 / 29.0 at 74,088.
-bool small_step(const Dev &d, uint32_t np)
+bool small_step(const Dev &d, uint32_t np, int model)
 {
-    return d.shape == 0 && d.topo_span == 0 && np <= small_np();
+    return d.shape == 0 && d.topo_span == 0 && div_up(np, SMALL_BLOCK) <= small_blocks(d, model);
 }
 
 // own_list: the kernel makes the cell list itself when it is due.
-void launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
-                  bool own_list, cudaStream_t st)
+cudaError_t launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
+                         bool own_list, cudaStream_t st)
 {
     const ForceArgs args{d, a, write_outputs, -1, force_consts(hp), law_params(hp)};
     // more blocks than chunks need where the cells are many: they share the list
-    const unsigned most = (unsigned)(small_np() / SMALL_BLOCK);
-    const unsigned grid = std::min(most, std::max(div_up(np, SMALL_BLOCK), div_up(d.ncells_all, 32 * SMALL_BLOCK)));
+    const unsigned grid = std::min(small_blocks(d, model),
+                                   std::max(div_up(np, SMALL_BLOCK), div_up(d.ncells_all, 32 * SMALL_BLOCK)));
     const int own = own_list ? 1 : 0;
-    if (d.inst) launch_together(k_small<2, true>, grid, SMALL_BLOCK, st, args, own);
-    else if (model == 1) launch_together(k_small<1, false>, grid, SMALL_BLOCK, st, args, own);
-    else if (model == 3) launch_together(k_small<3, false>, grid, SMALL_BLOCK, st, args, own);
-    else launch_together(k_small<2, false>, grid, SMALL_BLOCK, st, args, own);
+    if (d.inst) return launch_together(k_small<2, true>, grid, SMALL_BLOCK, st, args, own);
+    if (model == 1) return launch_together(k_small<1, false>, grid, SMALL_BLOCK, st, args, own);
+    if (model == 3) return launch_together(k_small<3, false>, grid, SMALL_BLOCK, st, args, own);
+    return launch_together(k_small<2, false>, grid, SMALL_BLOCK, st, args, own);
 }
 
-// A resident grid of k_contact: the SMs times the blocks of this
-// instantiation that fit on one (looked up once per instantiation).
+// A resident grid of k_contact: the blocks of this instantiation that the
+// device holds at once.
 template <int MODEL, bool BATCH, int CB>
 static unsigned contact_grid(uint32_t np)
 {
-    static int resident = 0;
-    if (resident == 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_contact<MODEL, BATCH, CB>, CB, 0);
-        resident = std::max(1, sms) * std::max(1, per_sm);
-    }
     const uint64_t chunks = div_up(np, 32);
-    return (unsigned)std::min<uint64_t>((uint64_t)resident, div_up(chunks, CB / 32));
+    return (unsigned)std::min<uint64_t>(resident_blocks<k_contact<MODEL, BATCH, CB>, CB>(), div_up(chunks, CB / 32));
 }
 
 // Particles per lane of k_topo's list decisions: 4 once the scene is four
@@ -2132,14 +2125,7 @@ static unsigned contact_grid(uint32_t np)
 // scene's searches run on as many lanes as it has particles.
 static uint32_t topo_span(uint32_t np)
 {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm < 1) nsm = 1;
-    }
-    const uint64_t resident = (uint64_t)nsm * TOPO_THREADS_PER_SM;
+    const uint64_t resident = (uint64_t)sm_count() * TOPO_THREADS_PER_SM;
     return (uint64_t)np >= 4 * resident ? 4u : ((uint64_t)np >= 2 * resident ? 2u : 1u);
 }
 
@@ -2179,16 +2165,8 @@ void launch_topo(const Dev &d, uint32_t np, bool visc, int a, cudaStream_t st)
 template <int MODEL, bool BATCH, bool SLOTS>
 static void launch_force_tiles(const ForceArgs &args, uint32_t np, cudaStream_t st)
 {
-    static int per_sm = 0, nsm = 0;
-    if (per_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_force_tiles<MODEL, BATCH, SLOTS>,
-                                                      32 * FORCE_WARPS, 0);
-        if (per_sm < 1) per_sm = 1;
-    }
-    const uint32_t grid = std::min<uint32_t>(div_up(np, FT_TILE * FORCE_WARPS), (uint32_t)(per_sm * nsm));
+    const uint32_t grid = std::min(div_up(np, FT_TILE * FORCE_WARPS),
+                                   resident_blocks<k_force_tiles<MODEL, BATCH, SLOTS>, 32 * FORCE_WARPS>());
     if (grid) k_force_tiles<MODEL, BATCH, SLOTS><<<grid, 32 * FORCE_WARPS, 0, st>>>(args);
 }
 

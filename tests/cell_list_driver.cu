@@ -70,6 +70,12 @@ int main()
     }
     check("no block ahead", fetch(behind, 1)[0] == 0u && fetch(d.status, 1)[0] == 0u);
 
+    // a grid that the device does not hold at once is refused, and said to be
+    const cudaError_t refused = launch_together(k_rounds, 1u << 20, 64, nullptr, d, filled(start), mark, behind, 1, 0u);
+    check("too large", refused == cudaErrorCooperativeLaunchTooLarge && cudaGetLastError() == refused);
+    const uint32_t most = resident_blocks<k_rebuild, REBUILD_BLOCK>();
+    check("resident", most >= sm_count() * REBUILD_BLOCKS_PER_SM && most <= SCAN_TILES / 2);
+
     // a cell list of 3,000 particles in 10 x 10 x 10 cells, in storage order
     // reversed against their indices
     const uint32_t np = 3000, nc = 1000;
