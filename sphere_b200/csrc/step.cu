@@ -1445,8 +1445,11 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
         const float fx = __double2float_ru(fabs(vel0.x * dt)), fy = __double2float_ru(fabs(vel0.y * dt)),
                     fz = __double2float_ru(fabs(vel0.z * dt));
         const float d2 = __fmaf_ru(fx, fx, __fmaf_ru(fy, fy, __fmul_ru(fz, fz)));
-        const uint32_t bits = __reduce_max_sync(__activemask(), __float_as_uint(d2) & 0x7fffffffu);
-        if ((threadIdx.x & 31u) == (uint32_t)(__ffs(__activemask()) - 1) &&
+        // one mask for both: a warp that is split here has a publishing lane in
+        // each part, whatever joins again between the two
+        const uint32_t on = __activemask();
+        const uint32_t bits = __reduce_max_sync(on, __float_as_uint(d2) & 0x7fffffffu);
+        if ((threadIdx.x & 31u) == (uint32_t)(__ffs(on) - 1) &&
             bits > *(volatile uint32_t *)&V.inc2_bits)
             atomicMax(&V.inc2_bits, bits);
     }

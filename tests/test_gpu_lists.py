@@ -103,3 +103,24 @@ def test_batched_scenes_of_either_kind(oracle_libs, span):
         rc, want, _ = run_oracle(oracle_libs["orc"], sb, 50)
         assert rc == 0
         assert mismatches(st, want, STATE_FIELDS + OUTPUT_FIELDS + ("contacts", "delta_t")) == []
+
+
+@both_kernels
+@pytest.mark.parametrize("fast", [0, 13, 31, 40])
+def test_the_fastest_grain_of_a_split_warp_sets_the_clock(oracle_libs, fast, span):
+    """One grain in motion among grains at rest, some of which touch walls or one
+    another, so that its warp takes different ways to the displacement's maximum:
+    it meets grains that were beyond its list's reach."""
+    sb = scenes.collision(n=96, seed=7, vmax=0.0, wmax=0.0, g=(0.0, 0.0, 0.0), phi_target=0.2)
+    lo = np.min(sb.x - sb.radius[:, None], axis=0)
+    sb.x = sb.x - lo - 1e-5
+    sb.L = np.max(sb.x + sb.radius[:, None], axis=0) - 1e-5
+    sb.num = np.maximum(1, np.floor(sb.L / 3.3e-3)).astype(np.uint32)
+    sb.vel[fast] = np.array([9.0, 7.0, 11.0]) * np.where(sb.x[fast] > 0.5 * sb.L, -1.0, 1.0)
+    rc, want, _ = run_oracle(oracle_libs["orc"], sb, 120)
+    assert rc == 0 and int((want.contacts != sb.np).sum()) > 0
+    with Simulation(config_from_spherebin(sb), verlet_skin=0.05, topo_span=span) as sim:
+        sim.upload(state_from_spherebin(sb))
+        sim.step(120)
+        sim.sync()
+        assert mismatches(sim.download(), want, ALL) == []
