@@ -705,7 +705,11 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
 // Sweep mode: the 27 stencil cells are scanned as in the reference (z, y, x;
 // members by particle index) and the list is recorded on the way, together
 // with the near candidates two cells away where cells are that small
-// (Params::wide).
+// (Params::wide).  What bounds it is latency, a chain of loads a row and one an
+// overlap: an x-row is one run of the cell list (a run a cell: 25 rows took 50
+// more), and the overlaps are tested when the sweep is over (where they are found
+// they come at different places in every lane).  k_topo sweeping in every step,
+// 50,000 grains in contact: 96 us -> 55.
 //
 // VISC (contact model 1): no slots; every candidate within ra + rb + db acts,
 // in visiting order: they are left in `va` and the lane's column of srow.
@@ -853,82 +857,6 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         bool list_overflow = false;
         held = 0u;
 
-        // A run [beg, end) of cell-list positions (one cell, or the three
-        // cells of an x-row whose inner boundaries are bnd1 <= bnd2), culled
-        // four candidates at a time so the four loads are in flight
-        // together; hits are handled in list order.  far: cells outside the
-        // stencil, whose candidates are only recorded.
-        auto scan_run = [&](uint32_t beg, uint32_t end, uint32_t code, uint32_t bnd1,
-                            uint32_t bnd2, bool far) {
-            const float sx = (code & 1u) ? Lf0 : ((code & 2u) ? -Lf0 : 0.0f);
-            const float sy = (code & 4u) ? Lf1 : ((code & 8u) ? -Lf1 : 0.0f);
-            uint32_t base = beg;
-            while (base < end) {
-                const uint32_t last = end - 1;
-                float4 c[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) c[j] = __ldca(&xs[min(base + (uint32_t)j, last)]);
-                uint32_t near = 0, hit = 0;
-                float gj[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float fx = (xaf.x - c[j].x) + sx;
-                    const float fy = (xaf.y - c[j].y) + sy;
-                    const float fz = xaf.z - c[j].z;
-                    const float d2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz * fz));
-                    const float rsum = VISC ? (xaf.w + c[j].w + extraf) : (xaf.w + c[j].w);
-                    const float rr = rsum * 1.000004f + eps;
-                    const float rs = (rsum + skinf) * 1.000004f + eps;
-                    const uint32_t k2 = base + (uint32_t)j;
-                    const bool ok = k2 < end && k2 != k;
-                    // the gap, with the cull's float slack taken against it
-                    gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
-                    if (ok && d2 < rs * rs) near |= 1u << j;
-                    if (ok && !far && d2 < rr * rr) hit |= 1u << j;
-                }
-                uint32_t next = base + 4;
-                while (near) {
-                    const int j = __ffs(near) - 1;
-                    near &= near - 1;
-                    const uint32_t k2 = base + (uint32_t)j;
-                    const uint32_t t = __ldca(&d.cellorder[k2]);
-                    const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
-                    float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
-                    if (VISC) {
-                        if ((hit >> j) & 1u) {
-                            act_on(t, code);
-                            w = -1.0f;
-                        }
-                    } else if ((hit >> j) & 1u) {
-                        double ln;
-                        if (pair_gap(P, xr[t], code, xa, ln) < 0.0f) {
-                            if (!topo_insert<TB>(d, srow, tid, s, t, code, ts)) {
-                                // nc > NC: skip the rest of this cell; the list
-                                // would not describe the skipped part
-                                next = (k2 < bnd1) ? bnd1 : ((k2 < bnd2) ? bnd2 : end);
-                                near = 0;
-                                list_overflow = true;
-                            }
-                            if (nlist < VL_CAP) held |= 1u << nlist;
-                            w = 3.0e38f;
-                        }
-                    }
-                    due = fminf(due, w);
-                    if (!use_lists) {
-                    } else if (nlist < VL_CAP) {
-                        const size_t at = vl_at(s, nlist);
-                        d.vl[at] = t;
-                        // a held entry that loses its slot is due at once
-                        d.vl_meta[at] = vl_meta_of(code, w > 1.0e38f ? S : fmaxf(w, 0.0f));
-                        ++nlist;
-                    } else {
-                        list_overflow = true;
-                    }
-                }
-                base = next;
-            }
-        };
-
         // Cell-level pruning: a stencil cell whose box lies farther from the
         // particle than ra + rmax + skin (plus the float slack of the
         // predicate) holds neither a contact nor a list candidate; skipping
@@ -959,6 +887,116 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         const float reach2 = prune ? reach * reach : 3.0e38f;
         const int R = (P.wide && use_lists) ? 2 : 1;
 
+        // A run of the cell list: cells c0, c0 + 1, ..., through image `code`;
+        // [in0, in1) is its part in the stencil, the rest, two cells away, is
+        // only recorded.
+        struct Run {
+            uint32_t beg, end, in0, in1, c0, code;
+        };
+        // The overlaps of the first VL_CAP near candidates are tested after the
+        // sweep, from the list: found here and there in a warp's lanes, each
+        // would make the whole warp wait for its two loads and its slot.  (A
+        // particle outside the grid has no list to keep them in.)
+        uint32_t later = 0;
+        auto test_later = [&]() {
+            for (; later; later &= later - 1u) {
+                const uint32_t e = (uint32_t)(__ffs(later) - 1);
+                const size_t at = vl_at(s, e);
+                const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
+                double ln;
+                if (pair_gap(P, xr[t], code, xa, ln) < 0.0f) {
+                    topo_insert<TB>(d, srow, tid, s, t, code, ts);   // nc <= VL_CAP: no cell ends
+                    held |= 1u << e;
+                } else {
+                    due = fminf(due, S);
+                }
+            }
+        };
+
+        // A run's candidates, culled four at a time so that their loads are in
+        // flight together; hits are handled in list order.
+        auto scan_run = [&](const Run &r) {
+            const float sx = (r.code & 1u) ? Lf0 : ((r.code & 2u) ? -Lf0 : 0.0f);
+            const float sy = (r.code & 4u) ? Lf1 : ((r.code & 8u) ? -Lf1 : 0.0f);
+            uint32_t base = r.beg;
+            while (base < r.end) {
+                const uint32_t last = r.end - 1;
+                float4 c[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) c[j] = xs[min(base + (uint32_t)j, last)];
+                uint32_t near = 0, hit = 0;
+                float gj[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float fx = (xaf.x - c[j].x) + sx;
+                    const float fy = (xaf.y - c[j].y) + sy;
+                    const float fz = xaf.z - c[j].z;
+                    const float d2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz * fz));
+                    const float rsum = VISC ? (xaf.w + c[j].w + extraf) : (xaf.w + c[j].w);
+                    const float rr = rsum * 1.000004f + eps;
+                    const float rs = (rsum + skinf) * 1.000004f + eps;
+                    const uint32_t k2 = base + (uint32_t)j;
+                    const bool ok = k2 < r.end && k2 != k;
+                    if (ok && d2 < rs * rs) {
+                        near |= 1u << j;
+                        // the gap, with the cull's float slack taken against it
+                        gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
+                    }
+                    if (ok && k2 >= r.in0 && k2 < r.in1 && d2 < rr * rr) hit |= 1u << j;
+                }
+                uint32_t next = base + 4;
+                while (near) {
+                    const int j = __ffs(near) - 1;
+                    near &= near - 1;
+                    const uint32_t t = d.cellorder[base + (uint32_t)j];
+                    const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
+                    // when it can overlap (a hit's gap is not positive)
+                    float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
+                    if (VISC) {
+                        if ((hit >> j) & 1u) {
+                            act_on(t, r.code);
+                            w = -1.0f;
+                        }
+                    } else if ((hit >> j) & 1u) {
+                        if (gp_in && nlist < VL_CAP) {
+                            later |= 1u << nlist;
+                            w = 3.0e38f;
+                        } else {
+                            test_later();   // in visiting order
+                            double ln;
+                            if (pair_gap(P, xr[t], r.code, xa, ln) < 0.0f) {
+                                if (!topo_insert<TB>(d, srow, tid, s, t, r.code, ts)) {
+                                    // nc > NC: skip the rest of this cell; the list
+                                    // would not describe the skipped part
+                                    uint32_t e = r.c0 + 1u;
+                                    while (d.cell_start[e] <= base + (uint32_t)j) ++e;
+                                    next = d.cell_start[e];
+                                    near = 0;
+                                    list_overflow = true;
+                                }
+                                w = 3.0e38f;
+                            }
+                        }
+                    }
+                    due = fminf(due, w);
+                    if (gp_in && nlist < VL_CAP) {
+                        const size_t at = vl_at(s, nlist);
+                        d.vl[at] = t;
+                        // a held entry that loses its slot is due at once
+                        d.vl_meta[at] = vl_meta_of(r.code, w > 1.0e38f ? S : fmaxf(w, 0.0f));
+                        ++nlist;
+                    } else {
+                        list_overflow = true;
+                    }
+                }
+                base = next;
+            }
+        };
+
+        // The cells in visiting order, of each x-row in up to three runs: those
+        // through the periodic boundary before it, those in the grid, those
+        // through the boundary after it (of a particle outside the grid its
+        // three cells one by one, as the reference's stencil names them).
         for (int oz = -R; oz <= R; ++oz) {
             const int32_t cz = (int32_t)((uint32_t)gp[2] + (uint32_t)oz);
             if (past_axis(cz, nz, R == 2)) continue;
@@ -969,45 +1007,51 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 if (dyz2 > reach2) continue;
                 int32_t cy = (int32_t)((uint32_t)gp[1] + (uint32_t)oy);
                 uint32_t ycode = 0;
-                if (P.periodic == 1) {
-                    wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
-                } else if (past_axis(cy, ny, R == 2)) {
-                    continue;
-                }
+                if (P.periodic == 1) wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
+                else if (past_axis(cy, ny, R == 2)) continue;
                 const uint32_t rowbase = (uint32_t)cy * nx + (nx * ny) * (uint32_t)cz;
                 const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
-                for (int ox = -R; ox <= R; ++ox) {
-                    int32_t cx = (int32_t)((uint32_t)gp[0] + (uint32_t)ox);
-                    uint32_t beg, end, b1, b2, code = ycode;
-                    const bool far = far_row || ox < -1 || ox > 1;
-                    if (!far && ox == -1 && cx >= 0 && (uint32_t)cx + 2 < nx) {
-                        // the three x cells are consecutive ids: one run of xs
-                        ox = 1;
-                        const uint32_t cid0 = (uint32_t)cx + rowbase;
-                        if (cid0 + 2 >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
-                        const uint32_t g0 = cid0 + P.cell_base;
-                        const uint32_t b0 = d.cell_start[g0], b3 = d.cell_start[g0 + 3];
-                        b1 = d.cell_start[g0 + 1];
-                        b2 = d.cell_start[g0 + 2];
-                        beg = (dyz2 + lo1[0] <= reach2) ? b0 : b1;
-                        end = (dyz2 + hi1[0] <= reach2) ? b3 : b2;
-                    } else {
-                        if (dyz2 + dist2(0, ox) > reach2) continue;
-                        if (P.periodic == 1 || P.periodic == 2) {
-                            wrap_axis(cx, nx, code, 1u, 2u, R == 2);
-                        } else if (past_axis(cx, nx, R == 2)) {
-                            continue;
+                for (int part = 0; part < 3; ++part) {
+                    int32_t a, b, cx;   // cells gp + a .. gp + b; the first one's x
+                    Run r;
+                    r.code = ycode;
+                    if (gp_in) {
+                        const int32_t g = gp[0], n = (int32_t)nx;
+                        if (part == 1) {
+                            a = max(-R, -g);
+                            b = min(R, n - 1 - g);
+                        } else {
+                            if (P.periodic != 1 && P.periodic != 2) continue;
+                            a = part == 0 ? -R : n - g;
+                            b = part == 0 ? -g - 1 : R;
                         }
-                        const uint32_t cid = (uint32_t)cx + rowbase;
-                        if (cid >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
-                        const uint32_t g = cid + P.cell_base;
-                        beg = d.cell_start[g];
-                        end = b1 = b2 = d.cell_start[g + 1];
+                        if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
+                        if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
+                        if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
+                        if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
+                        if (a > b) continue;
+                        cx = g + a + (part == 0 ? n : (part == 2 ? -n : 0));
+                        if (part != 1) r.code |= part == 0 ? 1u : 2u;
+                    } else {
+                        a = b = part - 1;
+                        cx = (int32_t)((uint32_t)gp[0] + (uint32_t)a);
+                        if (P.periodic == 1 || P.periodic == 2) wrap_axis(cx, nx, r.code, 1u, 2u, false);
+                        else if (past_axis(cx, nx, false)) continue;
                     }
-                    scan_run(beg, end, code, b1, b2, far);
+                    const uint32_t cid = (uint32_t)cx + rowbase;
+                    if (cid >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
+                    r.c0 = cid + P.cell_base;
+                    const uint32_t *const bounds = d.cell_start + r.c0;
+                    r.beg = bounds[0];
+                    r.end = bounds[b - a + 1];
+                    // the stencil's part: cells max(a, -1) .. min(b, 1)
+                    r.in0 = a < -1 ? bounds[-1 - a] : r.beg;
+                    r.in1 = far_row || a > 1 || b < -1 ? r.in0 : (b > 1 ? bounds[2 - a] : r.end);
+                    scan_run(r);
                 }
             }
         }
+        if (!VISC) test_later();
         const bool listed = use_lists && !list_overflow;
         d.vl_len[s] = listed ? (uint8_t)nlist : VL_NONE;
         if (!listed) {
