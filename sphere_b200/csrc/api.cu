@@ -18,7 +18,7 @@ void launch_force(const Dev &d, const Params &hp, uint32_t np, int model, int a,
                   bool slots, cudaStream_t st);
 void launch_contact(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                     cudaStream_t st);
-bool small_step(const Dev &d, uint32_t np, int model);
+bool small_step(const Dev &d, uint32_t np, int model, bool with_flow);
 cudaError_t launch_small(const Dev &d, const Params &hp, uint32_t np, int model, int a, int write_outputs,
                          bool own_list, cudaStream_t st);
 void launch_tail(const Dev &d, cudaStream_t st);
@@ -354,7 +354,7 @@ int enqueue_one_step(sph_ctx *c, int a, int write_outputs, cudaStream_t st, bool
 {
     // the small scenes' kernel makes its own cell list, unless the flow reads it too
     const int model = (int)c->hp.contactmodel;
-    const bool small = !c->diff && small_step(c->d, c->np_all, model);
+    const bool small = !c->diff && small_step(c->d, c->np_all, model, c->darcy_on);
     const bool own_list = small && !c->darcy_on;
     if (!own_list) CK(launch_rebuild(c->d, c->np_all, c->ncells_all, a, st));
     launch_bonds(c->d, c->hp, c->hp.nb0, a, st);

@@ -2137,9 +2137,17 @@ static uint32_t small_blocks(const Dev &d, int model)
 // split, on a B200: in a flow 24.7 / 29.0 at 1,000 grains, 32.6 / 38.3 at
 // 10,000, 37.8 / 45.0 at 50,000, 44.8 / 53.3 at 75,000; in a jammed packing
 // 20.1 / 20.9 at 1,000, 23.3 / 24.7 at 29,791, 28.5 / 29.0 at 74,088.
-bool small_step(const Dev &d, uint32_t np, int model)
+//
+// Beside a Darcy flow (with_flow) up to a block an SM: its blocks start all
+// together, so beyond that k_small waits for the porosity's to leave, which runs
+// at the same time.  One kernel against split, cells of 2.5 and 4 radii: 42.9 /
+// 47.0 and 60.6 / 60.9 at 10,000 grains, 66.0 / 54.1 and 108.8 / 69.0 at 20,000,
+// 69.5 / 60.5 and 113.0 / 73.1 at 50,000.
+bool small_step(const Dev &d, uint32_t np, int model, bool with_flow)
 {
-    return d.shape == 0 && d.topo_span == 0 && div_up(np, SMALL_BLOCK) <= small_blocks(d, model);
+    const uint32_t blocks = div_up(np, SMALL_BLOCK);
+    return d.shape == 0 && d.topo_span == 0 && blocks <= small_blocks(d, model) &&
+           !(with_flow && blocks > sm_count());
 }
 
 // own_list: the kernel makes the cell list itself when it is due.

@@ -75,6 +75,24 @@ def test_darcy_with_many_grains_a_cell(oracle_libs, num, periodic):
     assert mismatches(st, so, STATE_FIELDS) == []
 
 
+# a block of 128 grains an SM (148 of them): beside a flow the step in one kernel,
+# and past it split
+@pytest.mark.parametrize("n", [18944, 18945])
+def test_darcy_at_the_largest_scene_in_one_kernel(oracle_libs, n):
+    sb = scenes.collision(n=n, seed=29, box=(0.1, 0.1, 0.1), k_n=500.0, k_t=500.0, vmax=0.5)
+    sb.num = np.array([16, 16, 16], dtype=np.uint32)
+    start = seeded_grid(sb.num, 7)
+    _, so, o = run_darcy_oracle(oracle_libs["orc"], sb, 4, start.copy())
+    with Simulation(config_from_spherebin(sb)) as sim:
+        sim.upload(state_from_spherebin(sb))
+        sim.darcy_upload(start.copy(), NU)
+        sim.step(4)
+        sim.sync()
+        st, g = sim.download(), sim.darcy_download()
+    assert darcy_mismatches(g, o) == []
+    assert mismatches(st, so, STATE_FIELDS) == []
+
+
 def test_sessions_take_up_kept_arrays_or_replace_them():
     """Differentiable sessions of one context: the same checkpoint interval
     again, another, the first again, with plain steps and another scene's
