@@ -680,8 +680,8 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     AL(d.scan_tiles, SCAN_TILES);
     AL(d.alias_any, 1);
     AL(d.vl, tiled_size(np, VL_CAP)); AL(d.vl_meta, tiled_size(np, VL_CAP)); AL(d.vl_len, np);
-    AL(d.vl_held, np); AL(d.due, np);
-    AL(d.movers, MOVER_CAP); AL(d.dirty, ncells + 1); AL(d.vs, 1);
+    AL(d.vl_held, np); AL(d.due, np); AL(d.vl_tag, np); AL(d.outside, np);
+    AL(d.movers, MOVER_CAP); AL(d.dirty, ncells + 1); AL(d.look, ncells + 1); AL(d.vs, 1);
     AL(d.wf_pp, np); AL(d.wtouch, npad); AL(d.wf_partial, div_up(np, 256));
     AL(d.wf_flag, div_up(np, 256));
     AL(d.walls, 1);
@@ -831,12 +831,16 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
             const double reach = (2.0 * Q.rmax + Q.skin + Q.reach_extra) * (1.0 + 1e-5) + Q.prune_pad;
             Q.set_lists = Q.skin > 0.0 ? 1u : 0u;
             Q.wide = 0u;
+            Q.one_image = 1u;
             for (int k = 0; k < 3; ++k) {
                 const bool wraps = (k == 0 && Q.periodic != 0) || (k == 1 && Q.periodic == 1);
                 if (2.0 * Q.cellsize[k] < reach || (wraps && Q.num[k] < 3)) Q.set_lists = 0u;
                 if (Q.cellsize[k] < reach) Q.wide = 1u;
+                // (the wrap of the integration is a period only from a grid at 0)
+                if (wraps && !(Q.L[k] > 2.5 * reach && Q.origo[k] == 0.0)) Q.one_image = 0u;
             }
             if (!Q.set_lists) Q.wide = 0u;
+            if (!Q.set_lists || (Q.periodic != 1 && Q.periodic != 2)) Q.one_image = 0u;
             // without lists every step sweeps; the Darcy flow reads the cell list
             Q.eager = (!(Q.skin > 0.0) || c->darcy_on) ? 1u : 0u;
         }

@@ -64,8 +64,9 @@ __device__ __forceinline__ bool lists_given_up(const Dev &d)
 
 // Every cell of the neighbourhood of the cells that a move left and entered
 // (27 cells each, or with Params::wide 125) is stamped with this step's
-// number; particles in stamped cells sweep their stencil again.  Periodic axes
-// wrap as in findDistMod.
+// number; particles in stamped cells sweep their stencil again, or, around a
+// particle that is back from outside a periodic boundary, look at their lists.
+// Periodic axes wrap as in findDistMod.
 __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32_t stride)
 {
     Verlet &V = *d.vs;
@@ -74,6 +75,8 @@ __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32
         const uint2 mv = __ldcg(&d.movers[e >> 1]);
         const uint32_t cg = (e & 1u) ? mv.y : mv.x;
         if (cg >= d.ncells_all) continue;
+        uint32_t *const stamps = mv.x == LOOK ? d.look : d.dirty;
+        *(mv.x == LOOK ? &V.look_step : &V.dirty_step) = step;
         // the instance owning global cell cg (batched contexts)
         uint32_t inst = 0;
         if (d.inst) {
@@ -104,8 +107,7 @@ __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32
                         if (P.periodic != 1 && P.periodic != 2) continue;
                         x = (x + (int32_t)nx) % (int32_t)nx;
                     }
-                    d.dirty[P.cell_base + (uint32_t)x + (uint32_t)y * nx + (nx * ny) * (uint32_t)z] = step;
-                    V.dirty_step = step;
+                    stamps[P.cell_base + (uint32_t)x + (uint32_t)y * nx + (nx * ny) * (uint32_t)z] = step;
                 }
             }
         }

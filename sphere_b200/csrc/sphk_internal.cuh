@@ -72,6 +72,7 @@ struct Params {
     uint32_t esv_skip;  // no es/ev is -0.0: adding a zero rate may be skipped exactly
     uint32_t set_lists; // the candidate lists outlive moves between cells (see Verlet)
     uint32_t wide;      // with set_lists: a near pair may be two cells apart
+    uint32_t one_image; // with set_lists: a pair is near through one periodic image only (list_code)
     uint32_t eager;     // the cell list and xs are kept up to date in every step
     uint32_t cell_base; // batched contexts: first global cell id of this instance
     uint32_t uid_base;  // batched contexts: first global particle index of this instance
@@ -86,8 +87,7 @@ struct ForceConsts {
     uint32_t nw, nb0, ncells, cell_base;
     int32_t periodic;
     uint32_t num[3];
-    uint32_t esv_skip, set_lists, eager;
-    uint32_t pad;
+    uint32_t esv_skip, set_lists, eager, one_image;
     double origo[3], L[3], cellsize[3], rcell[3];
     double dt, g[3], rho, skin;
 };
@@ -102,6 +102,7 @@ __host__ __device__ inline ForceConsts force_consts(const Params &P)
     c.esv_skip = P.esv_skip;
     c.set_lists = P.set_lists;
     c.eager = P.eager;
+    c.one_image = P.one_image;
     for (int i = 0; i < 3; ++i) {
         c.num[i] = P.num[i];
         c.origo[i] = P.origo[i];
@@ -121,6 +122,7 @@ constexpr uint32_t SCAN_TILES = 4096;
 constexpr int VL_CAP = 32;              // candidates kept per particle
 constexpr uint8_t VL_NONE = 0xff;       // no usable list: sweep the stencil
 constexpr uint32_t MOVER_CAP = 1u << 16;
+constexpr uint32_t LOOK = 0xffffffffu;  // no cell
 
 // State of the Verlet-list epoch, device resident.
 //
@@ -137,6 +139,14 @@ constexpr uint32_t MOVER_CAP = 1u << 16;
 // the cell list then goes stale until a sweep needs it (`rebuild`).  Without,
 // they hold the pairs of the 27-cell stencils and every change of cell makes
 // the cells around it sweep again.
+//
+// A particle that crosses a periodic boundary stands outside the grid for one
+// step, in a cell that its id aliases, and is back in by one period in the next.
+// The pairs stay the same; with Params::one_image (axes longer than twice the
+// reach) an entry's image follows from the two positions.  What has to be done
+// is to look at the lists around it once it is back (`look` stamps): slots it
+// holds are now seen through another image.  A list recorded in the very step in
+// which it stood outside may miss it, and sweeps instead (vl_tag).
 struct Verlet {
     uint32_t step;          // number of the step about to run (dirty stamps)
     uint32_t all_rebuild;   // every particle sweeps in this step
@@ -145,6 +155,7 @@ struct Verlet {
     uint32_t nmovers;       // particles whose change of cell makes cells sweep
     uint32_t movers_overflow;
     uint32_t dirty_step;    // the last step in which any cell was stamped dirty
+    uint32_t look_step;     // and in which any was stamped to be looked at
     uint32_t rebuilds;      // cell-list rebuilds performed since upload
     uint32_t inc2_bits;     // float bits of the step's largest squared displacement
     uint32_t done_blocks;   // blocks of the step's force kernel that are through
@@ -244,8 +255,12 @@ struct Dev {
     uint8_t *vl_len;      // [np] list length or VL_NONE
     uint32_t *vl_held;    // [np] entries known to hold a slot through their image; 0 says nothing
     float *due;           // [np] the moment after which the particle is searched; below 0: next step
-    uint2 *movers;        // [MOVER_CAP] (old cell, new cell) of the last step's moves that make cells sweep
-    uint32_t *dirty;      // [ncells + 1] step stamp: a neighbour cell changed members
+    uint8_t *vl_tag;      // [np] the step in which the list was recorded, modulo 256
+    uint8_t *outside;     // [np] by uid, of a particle outside the grid: 1 since this step, 2 for longer
+    // [MOVER_CAP] of the last step's moves: (old cell, new cell) around which lists
+    // sweep, or (LOOK, new cell) around which they are looked at
+    uint2 *movers;
+    uint32_t *dirty, *look;   // [ncells + 1] step stamps of cells that sweep, that are looked at
     Verlet *vs;
     // walls
     double *wf_pp;        // [np] wall-0 force by uid
@@ -352,15 +367,21 @@ __device__ __forceinline__ bool grid_cell(const G &P, double x, double y, double
     return c < P.ncells && isfinite(x + y + z);
 }
 
-// Whether some floored cell coordinate of the position lies outside
-// [0, num): the particle is not inside its own cell's box (contact search
-// takes the reference's stencil from the floored coordinates, not the id).
+// The axes (bit k: axis k) on which the position's floored cell coordinate lies
+// outside [0, num): with any, the particle is not inside its own cell's box
+// (contact search takes the reference's stencil from the floored coordinates,
+// not the id).
+template <class G>
+__device__ __forceinline__ uint32_t outside_axes(const G &P, double x, double y, double z)
+{
+    const double f0 = cell_floor(P, 0, x), f1 = cell_floor(P, 1, y), f2 = cell_floor(P, 2, z);
+    return (f0 >= 0.0 && f0 < (double)P.num[0] ? 0u : 1u) | (f1 >= 0.0 && f1 < (double)P.num[1] ? 0u : 2u) |
+           (f2 >= 0.0 && f2 < (double)P.num[2] ? 0u : 4u);
+}
 template <class G>
 __device__ __forceinline__ bool cell_outside(const G &P, double x, double y, double z)
 {
-    const double f0 = cell_floor(P, 0, x), f1 = cell_floor(P, 1, y), f2 = cell_floor(P, 2, z);
-    return !(f0 >= 0.0 && f0 < (double)P.num[0] && f1 >= 0.0 && f1 < (double)P.num[1] &&
-             f2 >= 0.0 && f2 < (double)P.num[2]);
+    return outside_axes(P, x, y, z) != 0u;
 }
 
 // 1 / cellsize for cell_at, or 0 (which it takes for "divide") where that is

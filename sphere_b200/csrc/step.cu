@@ -451,17 +451,15 @@ __device__ __forceinline__ void topo_load_row(const Dev &d, uint32_t *srow, int 
     ts.loaded = true;
 }
 
-// Whether candidate t already holds a slot of the (loaded) row through the
-// periodic image `code`.
+// The slot of the (loaded) row that candidate t holds, or -1.
 template <int TB>
-__device__ __forceinline__ bool in_slot(const uint32_t *srow, int tid, const TopoSlots &ts,
-                                        uint32_t t, uint32_t code)
+__device__ __forceinline__ int slot_of(const uint32_t *srow, int tid, const TopoSlots &ts, uint32_t t)
 {
     for (uint32_t m = ts.occ; m; m &= m - 1) {
         const int i = __ffs(m) - 1;
-        if (srow[i * TB + tid] == t) return dm_get(ts.dm_lo, ts.dm_hi, i) == code;
+        if (srow[i * TB + tid] == t) return i;
     }
-    return false;
+    return -1;
 }
 
 // Overlapping candidate t (storage index) reached through a stencil cell
@@ -514,6 +512,21 @@ __device__ __forceinline__ double pair_gap(const Params &P, double4 xb, uint32_t
     const d3 xab = add(mk(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z), dm);
     len = flen(xab);
     return len - (xa.w + xb.w);
+}
+
+// The periodic image through which the candidate at xb of a list entry is seen
+// from xa: the entry's, or with Params::one_image the nearest, which is the one
+// of any near pair, whatever boundaries the two have crossed since.
+__device__ __forceinline__ uint32_t list_code(const Params &P, double4 xa, double4 xb, uint32_t meta)
+{
+    if (!P.one_image) return vl_code(meta);
+    const double dx = xa.x - xb.x, hx = 0.5 * P.L[0];
+    uint32_t code = dx < -hx ? 1u : (dx > hx ? 2u : 0u);
+    if (P.periodic == 1) {
+        const double dy = xa.y - xb.y, hy = 0.5 * P.L[1];
+        code |= dy < -hy ? 4u : (dy > hy ? 8u : 0u);
+    }
+    return code;
 }
 
 // Contact model 1 processes each candidate as soon as it is found
@@ -743,6 +756,14 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const bool gp_in = gp[0] >= 0 && (uint32_t)gp[0] < nx && gp[1] >= 0 && (uint32_t)gp[1] < ny &&
                        gp[2] >= 0 && (uint32_t)gp[2] < nz;
     const bool use_lists = P.skin > 0.0 && gp_in;
+    // around a particle that is back from outside a periodic boundary every entry
+    // is looked at; a list that was recorded while it stood outside is not used
+    const uint32_t step = __ldcg(&d.vs->step);
+    const bool new_list = d.vl_tag[s] == (uint8_t)(step - 1u);
+    if (__ldcg(&d.vs->look_step) == step && __ldcg(&d.look[d.cell[s]]) == step) {
+        held = 0u;
+        if (new_list) sweep = true;
+    }
     // one more acting pair of model 1
     auto act_on = [&](uint32_t t, uint32_t code) {
         if (va.n == VISC_CAP) visc_spill(d, P, A, s, srow + tid, TB, va);
@@ -775,18 +796,24 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 const uint32_t e = e0 + (uint32_t)j;
                 if (e >= len) break;
                 if ((held >> e) & 1u) continue;
-                const uint32_t t = tv[j], code = vl_code(mv[j]);
-                if (rows && in_slot<TB>(srow, tid, ts, t, code)) {
-                    held |= 1u << e;
-                    continue;
+                const uint32_t t = tv[j];
+                if (rows) {
+                    const int i = slot_of<TB>(srow, tid, ts, t);
+                    if (i >= 0 && dm_get(ts.dm_lo, ts.dm_hi, i) == list_code(P, xa, xr[t], mv[j])) {
+                        held |= 1u << e;
+                        continue;
+                    }
                 }
                 const float w = vl_when(mv[j]);
                 // (a pair of model 1 acts in every step, at rest too)
                 if (VISC ? !(S >= w) : !(S > w)) { due = fminf(due, w); continue; }
                 double ln;
-                const double gap = pair_gap(P, xr[t], code, xa, ln);
+                const double4 xb = xr[t];
+                const uint32_t code = list_code(P, xa, xb, mv[j]);
+                const double gap = pair_gap(P, xb, code, xa, ln);
                 if (VISC ? (gap < 0.0f || gap < P.db) : (gap < 0.0f)) {
                     act |= 1u << e;
+                    if (code != vl_code(mv[j])) d.vl_meta[vl_at(s, e)] = (mv[j] & ~0xfu) | code;
                 } else {
                     const uint32_t meta =
                         vl_meta_of(code, pair_when(S, gap, 1e-6 * ln + (VISC ? P.reach_extra : 0.0)));
@@ -1053,11 +1080,17 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
         }
         if (!VISC) test_later();
         const bool listed = use_lists && !list_overflow;
-        d.vl_len[s] = listed ? (uint8_t)nlist : VL_NONE;
         if (!listed) {
-            // sweeps again next step, over a cell list of that step
+            // searched again next step, over a cell list of that step.  The list of
+            // a particle that stands outside a periodic boundary stays for its
+            // return, unless it may miss another one that is back.
             due = -1.0f;
-            if (P.skin > 0.0) d.vs->want_cells = 1u;
+            const bool stays = P.one_image && !gp_in && !sweep && !new_list && __ldcg(&d.vs->dirty_step) != step;
+            if (!stays) d.vl_len[s] = VL_NONE;
+            if (P.skin > 0.0 && gp_in) d.vs->want_cells = 1u;   // (outside: particle_tail asks)
+        } else {
+            d.vl_len[s] = (uint8_t)nlist;
+            d.vl_tag[s] = (uint8_t)step;
         }
     }
 
@@ -1112,7 +1145,7 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
     const uint32_t lane = (uint32_t)tid & 31u;
     const uint32_t base = ((blockIdx.x * TB + (uint32_t)tid) >> 5) * (32u * span);
     const Verlet &V = *d.vs;
-    const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == V.step;
+    const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == V.step, look = V.look_step == V.step;
     const float S = V.moved;
     // bit j: particle base + 32 j + lane is searched / must sweep
     uint32_t need = 0, swp = 0;
@@ -1123,7 +1156,7 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
         if (s >= np) continue;
         const float due = d.due[s];
         const bool sw = all || (dirty && d.dirty[d.cell[s]] == V.step);
-        if (!sw && !(S > due)) {
+        if (!sw && !(S > due) && !(look && d.look[d.cell[s]] == V.step)) {
             if (VISC) d.c1acc[s] = make_double4(0.0, 0.0, 0.0, 0.0);
             continue;
         }
@@ -1461,6 +1494,7 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
         if (x.x < P.origo[0]) x.x += P.L[0];
         if (x.x > P.L[0]) x.x -= P.L[0];
     }
+    const uint32_t wrapped = (x.x != xa.x ? 1u : 0u) | (x.y != xa.y ? 2u : 0u);   // axes
     vel0.x += acc.x * dt;
     vel0.y += acc.y * dt;
     vel0.z += acc.z * dt;
@@ -1508,29 +1542,40 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
     const uint32_t c_old = R.cell();
     if (out) {
         // outside its cell's box: its own search sweeps, over a fresh list
-        d.rebuild[REBUILD_NEXT] = 1u;
+        // (past the last cell its stencil is empty)
+        if (c != d.ncells_all || c != c_old) d.rebuild[REBUILD_NEXT] = 1u;
         d.due[s] = -1.0f;
+        d.outside[d.uid[s]] = cell_outside(P, xa.x, xa.y, xa.z) ? 2 : 1;
     }
-    if (c != c_old) {
+    // (out through one side and into the next cell on another axis, a particle
+    // can come back into the cell that its id aliased)
+    if (c != c_old || (wrapped != 0u && c != d.ncells_all)) {
         d.cell[s] = c;
         // A move between neighbouring cells inside the grid leaves every
         // candidate list as it is (the lists are sets of near pairs, ordered
-        // by their cells only when needed).  Any other -- through a periodic
-        // boundary, or from or to a place outside the cells' boxes -- changes
+        // by their cells only when needed), and so does one out through a
+        // periodic boundary.  One back in by a period has the lists around
+        // looked at.  Any other -- or where axes are too short for that -- changes
         // images or what a stencil reaches: the cells around sweep again.
-        bool hard = out || !P.set_lists || c == d.ncells_all || c_old == d.ncells_all ||
-                    cell_outside(P, xa.x, xa.y, xa.z);
-        if (!hard) {
+        const uint32_t was = outside_axes(P, xa.x, xa.y, xa.z), is = out ? outside_axes(P, x.x, x.y, x.z) : 0u;
+        bool hard = !P.set_lists || c == d.ncells_all || c_old == d.ncells_all, look = false;
+        if (!hard && (was | is | wrapped)) {
+            const uint32_t sides = P.periodic == 1 ? 3u : 1u;   // with one_image
+            const bool leaves = !was && !wrapped && (is & ~sides) == 0u;
+            look = P.one_image && !is && wrapped == was && d.outside[d.uid[s]] == 1;
+            hard = !look && !(P.one_image && leaves);
+        }
+        if (!hard && !(was | is)) {
             const uint32_t p = c_old - P.cell_base, q = c - P.cell_base;
             const uint32_t nx = P.num[0], ny = P.num[1];
             const int dx = (int)(q % nx) - (int)(p % nx), dy = (int)(q / nx % ny) - (int)(p / nx % ny),
                       dz = (int)(q / (nx * ny)) - (int)(p / (nx * ny));
             hard = dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1;
         }
-        if (hard || P.eager) d.rebuild[REBUILD_NEXT] = 1u;
-        if (hard && P.skin > 0.0) {
+        if (hard || look || P.eager) d.rebuild[REBUILD_NEXT] = 1u;
+        if ((hard || look) && P.skin > 0.0) {
             const uint32_t m = atomicAdd(&V.nmovers, 1u);
-            if (m < MOVER_CAP) d.movers[m] = make_uint2(c_old, c);
+            if (m < MOVER_CAP) d.movers[m] = make_uint2(hard ? c_old : LOOK, c);
             else V.movers_overflow = 1u;
         }
     }
@@ -2058,7 +2103,8 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
             if (s < np) {
                 sweep = __ldcg(&V.all_rebuild) != 0u ||
                         (__ldcg(&V.dirty_step) == step && __ldcg(&d.dirty[d.cell[s]]) == step);
-                need = sweep || S > d.due[s];
+                need = sweep || S > d.due[s] ||
+                       (__ldcg(&V.look_step) == step && __ldcg(&d.look[d.cell[s]]) == step);
             }
             if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, S, va);
             __syncwarp();

@@ -124,3 +124,80 @@ def test_the_fastest_grain_of_a_split_warp_sets_the_clock(oracle_libs, fast, spa
         sim.step(120)
         sim.sync()
         assert mismatches(sim.download(), want, ALL) == []
+
+
+def _crossing_pairs(periodic, reach, sides, seed):
+    """Pairs in contact that travel out through a periodic side together or one
+    after the other, at every phase against the cells of the other axis: some cross
+    into the next cell in the step of their return."""
+    rng = np.random.default_rng(seed)
+    r, dt, num = 1e-3, 2e-6, 8 if reach == "one_image" else 3
+    cell = 2.05e-3 if reach == "one_image" else 1.7e-3   # an axis of 5.1 mm: under 2.5 reaches
+    L = num * cell
+    x, vel = [], []
+    for i in range(36):
+        hi = sides == "upper" or (sides == "both" and i % 2 == 0)
+        ax = (i // 2) % 2 if periodic == 1 else 0
+        k = 3 + i                                  # the step that takes it out
+        v = np.zeros(3)
+        p = np.array([0.0, 0.0, 2.5e-3 + 4.6e-3 * i])
+        v[ax] = 0.6 if hi else -0.6
+        p[ax] = (L if hi else 0.0) - (k - 0.5) * dt * v[ax]
+        v[1 - ax] = rng.choice([-0.7, 0.7])        # into the next cell one step later, or about then
+        p[1 - ax] = cell * rng.integers(1, num) - (k + 0.5 + rng.choice([0.0, 0.0, 1.0, -1.0])) * dt * v[1 - ax]
+        d = np.zeros(3)
+        d[rng.integers(0, 3)] = 2 * r - 1e-7
+        if d[ax] != 0.0 and hi:
+            d = -d
+        x += [p, p + d]
+        vel += [v, v]
+    sb = scenes.collision(n=len(x), seed=1, periodic=periodic, wmax=20.0, g=(0.0, 0.0, 0.0), dt=dt, k_n=500.0,
+                          k_t=500.0, gamma_n=0.0)
+    sb.L = np.array([L, L if periodic == 1 else 3 * L, 4.6e-3 * 37])
+    sb.num = np.array([num, num if periodic == 1 else 3 * num, 78], dtype=np.uint32)
+    sb.x, sb.vel, sb.radius = np.array(x) % np.where(np.arange(3) < 2, sb.L, 1e9), np.array(vel), np.full(len(x), r)
+    return sb
+
+
+@both_kernels
+@pytest.mark.parametrize("reach", ["one_image", "short_axis"])
+@pytest.mark.parametrize("periodic, sides", [(1, "upper"), (1, "lower"), (1, "both"), (2, "both")])
+@pytest.mark.parametrize("seed", [1, 2])
+def test_grains_that_cross_a_periodic_side(oracle_libs, periodic, sides, reach, seed, span):
+    """The images of list entries and slots, and the lists recorded while a grain
+    stood outside, with epochs that end in the steps of the crossings."""
+    sb = _crossing_pairs(periodic, reach, sides, seed)
+    rc, want, _ = run_oracle(oracle_libs["orc"], sb, 70)
+    assert rc == 0 and int((want.contacts != sb.np).sum()) >= sb.np // 2
+    for skin in (0.1, 0.01, 0.004):
+        with Simulation(config_from_spherebin(sb), verlet_skin=skin, topo_span=span) as sim:
+            sim.upload(state_from_spherebin(sb))
+            for k in (20, 1, 49):
+                sim.step(k)
+            sim.sync()
+            assert mismatches(sim.download(), want, ALL) == [], skin
+
+
+@both_kernels
+@pytest.mark.parametrize("model", [1, 2])
+@pytest.mark.parametrize("cell", [2.0, 2.4, 3.0])
+def test_sheared_beds_with_periodic_sides(oracle_libs, cell, model, span):
+    """Grains cross the sides in nearly every step, in a moving contact network."""
+    side = (1500 * 8.2e-9 / 0.35) ** (1 / 3)
+    sb = scenes.collision(n=1500, seed=6, periodic=1, box=(1.02 * side, 1.02 * side, 1.2 * side + 0.012),
+                          phi_target=0.35, k_n=500.0, k_t=500.0, gamma_n=0.01, vmax=2.0, straddle=True)
+    sb.vel = sb.vel + np.stack([6.0 * (2 * sb.x[:, 2] / sb.L[2] - 1), 0 * sb.x[:, 0], 0 * sb.x[:, 0]], 1)
+    sb.num = np.maximum(1, np.floor(sb.L / (cell * 1.6e-3))).astype(np.uint32)
+    if model == 1:
+        sb = with_model(sb, 1, kappa=0.05, V_b=1e-12, db=1e-4)
+    rc, want, orun = run_oracle(oracle_libs["orc"], sb, 150)
+    assert rc == 0
+    for skin in (0.1, 0.3):
+        with Simulation(config_from_spherebin(sb), verlet_skin=skin, topo_span=span) as sim:
+            sim.upload(state_from_spherebin(sb))
+            sim.step(150)
+            sim.sync()
+            got = sim.download()
+            _, perm, _, _ = sim.cells()
+        assert mismatches(got, want, ALL) == [], skin
+        assert np.array_equal(perm, orun.perm)
