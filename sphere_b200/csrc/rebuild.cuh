@@ -67,11 +67,15 @@ __device__ __forceinline__ bool lists_given_up(const Dev &d)
 // number; particles in stamped cells sweep their stencil again, or, around a
 // particle that is back from outside a periodic boundary, look at their lists.
 // Periodic axes wrap as in findDistMod.
+//
+// A thread a cell: one a move took 20 us for the one or two moves of a step, 125
+// stores after one another.
 __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32_t stride)
 {
     Verlet &V = *d.vs;
     const uint32_t n = min(__ldcg(&V.nmovers), MOVER_CAP), step = __ldcg(&V.step);
-    for (uint32_t e = first; e < 2 * n; e += stride) {
+    for (uint32_t w = first; w < 2u * 125u * n; w += stride) {
+        const uint32_t e = w / 125u;
         const uint2 mv = __ldcg(&d.movers[e >> 1]);
         const uint32_t cg = (e & 1u) ? mv.y : mv.x;
         if (cg >= d.ncells_all) continue;
@@ -88,29 +92,23 @@ __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32
             inst = lo;
         }
         const Params &P = d.prm[inst];
-        const uint32_t c = cg - P.cell_base;
-        const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
-        const int32_t cx = (int32_t)(c % nx), cy = (int32_t)((c / nx) % ny), cz = (int32_t)(c / (nx * ny));
-        const int R = P.wide ? 2 : 1;
-        for (int oz = -R; oz <= R; ++oz) {
-            const int32_t z = cz + oz;
-            if (z < 0 || z >= (int32_t)nz) continue;
-            for (int oy = -R; oy <= R; ++oy) {
-                int32_t y = cy + oy;
-                if (y < 0 || y >= (int32_t)ny) {
-                    if (P.periodic != 1) continue;
-                    y = (y + (int32_t)ny) % (int32_t)ny;
-                }
-                for (int ox = -R; ox <= R; ++ox) {
-                    int32_t x = cx + ox;
-                    if (x < 0 || x >= (int32_t)nx) {
-                        if (P.periodic != 1 && P.periodic != 2) continue;
-                        x = (x + (int32_t)nx) % (int32_t)nx;
-                    }
-                    stamps[P.cell_base + (uint32_t)x + (uint32_t)y * nx + (nx * ny) * (uint32_t)z] = step;
-                }
-            }
+        const uint32_t c = cg - P.cell_base, o = w % 125u;
+        const int32_t nx = (int32_t)P.num[0], ny = (int32_t)P.num[1], nz = (int32_t)P.num[2];
+        const int32_t ox = (int32_t)(o % 5u) - 2, oy = (int32_t)(o / 5u % 5u) - 2, oz = (int32_t)(o / 25u) - 2;
+        const int32_t R = P.wide ? 2 : 1;
+        if (max(max(abs(ox), abs(oy)), abs(oz)) > R) continue;
+        int32_t x = (int32_t)(c % (uint32_t)nx) + ox, y = (int32_t)(c / (uint32_t)nx % (uint32_t)ny) + oy;
+        const int32_t z = (int32_t)(c / (uint32_t)(nx * ny)) + oz;
+        if (z < 0 || z >= nz) continue;
+        if (y < 0 || y >= ny) {
+            if (P.periodic != 1) continue;
+            y = (y + ny) % ny;
         }
+        if (x < 0 || x >= nx) {
+            if (P.periodic != 1 && P.periodic != 2) continue;
+            x = (x + nx) % nx;
+        }
+        stamps[P.cell_base + (uint32_t)x + (uint32_t)y * (uint32_t)nx + (uint32_t)(nx * ny) * (uint32_t)z] = step;
     }
 }
 
