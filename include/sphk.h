@@ -271,7 +271,8 @@ int sph_render(sph_ctx *ctx, const sph_render_opts *opts, uint8_t *rgba);
  * the context keeps the checkpoints' memory, and the tape's while the
  * contexts of the process together keep no more of those than an eighth of
  * the device's memory, for its next sph_diff_begin (a calibration loop's);
- * sph_destroy frees both. */
+ * sph_destroy frees both, and a call of any context that runs out of device
+ * memory frees every kept tape before it gives up. */
 int sph_diff_begin(sph_ctx *ctx, const double *mu, uint32_t checkpoint_every);
 int sph_diff_backward(sph_ctx *ctx, const double *x_bar, const double *v_bar, double *grad_params,
                       double *grad_mu, double *x0_bar, double *v0_bar);

@@ -53,7 +53,7 @@ def _stale(target: Path, sources) -> bool:
 def build_lib(force=False, verbose_ptxas=False) -> Path:
     srcs = [CSRC / s for s in KERNEL_SOURCES]
     deps = srcs + [CSRC / "sphk_internal.cuh", CSRC / "diff_law.h", CSRC / "diff_step.cuh", CSRC / "rebuild.cuh",
-                   CSRC / "barrier_count.h",
+                   CSRC / "barrier_count.h", CSRC / "kept.h",
                    ROOT / "include" / "sphk.h"]
     if not force and not _stale(LIB, deps):
         return LIB

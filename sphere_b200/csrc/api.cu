@@ -1,10 +1,10 @@
 // api.cu -- the C ABI of libsphk (include/sphk.h): contexts, host<->device
 // transfer in the reference's host layout, and stepping through CUDA graphs.
 #include "diff_step.cuh"
+#include "kept.h"
 #include "../../include/sphk.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -119,13 +119,13 @@ struct sph_ctx {
     size_t rt_bytes = 0;
     size_t ckpt_bytes = 0;                // size of one pooled buffer
     cudaEvent_t ckpt_ev = nullptr;        // orders a checkpoint copy against the caller's stream
-    // the tape and the adjoint arrays; sph_diff_end keeps them (and the graphs
-    // that hold them) for the next session with the same checkpoint interval,
-    // within KEPT_SHARE of the device's memory over all contexts
+    // the tape and the adjoint arrays; sph_diff_end parks them in g_kept (and
+    // keeps the graphs that hold them) for the next session with the same
+    // checkpoint interval
     std::vector<void *> diff_allocs;
-    size_t diff_bytes = 0;
+    size_t diff_bytes = 0;                // of diff_allocs
+    size_t device_total = 0;              // the device's memory
     uint32_t diff_K = 0;                  // the interval they are sized for (0: none)
-    size_t kept_bytes = 0;                // counted in g_kept_bytes
     struct {
         double *mu_p;
         double4 *x, *v, *w;
@@ -144,10 +144,11 @@ struct sph_ctx {
 
 namespace {
 
-// Bytes of differentiable sessions kept after their end, over all contexts
-// of the process: at most 1 / KEPT_SHARE of the device's memory.
+// Arrays of differentiable sessions kept after their end, over all contexts
+// of the process: at most 1 / KEPT_SHARE of the device's memory, and only until
+// an allocation needs it.
 constexpr size_t KEPT_SHARE = 8;
-std::atomic<size_t> g_kept_bytes{0};
+KeptArrays g_kept;
 
 int fail(sph_ctx *c, int code, const std::string &msg)
 {
@@ -156,6 +157,26 @@ int fail(sph_ctx *c, int code, const std::string &msg)
         if (c->sticky == SPH_OK && code != SPH_ERR_BAD_INPUT) c->sticky = code;
     }
     return code;
+}
+
+// cudaMalloc, or cudaMallocAsync on a stream; out of memory it frees what ended
+// sessions have kept on the context's device, the current one, and tries again.
+cudaError_t device_malloc(sph_ctx *c, void **p, size_t bytes, cudaStream_t st = nullptr)
+{
+    return malloc_or_give_back(
+        [&] { return st ? cudaMallocAsync(p, bytes, st) : cudaMalloc(p, bytes); }, cudaErrorMemoryAllocation,
+        [&] {
+            cudaGetLastError();   // the failed try's
+            return g_kept.give_back(c->device, [](void *q) { cudaFree(q); });
+        });
+}
+template <typename T>
+cudaError_t device_malloc(sph_ctx *c, T **p, size_t bytes, cudaStream_t st = nullptr)
+{
+    void *q = nullptr;
+    const cudaError_t e = device_malloc(c, &q, bytes, st);
+    *p = static_cast<T *>(q);
+    return e;
 }
 
 #define CK(call)                                                                      \
@@ -170,7 +191,7 @@ int dalloc(sph_ctx *c, T **p, size_t count, std::vector<void *> *owner = nullptr
 {
     const size_t bytes = sizeof(T) * (count ? count : 1);
     void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, bytes);
+    cudaError_t e = device_malloc(c, &q, bytes);
     if (e != cudaSuccess) return fail(c, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     e = clear ? cudaMemsetAsync(q, 0, bytes, c->stream) : cudaSuccess;
     if (e != cudaSuccess) return fail(c, SPH_ERR_CUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
@@ -1197,9 +1218,9 @@ int sph_get_contacts(sph_ctx *c, uint32_t *contacts, double *distmod, double *de
     const size_t n = (size_t)np * NC;
     uint32_t *dc = nullptr;
     double4 *ddm = nullptr, *ddt = nullptr;
-    CK(cudaMallocAsync(&dc, n * 4, c->stream));
-    CK(cudaMallocAsync(&ddm, n * 32, c->stream));
-    CK(cudaMallocAsync(&ddt, n * 32, c->stream));
+    CK(device_malloc(c, &dc, n * 4, c->stream));
+    CK(device_malloc(c, &ddm, n * 32, c->stream));
+    CK(device_malloc(c, &ddt, n * 32, c->stream));
     k_rows_to_user<<<div_up(n, 256), 256, 0, c->stream>>>(c->d, dc, ddm, ddt, c->a);
     if (contacts) CK(cudaMemcpyAsync(contacts, dc, n * 4, cudaMemcpyDeviceToHost, c->stream));
     if (distmod) CK(cudaMemcpyAsync(distmod, ddm, n * 32, cudaMemcpyDeviceToHost, c->stream));
@@ -1220,7 +1241,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
     const uint32_t np = c->np_all, nc = c->ncells_all;
     uint32_t *b = nullptr;
     const size_t words = (size_t)np * 2 + (size_t)nc * 2;
-    CK(cudaMallocAsync(&b, words * 4, c->stream));
+    CK(device_malloc(c, &b, words * 4, c->stream));
     uint32_t *cs = b, *pm = b + np, *st = b + 2 * (size_t)np, *en = st + nc;
     const unsigned int n = (np > nc + 1 ? np : nc + 1);
     uint32_t made = 0;   // the status of a list made here
@@ -1238,7 +1259,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
                      o_members = part(np), o_start = part((size_t)nc + 2),
                      o_fill = part((size_t)nc + 1), o_scan = part(SCAN_TILES), o_word = part(4),
                      o_vs = part(sizeof(Verlet) / 4);
-        CK(cudaMallocAsync(&tmp, bytes, c->stream));
+        CK(device_malloc(c, &tmp, bytes, c->stream));
         CK(cudaMemsetAsync(tmp, 0, bytes, c->stream));   // a list given up stays in range
         auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
         q.cell = at(o_cell); q.cellorder = at(o_order); q.pos = at(o_pos);
@@ -1282,7 +1303,7 @@ int sph_get_stats(sph_ctx *c, sph_stats *out)
     memset(out, 0, sizeof(*out));
     if (c->uploaded) {
         unsigned long long *cnt = nullptr;
-        CK(cudaMallocAsync(&cnt, 8, c->stream));
+        CK(device_malloc(c, &cnt, 8, c->stream));
         CK(cudaMemsetAsync(cnt, 0, 8, c->stream));
         k_count_contacts<<<592, 256, 0, c->stream>>>(c->d.cmask, c->np_all, cnt);
         unsigned long long v = 0;
@@ -1298,7 +1319,7 @@ int sph_get_stats(sph_ctx *c, sph_stats *out)
     }
     out->steps = c->steps;
     out->relayouts = c->relayouts;
-    out->device_bytes = c->device_bytes + c->diff_bytes +
+    out->device_bytes = c->device_bytes + c->diff_bytes + g_kept.parked(c) +
                         (c->ckpts.size() + c->ckpt_pool.size()) * c->ckpt_bytes;
     CK(cudaStreamSynchronize(c->stream));   // the caller's arrays are complete
     return SPH_OK;
@@ -1359,7 +1380,7 @@ static int save_ckpt(sph_ctx *c, sph_ctx::Ckpt &k)
         c->ckpt_pool.pop_back();
     } else {
         // fully overwritten below, so no clearing
-        CK(cudaMalloc(&k.buf, bytes));
+        CK(device_malloc(c, &k.buf, bytes));
     }
     size_t off = 0;
     for (auto &f : ckpt_fields(c, c->a)) {
@@ -1449,14 +1470,13 @@ static void free_diff(sph_ctx *c)
 {
     leave_diff(c);
     drop_diff_graphs(c);
+    g_kept.take(c, c->diff_allocs);
     for (void *p : c->diff_allocs) cudaFree(p);
     c->diff_allocs.clear();
     c->bwd_scratch = nullptr;
     c->diff_bytes = 0;
     c->diff_K = 0;
     c->adj = AdjDev{};
-    g_kept_bytes -= c->kept_bytes;
-    c->kept_bytes = 0;
 }
 
 int sph_diff_begin(sph_ctx *c, const double *mu, uint32_t checkpoint_every)
@@ -1477,7 +1497,8 @@ int sph_diff_begin(sph_ctx *c, const double *mu, uint32_t checkpoint_every)
     auto &T = c->tape;
     std::vector<void *> *own = &c->diff_allocs;
     int rc = SPH_OK;
-    if (c->diff_K != checkpoint_every) {
+    c->diff_bytes = c->diff_K == checkpoint_every ? g_kept.take(c, c->diff_allocs) : 0;
+    if (c->diff_bytes == 0) {   // none kept for this interval, or given back since
         free_diff(c);
         // the tape's rows are written before they are read
 #define ALD(ptr, n, clear) \
@@ -1590,13 +1611,12 @@ int sph_diff_end(sph_ctx *c)
     leave_diff(c);
     // the session's arrays stay for the next one while all contexts together
     // keep no more than their share of the device's memory
-    if (c->kept_bytes != c->diff_bytes) {
-        size_t free_b = 0, total_b = 0;
-        CK(cudaMemGetInfo(&free_b, &total_b));
-        g_kept_bytes -= c->kept_bytes;
-        c->kept_bytes = c->diff_bytes;
-        if ((g_kept_bytes += c->kept_bytes) > total_b / KEPT_SHARE) free_diff(c);
+    if (c->device_total == 0) {
+        size_t free_b = 0;
+        CK(cudaMemGetInfo(&free_b, &c->device_total));
     }
+    if (g_kept.park(c, c->device, c->diff_allocs, c->diff_bytes, c->device_total / KEPT_SHARE)) c->diff_bytes = 0;
+    else free_diff(c);
     CK(cudaMemsetAsync(c->d.cflag, 1, div_up(c->np_all, 32), c->stream));
     // every list is looked at again (due below 0)
     CK(cudaMemsetAsync(c->d.due, 0xbf, (size_t)c->np_all * 4, c->stream));
@@ -1696,7 +1716,7 @@ int sph_render(sph_ctx *c, const sph_render_opts *o, uint8_t *rgba)
         if (c->rt_buf) cudaFree(c->rt_buf);
         c->rt_buf = nullptr;
         c->rt_bytes = 0;
-        CK(cudaMalloc(&c->rt_buf, need));
+        CK(device_malloc(c, &c->rt_buf, need));
         c->rt_bytes = need;
     }
     char *base = static_cast<char *>(c->rt_buf);

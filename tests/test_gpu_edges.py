@@ -124,6 +124,42 @@ def test_sessions_take_up_kept_arrays_or_replace_them():
             assert np.allclose(g["x0"], g_own["x0"], rtol=1e-9, atol=1e-12 * np.abs(g_own["x0"]).max())
 
 
+def test_a_kept_tape_gives_way_to_a_session_that_needs_the_memory():
+    """With less of the device free than a tape takes, a context's session gets the
+    tape that another context has kept since its own ended; that one's next session
+    allocates anew."""
+    torch = pytest.importorskip("torch")
+    sb = scenes.collision(n=4000, seed=3, vmax=0.2, wmax=50.0)
+    w = np.random.default_rng(8).normal(size=(4000, 3))
+
+    def session(sim):
+        sim.upload(state_from_spherebin(sb))
+        sim.diff_begin(checkpoint_every=64)
+        sim.step(20)
+        sim.sync()
+        g = sim.diff_backward(w, 1e-3 * w)
+        sim.diff_end()
+        return g
+
+    with Simulation(config_from_spherebin(sb)) as a, Simulation(config_from_spherebin(sb)) as b:
+        b.upload(state_from_spherebin(sb))
+        alone = a.stats()["device_bytes"]
+        first = session(a)
+        kept = a.stats()["device_bytes"] - alone
+        assert kept > 250e6   # 64 rows of 4000 particles, 1 KB each
+        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info()
+        fill = torch.empty(free - int(0.8 * kept), dtype=torch.uint8, device="cuda")
+        second = session(b)
+        assert a.stats()["device_bytes"] - alone < 0.2 * kept
+        del fill
+        torch.cuda.empty_cache()
+        third = session(a)
+    for g in (second, third):
+        for k in ("k_n", "k_t", "gamma_n"):   # only the order of atomic additions may differ
+            assert abs(g[k] - first[k]) <= 1e-11 * abs(first[k])
+
+
 # the terms the linear law leaves out: the capillary force where kappa is 0
 # (either sign), lengths only compared with zero (velocities 0, below and
 # above the smallest float square), the pressure of steps inside a call
