@@ -1239,11 +1239,23 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
     CK(cudaSetDevice(c->device));
     CK(cudaDeviceSynchronize());
     const uint32_t np = c->np_all, nc = c->ncells_all;
-    uint32_t *b = nullptr;
-    const size_t words = (size_t)np * 2 + (size_t)nc * 2;
-    CK(device_malloc(c, &b, words * 4, c->stream));
-    uint32_t *cs = b, *pm = b + np, *st = b + 2 * (size_t)np, *en = st + nc;
     const unsigned int n = (np > nc + 1 ? np : nc + 1);
+    size_t bytes = 0;
+    auto part = [&](size_t count) { const size_t at = bytes; bytes += (count + 31) / 32 * 128; return at; };
+    // the caller's four arrays, then the arrays of a list made here
+    const size_t o_cs = part(np), o_pm = part(np), o_st = part(nc), o_en = part(nc), o_list = bytes;
+    const size_t o_cell = part(np), o_order = part(np), o_pos = part(np), o_xs = part(4 * (size_t)np),
+                 o_members = part(np), o_start = part((size_t)nc + 2),
+                 o_fill = part((size_t)nc + 1), o_scan = part(SCAN_TILES), o_word = part(4),
+                 o_vs = part(sizeof(Verlet) / 4);
+    // in the context's scratch, which has the room unless the cells are many
+    char *own = nullptr, *tmp = static_cast<char *>(c->scratch);
+    if (bytes > c->scratch_bytes) {
+        CK(device_malloc(c, &own, bytes, c->stream));
+        tmp = own;
+    }
+    auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
+    uint32_t *cs = at(o_cs), *pm = at(o_pm), *st = at(o_st), *en = at(o_en);
     uint32_t made = 0;   // the status of a list made here
     if (c->since_relayout == 0) {
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(c->d, cs, pm, st, en);
@@ -1252,16 +1264,7 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         // here, in arrays of its own, from the start positions of the last
         // step, which that step left in the other buffer
         Dev q = c->d;
-        char *tmp = nullptr;
-        size_t bytes = 0;
-        auto part = [&](size_t count) { const size_t at = bytes; bytes += (count + 31) / 32 * 128; return at; };
-        const size_t o_cell = part(np), o_order = part(np), o_pos = part(np), o_xs = part(4 * (size_t)np),
-                     o_members = part(np), o_start = part((size_t)nc + 2),
-                     o_fill = part((size_t)nc + 1), o_scan = part(SCAN_TILES), o_word = part(4),
-                     o_vs = part(sizeof(Verlet) / 4);
-        CK(device_malloc(c, &tmp, bytes, c->stream));
-        CK(cudaMemsetAsync(tmp, 0, bytes, c->stream));   // a list given up stays in range
-        auto at = [&](size_t o) { return reinterpret_cast<uint32_t *>(tmp + o); };
+        CK(cudaMemsetAsync(tmp + o_list, 0, bytes - o_list, c->stream));   // a list given up stays in range
         q.cell = at(o_cell); q.cellorder = at(o_order); q.pos = at(o_pos);
         q.xs[c->a ^ 1] = reinterpret_cast<float4 *>(tmp + o_xs);
         q.xs[c->a] = reinterpret_cast<float4 *>(tmp + o_members);
@@ -1273,14 +1276,13 @@ int sph_get_cells(sph_ctx *c, uint32_t *cell_sorted, uint32_t *perm, uint32_t *c
         CK(launch_rebuild(q, np, nc, c->a ^ 1, c->stream));
         k_cells_out<<<div_up(n, 256), 256, 0, c->stream>>>(q, cs, pm, st, en);
         CK(cudaMemcpyAsync(&made, q.status, 4, cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaFreeAsync(tmp, c->stream));
     }
     CK(cudaGetLastError());
     if (cell_sorted) CK(cudaMemcpyAsync(cell_sorted, cs, (size_t)np * 4, cudaMemcpyDeviceToHost, c->stream));
     if (perm) CK(cudaMemcpyAsync(perm, pm, (size_t)np * 4, cudaMemcpyDeviceToHost, c->stream));
     if (cell_start) CK(cudaMemcpyAsync(cell_start, st, (size_t)nc * 4, cudaMemcpyDeviceToHost, c->stream));
     if (cell_end) CK(cudaMemcpyAsync(cell_end, en, (size_t)nc * 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaFreeAsync(b, c->stream));
+    if (own) CK(cudaFreeAsync(own, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     if (made & ST_TIMEOUT) return fail(c, SPH_ERR_TIMEOUT, status_msg(SPH_ERR_TIMEOUT));
     return SPH_OK;

@@ -71,10 +71,12 @@ def test_lists_past_2_32_arrivals(oracle_libs, span):
         sim.step(150)
         sim.sync()
         got, lists = sim.download(), sim.stats()["cell_rebuilds"] - lists
+        _, perm, _, _ = sim.cells()
     assert lists > 80
-    rc, want, _ = run_oracle(oracle_libs["orc"], sb, 150)
+    rc, want, orun = run_oracle(oracle_libs["orc"], sb, 150)
     assert rc == 0
     assert mismatches(got, want, fields) == []
+    assert np.array_equal(perm, orun.perm)
 
 
 @pytest.mark.gpu
