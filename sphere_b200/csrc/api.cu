@@ -1721,11 +1721,12 @@ int sph_render(sph_ctx *c, const sph_render_opts *o, uint8_t *rgba)
         CK(device_malloc(c, &c->rt_buf, need));
         c->rt_bytes = need;
     }
+    // doubles and keys first: the image may have an odd number of pixels
     char *base = static_cast<char *>(c->rt_buf);
     auto *mx = reinterpret_cast<unsigned long long *>(base);
     auto *keys = reinterpret_cast<unsigned long long *>(base + 32);
-    auto *img = reinterpret_cast<uchar4 *>(base + 32 + pixels * 8);
-    auto *values = reinterpret_cast<double *>(base + 32 + pixels * 12);
+    auto *values = reinterpret_cast<double *>(base + 32 + pixels * 8);
+    auto *img = reinterpret_cast<uchar4 *>(base + 32 + pixels * 8 + np * 8);
     auto *rays = reinterpret_cast<float *>(base + 32 + pixels * 12 + np * 8);
     cudaStream_t st = c->stream;
     // DEM::maxPos on the device, then the camera on the host

@@ -78,3 +78,14 @@ def test_gpu_render_rejects_oversized_images():
         with pytest.raises(SphError) as e:
             sim.render(0, 1.0, 0.0, 8192, 4096)
         assert e.value.code == -8
+
+
+@pytest.mark.parametrize("method", range(6))
+@pytest.mark.parametrize("w, h", [(33, 21), (151, 99), (31, 32), (1, 1)])
+def test_gpu_render_of_an_odd_number_of_pixels(oracle_libs, method, w, h):
+    """The colour-map values are doubles behind per-pixel words."""
+    import pyoracle
+    sb, st = render_scene()
+    want, _ = pyoracle.render(oracle_libs["orc"], oracle_libs["orc"], st, sb.L, method, 0.05, 0.0, w, h)
+    got = gpu_render(sb, st, method, 0.05, 0.0, w, h)
+    assert np.array_equal(got[..., :3], want[..., :3])
