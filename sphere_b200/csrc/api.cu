@@ -70,6 +70,7 @@ struct sph_ctx {
     std::vector<void *> allocs;
     size_t device_bytes = 0;
     // the graphs of a step, of the plain and of the differentiable one
+    // (step_graphs)
     struct StepGraphs {
         cudaGraphExec_t multi[2] = {nullptr, nullptr};
         cudaGraphExec_t single[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
@@ -488,12 +489,19 @@ void drop_graphs(sph_ctx *c)
     drop_diff_graphs(c);
 }
 
+// The graphs of the present kind of step: the differentiable one's, or with a
+// flow (which is never differentiable) the set for the pressure buffers' parity.
+sph_ctx::StepGraphs &step_graphs(sph_ctx *c)
+{
+    return c->graphs[c->diff ? 1 : (c->darcy_on ? c->dflip & 1 : 0)];
+}
+
 int ensure_graphs(sph_ctx *c)
 {
     // graphs carry the force kernel's constants: an upload that changed one
     // (the skin, esv_skip) captures them again
     const ForceConsts fc = force_consts(c->hp);
-    sph_ctx::StepGraphs &S = c->graphs[c->diff ? 1 : 0];
+    sph_ctx::StepGraphs &S = step_graphs(c);
     if (S.for_k == c->graph_steps && S.single[0][0] && std::memcmp(&fc, &S.fc, sizeof(fc)) == 0)
         return SPH_OK;
     drop_step_graphs(S);
@@ -811,9 +819,8 @@ int sph_upload(sph_ctx *c, const sph_host_state *h)
     const size_t np = c->np_all, nb0 = P.nb0;
     Dev &d = c->d;
     const int A = 0;
-    // the Darcy pressure buffers keep their roles across the parity reset;
-    // graphs hold the buffer of each step, so they are captured again
-    if (c->darcy_on && c->a != A) drop_graphs(c);
+    // the Darcy pressure buffers keep their roles across the parity reset
+    // (graphs hold the buffer of each step: there is a set for either)
     c->dflip ^= c->a ^ A;
     c->a = A;
     {
@@ -1107,14 +1114,14 @@ static int step_plain(sph_ctx *c, uint64_t nsteps, void *stream)
         const bool last_chunk = (i + room == nsteps);
         // multi-step graphs while more than one graph's worth remains
         while (room > K || (room == K && !last_chunk)) {
-            CK(cudaGraphLaunch(c->graphs[c->diff ? 1 : 0].multi[c->a], st));
+            CK(cudaGraphLaunch(step_graphs(c).multi[c->a], st));
             c->a ^= (int)(K & 1u);
             room -= K; i += K; c->since_relayout += K; c->steps += K;
             for (uint64_t k = 0; k < K; ++k) c->t_host += c->hp.dt;
         }
         while (room > 0) {
             const int w = (room == 1 && last_chunk) ? 1 : 0;
-            CK(cudaGraphLaunch(c->graphs[c->diff ? 1 : 0].single[c->a][w], st));
+            CK(cudaGraphLaunch(step_graphs(c).single[c->a][w], st));
             c->a ^= 1;
             room -= 1; i += 1; c->since_relayout += 1; c->steps += 1;
             c->t_host += c->hp.dt;

@@ -151,6 +151,7 @@ struct Verlet {
     uint32_t step;          // number of the step about to run (dirty stamps)
     uint32_t all_rebuild;   // every particle sweeps in this step
     float moved;            // the epoch's clock at the start of the step
+    uint32_t crossed;       // some particle has stood outside: look, images may change
     uint32_t want_cells;    // a particle without a list sweeps in the next step too
     uint32_t nmovers;       // particles whose change of cell makes cells sweep
     uint32_t movers_overflow;
@@ -374,6 +375,12 @@ __device__ __forceinline__ bool grid_cell(const G &P, double x, double y, double
 template <class G>
 __device__ __forceinline__ uint32_t outside_axes(const G &P, double x, double y, double z)
 {
+    // 2^-20 of a cell away from the grid's sides no quotient rounds past one
+    auto in = [&](int k, double v) {
+        const double q = (v - P.origo[k]) * P.rcell[k];
+        return q > 0x1p-20 && q < (double)P.num[k] - 0x1p-20 && q < 0x1p30;
+    };
+    if (in(0, x) && in(1, y) && in(2, z)) return 0u;
     const double f0 = cell_floor(P, 0, x), f1 = cell_floor(P, 1, y), f2 = cell_floor(P, 2, z);
     return (f0 >= 0.0 && f0 < (double)P.num[0] ? 0u : 1u) | (f1 >= 0.0 && f1 < (double)P.num[1] ? 0u : 2u) |
            (f2 >= 0.0 && f2 < (double)P.num[2] ? 0u : 4u);

@@ -515,11 +515,12 @@ __device__ __forceinline__ double pair_gap(const Params &P, double4 xb, uint32_t
 }
 
 // The periodic image through which the candidate at xb of a list entry is seen
-// from xa: the entry's, or with Params::one_image the nearest, which is the one
+// from xa: the entry's, or (with Params::one_image) the nearest, which is the one
 // of any near pair, whatever boundaries the two have crossed since.
-__device__ __forceinline__ uint32_t list_code(const Params &P, double4 xa, double4 xb, uint32_t meta)
+// one: whether it may have changed since it was recorded.
+__device__ __forceinline__ uint32_t list_code(const Params &P, bool one, double4 xa, double4 xb, uint32_t meta)
 {
-    if (!P.one_image) return vl_code(meta);
+    if (!one) return vl_code(meta);
     const double dx = xa.x - xb.x, hx = 0.5 * P.L[0];
     uint32_t code = dx < -hx ? 1u : (dx > hx ? 2u : 0u);
     if (P.periodic == 1) {
@@ -701,8 +702,255 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
     return best;
 }
 
+// What a sweep found: the particle's next moment, the entries known to hold a
+// slot, the entries recorded and whether they are a list.
+struct Swept {
+    float due;
+    uint32_t held, nlist;
+    bool listed;
+};
+
+// The sweep of particle s in grid cell gp (which need not be in the grid), for
+// topo_search: the 27 stencil cells are scanned as in the reference (z, y, x;
+// members by particle index) and the list is recorded on the way, together
+// with the near candidates two cells away where cells are that small
+// (Params::wide).  What bounds it is latency, a chain of loads a row and one an
+// overlap: an x-row is one run of the cell list (a run a cell: 25 rows took 50
+// more), and the overlaps are tested when the sweep is over (where they are found
+// they come at different places in every lane).  k_topo sweeping in every step,
+// 50,000 grains in contact: 96 us -> 55.
+//
+// Out of line: few steps sweep, and the decision and the lists' path keep their
+// registers (k_topo on 97,778 loose grains 5.9 us inline, 5.7 so; without lists, where
+// every particle sweeps, 500,000 grains take 276 us a step inline, 296 so).
+template <bool VISC, int TB>
+__device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, uint32_t s, int tid,
+                                         uint32_t *srow, float S, double4 xa, const int32_t gp[3],
+                                         bool use_lists, TopoSlots &ts, ViscAct &va)
+{
+    const double ra = xa.w;
+    const double4 *__restrict__ xr = d.xr[A];
+    const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
+    const bool gp_in = gp[0] >= 0 && (uint32_t)gp[0] < nx && gp[1] >= 0 && (uint32_t)gp[1] < ny &&
+                       gp[2] >= 0 && (uint32_t)gp[2] < nz;
+    // one more acting pair of model 1
+    auto act_on = [&](uint32_t t, uint32_t code) {
+        if (va.n == VISC_CAP) visc_spill(d, P, A, s, srow + tid, TB, va);
+        srow[va.n++ * TB + tid] = t | (code << 27);
+    };
+    uint32_t held = 0;
+    float due = 3.0e38f;
+    const float4 *xs = d.xs[A];
+    const uint32_t k = d.pos[s];
+    const float4 xaf = xs[k];
+    const float Lf0 = (float)P.L[0], Lf1 = (float)P.L[1];
+    const float eps = P.cull_eps;
+    const float skinf = (float)P.skin;
+    const float extraf = (float)P.reach_extra;
+    uint32_t nlist = 0;
+    bool list_overflow = false;
+
+    // Cell-level pruning: a stencil cell whose box lies farther from the
+    // particle than ra + rmax + skin (plus the float slack of the
+    // predicate) holds neither a contact nor a list candidate; skipping
+    // it leaves the visiting order of the others unchanged.  Used only
+    // while the particle's own cell is inside the grid and every
+    // particle sits inside its cell's box (alias_any clear).
+    const bool prune = gp_in && (__ldcg(d.alias_any) == 0u);
+    // squared distances to the cells one and two away on each axis
+    float lo1[3], hi1[3], lo2[3], hi2[3];
+    {
+        const double xc[3] = {xa.x, xa.y, xa.z};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double lo = xc[q] - (P.origo[q] + (double)gp[q] * P.cellsize[q]);
+            const double hi = (P.origo[q] + (double)(gp[q] + 1) * P.cellsize[q]) - xc[q];
+            const double l2 = lo + P.cellsize[q], h2 = hi + P.cellsize[q];
+            lo1[q] = lo > 0.0 ? (float)(lo * lo) * 0.99999f : 0.0f;
+            hi1[q] = hi > 0.0 ? (float)(hi * hi) * 0.99999f : 0.0f;
+            lo2[q] = l2 > 0.0 ? (float)(l2 * l2) * 0.99999f : 0.0f;
+            hi2[q] = h2 > 0.0 ? (float)(h2 * h2) * 0.99999f : 0.0f;
+        }
+    }
+    auto dist2 = [&](int q, int o) {
+        return o == 0 ? 0.0f : (o < 0 ? (o == -1 ? lo1[q] : lo2[q]) : (o == 1 ? hi1[q] : hi2[q]));
+    };
+    const double extra = VISC ? P.reach_extra : 0.0;
+    const float reach = (float)((ra + P.rmax + P.skin + extra) * (1.0 + 1e-5) + P.prune_pad);
+    const float reach2 = prune ? reach * reach : 3.0e38f;
+    const int R = (P.wide && use_lists) ? 2 : 1;
+
+    // A run of the cell list: cells c0, c0 + 1, ..., through image `code`;
+    // [in0, in1) is its part in the stencil, the rest, two cells away, is
+    // only recorded.
+    struct Run {
+        uint32_t beg, end, in0, in1, c0, code;
+    };
+    // The overlaps of the first VL_CAP near candidates are tested after the
+    // sweep, from the list: found here and there in a warp's lanes, each
+    // would make the whole warp wait for its two loads and its slot.  (A
+    // particle outside the grid has no list to keep them in.)
+    uint32_t later = 0;
+    auto test_later = [&]() {
+        for (; later; later &= later - 1u) {
+            const uint32_t e = (uint32_t)(__ffs(later) - 1);
+            const size_t at = vl_at(s, e);
+            const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
+            double ln;
+            if (pair_gap(P, xr[t], code, xa, ln) < 0.0f) {
+                topo_insert<TB>(d, srow, tid, s, t, code, ts);   // nc <= VL_CAP: no cell ends
+                held |= 1u << e;
+            } else {
+                due = fminf(due, S);
+            }
+        }
+    };
+
+    // A run's candidates, culled four at a time so that their loads are in
+    // flight together; hits are handled in list order.
+    auto scan_run = [&](const Run &r) {
+        const float sx = (r.code & 1u) ? Lf0 : ((r.code & 2u) ? -Lf0 : 0.0f);
+        const float sy = (r.code & 4u) ? Lf1 : ((r.code & 8u) ? -Lf1 : 0.0f);
+        uint32_t base = r.beg;
+        while (base < r.end) {
+            const uint32_t last = r.end - 1;
+            float4 c[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c[j] = xs[min(base + (uint32_t)j, last)];
+            uint32_t near = 0, hit = 0;
+            float gj[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float fx = (xaf.x - c[j].x) + sx;
+                const float fy = (xaf.y - c[j].y) + sy;
+                const float fz = xaf.z - c[j].z;
+                const float d2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz * fz));
+                const float rsum = VISC ? (xaf.w + c[j].w + extraf) : (xaf.w + c[j].w);
+                const float rr = rsum * 1.000004f + eps;
+                const float rs = (rsum + skinf) * 1.000004f + eps;
+                const uint32_t k2 = base + (uint32_t)j;
+                const bool ok = k2 < r.end && k2 != k;
+                if (ok && d2 < rs * rs) {
+                    near |= 1u << j;
+                    // the gap, with the cull's float slack taken against it
+                    gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
+                }
+                if (ok && k2 >= r.in0 && k2 < r.in1 && d2 < rr * rr) hit |= 1u << j;
+            }
+            uint32_t next = base + 4;
+            while (near) {
+                const int j = __ffs(near) - 1;
+                near &= near - 1;
+                const uint32_t t = d.cellorder[base + (uint32_t)j];
+                const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
+                // when it can overlap (a hit's gap is not positive)
+                float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
+                if (VISC) {
+                    if ((hit >> j) & 1u) {
+                        act_on(t, r.code);
+                        w = -1.0f;
+                    }
+                } else if ((hit >> j) & 1u) {
+                    if (gp_in && nlist < VL_CAP) {
+                        later |= 1u << nlist;
+                        w = 3.0e38f;
+                    } else {
+                        test_later();   // in visiting order
+                        double ln;
+                        if (pair_gap(P, xr[t], r.code, xa, ln) < 0.0f) {
+                            if (!topo_insert<TB>(d, srow, tid, s, t, r.code, ts)) {
+                                // nc > NC: skip the rest of this cell; the list
+                                // would not describe the skipped part
+                                uint32_t e = r.c0 + 1u;
+                                while (d.cell_start[e] <= base + (uint32_t)j) ++e;
+                                next = d.cell_start[e];
+                                near = 0;
+                                list_overflow = true;
+                            }
+                            w = 3.0e38f;
+                        }
+                    }
+                }
+                due = fminf(due, w);
+                if (gp_in && nlist < VL_CAP) {
+                    const size_t at = vl_at(s, nlist);
+                    d.vl[at] = t;
+                    // a held entry that loses its slot is due at once
+                    d.vl_meta[at] = vl_meta_of(r.code, w > 1.0e38f ? S : fmaxf(w, 0.0f));
+                    ++nlist;
+                } else {
+                    list_overflow = true;
+                }
+            }
+            base = next;
+        }
+    };
+
+    // The cells in visiting order, of each x-row in up to three runs: those
+    // through the periodic boundary before it, those in the grid, those
+    // through the boundary after it (of a particle outside the grid its
+    // three cells one by one, as the reference's stencil names them).
+    for (int oz = -R; oz <= R; ++oz) {
+        const int32_t cz = (int32_t)((uint32_t)gp[2] + (uint32_t)oz);
+        if (past_axis(cz, nz, R == 2)) continue;
+        const float dz2 = dist2(2, oz);
+        if (dz2 > reach2) continue;
+        for (int oy = -R; oy <= R; ++oy) {
+            const float dyz2 = dz2 + dist2(1, oy);
+            if (dyz2 > reach2) continue;
+            int32_t cy = (int32_t)((uint32_t)gp[1] + (uint32_t)oy);
+            uint32_t ycode = 0;
+            if (P.periodic == 1) wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
+            else if (past_axis(cy, ny, R == 2)) continue;
+            const uint32_t rowbase = (uint32_t)cy * nx + (nx * ny) * (uint32_t)cz;
+            const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
+            for (int part = 0; part < 3; ++part) {
+                int32_t a, b, cx;   // cells gp + a .. gp + b; the first one's x
+                Run r;
+                r.code = ycode;
+                if (gp_in) {
+                    const int32_t g = gp[0], n = (int32_t)nx;
+                    if (part == 1) {
+                        a = max(-R, -g);
+                        b = min(R, n - 1 - g);
+                    } else {
+                        if (P.periodic != 1 && P.periodic != 2) continue;
+                        a = part == 0 ? -R : n - g;
+                        b = part == 0 ? -g - 1 : R;
+                    }
+                    if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
+                    if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
+                    if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
+                    if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
+                    if (a > b) continue;
+                    cx = g + a + (part == 0 ? n : (part == 2 ? -n : 0));
+                    if (part != 1) r.code |= part == 0 ? 1u : 2u;
+                } else {
+                    a = b = part - 1;
+                    cx = (int32_t)((uint32_t)gp[0] + (uint32_t)a);
+                    if (P.periodic == 1 || P.periodic == 2) wrap_axis(cx, nx, r.code, 1u, 2u, false);
+                    else if (past_axis(cx, nx, false)) continue;
+                }
+                const uint32_t cid = (uint32_t)cx + rowbase;
+                if (cid >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
+                r.c0 = cid + P.cell_base;
+                const uint32_t *const bounds = d.cell_start + r.c0;
+                r.beg = bounds[0];
+                r.end = bounds[b - a + 1];
+                // the stencil's part: cells max(a, -1) .. min(b, 1)
+                r.in0 = a < -1 ? bounds[-1 - a] : r.beg;
+                r.in1 = far_row || a > 1 || b < -1 ? r.in0 : (b > 1 ? bounds[2 - a] : r.end);
+                scan_run(r);
+            }
+        }
+    }
+    if (!VISC) test_later();
+    return Swept{due, held, nlist, use_lists && !list_overflow};
+}
+
 // The contact search of one particle s that is due (k_topo); sweep: its
-// candidate list cannot be used; S: the epoch's clock.
+// candidate list cannot be used; S: the epoch's clock; step, crossed: as in
+// Verlet.
 //
 // List mode: the list holds every candidate that can overlap while the epoch
 // lasts, each with the earliest moment it can (vl_when).  Candidates known to
@@ -715,20 +963,13 @@ __device__ __noinline__ int first_visited(const Dev &d, const Params &P, int A, 
 // occupied slots plus the list length stay within NC none can (`simple`);
 // otherwise every overlap is walked in order, as the reference does.
 //
-// Sweep mode: the 27 stencil cells are scanned as in the reference (z, y, x;
-// members by particle index) and the list is recorded on the way, together
-// with the near candidates two cells away where cells are that small
-// (Params::wide).  What bounds it is latency, a chain of loads a row and one an
-// overlap: an x-row is one run of the cell list (a run a cell: 25 rows took 50
-// more), and the overlaps are tested when the sweep is over (where they are found
-// they come at different places in every lane).  k_topo sweeping in every step,
-// 50,000 grains in contact: 96 us -> 55.
+// Sweep mode: topo_sweep.
 //
 // VISC (contact model 1): no slots; every candidate within ra + rb + db acts,
 // in visiting order: they are left in `va` and the lane's column of srow.
 template <bool VISC, bool BATCH, int TB>
 __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int tid, uint32_t *srow,
-                                            bool sweep, float S, ViscAct &va)
+                                            bool sweep, bool crossed, uint32_t step, float S, ViscAct &va)
 {
     const Params &P = prm_at<BATCH>(d, s);
     const uint32_t len = d.vl_len[s];
@@ -744,8 +985,8 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const uint32_t occ_in = d.cmask[s];
     const double4 xa = d.xr[A][s];
     uint32_t held = VISC ? 0u : d.vl_held[s];
+    const bool one = crossed && P.one_image != 0u;   // else an entry's image is as recorded
     if (!BATCH && __ldcg(&d.vs->came_apart) != 0u) return;
-    const double ra = xa.w;
     const double4 *__restrict__ xr = d.xr[A];
     TopoSlots ts{occ_in, occ_in, 0u, 0ull, 0ull, 0, false, false};
     const uint32_t nx = P.num[0], ny = P.num[1], nz = P.num[2];
@@ -758,17 +999,11 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     const bool use_lists = P.skin > 0.0 && gp_in;
     // around a particle that is back from outside a periodic boundary every entry
     // is looked at; a list that was recorded while it stood outside is not used
-    const uint32_t step = __ldcg(&d.vs->step);
-    const bool new_list = d.vl_tag[s] == (uint8_t)(step - 1u);
-    if (__ldcg(&d.vs->look_step) == step && __ldcg(&d.look[d.cell[s]]) == step) {
+    auto new_list = [&]() { return d.vl_tag[s] == (uint8_t)(step - 1u); };
+    if (crossed && __ldcg(&d.vs->look_step) == step && __ldcg(&d.look[d.cell[s]]) == step) {
         held = 0u;
-        if (new_list) sweep = true;
+        if (new_list()) sweep = true;
     }
-    // one more acting pair of model 1
-    auto act_on = [&](uint32_t t, uint32_t code) {
-        if (va.n == VISC_CAP) visc_spill(d, P, A, s, srow + tid, TB, va);
-        srow[va.n++ * TB + tid] = t | (code << 27);
-    };
     float due = 3.0e38f;         // the particle's next moment
 
     if (use_lists && !sweep && len != VL_NONE) {
@@ -799,7 +1034,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 const uint32_t t = tv[j];
                 if (rows) {
                     const int i = slot_of<TB>(srow, tid, ts, t);
-                    if (i >= 0 && dm_get(ts.dm_lo, ts.dm_hi, i) == list_code(P, xa, xr[t], mv[j])) {
+                    if (i >= 0 && dm_get(ts.dm_lo, ts.dm_hi, i) == list_code(P, one, xa, xr[t], mv[j])) {
                         held |= 1u << e;
                         continue;
                     }
@@ -809,7 +1044,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
                 if (VISC ? !(S >= w) : !(S > w)) { due = fminf(due, w); continue; }
                 double ln;
                 const double4 xb = xr[t];
-                const uint32_t code = list_code(P, xa, xb, mv[j]);
+                const uint32_t code = list_code(P, one, xa, xb, mv[j]);
                 const double gap = pair_gap(P, xb, code, xa, ln);
                 if (VISC ? (gap < 0.0f || gap < P.db) : (gap < 0.0f)) {
                     act |= 1u << e;
@@ -873,223 +1108,20 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
             due = -1.0f;
         }
     } else {
-        const float4 *xs = d.xs[A];
-        const uint32_t k = d.pos[s];
-        const float4 xaf = xs[k];
-        const float Lf0 = (float)P.L[0], Lf1 = (float)P.L[1];
-        const float eps = P.cull_eps;
-        const float skinf = (float)P.skin;
-        const float extraf = (float)P.reach_extra;
-        uint32_t nlist = 0;
-        bool list_overflow = false;
-        held = 0u;
-
-        // Cell-level pruning: a stencil cell whose box lies farther from the
-        // particle than ra + rmax + skin (plus the float slack of the
-        // predicate) holds neither a contact nor a list candidate; skipping
-        // it leaves the visiting order of the others unchanged.  Used only
-        // while the particle's own cell is inside the grid and every
-        // particle sits inside its cell's box (alias_any clear).
-        const bool prune = gp_in && (__ldcg(d.alias_any) == 0u);
-        // squared distances to the cells one and two away on each axis
-        float lo1[3], hi1[3], lo2[3], hi2[3];
-        {
-            const double xc[3] = {xa.x, xa.y, xa.z};
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const double lo = xc[q] - (P.origo[q] + (double)gp[q] * P.cellsize[q]);
-                const double hi = (P.origo[q] + (double)(gp[q] + 1) * P.cellsize[q]) - xc[q];
-                const double l2 = lo + P.cellsize[q], h2 = hi + P.cellsize[q];
-                lo1[q] = lo > 0.0 ? (float)(lo * lo) * 0.99999f : 0.0f;
-                hi1[q] = hi > 0.0 ? (float)(hi * hi) * 0.99999f : 0.0f;
-                lo2[q] = l2 > 0.0 ? (float)(l2 * l2) * 0.99999f : 0.0f;
-                hi2[q] = h2 > 0.0 ? (float)(h2 * h2) * 0.99999f : 0.0f;
-            }
-        }
-        auto dist2 = [&](int q, int o) {
-            return o == 0 ? 0.0f : (o < 0 ? (o == -1 ? lo1[q] : lo2[q]) : (o == 1 ? hi1[q] : hi2[q]));
-        };
-        const double extra = VISC ? P.reach_extra : 0.0;
-        const float reach = (float)((ra + P.rmax + P.skin + extra) * (1.0 + 1e-5) + P.prune_pad);
-        const float reach2 = prune ? reach * reach : 3.0e38f;
-        const int R = (P.wide && use_lists) ? 2 : 1;
-
-        // A run of the cell list: cells c0, c0 + 1, ..., through image `code`;
-        // [in0, in1) is its part in the stencil, the rest, two cells away, is
-        // only recorded.
-        struct Run {
-            uint32_t beg, end, in0, in1, c0, code;
-        };
-        // The overlaps of the first VL_CAP near candidates are tested after the
-        // sweep, from the list: found here and there in a warp's lanes, each
-        // would make the whole warp wait for its two loads and its slot.  (A
-        // particle outside the grid has no list to keep them in.)
-        uint32_t later = 0;
-        auto test_later = [&]() {
-            for (; later; later &= later - 1u) {
-                const uint32_t e = (uint32_t)(__ffs(later) - 1);
-                const size_t at = vl_at(s, e);
-                const uint32_t t = d.vl[at], code = vl_code(d.vl_meta[at]);
-                double ln;
-                if (pair_gap(P, xr[t], code, xa, ln) < 0.0f) {
-                    topo_insert<TB>(d, srow, tid, s, t, code, ts);   // nc <= VL_CAP: no cell ends
-                    held |= 1u << e;
-                } else {
-                    due = fminf(due, S);
-                }
-            }
-        };
-
-        // A run's candidates, culled four at a time so that their loads are in
-        // flight together; hits are handled in list order.
-        auto scan_run = [&](const Run &r) {
-            const float sx = (r.code & 1u) ? Lf0 : ((r.code & 2u) ? -Lf0 : 0.0f);
-            const float sy = (r.code & 4u) ? Lf1 : ((r.code & 8u) ? -Lf1 : 0.0f);
-            uint32_t base = r.beg;
-            while (base < r.end) {
-                const uint32_t last = r.end - 1;
-                float4 c[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) c[j] = xs[min(base + (uint32_t)j, last)];
-                uint32_t near = 0, hit = 0;
-                float gj[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float fx = (xaf.x - c[j].x) + sx;
-                    const float fy = (xaf.y - c[j].y) + sy;
-                    const float fz = xaf.z - c[j].z;
-                    const float d2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz * fz));
-                    const float rsum = VISC ? (xaf.w + c[j].w + extraf) : (xaf.w + c[j].w);
-                    const float rr = rsum * 1.000004f + eps;
-                    const float rs = (rsum + skinf) * 1.000004f + eps;
-                    const uint32_t k2 = base + (uint32_t)j;
-                    const bool ok = k2 < r.end && k2 != k;
-                    if (ok && d2 < rs * rs) {
-                        near |= 1u << j;
-                        // the gap, with the cull's float slack taken against it
-                        gj[j] = __fsub_rd(__fmul_rd(__fsqrt_rd(d2), 0.999996f), rr);
-                    }
-                    if (ok && k2 >= r.in0 && k2 < r.in1 && d2 < rr * rr) hit |= 1u << j;
-                }
-                uint32_t next = base + 4;
-                while (near) {
-                    const int j = __ffs(near) - 1;
-                    near &= near - 1;
-                    const uint32_t t = d.cellorder[base + (uint32_t)j];
-                    const float g = j < 2 ? (j == 0 ? gj[0] : gj[1]) : (j == 2 ? gj[2] : gj[3]);
-                    // when it can overlap (a hit's gap is not positive)
-                    float w = g > 0.0f ? __fadd_rd(S, __fmul_rd(0.5f, g)) : S;
-                    if (VISC) {
-                        if ((hit >> j) & 1u) {
-                            act_on(t, r.code);
-                            w = -1.0f;
-                        }
-                    } else if ((hit >> j) & 1u) {
-                        if (gp_in && nlist < VL_CAP) {
-                            later |= 1u << nlist;
-                            w = 3.0e38f;
-                        } else {
-                            test_later();   // in visiting order
-                            double ln;
-                            if (pair_gap(P, xr[t], r.code, xa, ln) < 0.0f) {
-                                if (!topo_insert<TB>(d, srow, tid, s, t, r.code, ts)) {
-                                    // nc > NC: skip the rest of this cell; the list
-                                    // would not describe the skipped part
-                                    uint32_t e = r.c0 + 1u;
-                                    while (d.cell_start[e] <= base + (uint32_t)j) ++e;
-                                    next = d.cell_start[e];
-                                    near = 0;
-                                    list_overflow = true;
-                                }
-                                w = 3.0e38f;
-                            }
-                        }
-                    }
-                    due = fminf(due, w);
-                    if (gp_in && nlist < VL_CAP) {
-                        const size_t at = vl_at(s, nlist);
-                        d.vl[at] = t;
-                        // a held entry that loses its slot is due at once
-                        d.vl_meta[at] = vl_meta_of(r.code, w > 1.0e38f ? S : fmaxf(w, 0.0f));
-                        ++nlist;
-                    } else {
-                        list_overflow = true;
-                    }
-                }
-                base = next;
-            }
-        };
-
-        // The cells in visiting order, of each x-row in up to three runs: those
-        // through the periodic boundary before it, those in the grid, those
-        // through the boundary after it (of a particle outside the grid its
-        // three cells one by one, as the reference's stencil names them).
-        for (int oz = -R; oz <= R; ++oz) {
-            const int32_t cz = (int32_t)((uint32_t)gp[2] + (uint32_t)oz);
-            if (past_axis(cz, nz, R == 2)) continue;
-            const float dz2 = dist2(2, oz);
-            if (dz2 > reach2) continue;
-            for (int oy = -R; oy <= R; ++oy) {
-                const float dyz2 = dz2 + dist2(1, oy);
-                if (dyz2 > reach2) continue;
-                int32_t cy = (int32_t)((uint32_t)gp[1] + (uint32_t)oy);
-                uint32_t ycode = 0;
-                if (P.periodic == 1) wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
-                else if (past_axis(cy, ny, R == 2)) continue;
-                const uint32_t rowbase = (uint32_t)cy * nx + (nx * ny) * (uint32_t)cz;
-                const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
-                for (int part = 0; part < 3; ++part) {
-                    int32_t a, b, cx;   // cells gp + a .. gp + b; the first one's x
-                    Run r;
-                    r.code = ycode;
-                    if (gp_in) {
-                        const int32_t g = gp[0], n = (int32_t)nx;
-                        if (part == 1) {
-                            a = max(-R, -g);
-                            b = min(R, n - 1 - g);
-                        } else {
-                            if (P.periodic != 1 && P.periodic != 2) continue;
-                            a = part == 0 ? -R : n - g;
-                            b = part == 0 ? -g - 1 : R;
-                        }
-                        if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
-                        if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
-                        if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
-                        if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
-                        if (a > b) continue;
-                        cx = g + a + (part == 0 ? n : (part == 2 ? -n : 0));
-                        if (part != 1) r.code |= part == 0 ? 1u : 2u;
-                    } else {
-                        a = b = part - 1;
-                        cx = (int32_t)((uint32_t)gp[0] + (uint32_t)a);
-                        if (P.periodic == 1 || P.periodic == 2) wrap_axis(cx, nx, r.code, 1u, 2u, false);
-                        else if (past_axis(cx, nx, false)) continue;
-                    }
-                    const uint32_t cid = (uint32_t)cx + rowbase;
-                    if (cid >= P.ncells) { ts.err |= ST_OUT_OF_GRID; continue; }
-                    r.c0 = cid + P.cell_base;
-                    const uint32_t *const bounds = d.cell_start + r.c0;
-                    r.beg = bounds[0];
-                    r.end = bounds[b - a + 1];
-                    // the stencil's part: cells max(a, -1) .. min(b, 1)
-                    r.in0 = a < -1 ? bounds[-1 - a] : r.beg;
-                    r.in1 = far_row || a > 1 || b < -1 ? r.in0 : (b > 1 ? bounds[2 - a] : r.end);
-                    scan_run(r);
-                }
-            }
-        }
-        if (!VISC) test_later();
-        const bool listed = use_lists && !list_overflow;
+        const Swept w = topo_sweep<VISC, TB>(d, P, A, s, tid, srow, S, xa, gp, use_lists, ts, va);
+        due = w.due;
+        held = w.held;
+        const bool listed = w.listed;
         if (!listed) {
             // searched again next step, over a cell list of that step.  The list of
             // a particle that stands outside a periodic boundary stays for its
             // return, unless it may miss another one that is back.
             due = -1.0f;
-            const bool stays = P.one_image && !gp_in && !sweep && !new_list && __ldcg(&d.vs->dirty_step) != step;
+            const bool stays = one && !gp_in && !sweep && !new_list() && __ldcg(&d.vs->dirty_step) != step;
             if (!stays) d.vl_len[s] = VL_NONE;
             if (P.skin > 0.0 && gp_in) d.vs->want_cells = 1u;   // (outside: particle_tail asks)
         } else {
-            d.vl_len[s] = (uint8_t)nlist;
+            d.vl_len[s] = (uint8_t)w.nlist;
             d.vl_tag[s] = (uint8_t)step;
         }
     }
@@ -1145,7 +1177,9 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
     const uint32_t lane = (uint32_t)tid & 31u;
     const uint32_t base = ((blockIdx.x * TB + (uint32_t)tid) >> 5) * (32u * span);
     const Verlet &V = *d.vs;
-    const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == V.step, look = V.look_step == V.step;
+    const uint32_t step = V.step;
+    const bool all = V.all_rebuild != 0u, dirty = V.dirty_step == step, crossed = V.crossed != 0u;
+    const bool look = crossed && V.look_step == step;
     const float S = V.moved;
     // bit j: particle base + 32 j + lane is searched / must sweep
     uint32_t need = 0, swp = 0;
@@ -1155,8 +1189,8 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
         if (j >= span) break;
         if (s >= np) continue;
         const float due = d.due[s];
-        const bool sw = all || (dirty && d.dirty[d.cell[s]] == V.step);
-        if (!sw && !(S > due) && !(look && d.look[d.cell[s]] == V.step)) {
+        const bool sw = all || (dirty && d.dirty[d.cell[s]] == step);
+        if (!sw && !(S > due) && !(look && d.look[d.cell[s]] == step)) {
             if (VISC) d.c1acc[s] = make_double4(0.0, 0.0, 0.0, 0.0);
             continue;
         }
@@ -1197,7 +1231,7 @@ k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
             }
             const uint32_t bit = __fns(sel, 0, (int)rem + 1);
             s = base + 32u * selj + bit;
-            topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u, S, va);
+            topo_search<VISC, BATCH, TB>(d, A, s, tid, srow, (sel_s >> bit) & 1u, crossed, step, S, va);
         }
         if constexpr (VISC) {
             __syncwarp();
@@ -1545,6 +1579,7 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
         // (past the last cell its stencil is empty)
         if (c != d.ncells_all || c != c_old) d.rebuild[REBUILD_NEXT] = 1u;
         d.due[s] = -1.0f;
+        V.crossed = 1u;
         d.outside[d.uid[s]] = cell_outside(P, xa.x, xa.y, xa.z) ? 2 : 1;
     }
     // (out through one side and into the next cell on another axis, a particle
@@ -1573,6 +1608,7 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
             hard = dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1;
         }
         if (hard || look || P.eager) d.rebuild[REBUILD_NEXT] = 1u;
+        if (look) V.crossed = 1u;   // (outside since the upload)
         if ((hard || look) && P.skin > 0.0) {
             const uint32_t m = atomicAdd(&V.nmovers, 1u);
             if (m < MOVER_CAP) d.movers[m] = make_uint2(hard ? c_old : LOOK, c);
@@ -2085,9 +2121,8 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
     const uint32_t chunk = blockIdx.x * WARPS + w, s0 = chunk * 32u, s = s0 + lane;
     // the cell list first, where this step needs it (REBUILD_NOW does not
     // change before the step ends)
-    const bool due = *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u;
-    if (lists_given_up(d)) return;
-    if (own_list && due) {
+    if (own_list && *(volatile const uint32_t *)&d.rebuild[REBUILD_NOW] != 0u) {
+        if (lists_given_up(d)) return;
         GridBar bar{&d.vs->bar_small, 0};
         if (!rebuild_grid<SMALL_BLOCK>(d, A, bar) || !grid_barrier(d, bar)) return;
     }
@@ -2099,14 +2134,15 @@ k_small(const __grid_constant__ ForceArgs args, int own_list)
             const Verlet &V = *d.vs;
             const uint32_t step = __ldcg(&V.step);
             const float S = __ldcg(&V.moved);
+            const bool crossed = __ldcg(&V.crossed) != 0u;
+            const bool look = crossed && __ldcg(&V.look_step) == step;
             bool need = false, sweep = false;
             if (s < np) {
                 sweep = __ldcg(&V.all_rebuild) != 0u ||
                         (__ldcg(&V.dirty_step) == step && __ldcg(&d.dirty[d.cell[s]]) == step);
-                need = sweep || S > d.due[s] ||
-                       (__ldcg(&V.look_step) == step && __ldcg(&d.look[d.cell[s]]) == step);
+                need = sweep || S > d.due[s] || (look && __ldcg(&d.look[d.cell[s]]) == step);
             }
-            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, S, va);
+            if (need) topo_search<VISC, BATCH, 32>(d, A, s, (int)lane, srow[w], sweep, crossed, step, S, va);
             __syncwarp();
             if constexpr (VISC) visc_warp(d, A, s, srow[w], 32u, visc[w], va);
         }
