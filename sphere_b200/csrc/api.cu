@@ -708,9 +708,12 @@ int create_impl(const sph_config *cfgs, uint32_t ninst, bool batched, sph_ctx **
     AL(d.cell_start, ncells + 2); AL(d.cellorder, np); AL(d.pos, npad); AL(d.cell_fill, ncells + 1);
     AL(d.scan_tiles, SCAN_TILES);
     AL(d.alias_any, 1);
-    AL(d.vl, tiled_size(np, VL_CAP)); AL(d.vl_meta, tiled_size(np, VL_CAP)); AL(d.vl_len, np);
-    AL(d.vl_held, np); AL(d.due, np); AL(d.vl_tag, np); AL(d.outside, np);
-    AL(d.movers, MOVER_CAP); AL(d.dirty, ncells + 1); AL(d.look, ncells + 1); AL(d.vs, 1);
+    AL(d.vl, tiled_size(np, VL_CAP)); AL(d.vl_meta, tiled_size(np, VL_CAP)); AL(d.vl_len, 3 * np);
+    d.vl_tag = d.vl_len + np;   // (an allocation less each)
+    d.outside = d.vl_tag + np;
+    AL(d.vl_held, np); AL(d.due, np);
+    AL(d.movers, MOVER_CAP); AL(d.dirty, 2 * (ncells + 1)); AL(d.vs, 1);
+    d.look = d.dirty + ncells + 1;
     AL(d.wf_pp, np); AL(d.wtouch, npad); AL(d.wf_partial, div_up(np, 256));
     AL(d.wf_flag, div_up(np, 256));
     AL(d.walls, 1);

@@ -178,26 +178,65 @@ def test_grains_that_cross_a_periodic_side(oracle_libs, periodic, sides, reach, 
             assert mismatches(sim.download(), want, ALL) == [], skin
 
 
+def _sheared(n=1500, cell=2.0, seed=6, periodic=1):
+    """A dense bed in fast shear: grains cross the sides in nearly every step, in a
+    moving contact network."""
+    side = (n * 8.2e-9 / 0.35) ** (1 / 3)
+    sb = scenes.collision(n=n, seed=seed, periodic=periodic, box=(1.02 * side, 1.02 * side, 1.2 * side + 0.012),
+                          phi_target=0.35, k_n=500.0, k_t=500.0, gamma_n=0.01, vmax=2.0, straddle=True)
+    sb.vel = sb.vel + np.stack([6.0 * (2 * sb.x[:, 2] / sb.L[2] - 1), 0 * sb.x[:, 0], 0 * sb.x[:, 0]], 1)
+    sb.num = np.maximum(1, np.floor(sb.L / (cell * 1.6e-3))).astype(np.uint32)
+    return sb
+
+
 @both_kernels
 @pytest.mark.parametrize("model", [1, 2])
 @pytest.mark.parametrize("cell", [2.0, 2.4, 3.0])
 def test_sheared_beds_with_periodic_sides(oracle_libs, cell, model, span):
-    """Grains cross the sides in nearly every step, in a moving contact network."""
-    side = (1500 * 8.2e-9 / 0.35) ** (1 / 3)
-    sb = scenes.collision(n=1500, seed=6, periodic=1, box=(1.02 * side, 1.02 * side, 1.2 * side + 0.012),
-                          phi_target=0.35, k_n=500.0, k_t=500.0, gamma_n=0.01, vmax=2.0, straddle=True)
-    sb.vel = sb.vel + np.stack([6.0 * (2 * sb.x[:, 2] / sb.L[2] - 1), 0 * sb.x[:, 0], 0 * sb.x[:, 0]], 1)
-    sb.num = np.maximum(1, np.floor(sb.L / (cell * 1.6e-3))).astype(np.uint32)
+    sb = _sheared(cell=cell)
     if model == 1:
         sb = with_model(sb, 1, kappa=0.05, V_b=1e-12, db=1e-4)
     rc, want, orun = run_oracle(oracle_libs["orc"], sb, 150)
     assert rc == 0
-    for skin in (0.1, 0.3):
-        with Simulation(config_from_spherebin(sb), verlet_skin=skin, topo_span=span) as sim:
+    for kw in (dict(verlet_skin=0.1), dict(verlet_skin=0.3), dict(relayout_every=7, graph_steps=3)):
+        with Simulation(config_from_spherebin(sb), topo_span=span, **kw) as sim:
             sim.upload(state_from_spherebin(sb))
             sim.step(150)
             sim.sync()
             got = sim.download()
             _, perm, _, _ = sim.cells()
-        assert mismatches(got, want, ALL) == [], skin
+        assert mismatches(got, want, ALL) == [], kw
         assert np.array_equal(perm, orun.perm)
+
+
+@both_kernels
+def test_batched_scenes_with_periodic_sides(oracle_libs, span):
+    """Crossings of several scenes in a step, of scenes whose axes are too short to
+    follow an image beside ones that do."""
+    sbs = [_crossing_pairs(1, "one_image", "both", 3), _sheared(n=800, seed=7), _crossing_pairs(1, "short_axis", "both", 4),
+           _sheared(n=700, seed=10, cell=2.4), _crossing_pairs(2, "one_image", "both", 5)]
+    with BatchSimulation([config_from_spherebin(sb) for sb in sbs], topo_span=span) as sim:
+        for _ in range(2):   # another run of the same context
+            sim.upload([state_from_spherebin(sb) for sb in sbs])
+            sim.step(70)
+            sim.sync()
+        got = sim.download_all()
+    for sb, st in zip(sbs, got):
+        rc, want, _ = run_oracle(oracle_libs["orc"], sb, 70)
+        assert rc == 0
+        assert mismatches(st, want, STATE_FIELDS + OUTPUT_FIELDS + ("contacts", "delta_t")) == []
+
+
+def test_differentiable_steps_with_periodic_sides():
+    """The forward with lists and with a sweep in every step, bit for bit."""
+    sb = _sheared(n=900, seed=9)
+    x = []
+    for skin in (0.0, 0.1):
+        with Simulation(config_from_spherebin(sb), verlet_skin=skin) as sim:
+            sim.upload(state_from_spherebin(sb))
+            sim.diff_begin(checkpoint_every=16)
+            sim.step(120)
+            sim.sync()
+            x.append(sim.download())
+            sim.diff_end()
+    assert mismatches(x[1], x[0], STATE_FIELDS + ("force", "torque", "contacts", "delta_t")) == []
