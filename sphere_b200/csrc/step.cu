@@ -591,7 +591,7 @@ struct ViscWarp {
 
 // The pairs of the warp's particles (lane's particle s, its column act),
 // evaluated 32 at a time, one a lane, and added up by each particle's own lane
-// in visiting order, as contact_chunk does for the slots.  All lanes.
+// in visiting order.  All lanes.
 __device__ __forceinline__ void visc_warp(const Dev &d, int A, uint32_t s, const uint32_t *act,
                                           uint32_t stride, ViscWarp &vs, ViscAct &v)
 {
@@ -1162,9 +1162,9 @@ constexpr uint32_t TOPO_SPAN_MAX = 4;
 // the 54 cells around it sweep, and the cell list was sorted anew in each
 // such step) and tested against the largest displacement in every step.  Per
 // step, search + cell list, then and now: 1M loose grains in motion 44 + 60
-// -> 11.3 + 0.1 us; 50k in a rapid flow 36 + 25 -> 15 + 2 us; 64 jammed
-// scenes of 330k grains 233 + 62 -> 5.3 + 0.1 us; the 1M jammed column 13.9
-// -> 8.7 us.
+// -> 12.0 + 0.1 us; 50k in a rapid flow 36 + 25 -> 15.5 + 0.7 us; 64 jammed
+// scenes of 330k grains 233 + 62 -> 5.1 + 0.1 us; the 1M jammed column 13.9
+// -> 9.5 us.
 template <bool VISC, bool BATCH, int TB>
 __global__ void __launch_bounds__(TB, TOPO_THREADS_PER_SM / TB)
 k_topo(const __grid_constant__ Dev d, int A, uint32_t span)
@@ -2093,8 +2093,8 @@ struct RegRows {
 // has a warp of its own on the device at once.  A particle's search, contact
 // forces and integration need its neighbours' start-of-step rows (buffer A)
 // and its own results only, so the warp of a chunk runs all three, and the
-// step is one launch: the slot sums stay in shared memory, the last block
-// ends the step.
+// step is one launch: the slot sums stay in registers, the last block ends
+// the step.
 //
 // What bounds it: latency, one chain of the search, the laws' rounds and the
 // integration.  As three kernels each of their launches, ramps and drains
@@ -2216,9 +2216,9 @@ static uint32_t small_blocks(const Dev &d, int model)
 // each (75,776 particles on 148 SMs), and no shape or span of the split
 // kernels was asked for.  Above, the split kernels balance the work over the
 // device and stream the integration.  Microseconds a step, one kernel against
-// split, on a B200: in a flow 24.7 / 29.0 at 1,000 grains, 32.6 / 38.3 at
-// 10,000, 37.8 / 45.0 at 50,000, 44.8 / 53.3 at 75,000; in a jammed packing
-// 20.1 / 20.9 at 1,000, 23.3 / 24.7 at 29,791, 28.5 / 29.0 at 74,088.
+// split, on a B200: in a flow 20.0 / 24.0 at 1,000 grains, 25.3 / 30.7 at
+// 10,000, 30.3 / 36.0 at 50,000, 36.0 / 42.0 at 75,000; in a jammed packing
+// 20.9 / 20.7 at 1,000, 22.8 / 23.2 at 29,791, 28.8 / 27.0 at 74,088.
 //
 // Beside a Darcy flow (with_flow) up to a block an SM: its blocks start all
 // together, so beyond that k_small waits for the porosity's to leave, which runs
