@@ -147,10 +147,12 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rt_maxpos(Dev d, int A, unsigned l
 }
 
 // A sphere's pixels.  What bounds it: instructions, a discriminant for each
-// pixel of the box.  A pixel whose key is already nearer than the sphere can
-// be (a plain read, possibly out of date: keys only fall) takes no root and
-// no atomic.  1M spheres, 800 x 800: 542 us with a box four times the bound's
-// and a root and an atomic for every hit, 164 us now.
+// pixel of the box and a root for each hit; for few spheres that cover many
+// pixels, one thread's.  A hit only issues its atomic minimum: reading the key
+// first, to leave out what is already covered, made every hit wait for L2 (a
+// frame of 2,000 spheres, 800 x 800 and 2000 x 3000: 1.57 and 24.5 ms with the
+// read, 0.86 and 10.4 without; of 1M 0.62 and 4.4 against 0.60 and 4.2).  A box
+// four times the bound's took 1.09 and 13.3 ms, and 1.06 and 6.5.
 __global__ void __launch_bounds__(RT_BLOCK)
 k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderArgs g,
            const double *values, const fl3 *__restrict__ colA, const fl3 *__restrict__ rowB,
@@ -190,19 +192,13 @@ k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderA
     const int W = (int)g.W;
     int i0 = 0, i1 = W - 1, j0 = 0, j1 = W - 1;   // j: the wrapped row index
     const double r2 = rho * (1.0 + 1e-6);
-    // no hit's |t| is below this (0: not known).  The ray t d passes within
-    // rho of c, and the float root errs on t by less than rho / |d| more, so
-    // |t| |d| > |ec| - 3 rho; |d| is at most its length at the box's far corner.
-    float t_low = 0.0f;
     if (c0 * c0 > r2 * r2) {
         // image-plane coordinate -D * (along / depth) over the ball
-        double far2 = 0.0;   // squares of the box's largest plane coordinates
         auto range = [&](double p0, double lo_img, double hi_img, int n, int &lo, int &hi) {
             const double den = c0 * c0 - r2 * r2;
             const double root = r2 * sqrt(p0 * p0 + c0 * c0 - r2 * r2);
             const double k1 = (p0 * c0 + root) / den, k2 = (p0 * c0 - root) / den;
             const double pa = -D * k1, pb = -D * k2;
-            far2 += isfinite(pa) && isfinite(pb) ? fmax(pa * pa, pb * pb) : 1e300;
             if (!isfinite(pa) || !isfinite(pb)) return;   // keep the whole range
             const double plo = fmin(pa, pb), phi = fmax(pa, pb);
             const double span = hi_img - lo_img;
@@ -214,7 +210,7 @@ k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderA
                 return;
             }
             const double f_lo = (plo - lo_img) * n / span - 0.5, f_hi = (phi - lo_img) * n / span - 0.5;
-            if (!isfinite(f_lo) || !isfinite(f_hi)) { far2 = 1e300; return; }
+            if (!isfinite(f_lo) || !isfinite(f_hi)) return;
             const double a = fmin(f_lo, f_hi), b = fmax(f_lo, f_hi);
             lo = (int)fmax(-1.0, fmin((double)n, ceil(a - 0.5)));
             hi = (int)fmax(-1.0, fmin((double)n, floor(b + 0.5)));
@@ -225,15 +221,8 @@ k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderA
         i1 = min(i1, W - 1);
         j0 = max(j0, 0);
         j1 = min(j1, W - 1);
-        // the widening by half a pixel and the float directions: one more
-        // pixel's extent and 1e-5
-        const double px = fmax(fabs((double)ip[1] - ip[0]) / g.W, fabs((double)ip[3] - ip[2]) / g.H);
-        const double dmax = sqrt(D * D + far2) + 2.0 * px;
-        const double low = (nb - 3.0 * rho) / dmax * (1.0 - 1e-5);
-        if (low > 0.0 && low < 1e30) t_low = __double2float_rd(low);
     }
     if (i0 > i1 || j0 > j1) return;
-    const float *key_t = reinterpret_cast<const float *>(keys) + 1;   // the |t| of a key
     // Rows y with y mod W in [j0, j1].  The reference's row index of pixel m
     // is floor((float)m / W) mod W: m is below 2^24, so the quotient errs by
     // at most H 2^-24 < 1 / W and the floor is y for every pixel of row y.
@@ -250,8 +239,6 @@ k_rt_splat(const __grid_constant__ Dev d, int A, const __grid_constant__ RenderA
                 const float Delta = (2.0f * fdot(dir, ec)) * (2.0f * fdot(dir, ec)) -
                                     4.0f * fdot(dir, dir) * (fdot(ec, ec) - R * R);
                 if (!(Delta > 0.0f)) continue;
-                // no hit yet reads as NaN, which is not below
-                if (key_t[2 * (size_t)m] < t_low) continue;
                 const float t_minus =
                     ((fdot(-dir, ec) -
                       sqrtf(fdot(dir, ec) * fdot(dir, ec) - fdot(dir, dir) * (fdot(ec, ec) - R * R))) /
