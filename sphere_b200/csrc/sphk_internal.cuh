@@ -120,7 +120,8 @@ __host__ __device__ inline ForceConsts force_consts(const Params &P)
 // Twice the blocks that a rebuild's grid can have (8 an SM, with room).
 constexpr uint32_t SCAN_TILES = 4096;
 constexpr int VL_CAP = 32;              // candidates kept per particle
-constexpr uint8_t VL_NONE = 0xff;       // no usable list: sweep the stencil
+constexpr uint8_t VL_NONE = 0xff;       // no list yet: sweep and record one
+constexpr uint8_t VL_OVER = 0xfe;       // more candidates than that: sweep in every step
 constexpr uint32_t MOVER_CAP = 1u << 16;
 constexpr uint32_t LOOK = 0xffffffffu;  // no cell
 
@@ -253,7 +254,7 @@ struct Dev {
     // Verlet lists
     uint32_t *vl;         // tiled, VL_CAP per particle: candidate storage indices, in visiting order
     uint32_t *vl_meta;    // tiled, VL_CAP per particle: vl_meta_of(shift code, moment)
-    uint8_t *vl_len;      // [np] list length or VL_NONE
+    uint8_t *vl_len;      // [np] list length, VL_NONE or VL_OVER
     uint32_t *vl_held;    // [np] entries known to hold a slot through their image; 0 says nothing
     float *due;           // [np] the moment after which the particle is searched; below 0: next step
     uint8_t *vl_tag;      // [np] the step in which the list was recorded, modulo 256

@@ -714,7 +714,7 @@ struct Swept {
 // topo_search: the 27 stencil cells are scanned as in the reference (z, y, x;
 // members by particle index) and the list is recorded on the way, together
 // with the near candidates two cells away where cells are that small
-// (Params::wide).  What bounds it is latency, a chain of loads a row and one an
+// (Params::wide), or with `record` not set only searched.  What bounds it is latency, a chain of loads a row and one an
 // overlap: an x-row is one run of the cell list (a run a cell: 25 rows took 50
 // more), and the overlaps are tested when the sweep is over (where they are found
 // they come at different places in every lane).  k_topo sweeping in every step,
@@ -726,7 +726,7 @@ struct Swept {
 template <bool VISC, int TB>
 __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, uint32_t s, int tid,
                                          uint32_t *srow, float S, double4 xa, const int32_t gp[3],
-                                         bool use_lists, TopoSlots &ts, ViscAct &va)
+                                         bool record, TopoSlots &ts, ViscAct &va)
 {
     const double ra = xa.w;
     const double4 *__restrict__ xr = d.xr[A];
@@ -745,7 +745,8 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
     const float4 xaf = xs[k];
     const float Lf0 = (float)P.L[0], Lf1 = (float)P.L[1];
     const float eps = P.cull_eps;
-    const float skinf = (float)P.skin;
+    const double skin = record ? P.skin : 0.0;
+    const float skinf = (float)skin;
     const float extraf = (float)P.reach_extra;
     uint32_t nlist = 0;
     bool list_overflow = false;
@@ -776,9 +777,11 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
         return o == 0 ? 0.0f : (o < 0 ? (o == -1 ? lo1[q] : lo2[q]) : (o == 1 ? hi1[q] : hi2[q]));
     };
     const double extra = VISC ? P.reach_extra : 0.0;
-    const float reach = (float)((ra + P.rmax + P.skin + extra) * (1.0 + 1e-5) + P.prune_pad);
-    const float reach2 = prune ? reach * reach : 3.0e38f;
-    const int R = (P.wide && use_lists) ? 2 : 1;
+    const float reach = (float)((ra + P.rmax + skin + extra) * (1.0 + 1e-5) + P.prune_pad);
+    // (cells two away, which the reference does not visit, are only looked into for
+    // the list: their distance counts in any case)
+    const float far2 = reach * reach, reach2 = prune ? far2 : 3.0e38f;
+    const int R = (P.wide && record) ? 2 : 1;
 
     // A run of the cell list: cells c0, c0 + 1, ..., through image `code`;
     // [in0, in1) is its part in the stencil, the rest, two cells away, is
@@ -894,16 +897,17 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
         const int32_t cz = (int32_t)((uint32_t)gp[2] + (uint32_t)oz);
         if (past_axis(cz, nz, R == 2)) continue;
         const float dz2 = dist2(2, oz);
-        if (dz2 > reach2) continue;
+        if (dz2 > (oz < -1 || oz > 1 ? far2 : reach2)) continue;
         for (int oy = -R; oy <= R; ++oy) {
             const float dyz2 = dz2 + dist2(1, oy);
-            if (dyz2 > reach2) continue;
+            const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
+            const float most = far_row ? far2 : reach2;
+            if (dyz2 > most) continue;
             int32_t cy = (int32_t)((uint32_t)gp[1] + (uint32_t)oy);
             uint32_t ycode = 0;
             if (P.periodic == 1) wrap_axis(cy, ny, ycode, 4u, 8u, R == 2);
             else if (past_axis(cy, ny, R == 2)) continue;
             const uint32_t rowbase = (uint32_t)cy * nx + (nx * ny) * (uint32_t)cz;
-            const bool far_row = oz < -1 || oz > 1 || oy < -1 || oy > 1;
             for (int part = 0; part < 3; ++part) {
                 int32_t a, b, cx;   // cells gp + a .. gp + b; the first one's x
                 Run r;
@@ -918,10 +922,10 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
                         a = part == 0 ? -R : n - g;
                         b = part == 0 ? -g - 1 : R;
                     }
-                    if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
-                    if (a < 0 && a <= b && dyz2 + dist2(0, a) > reach2) ++a;
-                    if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
-                    if (b > 0 && a <= b && dyz2 + dist2(0, b) > reach2) --b;
+                    if (a == -2 && a <= b && dyz2 + lo2[0] > far2) ++a;
+                    if (a == -1 && a <= b && dyz2 + lo1[0] > most) ++a;
+                    if (b == 2 && a <= b && dyz2 + hi2[0] > far2) --b;
+                    if (b == 1 && a <= b && dyz2 + hi1[0] > most) --b;
                     if (a > b) continue;
                     cx = g + a + (part == 0 ? n : (part == 2 ? -n : 0));
                     if (part != 1) r.code |= part == 0 ? 1u : 2u;
@@ -945,7 +949,7 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
         }
     }
     if (!VISC) test_later();
-    return Swept{due, held, nlist, use_lists && !list_overflow};
+    return Swept{due, held, nlist, record && !list_overflow};
 }
 
 // The contact search of one particle s that is due (k_topo); sweep: its
@@ -1006,7 +1010,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
     }
     float due = 3.0e38f;         // the particle's next moment
 
-    if (use_lists && !sweep && len != VL_NONE) {
+    if (use_lists && !sweep && len < VL_OVER) {
         const bool simple = VISC || len + (uint32_t)__popc(ts.occ) <= (uint32_t)NC;
         if (!simple) held = 0u;
         const bool rows = !VISC && simple && held == 0u && ts.occ != 0u;
@@ -1108,7 +1112,10 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
             due = -1.0f;
         }
     } else {
-        const Swept w = topo_sweep<VISC, TB>(d, P, A, s, tid, srow, S, xa, gp, use_lists, ts, va);
+        // a list that had too many entries is tried again with the cells around
+        // or in the next epoch; until then the reference's stencil is enough
+        const bool record = use_lists && (sweep || len != VL_OVER);
+        const Swept w = topo_sweep<VISC, TB>(d, P, A, s, tid, srow, S, xa, gp, record, ts, va);
         due = w.due;
         held = w.held;
         const bool listed = w.listed;
@@ -1118,7 +1125,7 @@ __device__ __forceinline__ void topo_search(const Dev &d, int A, uint32_t s, int
             // return, unless it may miss another one that is back.
             due = -1.0f;
             const bool stays = one && !gp_in && !sweep && !new_list() && __ldcg(&d.vs->dirty_step) != step;
-            if (!stays) d.vl_len[s] = VL_NONE;
+            if (!stays) d.vl_len[s] = gp_in ? VL_OVER : VL_NONE;
             if (P.skin > 0.0 && gp_in) d.vs->want_cells = 1u;   // (outside: particle_tail asks)
         } else {
             d.vl_len[s] = (uint8_t)w.nlist;

@@ -43,7 +43,20 @@ SCENES = {
     "two_cells": lambda: _flow(4.5, 1, n=400, box=(0.0165, 0.0165, 0.05)),
     # grains four times their neighbours' size: more candidates than a list holds
     "overflow": lambda: _flow(2.0, 0, n=1200, r=(0.35e-3, 2.0e-3)),
+    # and among them grains that cross a side
+    "overflow_periodic": lambda: _few_large(),
 }
+
+
+def _few_large():
+    """A sheared periodic bed of fine grains with a few large ones, whose candidates
+    are more than a list holds in nearly every step."""
+    sb = _sheared(n=1500, seed=12)
+    r = 0.4 * sb.radius
+    r[np.random.default_rng(12).choice(1500, 12, replace=False)] = 2.6e-3
+    sb.radius = r
+    sb.num = np.maximum(3, np.floor(sb.L / 5.2e-3)).astype(np.uint32)
+    return sb
 
 
 both_kernels = pytest.mark.parametrize("span", [None, 1], ids=["one_kernel", "split"])
