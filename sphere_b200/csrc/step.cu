@@ -722,7 +722,7 @@ struct Swept {
 //
 // Out of line: few steps sweep, and the decision and the lists' path keep their
 // registers (k_topo on 97,778 loose grains 5.9 us inline, 5.7 so; without lists, where
-// every particle sweeps, 500,000 grains take 276 us a step inline, 296 so).
+// every particle sweeps, 500,000 grains take 276 us a step inline, 298 so).
 template <bool VISC, int TB>
 __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, uint32_t s, int tid,
                                          uint32_t *srow, float S, double4 xa, const int32_t gp[3],
