@@ -80,7 +80,6 @@ __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32
         const uint32_t cg = (e & 1u) ? mv.y : mv.x;
         if (cg >= d.ncells_all) continue;
         uint32_t *const stamps = mv.x == LOOK ? d.look : d.dirty;
-        *(mv.x == LOOK ? &V.look_step : &V.dirty_step) = step;
         // the instance owning global cell cg (batched contexts)
         uint32_t inst = 0;
         if (d.inst) {
@@ -97,6 +96,10 @@ __device__ __forceinline__ void stamp_moves(const Dev &d, uint32_t first, uint32
         const int32_t ox = (int32_t)(o % 5u) - 2, oy = (int32_t)(o / 5u % 5u) - 2, oz = (int32_t)(o / 25u) - 2;
         const int32_t R = P.wide ? 2 : 1;
         if (max(max(abs(ox), abs(oy)), abs(oz)) > R) continue;
+        if (o == 62u) {   // the cell itself
+            uint32_t *const when = mv.x == LOOK ? &V.look_step : &V.dirty_step;
+            if (__ldcg(when) != step) *when = step;
+        }
         int32_t x = (int32_t)(c % (uint32_t)nx) + ox, y = (int32_t)(c / (uint32_t)nx % (uint32_t)ny) + oy;
         const int32_t z = (int32_t)(c / (uint32_t)(nx * ny)) + oz;
         if (z < 0 || z >= nz) continue;
@@ -212,7 +215,7 @@ __device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
         // a particle whose floored coordinates leave the grid sits outside
         // its cell's box (saturated or aliased cell id): contact search must
         // then not prune cells by geometry
-        if (cell_outside(P, x.x, x.y, x.z)) atomicOr(d.alias_any, 1u);
+        if (cell_outside(P, x.x, x.y, x.z)) *d.alias_any = 1u;
     };
     for (uint32_t k = first; k < np; k += stride) {
         const uint32_t s = members[k], c = d.cell[s], key = d.uid[s];

@@ -369,22 +369,25 @@ __device__ __forceinline__ bool grid_cell(const G &P, double x, double y, double
     return c < P.ncells && isfinite(x + y + z);
 }
 
-// The axes (bit k: axis k) on which the position's floored cell coordinate lies
-// outside [0, num): with any, the particle is not inside its own cell's box
-// (contact search takes the reference's stencil from the floored coordinates,
-// not the id).
+// The axes on which the position's floored cell coordinate lies below 0 (bit k:
+// axis k) or at num or above, or is none (bit 3 + k): with any, the particle is
+// not inside its own cell's box (contact search takes the reference's stencil
+// from the floored coordinates, not the id).  Below 0 the id saturates to the
+// cell next to the position; above it aliases one elsewhere.
 template <class G>
 __device__ __forceinline__ uint32_t outside_axes(const G &P, double x, double y, double z)
 {
-    // 2^-20 of a cell away from the grid's sides no quotient rounds past one
-    auto in = [&](int k, double v) {
-        const double q = (v - P.origo[k]) * P.rcell[k];
-        return q > 0x1p-20 && q < (double)P.num[k] - 0x1p-20 && q < 0x1p30;
+    auto axis = [&](int k, double v) -> uint32_t {
+        // 2^-20 of a cell away from the grid's sides the product with 1 / cellsize
+        // is on the same side as the quotient (see cell_at)
+        const double q = (v - P.origo[k]) * P.rcell[k], n = (double)P.num[k];
+        if (q > 0x1p-20 && q < n - 0x1p-20 && q < 0x1p30) return 0u;
+        if (q < -0x1p-20 && q > -0x1p30) return 1u << k;
+        if (q > n + 0x1p-20 && q < 0x1p30) return 8u << k;
+        const double f = cell_floor(P, k, v);
+        return f < 0.0 ? 1u << k : (f < n ? 0u : 8u << k);
     };
-    if (in(0, x) && in(1, y) && in(2, z)) return 0u;
-    const double f0 = cell_floor(P, 0, x), f1 = cell_floor(P, 1, y), f2 = cell_floor(P, 2, z);
-    return (f0 >= 0.0 && f0 < (double)P.num[0] ? 0u : 1u) | (f1 >= 0.0 && f1 < (double)P.num[1] ? 0u : 2u) |
-           (f2 >= 0.0 && f2 < (double)P.num[2] ? 0u : 4u);
+    return axis(0, x) | axis(1, y) | axis(2, z);
 }
 template <class G>
 __device__ __forceinline__ bool cell_outside(const G &P, double x, double y, double z)

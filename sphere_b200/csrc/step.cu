@@ -1599,13 +1599,16 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
         // periodic boundary.  One back in by a period has the lists around
         // looked at.  Any other -- or where axes are too short for that -- changes
         // images or what a stencil reaches: the cells around sweep again.
+        // While a particle stays outside nobody's list changes: below the grid it
+        // is found in the cell next to it all along, above it nowhere near.
         const uint32_t was = outside_axes(P, xa.x, xa.y, xa.z), is = out ? outside_axes(P, x.x, x.y, x.z) : 0u;
         bool hard = !P.set_lists || c == d.ncells_all || c_old == d.ncells_all, look = false;
         if (!hard && (was | is | wrapped)) {
-            const uint32_t sides = P.periodic == 1 ? 3u : 1u;   // with one_image
-            const bool leaves = !was && !wrapped && (is & ~sides) == 0u;
-            look = P.one_image && !is && wrapped == was && d.outside[d.uid[s]] == 1;
-            hard = !look && !(P.one_image && leaves);
+            const uint32_t sides = P.periodic == 1 ? 033u : 011u;   // with one_image
+            const bool leaves = P.one_image && !was && !wrapped && (is & ~sides) == 0u;
+            const bool stays = was && is && !wrapped && !((was >> 3) && !(is >> 3));
+            look = P.one_image && !is && wrapped == ((was | was >> 3) & 7u) && d.outside[d.uid[s]] == 1;
+            hard = !look && !leaves && !stays;
         }
         if (!hard && !(was | is)) {
             const uint32_t p = c_old - P.cell_base, q = c - P.cell_base;

@@ -253,3 +253,28 @@ def test_differentiable_steps_with_periodic_sides():
             x.append(sim.download())
             sim.diff_end()
     assert mismatches(x[1], x[0], STATE_FIELDS + ("force", "torque", "contacts", "delta_t")) == []
+
+
+@both_kernels
+@pytest.mark.parametrize("skin", [0.0, 0.1, 0.4])
+@pytest.mark.parametrize("shift", [0.0, -0.07, 0.05])
+@pytest.mark.parametrize("periodic", [0, 1])
+def test_beds_that_stand_out_of_their_grid(oracle_libs, periodic, shift, skin, span):
+    """Grains beyond the sides for the whole run, in cells that their ids saturate
+    to or alias, some on their way in or out."""
+    sb = scenes.settling(4, 11, 11, 6)
+    sb.L, sb.num = np.array([0.2, 0.18, 2.0]), np.array([9, 8, 96], dtype=np.uint32)
+    sb.periodic = periodic
+    sb.x = sb.x + np.array([shift, 0.7 * shift, 0.02])
+    sb.vel = np.random.default_rng(3).uniform(-3.0, 3.0, sb.x.shape) * np.array([1.0, 1.0, 0.2])
+    rc, want, orun = run_oracle(oracle_libs["orc"], sb, 60)
+    assert rc == 0
+    with Simulation(config_from_spherebin(sb), verlet_skin=skin, topo_span=span) as sim:
+        sim.upload(state_from_spherebin(sb))
+        for k in (7, 53):
+            sim.step(k)
+        sim.sync()
+        got = sim.download()
+        _, perm, _, _ = sim.cells()
+    assert mismatches(got, want, ALL) == []
+    assert np.array_equal(perm, orun.perm)
