@@ -791,8 +791,9 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
     };
     // The overlaps of the first VL_CAP near candidates are tested after the
     // sweep, from the list: found here and there in a warp's lanes, each
-    // would make the whole warp wait for its two loads and its slot.  (A
-    // particle outside the grid has no list to keep them in.)
+    // would make the whole warp wait for its two loads and its slot.  (With
+    // Params::one_image the list of a particle outside the grid may have to stay.)
+    const bool room = gp_in || !P.one_image;
     uint32_t later = 0;
     auto test_later = [&]() {
         for (; later; later &= later - 1u) {
@@ -854,7 +855,7 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
                         w = -1.0f;
                     }
                 } else if ((hit >> j) & 1u) {
-                    if (gp_in && nlist < VL_CAP) {
+                    if (room && nlist < VL_CAP) {
                         later |= 1u << nlist;
                         w = 3.0e38f;
                     } else {
@@ -875,7 +876,7 @@ __device__ __noinline__ Swept topo_sweep(const Dev &d, const Params &P, int A, u
                     }
                 }
                 due = fminf(due, w);
-                if (gp_in && nlist < VL_CAP) {
+                if (room && nlist < VL_CAP) {
                     const size_t at = vl_at(s, nlist);
                     d.vl[at] = t;
                     // a held entry that loses its slot is due at once
@@ -1586,7 +1587,8 @@ __device__ __forceinline__ void particle_tail(const Dev &d, const PS &P, uint32_
         // (past the last cell its stencil is empty)
         if (c != d.ncells_all || c != c_old) d.rebuild[REBUILD_NEXT] = 1u;
         d.due[s] = -1.0f;
-        V.crossed = 1u;
+        // (a store by every such particle holds up the readers of V)
+        if (*(volatile uint32_t *)&V.crossed == 0u) V.crossed = 1u;
         d.outside[d.uid[s]] = cell_outside(P, xa.x, xa.y, xa.z) ? 2 : 1;
     }
     // (out through one side and into the next cell on another axis, a particle
