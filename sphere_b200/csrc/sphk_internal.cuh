@@ -539,18 +539,11 @@ __device__ __forceinline__ uint32_t vl_code(uint32_t meta) { return meta & 0xfu;
 __device__ __forceinline__ float vl_when(uint32_t meta) { return __uint_as_float(meta & 0xfffffff0u); }
 
 // Entry e of particle s's Verlet list (Dev::vl, Dev::vl_meta): tiled like
-// the slots, or (SPHK_VL_ROWS) one row of VL_CAP entries per particle.
-#ifdef SPHK_VL_ROWS
-__host__ __device__ __forceinline__ size_t vl_at(uint32_t s, uint32_t e)
-{
-    return (size_t)s * VL_CAP + e;
-}
-#else
+// the slots.
 __host__ __device__ __forceinline__ size_t vl_at(uint32_t s, uint32_t e)
 {
     return tile_at(s, e, VL_CAP);
 }
-#endif
 // Entries of a tiled array for np particles (the last tile is padded).
 __host__ __device__ __forceinline__ size_t tiled_size(size_t np, uint32_t width)
 {

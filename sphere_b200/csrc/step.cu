@@ -1743,7 +1743,6 @@ k_force_diff(ForceArgs args)
     const uint32_t np = d.np_all;
     const uint32_t s = blockIdx.x * FORCE_BLOCK + threadIdx.x;
     if (s >= np) return;
-#ifndef SPHK_NO_PREFETCH
     // The state the integration reads comes after the contact work and
     // after stores the compiler may not move loads across, so each of its
     // loads would wait out a full DRAM latency in turn.  Lane 0 of every
@@ -1757,7 +1756,6 @@ k_force_diff(ForceArgs args)
         bulk_prefetch_l2(d.fixed + s, 32);
         bulk_prefetch_l2(d.wtouch + s, 32);
     }
-#endif
     const GlobalRows R{d, args.a, s};
     {
         const Params &P = *d.prm;
