@@ -143,21 +143,24 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t &total)
 
 // A cell with more members than this is put in order by one block, which looks
 // for them among all particles in index order; below, every member counts the
-// smaller indices of its cell for itself.  The first costs a pass over the
-// particles (1.5 us per 512 of them), the second the square of the members
-// shared by the whole grid: 65,536 of them 2 ms of a million particles' list,
-// and all particles in one cell still well inside the barrier's limit.
-constexpr uint32_t CROWD = 1u << 16;
-// the crowded cells, in the half of scan_tiles that no grid's totals reach
-constexpr uint32_t CROWDED_AT = SCAN_TILES / 2, CROWDED_CAP = SCAN_TILES / 2;
+// smaller indices of its cell for itself.  The first takes 2.4 us for each 512
+// particles of the context, whatever the members, the second 0.5 us a member of
+// the cell for a million particles, so they meet at about 10,000 members: a
+// million particles in 16 cells 28.5 ms by counting, 4.6 by blocks, all in one
+// cell 4.8.
+constexpr uint32_t CROWD = 1u << 14;
+// the crowded cells (at most 2^27 / CROWD), past the part of scan_tiles that the
+// blocks' totals take
+constexpr uint32_t CROWDED_AT = SCAN_TILES / 4, CROWDED_CAP = SCAN_TILES - CROWDED_AT;
+static_assert(CROWDED_CAP >= (1u << 27) / CROWD, "every crowded cell has a place");
 
 // The cell list of the positions in buffer A, by all blocks of the grid; false
 // after a timeout.  BLOCK: the threads of a block.
 //
-// What bounds it: the barriers (about 2 us each) and L2 latency.  One thread
-// used to sort each cell's members by insertion, one load after another: 190 us
-// a list where cells of four radii hold 12 grains each, 13 ms at 300, and past
-// the barrier's limit of 1 s at about 3,000.
+// What bounds it: the barriers and L2 latency (17 us at 50,000 particles, 47 at a
+// million).  One thread used to sort each cell's members by insertion, one load
+// after another: 189 us a list where cells of four radii hold 12 grains each, and
+// past the barrier's limit of 1 s at a few thousand.
 template <int BLOCK>
 __device__ __noinline__ bool rebuild_grid(const Dev &d, int A, GridBar &bar)
 {

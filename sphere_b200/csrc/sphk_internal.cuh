@@ -117,8 +117,8 @@ __host__ __device__ inline ForceConsts force_consts(const Params &P)
     return c;
 }
 
-// Twice the blocks that a rebuild's grid can have (8 an SM, with room).
-constexpr uint32_t SCAN_TILES = 4096;
+// Four times the blocks that a rebuild's grid can have (8 an SM, with room).
+constexpr uint32_t SCAN_TILES = 16384;
 constexpr int VL_CAP = 32;              // candidates kept per particle
 constexpr uint8_t VL_NONE = 0xff;       // no list yet: sweep and record one
 constexpr uint8_t VL_OVER = 0xfe;       // more candidates than that: sweep in every step

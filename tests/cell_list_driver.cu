@@ -74,7 +74,7 @@ int main()
     const cudaError_t refused = launch_together(k_rounds, 1u << 20, 64, nullptr, d, filled(start), mark, behind, 1, 0u);
     check("too large", refused == cudaErrorCooperativeLaunchTooLarge && cudaGetLastError() == refused);
     const uint32_t most = resident_blocks<k_rebuild, REBUILD_BLOCK>();
-    check("resident", most >= sm_count() * REBUILD_BLOCKS_PER_SM && most <= SCAN_TILES / 2);
+    check("resident", most >= sm_count() * REBUILD_BLOCKS_PER_SM && most <= CROWDED_AT);
 
     // a cell list of 3,000 particles in 10 x 10 x 10 cells, in storage order
     // reversed against their indices

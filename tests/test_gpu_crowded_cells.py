@@ -1,5 +1,5 @@
 """Cells with many members: the cell list's order from two members a cell to all
-grains in one (past 65,536 a block looks for them in index order), the bucket of
+grains in one (past 16,384 a block looks for them in index order), the bucket of
 the outside among them, and steps over such cells against the oracle."""
 import numpy as np
 import pytest
@@ -24,8 +24,8 @@ def _cloud(n, num):
 
 
 @pytest.mark.parametrize("outside", [0.0, 0.5, 1.0])
-@pytest.mark.parametrize("n, num", [(33, (1, 1, 1)), (5000, (2, 1, 1)), (65536, (1, 1, 1)),
-                                    (65537, (1, 1, 1)), (200000, (3, 1, 1)), (300000, (40, 40, 40))],
+@pytest.mark.parametrize("n, num", [(33, (1, 1, 1)), (5000, (2, 1, 1)), (16384, (1, 1, 1)),
+                                    (16385, (1, 1, 1)), (70000, (1, 1, 1)), (200000, (3, 1, 1)), (300000, (18, 1, 1)), (300000, (40, 40, 40))],
                          ids=lambda v: str(v if isinstance(v, int) else v[0] * v[1] * v[2]))
 def test_order_of_crowded_cells(n, num, outside):
     sb = _cloud(n, num)
